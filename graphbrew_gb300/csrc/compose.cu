@@ -124,42 +124,75 @@ __global__ void k_positions(const uint32_t* __restrict__ order_v, const uint32_t
     }
 }
 
-// Community classes: 1 = Gorder (thread), 2 = Gorder (warp, shared memory),
-// 3 = Gorder (warp, global workspace), 4 = BFS.  Lists hold ranks.
+// Community classes.  Gorder communities by size: a thread, a warp, a small
+// and a large CTA (scan heap in shared memory), and a warp over a global
+// workspace for the sizes whose scan heap shared memory does not hold.
+// Lists hold ranks.
+enum Class { kClsThread = 1, kClsWarp = 2, kClsCta = 3, kClsBfs = 4, kClsBigCta = 5, kClsGlobal = 6, kClasses = 7 };
+
 struct ClassCounts {
-    int32_t n[5];
+    int32_t n[kClasses];
     unsigned long long gorder_communities, gorder_vertices, fallback_communities, fallback_vertices;
     uint32_t gorder_max, largest;
 };
 
 constexpr int kThreadGorderMax = 32;
-constexpr int kSmemGorderMax = 4096;
+constexpr int kWarpGorderMax = 512;     // a lane holds up to 16 vertices
+constexpr int kCtaGorderMax = 2048;     // 128 threads, up to 16 vertices each
+constexpr int kBigCtaGorderMax = 16384; // 512 threads, up to 32 each; 12 bytes of shared memory a vertex
 constexpr int kMaxGorderWindow = 100;   // the thread variant's bound (kMaxB) too
 
+// Counters are added once per warp (millions of tiny communities share them).
 __global__ void k_classify(const int64_t* __restrict__ ssize, int64_t C, int intra, int fallback,
                            int32_t* __restrict__ lists, ClassCounts* __restrict__ cc) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < C; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t sz = ssize[i];
-        if (sz == 0) continue;
-        atomicMax(&cc->largest, (uint32_t)sz);
+    const int lane = threadIdx.x & 31;
+    for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; i0 < C;
+         i0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = i0 + lane;
+        const int64_t sz = i < C ? ssize[i] : 0;
+        const uint32_t sz32 = (uint32_t)sz;
         int cls = 0;
-        if (intra == kIntraGorder) {
-            if (fallback > 0 && sz > fallback) {
-                atomicAdd(&cc->fallback_communities, 1ull);
-                atomicAdd(&cc->fallback_vertices, (unsigned long long)sz);
-                cls = 4;
-            } else if (sz > 3) {
-                atomicAdd(&cc->gorder_communities, 1ull);
-                atomicAdd(&cc->gorder_vertices, (unsigned long long)sz);
-                atomicMax(&cc->gorder_max, (uint32_t)sz);
-                cls = sz <= kThreadGorderMax ? 1 : (sz <= kSmemGorderMax ? 2 : 3);
+        bool gorder = false, fell = false;
+        if (sz > 0) {
+            if (intra == kIntraGorder) {
+                fell = fallback > 0 && sz > fallback;
+                gorder = !fell && sz > 3;
+                if (fell) cls = kClsBfs;
+                else if (gorder)
+                    cls = sz <= kThreadGorderMax ? kClsThread
+                          : sz <= kWarpGorderMax ? kClsWarp
+                          : sz <= kCtaGorderMax  ? kClsCta
+                          : sz <= kBigCtaGorderMax ? kClsBigCta : kClsGlobal;
+            } else {
+                cls = sz >= 2 ? kClsBfs : 0;
             }
-        } else {
-            cls = sz >= 2 ? 4 : 0;
         }
-        if (cls) {
-            const int32_t slot = atomicAdd(&cc->n[cls], 1);
-            lists[(int64_t)cls * C + slot] = (int32_t)i;
+        const unsigned peers = __match_any_sync(0xFFFFFFFFu, cls);
+        const int leader = __ffs(peers) - 1;
+        int32_t slot = 0;
+        if (cls && lane == leader) slot = atomicAdd(&cc->n[cls], __popc(peers));
+        slot = __shfl_sync(0xFFFFFFFFu, slot, leader) + __popc(peers & ((1u << lane) - 1u));
+        if (cls) lists[(int64_t)cls * C + slot] = (int32_t)i;
+        const uint32_t largest = __reduce_max_sync(0xFFFFFFFFu, sz32);
+        const uint32_t gmax = __reduce_max_sync(0xFFFFFFFFu, gorder ? sz32 : 0u);
+        const unsigned gb = __ballot_sync(0xFFFFFFFFu, gorder), fb = __ballot_sync(0xFFFFFFFFu, fell);
+        unsigned long long gv = gorder ? (unsigned long long)sz : 0ull, fv = fell ? (unsigned long long)sz : 0ull;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            gv += __shfl_xor_sync(0xFFFFFFFFu, gv, o);
+            fv += __shfl_xor_sync(0xFFFFFFFFu, fv, o);
+        }
+        if (lane == 0) {
+            if (largest) atomicMax(&cc->largest, largest);
+            if (gb) {
+                atomicAdd(&cc->gorder_communities, (unsigned long long)__popc(gb));
+                atomicAdd(&cc->gorder_vertices, gv);
+                atomicMax(&cc->gorder_max, gmax);
+            }
+            if (fb) {
+                atomicAdd(&cc->fallback_communities, (unsigned long long)__popc(fb));
+                atomicAdd(&cc->fallback_vertices, fv);
+            }
         }
     }
 }
@@ -179,18 +212,62 @@ __global__ void k_mark_gorder_positions(const int32_t* __restrict__ list, const 
     }
 }
 
+// Both passes: eight lanes a row (four rows per warp), rows above kOctetRow
+// entries by the whole warp afterwards, so that neither the many short rows
+// idle a warp nor a hub's row waits on one thread (a thread a row took 224 us
+// for the two passes on RMAT scale 12, where one row has 800 entries).
+constexpr int kOctetRow = 64;
+
+template <typename Short, typename Long>
+__device__ __forceinline__ void for_marked_rows(const int64_t* __restrict__ rp, const uint32_t* __restrict__ memb,
+                                                const uint32_t* __restrict__ order_v,
+                                                const uint8_t* __restrict__ mark, int64_t nn, Short&& short_row,
+                                                Long&& long_row) {
+    const int lane = threadIdx.x & 31, g = lane >> 3;
+    const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t p0 = 4 * w; p0 < nn; p0 += 4 * nw) {
+        const int64_t p = p0 + g;
+        int64_t b = 0, e = 0;
+        uint32_t cu = 0;
+        if (p < nn && mark[p]) {
+            const uint32_t u = order_v[p];
+            b = rp[u];
+            e = rp[u + 1];
+            cu = memb[u];
+        }
+        const bool is_long = e - b > kOctetRow;
+        short_row(p, b, is_long ? b : e, cu, is_long);
+        unsigned todo = __ballot_sync(0xFFFFFFFFu, is_long && (lane & 7) == 0);
+        while (todo) {
+            const int src = __ffs(todo) - 1;
+            todo &= todo - 1;
+            long_row(p0 + (src >> 3), __shfl_sync(0xFFFFFFFFu, b, src), __shfl_sync(0xFFFFFFFFu, e, src),
+                     __shfl_sync(0xFFFFFFFFu, cu, src));
+        }
+    }
+}
+
 __global__ void k_local_count(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
                               const uint32_t* __restrict__ memb, const uint32_t* __restrict__ order_v,
                               const uint8_t* __restrict__ mark, int64_t nn, int64_t* __restrict__ cnt) {
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < nn; p += (int64_t)gridDim.x * blockDim.x) {
-        int64_t c = 0;
-        if (mark[p]) {
-            const uint32_t u = order_v[p];
-            const uint32_t cu = memb[u];
-            for (int64_t e = rp[u]; e < rp[u + 1]; ++e) c += (memb[col[e]] == cu);
-        }
-        cnt[p] = c;
-    }
+    const int lane = threadIdx.x & 31, j = lane & 7;
+    for_marked_rows(
+        rp, memb, order_v, mark, nn,
+        [&](int64_t p, int64_t b, int64_t e, uint32_t cu, bool is_long) {
+            int c = 0;
+            for (int64_t x = b + j; x < e; x += 8) c += memb[col[x]] == cu;
+            c += __shfl_xor_sync(0xFFFFFFFFu, c, 4);
+            c += __shfl_xor_sync(0xFFFFFFFFu, c, 2);
+            c += __shfl_xor_sync(0xFFFFFFFFu, c, 1);
+            if (j == 0 && p < nn && !is_long) cnt[p] = c;
+        },
+        [&](int64_t p, int64_t b, int64_t e, uint32_t cu) {
+            int c = 0;
+            for (int64_t x = b + lane; x < e; x += 32) c += memb[col[x]] == cu;
+            c = __reduce_add_sync(0xFFFFFFFFu, c);
+            if (lane == 0) cnt[p] = c;
+        });
 }
 
 __global__ void k_local_fill(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
@@ -198,19 +275,34 @@ __global__ void k_local_fill(const int64_t* __restrict__ rp, const int32_t* __re
                              const uint8_t* __restrict__ mark, const uint32_t* __restrict__ local,
                              const int64_t* __restrict__ loff, int64_t nn, uint16_t* __restrict__ ladj16,
                              uint32_t* __restrict__ ladj32) {
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < nn; p += (int64_t)gridDim.x * blockDim.x) {
-        if (!mark[p]) continue;
-        const uint32_t u = order_v[p];
-        const uint32_t cu = memb[u];
-        int64_t o = loff[p];
-        for (int64_t e = rp[u]; e < rp[u + 1]; ++e) {
-            const int32_t w = col[e];
-            if (memb[w] == cu) {
-                if (ladj32) ladj32[o++] = local[w];
-                else ladj16[o++] = (uint16_t)local[w];
+    const int lane = threadIdx.x & 31, j = lane & 7;
+    auto put = [&](int64_t o, int32_t w) {
+        if (ladj32) ladj32[o] = local[w];
+        else ladj16[o] = (uint16_t)local[w];
+    };
+    for_marked_rows(
+        rp, memb, order_v, mark, nn,
+        [&](int64_t p, int64_t b, int64_t e, uint32_t cu, bool) {
+            int64_t o = e > b ? loff[p] : 0;
+            for (int64_t x = b + j; __any_sync(0xFFFFFFFFu, x < e); x += 8) {
+                const int32_t w = x < e ? col[x] : -1;
+                const bool keep = w >= 0 && memb[w] == cu;
+                const unsigned bal = (__ballot_sync(0xFFFFFFFFu, keep) >> (lane & 24)) & 0xFFu;
+                if (keep) put(o + __popc(bal & ((1u << j) - 1u)), w);
+                o += __popc(bal);
             }
-        }
-    }
+        },
+        [&](int64_t p, int64_t b, int64_t e, uint32_t cu) {
+            int64_t o = loff[p];
+            for (int64_t x0 = b; x0 < e; x0 += 32) {
+                const int64_t x = x0 + lane;
+                const int32_t w = x < e ? col[x] : -1;
+                const bool keep = w >= 0 && memb[w] == cu;
+                const unsigned bal = __ballot_sync(0xFFFFFFFFu, keep);
+                if (keep) put(o + __popc(bal & ((1u << lane) - 1u)), w);
+                o += __popc(bal);
+            }
+        });
 }
 
 // ---------------------------------------------------------------------------
@@ -569,21 +661,18 @@ __device__ void gorder_lazy_warp(const LazyHeap& h, int sz, int nb, int window, 
     __syncwarp();
 }
 
-// One warp per community of 33..gordf vertices; its workspace in shared
-// memory (capacity S of the launch) or, for the largest class, in global
-// memory (one slice per CTA).
-template <typename LAdj, bool kShared>
+// One warp per community above kBigCtaGorderMax vertices, its workspace in
+// global memory (one slice per CTA).
+template <typename LAdj>
 __global__ void k_gorder_warp(const int32_t* __restrict__ list, const int32_t* __restrict__ count_p,
                               const int64_t* __restrict__ offs, const int64_t* __restrict__ ssize,
                               const uint32_t* __restrict__ order_v, const int64_t* __restrict__ rp,
                               const LAdj* __restrict__ ladj, const int64_t* __restrict__ loff, int window,
                               uint32_t* __restrict__ local_by_pos, int* __restrict__ gws, int64_t cap) {
-    extern __shared__ int smem[];
     const int32_t count = *count_p;
     const int lane = threadIdx.x & 31;
     const int nb = window + 2;
-    int* ws = kShared ? smem : gws + (int64_t)blockIdx.x * lazy_ws_ints(cap, nb, window);
-    const LazyHeap h = lazy_view(ws, cap, nb, window);
+    const LazyHeap h = lazy_view(gws + (int64_t)blockIdx.x * lazy_ws_ints(cap, nb, window), cap, nb, window);
     for (int32_t j = blockIdx.x; j < count; j += gridDim.x) {
         const int32_t r = list[j];
         const int64_t base = offs[r];
@@ -595,6 +684,183 @@ __global__ void k_gorder_warp(const int32_t* __restrict__ list, const int32_t* _
         __syncwarp();
         gorder_lazy_warp<LAdj>(h, sz, nb, window, ladj, loff + base, local_by_pos + base);
         __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The same greedy order without linked buckets (33..kBigCtaGorderMax vertices).
+//
+// The UnitHeap's next vertex is the unplaced one of the highest key that was
+// moved into its bucket last.  A placed vertex moves its neighbours in
+// adjacency order, and adjacency rows ascend in local index, so "last" is the
+// larger (placement, bump sign) stamp and, within one stamp, the larger local
+// index; vertices never moved (stamp 0) stand in local order behind all
+// others of bucket 0.  The heap is therefore just a key and a stamp per vertex,
+// and the next vertex the maximum of (key, stamp, index).
+//
+// Bumps are fire-and-forget shared-memory reductions (key += +-1, stamp =
+// max): the key of an unplaced neighbour of a vertex leaving the window is at
+// least 1, because that vertex raised it when it was placed, so the +1 and -1
+// bumps of one placement commute and the reference's "no bump below 0" never
+// applies.  Placed vertices carry a bias that keeps their key negative.  Each
+// thread owns a run of vertices and keeps their maximum in registers; it scans
+// them again only when one of them was bumped.  A placement is two barriers
+// (none for the warp variant) and one hardware max-reduction per level.
+//
+// What bounds it is that chain's latency, one placement after another: the
+// linked form (a warp, push stacks with lazy deletion) took 9.5 ms for the
+// 3,267-vertex community of an RMAT graph of scale 12.
+// ---------------------------------------------------------------------------
+constexpr int kStampBits = 25;              // stamps < 2 * kBigCtaGorderMax + 4, keys <= window + 1 < 128
+constexpr int kPlacedBias = -(1 << 20);     // keys move by at most 2 * kBigCtaGorderMax after it
+static_assert(2 * kBigCtaGorderMax + 4 < (1 << kStampBits) && 2 * kBigCtaGorderMax < (1 << 20), "heap fields");
+static_assert(kMaxGorderWindow + 2 < (1 << (32 - kStampBits)), "heap key field");
+
+__host__ __device__ constexpr int scan_smem_ints(int cap, int threads, int window) {
+    return 3 * ((cap + 3) & ~3) + 4 + threads + window + 1;
+}
+
+template <int T>
+__device__ __forceinline__ void gorder_barrier() {
+    if (T == 32) __syncwarp(); else __syncthreads();
+}
+
+// Maximum of (hi, lo) over the CTA, in every thread.
+template <int T>
+__device__ __forceinline__ void gorder_max(uint32_t& hi, uint32_t& lo, uint32_t* wm) {
+    const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, hi);
+    uint32_t l = __reduce_max_sync(0xFFFFFFFFu, hi == m ? lo : 0u);
+    hi = m;
+    lo = l;
+    if (T > 32) {
+        constexpr int kW = T / 32;
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        if (lane == 0) {
+            wm[2 * w] = hi;
+            wm[2 * w + 1] = lo;
+        }
+        __syncthreads();
+        const uint32_t h2 = lane < kW ? wm[2 * lane] : 0u, l2 = lane < kW ? wm[2 * lane + 1] : 0u;
+        hi = __reduce_max_sync(0xFFFFFFFFu, h2);
+        lo = __reduce_max_sync(0xFFFFFFFFu, h2 == hi ? l2 : 0u);
+    }
+}
+
+template <typename LAdj, int T>
+__global__ void __launch_bounds__(T)
+k_gorder_scan(const int32_t* __restrict__ list, const int64_t* __restrict__ offs, const int64_t* __restrict__ ssize,
+              const uint32_t* __restrict__ order_v, const int64_t* __restrict__ rp, const LAdj* __restrict__ ladj,
+              const int64_t* __restrict__ loff, int window, int cap, uint32_t* __restrict__ local_by_pos) {
+    extern __shared__ __align__(16) int smem[];
+    __shared__ uint32_t wm[2 * (T / 32)];
+    const int cap4 = (cap + 3) & ~3;
+    int* key = smem;
+    uint32_t* stamp = reinterpret_cast<uint32_t*>(key + cap4);
+    uint32_t* off = stamp + cap4;                 // adjacency offsets, relative to the community's first
+    uint32_t* touched = off + cap4 + 4;           // per thread: last placement that bumped one of its vertices
+    int* ring = reinterpret_cast<int*>(touched + T);
+    const int tid = threadIdx.x;
+    const int32_t r = list[blockIdx.x];
+    const int64_t base = offs[r];
+    const int sz = (int)ssize[r], sz4 = (sz + 3) & ~3;
+    int sh = 2;                                   // a thread owns 1 << sh vertices
+    while ((T << sh) < sz) ++sh;
+    const int64_t l0 = loff[base];
+    const LAdj* adj = ladj + l0;
+    uint32_t* out = local_by_pos + base;
+    // Seed: largest degree, first in local order.
+    uint32_t hi = 0, lo = 0;
+    for (int i = tid; i < sz4; i += T) {
+        key[i] = i < sz ? 0 : kPlacedBias;
+        stamp[i] = 0;
+        if (i < sz) {
+            const uint32_t u = order_v[base + i];
+            const uint32_t d = (uint32_t)(rp[u + 1] - rp[u]), first = (uint32_t)(sz - i);
+            if (lo == 0 || d > hi) {              // indices ascend: the first of equal degrees stays
+                hi = d;
+                lo = first;
+            }
+        }
+    }
+    for (int i = tid; i <= sz; i += T) off[i] = (uint32_t)(loff[base + i] - l0);
+    touched[tid] = 0;
+    gorder_barrier<T>();
+    // First touch of the community's adjacency, all loads in flight together:
+    // the chain below then finds most rows in L1.
+    {
+        constexpr int kPer = 32 / sizeof(LAdj);
+        uint32_t sink = 0;
+        for (uint32_t i = tid * kPer; i < off[sz]; i += T * kPer) sink ^= adj[i];
+        asm volatile("" ::"r"(sink));
+    }
+    gorder_max<T>(hi, lo, wm);
+    int best = sz - (int)lo;
+    const int own0 = tid << sh, own1 = min(sz4, own0 + (1 << sh));
+    // Maximum over the thread's own vertices.
+    auto scan_own = [&]() {
+        hi = lo = 0;
+        for (int i = own0; i < own1; i += 4) {
+            const int4 k = *reinterpret_cast<const int4*>(key + i);
+            const uint4 st = *reinterpret_cast<const uint4*>(stamp + i);
+            const int kk[4] = {k.x, k.y, k.z, k.w};
+            const uint32_t ss[4] = {st.x, st.y, st.z, st.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t h = (uint32_t)kk[q] << kStampBits | ss[q];
+                const uint32_t l = ss[q] ? (uint32_t)(i + q + 1) : (uint32_t)(sz - i - q);
+                if (kk[q] >= 0 && (h > hi || (h == hi && l > lo))) {
+                    hi = h;
+                    lo = l;
+                }
+            }
+        }
+    };
+    auto bump = [&](int n, int delta, uint32_t st, uint32_t mark) {
+        atomicAdd(&key[n], delta);
+        atomicMax(&stamp[n], st);
+        touched[n >> sh] = mark;
+    };
+    scan_own();
+    uint32_t ohi = hi, olo = lo;                  // kept over placements
+    uint32_t o0 = 0, o1 = 0;                      // adjacency of the vertex that leaves the window
+    int m0 = -1;
+    gorder_barrier<T>();                          // scans done before the first bumps
+    for (int lid = 0;; ++lid) {
+        const uint32_t mark = (uint32_t)lid + 1, st = 2u * (uint32_t)lid + 2u;
+        const uint32_t e0 = off[best], e1 = off[best + 1];
+        int n0 = e0 + tid < e1 ? (int)adj[e0 + tid] : -1;
+        if (tid == 0) {
+            out[best] = (uint32_t)lid;
+            ring[lid % (window + 1)] = best;
+            atomicAdd(&key[best], kPlacedBias);
+            touched[best >> sh] = mark;
+        }
+        if (lid + 1 == sz) break;
+        if (m0 >= 0) bump(m0, -1, st + 1, mark);
+        for (uint32_t i = o0 + tid + T; i < o1; i += T) bump((int)adj[i], -1, st + 1, mark);
+        if (n0 >= 0) bump(n0, 1, st, mark);
+        for (uint32_t i = e0 + tid + T; i < e1; i += T) bump((int)adj[i], 1, st, mark);
+        // The next placement's leaving vertex is known already: its row is
+        // fetched while this placement's maximum is formed.
+        m0 = -1;
+        o0 = o1 = 0;
+        if (lid + 1 >= window) {
+            const int old = window == 1 ? best : ring[(lid + 1 - window) % (window + 1)];
+            o0 = off[old];
+            o1 = off[old + 1];
+            if (o0 + tid < o1) m0 = (int)adj[o0 + tid];
+        }
+        gorder_barrier<T>();
+        if (touched[tid] == mark) {
+            scan_own();
+            ohi = hi;
+            olo = lo;
+        }
+        hi = ohi;
+        lo = olo;
+        gorder_max<T>(hi, lo, wm);
+        best = (hi & ((1u << kStampBits) - 1u)) ? (int)lo - 1 : sz - (int)lo;
+        if (T == 32) __syncwarp();
     }
 }
 
@@ -1322,7 +1588,7 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
     launches += 6 + 3 * ((vbits + 7) / 8);
 
     // Classify communities.
-    DevBuf<int32_t> lists(5 * C, s);
+    DevBuf<int32_t> lists(kClasses * C, s);
     DevBuf<ClassCounts> cc(1, s);
     GB_CUDA(cudaMemsetAsync(cc, 0, sizeof(ClassCounts), s));
     k_classify<<<grid_for(C, kT), kT, 0, s>>>(ssize, C, intra, p.gorder_fallback, lists, cc);
@@ -1336,25 +1602,25 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
     GB_CUDA(cudaEventRecord(ev_intra0, s));
 
     // ---- Gorder communities ----
-    const int32_t ng = hc.n[1] + hc.n[2] + hc.n[3];
+    const int32_t ng = hc.n[kClsThread] + hc.n[kClsWarp] + hc.n[kClsCta] + hc.n[kClsBigCta] + hc.n[kClsGlobal];
     if (ng > 0) {
         DevBuf<uint8_t> mark(nn, s);
         GB_CUDA(cudaMemsetAsync(mark, 0, nn, s));
-        for (int cls = 1; cls <= 3; ++cls) {
-            if (hc.n[cls] == 0) continue;
+        for (int cls = 1; cls < kClasses; ++cls) {
+            if (cls == kClsBfs || hc.n[cls] == 0) continue;
             k_mark_gorder_positions<<<kNumSMs * 8, kT, 0, s>>>(lists.get() + cls * C, cc.get()->n + cls, offs, ssize, mark);
             GB_LAUNCH_CHECK();
             ++launches;
         }
         DevBuf<int64_t> loff(nn + 1, s);
-        k_local_count<<<grid_for(nn, kT), kT, 0, s>>>(g.row_ptr, g.col, memb, order_v, mark, nn, loff);
+        k_local_count<<<grid_for(nn * 8, kT), kT, 0, s>>>(g.row_ptr, g.col, memb, order_v, mark, nn, loff);
         GB_LAUNCH_CHECK();
         exclusive_scan_i64_total(loff, loff, nn, loff.get() + nn, s);
         const int64_t ltot = read_dev(loff.get() + nn, s);
         const bool wide = hc.gorder_max > 65535;
         DevBuf<uint16_t> l16(wide ? 0 : (ltot > 0 ? ltot : 1), s);
         DevBuf<uint32_t> l32(wide ? (ltot > 0 ? ltot : 1) : 0, s);
-        k_local_fill<<<grid_for(nn, kT), kT, 0, s>>>(g.row_ptr, g.col, memb, order_v, mark, local, loff, nn,
+        k_local_fill<<<grid_for(nn * 8, kT), kT, 0, s>>>(g.row_ptr, g.col, memb, order_v, mark, local, loff, nn,
                                                      l16.get(), wide ? l32.get() : nullptr);
         GB_LAUNCH_CHECK();
         DevBuf<uint32_t> local_by_pos(nn, s);
@@ -1362,40 +1628,41 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
         launches += 5;
         auto run = [&](auto* ladj) {
             using LT = std::remove_pointer_t<decltype(ladj)>;
-            if (hc.n[1] > 0) {
-                k_gorder_thread<LT><<<grid_for(hc.n[1], 64), 64, 0, s>>>(lists.get() + 1 * C, cc.get()->n + 1, offs,
-                                                                          ssize, order_v, g.row_ptr, ladj, loff,
-                                                                          p.gorder_window, local_by_pos);
+            // Largest communities first: theirs is the longest chain.
+            auto scan = [&](auto threads, int cls, int max_size) {
+                constexpr int T = decltype(threads)::value;
+                if (hc.n[cls] == 0) return;
+                // Shared memory sized by this call's largest community of the
+                // class; the attribute is the one constant maximum, so
+                // concurrent callers never race on it.
+                const int cap = (int)std::min<int64_t>(max_size, hc.gorder_max);
+                const int smem = (int)sizeof(int) * scan_smem_ints(cap, T, p.gorder_window);
+                GB_CUDA(cudaFuncSetAttribute(k_gorder_scan<LT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(int) * scan_smem_ints(max_size, T, kMaxGorderWindow)));
+                k_gorder_scan<LT, T><<<(unsigned)hc.n[cls], T, smem, s>>>(lists.get() + cls * C, offs, ssize, order_v,
+                                                                         g.row_ptr, ladj, loff, p.gorder_window, cap,
+                                                                         local_by_pos);
                 GB_LAUNCH_CHECK();
                 ++launches;
-            }
-            if (hc.n[2] > 0) {
-                // Workspace sized by this call's largest community of the class
-                // (occupancy follows it); the attribute is the one constant
-                // maximum, so concurrent callers never race on it.
-                const int nb = p.gorder_window + 2;
-                const int64_t cap = std::min<int64_t>(kSmemGorderMax, std::max<int64_t>(hc.gorder_max, 33));
-                const int smem = (int)(sizeof(int) * lazy_ws_ints(cap, nb, p.gorder_window));
-                GB_CUDA(cudaFuncSetAttribute(k_gorder_warp<LT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)(sizeof(int) * lazy_ws_ints(kSmemGorderMax, kMaxGorderWindow + 2,
-                                                                              kMaxGorderWindow))));
-                int per_sm = 1;
-                GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gorder_warp<LT, true>, 32, smem));
-                const int grid = std::min<int>(hc.n[2], kNumSMs * std::max(1, per_sm));
-                k_gorder_warp<LT, true><<<grid, 32, smem, s>>>(lists.get() + 2 * C, cc.get()->n + 2, offs, ssize,
-                                                               order_v, g.row_ptr, ladj, loff, p.gorder_window,
-                                                               local_by_pos, nullptr, cap);
-                GB_LAUNCH_CHECK();
-                ++launches;
-            }
-            if (hc.n[3] > 0) {
-                const int grid = std::min<int>(hc.n[3], kNumSMs * 4);
+            };
+            if (hc.n[kClsGlobal] > 0) {
+                const int grid = std::min<int>(hc.n[kClsGlobal], kNumSMs * 4);
                 const int64_t cap = hc.gorder_max;
                 const int nb = p.gorder_window + 2;
                 DevBuf<int> gws((int64_t)grid * lazy_ws_ints(cap, nb, p.gorder_window), s);
-                k_gorder_warp<LT, false><<<grid, 32, 0, s>>>(lists.get() + 3 * C, cc.get()->n + 3, offs, ssize,
-                                                             order_v, g.row_ptr, ladj, loff, p.gorder_window,
-                                                             local_by_pos, gws, cap);
+                k_gorder_warp<LT><<<grid, 32, 0, s>>>(lists.get() + kClsGlobal * C, cc.get()->n + kClsGlobal, offs,
+                                                      ssize, order_v, g.row_ptr, ladj, loff, p.gorder_window,
+                                                      local_by_pos, gws, cap);
+                GB_LAUNCH_CHECK();
+                ++launches;
+            }
+            scan(std::integral_constant<int, 512>{}, kClsBigCta, kBigCtaGorderMax);
+            scan(std::integral_constant<int, 128>{}, kClsCta, kCtaGorderMax);
+            scan(std::integral_constant<int, 32>{}, kClsWarp, kWarpGorderMax);
+            if (hc.n[kClsThread] > 0) {
+                k_gorder_thread<LT><<<grid_for(hc.n[kClsThread], 64), 64, 0, s>>>(
+                    lists.get() + kClsThread * C, cc.get()->n + kClsThread, offs, ssize, order_v, g.row_ptr, ladj,
+                    loff, p.gorder_window, local_by_pos);
                 GB_LAUNCH_CHECK();
                 ++launches;
             }
@@ -1407,26 +1674,26 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
     }
 
     // ---- RCM: every community of two or more vertices ----
-    const int32_t nbfs = hc.n[4];
+    const int32_t nbfs = hc.n[kClsBfs];
     int64_t levels = 0;
     if (nbfs > 0 && (intra == kIntraRCM || intra == kIntraRCMpp)) {
-        levels = rcm_communities(g, memb, lists.get() + 4 * C, cc.get()->n + 4, nbfs, order_v, vkeys, offs, ssize, C,
+        levels = rcm_communities(g, memb, lists.get() + kClsBfs * C, cc.get()->n + kClsBfs, nbfs, order_v, vkeys, offs, ssize, C,
                                  nn, hc.largest, intra == kIntraRCMpp, local, s, &launches);
     }
     // ---- sorted orders: every community ----
     if (sorted_intra) sorted_communities(g, memb, intra, order_v, vkeys, offs, ssize, nn, local, s, &launches);
     // ---- intra_random: every community of two or more vertices ----
     if (random_intra)
-        random_communities(memb, order_v, vkeys, offs, ssize, lists.get() + 4 * C, cc.get()->n + 4, nbfs, nn, local, s,
+        random_communities(memb, order_v, vkeys, offs, ssize, lists.get() + kClsBfs * C, cc.get()->n + kClsBfs, nbfs, nn, local, s,
                            &launches);
     // ---- BFS communities ----
     if (nbfs > 0 && intra != kIntraRCM && intra != kIntraRCMpp && !sorted_intra && !random_intra) {
-        const int32_t* blist = lists.get() + 4 * C;
+        const int32_t* blist = lists.get() + kClsBfs * C;
         DevBuf<int32_t> slot_of_comm(C, s);
         GB_CUDA(cudaMemsetAsync(slot_of_comm, 0xFF, C * sizeof(int32_t), s));
         DevBuf<int64_t> slot_base(nbfs, s), slot_size(nbfs, s), qlen(nbfs, s), fs(nbfs, s), fe(nbfs, s),
             bbase(nbfs, s), bend(nbfs, s);
-        k_bfs_slots<<<grid_for(nbfs, kT), kT, 0, s>>>(blist, cc.get()->n + 4, order_v, offs, memb, slot_of_comm,
+        k_bfs_slots<<<grid_for(nbfs, kT), kT, 0, s>>>(blist, cc.get()->n + kClsBfs, order_v, offs, memb, slot_of_comm,
                                                       slot_base, slot_size, ssize);
         GB_LAUNCH_CHECK();
         DevBuf<unsigned long long> hubkey(nbfs, s);
