@@ -124,11 +124,10 @@ __global__ void k_positions(const uint32_t* __restrict__ order_v, const uint32_t
     }
 }
 
-// Community classes.  Gorder communities by size: a thread, a warp, a small
-// and a large CTA (scan heap in shared memory), and a warp over a global
-// workspace for the sizes whose scan heap shared memory does not hold.
-// Lists hold ranks.
-enum Class { kClsThread = 1, kClsWarp = 2, kClsCta = 3, kClsBfs = 4, kClsBigCta = 5, kClsGlobal = 6, kClasses = 7 };
+// Community classes.  Gorder communities by size: a thread, a warp or a CTA
+// over a scan heap in shared memory, and a warp over a global workspace for the
+// sizes whose scan heap shared memory does not hold.  Lists hold ranks.
+enum Class { kClsThread = 1, kClsWarp = 2, kClsCta = 3, kClsBfs = 4, kClsGlobal = 5, kClasses = 6 };
 
 struct ClassCounts {
     int32_t n[kClasses];
@@ -137,9 +136,8 @@ struct ClassCounts {
 };
 
 constexpr int kThreadGorderMax = 32;
-constexpr int kWarpGorderMax = 512;     // a lane holds up to 16 vertices
-constexpr int kCtaGorderMax = 2048;     // 128 threads, up to 16 vertices each
-constexpr int kBigCtaGorderMax = 16384; // 512 threads, up to 32 each; 12 bytes of shared memory a vertex
+constexpr int kWarpGorderMax = 1024;    // a lane scans up to 32 vertices
+constexpr int kCtaGorderMax = 16384;    // 256 threads; up to 12 bytes of shared memory a vertex
 constexpr int kMaxGorderWindow = 100;   // the thread variant's bound (kMaxB) too
 
 // Counters are added once per warp (millions of tiny communities share them).
@@ -161,8 +159,7 @@ __global__ void k_classify(const int64_t* __restrict__ ssize, int64_t C, int int
                 else if (gorder)
                     cls = sz <= kThreadGorderMax ? kClsThread
                           : sz <= kWarpGorderMax ? kClsWarp
-                          : sz <= kCtaGorderMax  ? kClsCta
-                          : sz <= kBigCtaGorderMax ? kClsBigCta : kClsGlobal;
+                          : sz <= kCtaGorderMax  ? kClsCta : kClsGlobal;
             } else {
                 cls = sz >= 2 ? kClsBfs : 0;
             }
@@ -661,7 +658,7 @@ __device__ void gorder_lazy_warp(const LazyHeap& h, int sz, int nb, int window, 
     __syncwarp();
 }
 
-// One warp per community above kBigCtaGorderMax vertices, its workspace in
+// One warp per community above kCtaGorderMax vertices, its workspace in
 // global memory (one slice per CTA).
 template <typename LAdj>
 __global__ void k_gorder_warp(const int32_t* __restrict__ list, const int32_t* __restrict__ count_p,
@@ -688,180 +685,197 @@ __global__ void k_gorder_warp(const int32_t* __restrict__ list, const int32_t* _
 }
 
 // ---------------------------------------------------------------------------
-// The same greedy order without linked buckets (33..kBigCtaGorderMax vertices).
+// The same greedy order without linked buckets (33..kCtaGorderMax vertices).
 //
 // The UnitHeap's next vertex is the unplaced one of the highest key that was
 // moved into its bucket last.  A placed vertex moves its neighbours in
 // adjacency order, and adjacency rows ascend in local index, so "last" is the
 // larger (placement, bump sign) stamp and, within one stamp, the larger local
-// index; vertices never moved (stamp 0) stand in local order behind all
-// others of bucket 0.  The heap is therefore just a key and a stamp per vertex,
-// and the next vertex the maximum of (key, stamp, index).
+// index; vertices never moved stand in local order behind all others of bucket
+// 0, which initial stamps sz - i below every later one express.  So a vertex is
+// one word, key | stamp | index (0 once placed), a bump rewrites one word, and
+// the next vertex is the largest word.
 //
-// Bumps are fire-and-forget shared-memory reductions (key += +-1, stamp =
-// max): the key of an unplaced neighbour of a vertex leaving the window is at
-// least 1, because that vertex raised it when it was placed, so the +1 and -1
-// bumps of one placement commute and the reference's "no bump below 0" never
-// applies.  Placed vertices carry a bias that keeps their key negative.  Each
-// thread owns a run of vertices and keeps their maximum in registers; it scans
-// them again only when one of them was bumped.  A placement is two barriers
-// (none for the warp variant) and one hardware max-reduction per level.
+// Per placement: the vertex leaving the window lowers its neighbours, the
+// placed one raises its own (each row's vertices are distinct, so plain stores;
+// the lowering first but with the later stamp, which leaves the same words, as
+// an unplaced neighbour of a leaving vertex has key >= 1: that vertex raised it
+// when it was placed), then the maximum over all words, by one hardware
+// reduction per level, gives the next vertex.  Short rows are bumped by the
+// first warp alone, long ones by the CTA.
 //
-// What bounds it is that chain's latency, one placement after another: the
-// linked form (a warp, push stacks with lazy deletion) took 9.5 ms for the
-// 3,267-vertex community of an RMAT graph of scale 12.
+// What bounds it is that chain's latency, one placement after another, so the
+// code is laid out for it: one warp without a barrier up to 1,024 vertices
+// (eight vector loads a lane), 256 threads above; rows in shared memory; no
+// branch on the chain (a lane without an entry bumps the dummy word, which is 0
+// and stays so); the leaving vertex's row kept by the ring and fetched a
+// placement ahead.  3,267 vertices of an RMAT graph of scale 12 took 9.5 ms with
+// linked buckets (a warp, push stacks with lazy deletion), 3.3 ms with key and
+// stamp in two arrays bumped by atomics over 512 threads, and 1.8 ms so.
 // ---------------------------------------------------------------------------
-constexpr int kStampBits = 25;              // stamps < 2 * kBigCtaGorderMax + 4, keys <= window + 1 < 128
-constexpr int kPlacedBias = -(1 << 20);     // keys move by at most 2 * kBigCtaGorderMax after it
-static_assert(2 * kBigCtaGorderMax + 4 < (1 << kStampBits) && 2 * kBigCtaGorderMax < (1 << 20), "heap fields");
-static_assert(kMaxGorderWindow + 2 < (1 << (32 - kStampBits)), "heap key field");
+constexpr int kShortRow = 128;              // rows the first warp bumps alone
+constexpr int kMaxSmem = 226 * 1024;        // dynamic shared memory of a CTA (227 KB less the static part)
 
-__host__ __device__ constexpr int scan_smem_ints(int cap, int threads, int window) {
-    return 3 * ((cap + 3) & ~3) + 4 + threads + window + 1;
+// Words padded to whole vector loads of the CTA; the dummy word follows.
+__host__ __device__ constexpr int64_t scan_words(int64_t cap, int threads) {
+    return (cap + 4 * threads - 1) / (4 * threads) * (4 * threads);
+}
+__host__ __device__ constexpr int64_t scan_smem_bytes(int64_t cap, int threads, int window, int word) {
+    return (((scan_words(cap, threads) + 4) * word + (cap + 2) / 2 * 8 + (window + 1) * 8) + 15) & ~15ll;
 }
 
-template <int T>
-__device__ __forceinline__ void gorder_barrier() {
-    if (T == 32) __syncwarp(); else __syncthreads();
+__device__ __forceinline__ uint32_t warp_max_word(uint32_t v) { return __reduce_max_sync(0xFFFFFFFFu, v); }
+__device__ __forceinline__ unsigned long long warp_max_word(unsigned long long v) {
+    const uint32_t hi = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)(v >> 32));
+    const uint32_t lo = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)(v >> 32) == hi ? (uint32_t)v : 0u);
+    return (unsigned long long)hi << 32 | lo;
 }
 
-// Maximum of (hi, lo) over the CTA, in every thread.
-template <int T>
-__device__ __forceinline__ void gorder_max(uint32_t& hi, uint32_t& lo, uint32_t* wm) {
-    const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, hi);
-    uint32_t l = __reduce_max_sync(0xFFFFFFFFu, hi == m ? lo : 0u);
-    hi = m;
-    lo = l;
+// Maximum over the CTA, in every thread (wm: a slot per warp).
+template <int T, typename W>
+__device__ __forceinline__ W cta_max_word(W v, W* wm) {
+    v = warp_max_word(v);
     if (T > 32) {
-        constexpr int kW = T / 32;
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-        if (lane == 0) {
-            wm[2 * w] = hi;
-            wm[2 * w + 1] = lo;
-        }
+        if (lane == 0) wm[w] = v;
         __syncthreads();
-        const uint32_t h2 = lane < kW ? wm[2 * lane] : 0u, l2 = lane < kW ? wm[2 * lane + 1] : 0u;
-        hi = __reduce_max_sync(0xFFFFFFFFu, h2);
-        lo = __reduce_max_sync(0xFFFFFFFFu, h2 == hi ? l2 : 0u);
+        v = warp_max_word(wm[lane & (T / 32 - 1)]);
     }
+    return v;
 }
 
-template <typename LAdj, int T>
+// Maximum of four consecutive words.
+__device__ __forceinline__ uint32_t quad_max(const uint32_t* p) {
+    const uint4 v = *reinterpret_cast<const uint4*>(p);
+    return max(max(v.x, v.y), max(v.z, v.w));
+}
+__device__ __forceinline__ unsigned long long quad_max(const unsigned long long* p) {
+    const ulonglong2 v = reinterpret_cast<const ulonglong2*>(p)[0], w = reinterpret_cast<const ulonglong2*>(p)[1];
+    return max(max(v.x, v.y), max(w.x, w.y));
+}
+
+// One community's placements; row(i) is entry i of its local adjacency.  ib /
+// sb: bits of the index and stamp fields of a word (the key above them).
+template <typename LAdj, int T, typename W>
+struct GorderScan {
+    static constexpr int kW = T / 32;
+    W *word, *wm;
+    uint32_t* off;        // adjacency offsets relative to the community's first
+    uint2* ring;          // rows of the last window + 1 placed vertices
+    uint32_t* out;
+    int sz, window, ib, sb;
+
+    template <typename Row>
+    __device__ __forceinline__ void run(int best, Row row) const {
+        const int tid = threadIdx.x, lane = tid & 31;
+        const bool first_warp = T == 32 || tid < 32;
+        const W unit = (W)1 << (ib + sb), imask = ((W)1 << ib) - 1, smask = (((W)1 << sb) - 1) << ib;
+        const int nwords = (int)scan_words(sz, T), dummy = nwords;
+        auto bumped = [&](W v, W delta, W st) {   // the later stamp of this placement stays
+            return v ? ((v & ~smask) + delta) | max(v & smask, st) : (W)0;
+        };
+        auto bump = [&](int n, W delta, W st) { word[n] = bumped(word[n], delta, st); };
+        uint2 leave = make_uint2(0, 0);   // row of the vertex that leaves the window
+        int m = dummy;                    // its entry of this lane (first warp)
+        int wpos = 0;                     // ring slot of this placement
+        W st = (W)(sz + 1) << ib;
+        const W one = (W)1 << ib;
+        W top = 0;
+        for (int lid = 0;; ++lid, st += 2 * one) {
+            // Here every thread has scanned; top: this warp's maximum (lid > 0).
+            const uint32_t olen = leave.y - leave.x;
+            const bool olong = T > 32 && olen > (uint32_t)kShortRow;
+            if (olong) {
+                for (uint32_t i = leave.x + tid; i < leave.y; i += T) bump(row(i), (W)0 - unit, st + one);
+            } else if (first_warp) {
+                bump(m, (W)0 - unit, st + one);
+                if (olen > 32u)
+                    for (uint32_t i = leave.x + lane + 32; i < leave.y; i += 32) bump(row(i), (W)0 - unit, st + one);
+            }
+            if (lid > 0) {
+                if (T > 32) top = warp_max_word(wm[lane & (kW - 1)]);
+                best = (int)(top & imask);
+            }
+            const uint32_t e0 = off[best], e1 = off[best + 1], elen = e1 - e0;
+            const bool elong = T > 32 && elen > (uint32_t)kShortRow;
+            if (tid == 0) {
+                out[best] = (uint32_t)lid;
+                ring[wpos] = make_uint2(e0, e1);
+            }
+            if (lid + 1 == sz) break;
+            if (olong || elong) __syncthreads(); else __syncwarp();
+            if (tid == 0) word[best] = 0;
+            if (elong) {
+                for (uint32_t i = e0 + tid; i < e1; i += T) bump(row(i), unit, st);
+            } else if (first_warp) {
+                bump((uint32_t)lane < elen ? row(e0 + lane) : dummy, unit, st);
+                if (elen > 32u)
+                    for (uint32_t i = e0 + lane + 32; i < e1; i += 32) bump(row(i), unit, st);
+            }
+            if (T > 32) __syncthreads(); else __syncwarp();
+            // The next placement's leaving vertex is known: its row is fetched
+            // while the maximum is formed.
+            if (++wpos > window) wpos = 0;
+            if (lid + 1 >= window) {
+                leave = ring[wpos == window ? 0 : wpos + 1];
+                m = first_warp && leave.x + lane < leave.y ? row(leave.x + lane) : dummy;
+            }
+            top = 0;
+#pragma unroll 4
+            for (int i = 4 * tid; i < nwords; i += 4 * T) top = max(top, quad_max(word + i));
+            top = warp_max_word(top);
+            if (T > 32) {
+                if (lane == 0) wm[tid >> 5] = top;
+                __syncthreads();
+            }
+        }
+    }
+};
+
+template <typename LAdj, int T, typename W>
 __global__ void __launch_bounds__(T)
 k_gorder_scan(const int32_t* __restrict__ list, const int64_t* __restrict__ offs, const int64_t* __restrict__ ssize,
               const uint32_t* __restrict__ order_v, const int64_t* __restrict__ rp, const LAdj* __restrict__ ladj,
-              const int64_t* __restrict__ loff, int window, int cap, uint32_t* __restrict__ local_by_pos) {
-    extern __shared__ __align__(16) int smem[];
-    __shared__ uint32_t wm[2 * (T / 32)];
-    const int cap4 = (cap + 3) & ~3;
-    int* key = smem;
-    uint32_t* stamp = reinterpret_cast<uint32_t*>(key + cap4);
-    uint32_t* off = stamp + cap4;                 // adjacency offsets, relative to the community's first
-    uint32_t* touched = off + cap4 + 4;           // per thread: last placement that bumped one of its vertices
-    int* ring = reinterpret_cast<int*>(touched + T);
+              const int64_t* __restrict__ loff, int window, int cap, int ib, int sb, uint32_t sadj_cap,
+              uint32_t* __restrict__ local_by_pos) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned long long wm64[T / 32];
+    GorderScan<LAdj, T, W> h;
     const int tid = threadIdx.x;
     const int32_t r = list[blockIdx.x];
     const int64_t base = offs[r];
-    const int sz = (int)ssize[r], sz4 = (sz + 3) & ~3;
-    int sh = 2;                                   // a thread owns 1 << sh vertices
-    while ((T << sh) < sz) ++sh;
+    h.sz = (int)ssize[r];
+    h.window = window;
+    h.ib = ib;
+    h.sb = sb;
+    h.wm = reinterpret_cast<W*>(wm64);
+    h.word = reinterpret_cast<W*>(smem_raw);
+    h.ring = reinterpret_cast<uint2*>(h.word + scan_words(cap, T) + 4);
+    h.off = reinterpret_cast<uint32_t*>(h.ring + window + 1);
+    h.out = local_by_pos + base;
+    LAdj* sadj = reinterpret_cast<LAdj*>(smem_raw + scan_smem_bytes(cap, T, window, sizeof(W)));
+    const int sz = h.sz;
     const int64_t l0 = loff[base];
     const LAdj* adj = ladj + l0;
-    uint32_t* out = local_by_pos + base;
     // Seed: largest degree, first in local order.
-    uint32_t hi = 0, lo = 0;
-    for (int i = tid; i < sz4; i += T) {
-        key[i] = i < sz ? 0 : kPlacedBias;
-        stamp[i] = 0;
+    unsigned long long seed = 0;
+    for (int i = tid; i < (int)scan_words(sz, T) + 4; i += T) {
+        h.word[i] = i < sz ? (W)(sz - i) << ib | (W)i : (W)0;
         if (i < sz) {
             const uint32_t u = order_v[base + i];
-            const uint32_t d = (uint32_t)(rp[u + 1] - rp[u]), first = (uint32_t)(sz - i);
-            if (lo == 0 || d > hi) {              // indices ascend: the first of equal degrees stays
-                hi = d;
-                lo = first;
-            }
+            const unsigned long long d = (unsigned long long)(rp[u + 1] - rp[u]) << 32 | (uint32_t)(sz - i);
+            seed = d > seed ? d : seed;
         }
     }
-    for (int i = tid; i <= sz; i += T) off[i] = (uint32_t)(loff[base + i] - l0);
-    touched[tid] = 0;
-    gorder_barrier<T>();
-    // First touch of the community's adjacency, all loads in flight together:
-    // the chain below then finds most rows in L1.
-    {
-        constexpr int kPer = 32 / sizeof(LAdj);
-        uint32_t sink = 0;
-        for (uint32_t i = tid * kPer; i < off[sz]; i += T * kPer) sink ^= adj[i];
-        asm volatile("" ::"r"(sink));
-    }
-    gorder_max<T>(hi, lo, wm);
-    int best = sz - (int)lo;
-    const int own0 = tid << sh, own1 = min(sz4, own0 + (1 << sh));
-    // Maximum over the thread's own vertices.
-    auto scan_own = [&]() {
-        hi = lo = 0;
-        for (int i = own0; i < own1; i += 4) {
-            const int4 k = *reinterpret_cast<const int4*>(key + i);
-            const uint4 st = *reinterpret_cast<const uint4*>(stamp + i);
-            const int kk[4] = {k.x, k.y, k.z, k.w};
-            const uint32_t ss[4] = {st.x, st.y, st.z, st.w};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint32_t h = (uint32_t)kk[q] << kStampBits | ss[q];
-                const uint32_t l = ss[q] ? (uint32_t)(i + q + 1) : (uint32_t)(sz - i - q);
-                if (kk[q] >= 0 && (h > hi || (h == hi && l > lo))) {
-                    hi = h;
-                    lo = l;
-                }
-            }
-        }
-    };
-    auto bump = [&](int n, int delta, uint32_t st, uint32_t mark) {
-        atomicAdd(&key[n], delta);
-        atomicMax(&stamp[n], st);
-        touched[n >> sh] = mark;
-    };
-    scan_own();
-    uint32_t ohi = hi, olo = lo;                  // kept over placements
-    uint32_t o0 = 0, o1 = 0;                      // adjacency of the vertex that leaves the window
-    int m0 = -1;
-    gorder_barrier<T>();                          // scans done before the first bumps
-    for (int lid = 0;; ++lid) {
-        const uint32_t mark = (uint32_t)lid + 1, st = 2u * (uint32_t)lid + 2u;
-        const uint32_t e0 = off[best], e1 = off[best + 1];
-        int n0 = e0 + tid < e1 ? (int)adj[e0 + tid] : -1;
-        if (tid == 0) {
-            out[best] = (uint32_t)lid;
-            ring[lid % (window + 1)] = best;
-            atomicAdd(&key[best], kPlacedBias);
-            touched[best >> sh] = mark;
-        }
-        if (lid + 1 == sz) break;
-        if (m0 >= 0) bump(m0, -1, st + 1, mark);
-        for (uint32_t i = o0 + tid + T; i < o1; i += T) bump((int)adj[i], -1, st + 1, mark);
-        if (n0 >= 0) bump(n0, 1, st, mark);
-        for (uint32_t i = e0 + tid + T; i < e1; i += T) bump((int)adj[i], 1, st, mark);
-        // The next placement's leaving vertex is known already: its row is
-        // fetched while this placement's maximum is formed.
-        m0 = -1;
-        o0 = o1 = 0;
-        if (lid + 1 >= window) {
-            const int old = window == 1 ? best : ring[(lid + 1 - window) % (window + 1)];
-            o0 = off[old];
-            o1 = off[old + 1];
-            if (o0 + tid < o1) m0 = (int)adj[o0 + tid];
-        }
-        gorder_barrier<T>();
-        if (touched[tid] == mark) {
-            scan_own();
-            ohi = hi;
-            olo = lo;
-        }
-        hi = ohi;
-        lo = olo;
-        gorder_max<T>(hi, lo, wm);
-        best = (hi & ((1u << kStampBits) - 1u)) ? (int)lo - 1 : sz - (int)lo;
-        if (T == 32) __syncwarp();
-    }
+    for (int i = tid; i <= sz; i += T) h.off[i] = (uint32_t)(loff[base + i] - l0);
+    const uint32_t total = (uint32_t)(loff[base + sz] - l0);
+    const bool staged = total <= sadj_cap;
+    if (staged)
+        for (uint32_t i = tid; i < total; i += T) sadj[i] = adj[i];
+    const int first = sz - (int)(uint32_t)cta_max_word<T, unsigned long long>(seed, wm64);
+    if (T > 32) __syncthreads(); else __syncwarp();
+    if (staged) h.run(first, [&](uint32_t i) { return (int)sadj[i]; });
+    else h.run(first, [&](uint32_t i) { return (int)adj[i]; });
 }
 
 // ---------------------------------------------------------------------------
@@ -1602,7 +1616,7 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
     GB_CUDA(cudaEventRecord(ev_intra0, s));
 
     // ---- Gorder communities ----
-    const int32_t ng = hc.n[kClsThread] + hc.n[kClsWarp] + hc.n[kClsCta] + hc.n[kClsBigCta] + hc.n[kClsGlobal];
+    const int32_t ng = hc.n[kClsThread] + hc.n[kClsWarp] + hc.n[kClsCta] + hc.n[kClsGlobal];
     if (ng > 0) {
         DevBuf<uint8_t> mark(nn, s);
         GB_CUDA(cudaMemsetAsync(mark, 0, nn, s));
@@ -1629,19 +1643,25 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
         auto run = [&](auto* ladj) {
             using LT = std::remove_pointer_t<decltype(ladj)>;
             // Largest communities first: theirs is the longest chain.
-            auto scan = [&](auto threads, int cls, int max_size) {
+            auto scan = [&](auto threads, auto word, int cls, int max_size) {
                 constexpr int T = decltype(threads)::value;
+                using W = decltype(word);
                 if (hc.n[cls] == 0) return;
-                // Shared memory sized by this call's largest community of the
-                // class; the attribute is the one constant maximum, so
-                // concurrent callers never race on it.
+                // Shared memory: the words of this call's largest community of
+                // the class, and an equal share of what an SM has for the
+                // adjacency, as far as all communities still run at once.  The
+                // attribute is a constant, so concurrent callers never race on it.
                 const int cap = (int)std::min<int64_t>(max_size, hc.gorder_max);
-                const int smem = (int)sizeof(int) * scan_smem_ints(cap, T, p.gorder_window);
-                GB_CUDA(cudaFuncSetAttribute(k_gorder_scan<LT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)sizeof(int) * scan_smem_ints(max_size, T, kMaxGorderWindow)));
-                k_gorder_scan<LT, T><<<(unsigned)hc.n[cls], T, smem, s>>>(lists.get() + cls * C, offs, ssize, order_v,
-                                                                         g.row_ptr, ladj, loff, p.gorder_window, cap,
-                                                                         local_by_pos);
+                const int ib = bits_for((uint64_t)cap - 1), sb = bits_for(3 * (uint64_t)cap + 2);
+                const int64_t need = scan_smem_bytes(cap, T, p.gorder_window, sizeof(W));
+                const int64_t per_sm = ceil_div(hc.n[cls], kNumSMs);
+                const int64_t share = std::min<int64_t>(kMaxSmem, kMaxSmem / per_sm - 1024) - need;
+                const int64_t sadj = std::max<int64_t>(0, std::min<int64_t>(share / (int64_t)sizeof(LT), ltot));
+                const auto fn = k_gorder_scan<LT, T, W>;
+                GB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
+                fn<<<(unsigned)hc.n[cls], T, need + sadj * (int64_t)sizeof(LT), s>>>(
+                    lists.get() + cls * C, offs, ssize, order_v, g.row_ptr, ladj, loff, p.gorder_window, cap, ib, sb,
+                    (uint32_t)sadj, local_by_pos);
                 GB_LAUNCH_CHECK();
                 ++launches;
             };
@@ -1656,9 +1676,14 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
                 GB_LAUNCH_CHECK();
                 ++launches;
             }
-            scan(std::integral_constant<int, 512>{}, kClsBigCta, kBigCtaGorderMax);
-            scan(std::integral_constant<int, 128>{}, kClsCta, kCtaGorderMax);
-            scan(std::integral_constant<int, 32>{}, kClsWarp, kWarpGorderMax);
+            // One 32-bit word holds key, stamp and index of the warp class at any
+            // window and of 5,000 vertices at the default one; else 64 bits.
+            const uint64_t cap = std::min<uint64_t>(kCtaGorderMax, hc.gorder_max);
+            if (bits_for(cap - 1) + bits_for(3 * cap + 2) + bits_for(p.gorder_window + 1) <= 32)
+                scan(std::integral_constant<int, 256>{}, uint32_t{}, kClsCta, kCtaGorderMax);
+            else
+                scan(std::integral_constant<int, 256>{}, (unsigned long long){}, kClsCta, kCtaGorderMax);
+            scan(std::integral_constant<int, 32>{}, uint32_t{}, kClsWarp, kWarpGorderMax);
             if (hc.n[kClsThread] > 0) {
                 k_gorder_thread<LT><<<grid_for(hc.n[kClsThread], 64), 64, 0, s>>>(
                     lists.get() + kClsThread * C, cc.get()->n + kClsThread, offs, ssize, order_v, g.row_ptr, ladj,
