@@ -43,7 +43,10 @@ namespace gb {
 namespace {
 
 constexpr int kT = 256;
-constexpr uint8_t kUnknown = 2;
+// Decision word of a window vertex: the community it moves to, or kNoMove, and
+// whether the last evaluation changed it (vertex ids are below 2^31 - 1).
+constexpr uint32_t kNoMove = 0x7FFFFFFFu;
+constexpr uint32_t kChanged = 0x80000000u;
 constexpr int kWindowMax = 65536;             // window vertices (events <= 2 x window)
 constexpr int kEventsMax = 2 * kWindowMax;    // event index = 2 x window offset (+1)
 constexpr int kSlotBits = 18;
@@ -76,6 +79,10 @@ constexpr int kZMax = 8;                      // designated communities at most
 constexpr int kZKeep = 64;                    // events a designated community needs to stay / be chosen
 constexpr int kZCand = 128;                   // hot slots of the sorted table considered
 static_assert(kEventsMax < (1 << kEndBits), "event positions fit the end field");
+// CommRec.slotw: where the community's events of the current table are -- low
+// bits of the table's generation, then a designated index or a hash slot.
+constexpr int kSlotwTagShift = kSlotBits + 1;
+constexpr uint32_t kSlotwDesig = 1u << kSlotBits;
 constexpr int kHubThreads2 = 256;             // threads of the hub kernels
 constexpr int kBigMaxDeg = 2048;              // rows above kWarpMaxDeg up to this: one CTA each
 constexpr int kBigThreads = 256;
@@ -97,6 +104,7 @@ struct Ctl {
     long long cP, cX;         // committed range of the last decided window
     long long c_es0, c_es1;   // its hub edge-segment range
     long long c_ts0, c_ts1;   // its hub table-segment range
+    long long pE;             // end of the last decided window: vertices from here on are new to this one
     long long max_rounds;     // bound on rounds per iteration (n + 1 always suffices)
     long long error;          // nonzero: the round loop stopped without finishing
     unsigned long long tag;   // generation of the event table (slots of older tags are empty)
@@ -114,6 +122,15 @@ struct __align__(16) SlotMeta {
     uint32_t endh;            // one past its last event | (hot index + 1) << kEndBits
 };
 
+// What an evaluation needs of a community, in one 16-byte load: its committed
+// total, where its events of the current table are (if it has any) and the last
+// round in which those events differ from the round before's.
+struct __align__(16) CommRec {
+    unsigned long long total;
+    uint32_t slotw;
+    uint32_t cver;
+};
+
 struct HubSeg {
     int32_t hub;      // index into the hub arrays
     int32_t part;     // segment number within the hub
@@ -124,14 +141,12 @@ struct ExactState {
     const int32_t* col;
     const uint32_t* vcob;  // refinement bounds (localMovingPhase<true>), null otherwise
     uint32_t* vcom;
-    unsigned long long* ctot;
+    CommRec* rec;         // per community
     uint8_t* vaff;
     uint8_t* mv;          // committed vertex moved (read by the affected-flag kernels)
     Ctl* ctl;
-    // decisions, double-buffered by round parity
-    uint32_t* best[2];
-    uint8_t* act[2];
-    double* delta[2];
+    uint32_t* dec[2];     // decision words, double-buffered by round parity
+    double* delta;        // delta of the current decision (movers)
     double* final_delta;
     // event table
     SlotMeta* slots;      // kTableSlots: community key and its sorted-event range
@@ -187,56 +202,62 @@ __device__ __forceinline__ uint32_t slot_hash(uint32_t c) {
     return (uint32_t)(((uint64_t)c * 0x9E3779B97F4A7C15ull) >> 40);
 }
 
+__device__ __forceinline__ CommRec load_rec(const ExactState& a, uint32_t c) {
+    const uint4 v = *reinterpret_cast<const uint4*>(a.rec + c);
+    CommRec r;
+    r.total = (unsigned long long)v.y << 32 | v.x;
+    r.slotw = v.z;
+    r.cver = v.w;
+    return r;
+}
+
 // Community totals at time u for K communities: the committed total plus the
-// speculative events of c before u -- a 16-byte probe per hash step, then a
-// binary search over the slot's time-sorted events.  The K probe chains and
-// searches advance in lockstep so their loads are in flight together.
-// Designated communities read their dense row instead (their probe, issued
-// alongside, finds no slot: they are not in the table).
-// valid[k] = false entries return 0.
+// speculative events of c before u.  The community's record says whether it has
+// events in this table at all -- most candidates have none, and their total is
+// this one load (probing the hash for each cost a 16-byte read per candidate
+// more, and the total and the designated index one read each: uniform 2^23
+// took 225 us a round so) -- and where they are: a slot's time-sorted events,
+// binary-searched for the last before u, or a designated community's dense row.
+// The K chains advance in lockstep so their loads are in flight together.  The
+// record's generation is cut to its low bits, so what it points at is checked
+// against the full one.  valid[k] = false entries return 0.
 template <int K>
 __device__ __forceinline__ void sigma_at_k(const ExactState& a, unsigned long long tag, long long P, int par,
-                                           const uint32_t (&c)[K], const bool (&valid)[K], uint32_t u,
-                                           long long (&out)[K]) {
-    uint32_t h[K], hot[K];
+                                           const uint32_t (&c)[K], const bool (&valid)[K], const CommRec (&rec)[K],
+                                           uint32_t u, long long (&out)[K]) {
+    uint32_t hot[K];
     int lo[K], l[K], r[K];
-    bool pending[K];
-    uint32_t zd[K];
+    int zd[K];
+    SlotMeta sm[K];
+    bool slot[K];
+    bool any = false;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        out[k] = valid[k] ? (long long)a.ctot[c[k]] : 0;
-        zd[k] = valid[k] ? a.zof[c[k]] : 0u;
-        h[k] = slot_hash(c[k]) & (kTableSlots - 1);
-        pending[k] = valid[k];
+        out[k] = valid[k] ? (long long)rec[k].total : 0;
+        const bool ev = valid[k] && (rec[k].slotw >> kSlotwTagShift) ==
+                                        ((uint32_t)tag & ((1u << (32 - kSlotwTagShift)) - 1u));
+        zd[k] = ev && (rec[k].slotw & kSlotwDesig) ? (int)(rec[k].slotw & (kZMax - 1)) : -1;
+        slot[k] = ev && zd[k] < 0;
+        any = any || ev;
+    }
+    if (!any) return;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (slot[k]) sm[k] = a.slots[rec[k].slotw & (kTableSlots - 1)];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
         lo[k] = l[k] = r[k] = 0;
         hot[k] = 0;
-    }
-    bool any = true;
-    while (any) {
-        SlotMeta sm[K];
-#pragma unroll
-        for (int k = 0; k < K; ++k)
-            if (pending[k]) sm[k] = a.slots[h[k]];
-        any = false;
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            if (!pending[k]) continue;
-            if (sm[k].tkey == (tag << 32 | c[k])) {
-                lo[k] = l[k] = sm[k].start;
-                r[k] = (int)(sm[k].endh & ((1u << kEndBits) - 1u));
-                hot[k] = sm[k].endh >> kEndBits;
-                if (hot[k] > (uint32_t)kHotMax) {   // never written by a finished table
-                    a.ctl->error = 2;
-                    hot[k] = 0;
-                }
-                pending[k] = false;
-            } else if ((sm[k].tkey >> 32) != tag) {   // a slot of an older table: empty
-                pending[k] = false;
-            } else {
-                h[k] = (h[k] + 1) & (kTableSlots - 1);
-                any = true;
+        if (slot[k] && sm[k].tkey == (tag << 32 | c[k])) {
+            lo[k] = l[k] = sm[k].start;
+            r[k] = (int)(sm[k].endh & ((1u << kEndBits) - 1u));
+            hot[k] = sm[k].endh >> kEndBits;
+            if (hot[k] > (uint32_t)kHotMax) {   // never written by a finished table
+                a.ctl->error = 2;
+                hot[k] = 0;
             }
         }
+        if (zd[k] >= 0 && (zd[k] >= (int)a.ctl->nz || a.ctl->zc[zd[k]] != c[k])) zd[k] = -1;
     }
     // Hot slots: narrow [l, r) to u's time bucket.
     {
@@ -253,7 +274,6 @@ __device__ __forceinline__ void sigma_at_k(const ExactState& a, unsigned long lo
         for (int k = 0; k < K; ++k)
             if (hot[k]) { l[k] = bl[k]; r[k] = br[k]; }
     }
-    any = true;
     while (any) {
         uint32_t t[K];
         int mid[K];
@@ -278,8 +298,8 @@ __device__ __forceinline__ void sigma_at_k(const ExactState& a, unsigned long lo
     const int off = (int)((long long)u - P), bk = off >> 4, rem = off & 15;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        if (!zd[k]) continue;
-        const size_t row = (size_t)(par * kZMax + (int)zd[k] - 1);
+        if (zd[k] < 0) continue;
+        const size_t row = (size_t)(par * kZMax + zd[k]);
         const int4* q = reinterpret_cast<const int4*>(a.zcontrib + row * kWindowMax + ((size_t)bk << 4));
         long long sum = a.zpre[row * kHotStride + bk];
 #pragma unroll
@@ -296,38 +316,69 @@ __device__ __forceinline__ void sigma_at_k(const ExactState& a, unsigned long lo
 
 struct Round {
     long long P, E;
+    long long cP, pE;     // start and end of the window before
     unsigned long long tag;
     int par;              // parity of the round (decision buffers and dense rows)
-    const uint32_t* pbest;
-    const uint8_t* pact;
-    uint32_t* nbest;
-    uint8_t* nact;
-    double* ndelta;
+    const uint32_t* pdec;
+    uint32_t* ndec;
 };
 
 __device__ __forceinline__ Round round_view(const ExactState& a, const Ctl* c) {
     Round r;
     r.P = c->P;
     r.E = c->E;
+    r.cP = c->cP;
+    r.pE = c->pE;
     r.tag = c->tag;
     const int par = (int)(c->round & 1);
     r.par = par;
-    r.pbest = a.best[par];
-    r.pact = a.act[par];
-    r.nbest = a.best[par ^ 1];
-    r.nact = a.act[par ^ 1];
-    r.ndelta = a.delta[par ^ 1];
+    r.pdec = a.dec[par];
+    r.ndec = a.dec[par ^ 1];
     return r;
 }
 
+// What u sees of its neighbour v: v's community at time u, whether v moves
+// before u in this window, and whether v's decision is another one than in the
+// round before (v may have been committed since: the window before reaches
+// back to cP).
+struct Seen {
+    uint32_t c;
+    bool moved, changed;
+};
+
+__device__ __forceinline__ Seen see(const ExactState& a, const Round& r, int64_t v, int64_t u) {
+    Seen s{a.vcom[v], false, false};
+    if (v >= r.cP && v < u) {
+        const uint32_t w = r.pdec[v], to = w & kNoMove;
+        s.changed = (w & kChanged) != 0;
+        if (v >= r.P && to != kNoMove) {
+            s.moved = true;
+            s.c = to;
+        }
+    }
+    return s;
+}
+
 __device__ __forceinline__ bool prev_mover(const ExactState& a, const Round& r, int64_t v) {
-    return r.pact[v] == 1 && r.pbest[v] != a.vcom[v];
+    return (r.pdec[v] & kNoMove) != kNoMove;
 }
 
 __device__ __forceinline__ uint32_t comm_at(const ExactState& a, const Round& r, int64_t v, int64_t u) {
-    if (v >= r.P && v < u && prev_mover(a, r, v)) return r.pbest[v];
+    if (v >= r.P && v < u) {
+        const uint32_t to = r.pdec[v] & kNoMove;
+        if (to != kNoMove) return to;
+    }
     return a.vcom[v];
 }
+
+// Whether the events of a community differ from the round before's (a mark of
+// this round for the next may be there already: then once too often).
+__device__ __forceinline__ bool comm_changed(const Round& r, const CommRec& rec) { return rec.cver >= (uint32_t)r.tag; }
+
+// A vertex that the round before evaluated, with unchanged neighbours and
+// unchanged communities, decides as it did: every input is the same, as a
+// commit only turns decisions into state.
+__device__ __forceinline__ void keep_decision(const Round& r, int64_t u) { r.ndec[u] = r.pdec[u] & kNoMove; }
 
 // Refinement (scanCommunities<true>, RG:1392-1437): only neighbours inside
 // u's bound count; ub = vcob[u] (0 when not refining).
@@ -341,19 +392,31 @@ __device__ __forceinline__ bool refine_stays(const ExactState& a, double sigma_d
     return a.vcob != nullptr && sigma_d > __dmul_rn(ku, 1.001);
 }
 
-__device__ __forceinline__ void record(const ExactState& a, const Round& r, int64_t u, uint8_t act, uint32_t best,
+// Marks c as changed for the next round.  Designated communities change in
+// nearly every round and are marked once by the advance (every mover storing
+// to the one record of RMAT-22's giant community cost 80 us a round).
+__device__ __forceinline__ void mark_changed(const ExactState& a, const Round& r, uint32_t c) {
+    const uint32_t next = (uint32_t)r.tag + 1u;
+    if (a.rec[c].cver != next && a.zof[c] == 0) a.rec[c].cver = next;
+}
+
+// cur: u's committed community; to: the community it moves to, or kNoMove.
+__device__ __forceinline__ void record(const ExactState& a, const Round& r, int64_t u, uint32_t cur, uint32_t to,
                                        double delta) {
-    r.nact[u] = act;
-    r.nbest[u] = best;
-    r.ndelta[u] = delta;
     // Only the move itself is visible to later vertices: "inactive",
-    // "evaluated, stays" and "not yet evaluated" (kUnknown) are the same
-    // input to them, so only a different move is a change.
-    const uint32_t cur = a.vcom[u];
-    const bool moves = act == 1 && best != cur;
-    const bool pmoves = r.pact[u] == 1 && r.pbest[u] != cur;
-    if (moves != pmoves || (moves && best != r.pbest[u]))
+    // "evaluated, stays" and "not yet evaluated" are the same input to them,
+    // so only a different move is a change.
+    const uint32_t prev = r.pdec[u] & kNoMove;
+    const bool changed = to != prev;
+    r.ndec[u] = to | (changed ? kChanged : 0u);
+    if (to != kNoMove) a.delta[u] = delta;
+    if (changed) {
         atomicMin(&a.ctl->first_change, (unsigned long long)u);
+        // The events of these differ in the next table.
+        if (to == kNoMove || prev == kNoMove) mark_changed(a, r, cur);
+        if (to != kNoMove) mark_changed(a, r, to);
+        if (prev != kNoMove) mark_changed(a, r, prev);
+    }
 }
 
 __device__ __forceinline__ long long lower_bound_u32(const uint32_t* a, long long n, uint32_t key) {
@@ -442,8 +505,10 @@ __device__ __forceinline__ SegSum seg_shfl_up(SegSum x, int o) {
                   __shfl_up_sync(0xFFFFFFFFu, x.head, o)};
 }
 
-// Slot of community c in the generation-`tag` table, inserting it if absent.
-__device__ __forceinline__ uint32_t table_insert(SlotMeta* slots, unsigned long long tag, uint32_t c) {
+// Slot of community c in the generation-`tag` table, inserting it if absent;
+// the thread that inserts it notes the slot in the community's record.
+__device__ __forceinline__ uint32_t table_insert(const ExactState& a, unsigned long long tag, uint32_t c) {
+    SlotMeta* slots = a.slots;
     const unsigned long long want = tag << 32 | c;
     uint32_t h = slot_hash(c) & (kTableSlots - 1);
     while (true) {
@@ -451,6 +516,7 @@ __device__ __forceinline__ uint32_t table_insert(SlotMeta* slots, unsigned long 
         if (cur == want) return h;
         if ((cur >> 32) != tag) {
             const unsigned long long prev = atomicCAS(&slots[h].tkey, cur, want);
+            if (prev == cur) a.rec[c].slotw = (uint32_t)tag << kSlotwTagShift | h;
             if (prev == cur || prev == want) return h;
             continue;   // another community took the slot: look at it again
         }
@@ -473,22 +539,21 @@ __device__ __forceinline__ void tb_insert_chunk(const ExactState& a, const Ctl* 
     int dg = 0;
     if (i < W) {
         const int64_t wv = P + i;
-        const uint8_t pa = r.pact[wv];
-        const uint32_t pb = r.pbest[wv], vc = a.vcom[wv];
+        const uint32_t pb = r.pdec[wv] & kNoMove, vc = a.vcom[wv];
         const int64_t r0 = a.rp[wv], r1 = a.rp[wv + 1];
         uint32_t s0 = kPadSlot, s1 = kPadSlot;
-        if (pa == 1 && pb != vc) {
+        if (pb != kNoMove) {
             dg = (int)(r1 - r0);
             if (nz) {
                 z0 = a.zof[vc];
                 z1 = a.zof[pb];
             }
             if (!z0) {
-                s0 = table_insert(a.slots, r.tag, vc);
+                s0 = table_insert(a, r.tag, vc);
                 atomicAdd(&hist[s0 >> kFineBits], 1);
             }
             if (!z1) {
-                s1 = table_insert(a.slots, r.tag, pb);
+                s1 = table_insert(a, r.tag, pb);
                 atomicAdd(&hist[s1 >> kFineBits], 1);
             }
         }
@@ -949,45 +1014,88 @@ __device__ __forceinline__ void eval_vertex(const ExactState& a, const Round& r,
     }
     const uint32_t d = a.vcom[u];
     if (!act) {
-        if (lane == 0) record(a, r, u, 0, d, 0.0);
+        if (lane == 0) record(a, r, u, d, kNoMove, 0.0);
         return;
     }
+    const bool known = u < r.pE;
+    const CommRec rd = load_rec(a, d);
     const double ku = (double)deg;
     const uint32_t ub = bound_of(a, (uint32_t)u);
     double best_d = 0.0;
     uint32_t best_c = kNone;
     if (!kMid) {
+        uint32_t c = kNone;
+        CommRec rc = rd;
+        bool dirty = !known || comm_changed(r, rd);
+        if (lane < deg) {
+            const int32_t v = a.col[rb + lane];
+            const Seen sv = see(a, r, v, u);
+            if (counts(a, v, (uint32_t)u, ub)) {
+                c = sv.c;
+                rc = load_rec(a, c);
+                dirty = dirty || comm_changed(r, rc);
+            }
+            dirty = dirty || sv.changed;
+        }
+        if (!__any_sync(0xFFFFFFFFu, dirty)) {
+            if (lane == 0) keep_decision(r, u);
+            return;
+        }
         if (a.vcob) {
             long long sg1 = 0;
             if (lane == 0) {
                 const uint32_t cc[1] = {d};
                 const bool vv[1] = {true};
+                const CommRec rr[1] = {rd};
                 long long o[1];
-                sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, (uint32_t)u, o);
+                sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, rr, (uint32_t)u, o);
                 sg1 = o[0];
             }
             sg1 = __shfl_sync(0xFFFFFFFFu, sg1, 0);
             if (refine_stays(a, (double)sg1, ku)) {
-                if (lane == 0) record(a, r, u, 1, d, 0.0);
+                if (lane == 0) record(a, r, u, d, kNoMove, 0.0);
                 return;
             }
-        }
-        uint32_t c = kNone;
-        if (lane < deg) {
-            const int32_t v = a.col[rb + lane];
-            if (counts(a, v, (uint32_t)u, ub)) c = comm_at(a, r, v, u);
         }
         const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
         const int kud = __popc(__ballot_sync(0xFFFFFFFFu, c == d));
         if (c != kNone && c != d && lane == __ffs(peers) - 1) {
             const uint32_t cc[2] = {c, d};
             const bool vv[2] = {true, true};
+            const CommRec rr[2] = {rc, rd};
             long long sg[2];
-            sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, (uint32_t)u, sg);
+            sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, rr, (uint32_t)u, sg);
             const double dl = delta_qi(a.dq, __popc(peers), kud, deg, sg[0], sg[1]);
             if (dpos(dl)) { best_d = dl; best_c = c; }
         }
     } else {
+        // Has anything changed that the vertex sees?  Asked of rows of up to 128
+        // entries (longer ones see a community that changes every round), in a
+        // gather of its own: with the question inside the accumulation below
+        // its loads no longer overlapped (RMAT-22: 143 -> 188 us a round).
+        if (known && deg <= 128 && !comm_changed(r, rd)) {
+            bool dirty = false;
+            uint32_t c[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int e = 32 * k + lane;
+                c[k] = d;
+                if (e < deg) {
+                    const Seen sv = see(a, r, a.col[rb + e], u);
+                    dirty |= sv.changed;
+                    c[k] = sv.c;
+                }
+            }
+            uint32_t ver[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) ver[k] = 32 * k < deg ? a.rec[c[k]].cver : 0u;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) dirty |= ver[k] >= (uint32_t)r.tag;
+            if (!__any_sync(0xFFFFFFFFu, dirty)) {
+                if (lane == 0) keep_decision(r, u);
+                return;
+            }
+        }
         uint32_t H = 64;
         while (H < 2u * (uint32_t)deg) H <<= 1;
         const uint32_t mask = H - 1;
@@ -1038,8 +1146,9 @@ __device__ __forceinline__ void eval_vertex(const ExactState& a, const Round& r,
             const uint32_t i = i0 + lane;
             const uint32_t cc[2] = {i < cnt ? tk[i] : kNone, d};
             const bool vv[2] = {i < cnt, i0 == 0};
+            const CommRec rr[2] = {vv[0] ? load_rec(a, cc[0]) : rd, rd};
             long long sg[2];
-            sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, (uint32_t)u, sg);
+            sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, rr, (uint32_t)u, sg);
             if (i0 == 0) sd = sg[1];
             if (vv[0]) {
                 const double dl = delta_qi(a.dq, tv[i], kud, deg, sg[0], sd);
@@ -1052,8 +1161,8 @@ __device__ __forceinline__ void eval_vertex(const ExactState& a, const Round& r,
     }
     warp_argmax_pos(best_d, best_c);
     if (lane == 0) {
-        if (best_d > 0.0 && best_c != kNone && best_c != d) record(a, r, u, 1, best_c, best_d);
-        else record(a, r, u, 1, d, 0.0);
+        if (best_d > 0.0 && best_c != kNone && best_c != d) record(a, r, u, d, best_c, best_d);
+        else record(a, r, u, d, kNoMove, 0.0);
     }
 }
 
@@ -1080,7 +1189,8 @@ __device__ __forceinline__ void eval_small_body(const ExactState& a, const Ctl* 
             deg = (int)(a.rp[u + 1] - rb);
         }
         const bool tiny = inwin && deg <= kTinyDeg;
-        // One load round for the row, its vertex state and its neighbours' states.
+        // One load round for the row and its vertex state, one for its
+        // neighbours' states, one for the communities they are in.
         int32_t v = -1;
         uint32_t d = kNone;
         bool aff = false;
@@ -1091,45 +1201,59 @@ __device__ __forceinline__ void eval_small_body(const ExactState& a, const Ctl* 
             aff = a.vaff[u] != 0;
             ub = bound_of(a, (uint32_t)u);
         }
+        bool dirty = tiny && u >= r.pE;
         bool pm = false;
         uint32_t cv = kNone;
-        if (v >= 0) {
-            const uint32_t vc = a.vcom[v];
-            cv = vc;
-            if (v >= r.P && v < u) {
-                pm = r.pact[v] == 1 && r.pbest[v] != vc;
-                if (pm) cv = r.pbest[v];
-            }
-            if (!counts(a, v, (uint32_t)u, ub)) cv = kNone;   // self loops (and, refining, other bounds)
+        CommRec rc{0ull, 0u, 0u}, rd = rc;
+        if (tiny) {
+            rd = load_rec(a, d);
+            dirty = dirty || comm_changed(r, rd);
         }
+        if (v >= 0) {
+            const Seen sv = see(a, r, v, u);
+            pm = sv.moved;
+            dirty = dirty || sv.changed;
+            if (counts(a, v, (uint32_t)u, ub)) {   // not self loops (nor, refining, other bounds)
+                cv = sv.c;
+                rc = load_rec(a, cv);
+                dirty = dirty || comm_changed(r, rc);
+            }
+        }
+        const unsigned dirtyb = __ballot_sync(0xFFFFFFFFu, dirty);
+        const bool redo = tiny && (dirtyb & gmask) != 0;
+        if (tiny && !redo && j == 0) keep_decision(r, u);
+        const unsigned pmb = __ballot_sync(0xFFFFFFFFu, pm);
+        const bool act = redo && (aff || (pmb & gmask) != 0);
         // Refinement: the group's vertex stays when its community already holds more.
         bool stays = false;
         if (a.vcob) {
             long long sg1 = 0;
-            if (tiny && j == 0) {
+            if (redo && j == 0) {
                 const uint32_t cc[1] = {d};
                 const bool vv[1] = {true};
+                const CommRec rr[1] = {rd};
                 long long o[1];
-                sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, (uint32_t)u, o);
+                sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, rr, (uint32_t)u, o);
                 sg1 = o[0];
             }
             sg1 = __shfl_sync(0xFFFFFFFFu, sg1, lane & ~7);
-            stays = tiny && refine_stays(a, (double)sg1, (double)deg);
+            stays = redo && refine_stays(a, (double)sg1, (double)deg);
         }
-        const unsigned pmb = __ballot_sync(0xFFFFFFFFu, pm);
-        const bool act = tiny && (aff || (pmb & gmask) != 0);
         const uint32_t c = act ? cv : kNone;
-        const unsigned peers = __match_any_sync(0xFFFFFFFFu, ((unsigned long long)g << 32) | c);
-        const unsigned eqd = __ballot_sync(0xFFFFFFFFu, act && c != kNone && c == d) & gmask;
         double best_d = 0.0;
         uint32_t best_c = kNone;
-        if (act && c != kNone && c != d && lane == __ffs(peers) - 1) {
-            const uint32_t cc[2] = {c, d};
-            const bool vv[2] = {true, true};
-            long long sg[2];
-            sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, (uint32_t)u, sg);
-            const double dl = delta_qi(a.dq, __popc(peers), __popc(eqd), deg, sg[0], sg[1]);
-            if (dpos(dl)) { best_d = dl; best_c = c; }
+        if (dirtyb) {
+            const unsigned peers = __match_any_sync(0xFFFFFFFFu, ((unsigned long long)g << 32) | c);
+            const unsigned eqd = __ballot_sync(0xFFFFFFFFu, act && c != kNone && c == d) & gmask;
+            if (act && c != kNone && c != d && lane == __ffs(peers) - 1) {
+                const uint32_t cc[2] = {c, d};
+                const bool vv[2] = {true, true};
+                const CommRec rr[2] = {rc, rd};
+                long long sg[2];
+                sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, rr, (uint32_t)u, sg);
+                const double dl = delta_qi(a.dq, __popc(peers), __popc(eqd), deg, sg[0], sg[1]);
+                if (dpos(dl)) { best_d = dl; best_c = c; }
+            }
         }
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) {   // argmax inside each 8-lane group
@@ -1137,10 +1261,9 @@ __device__ __forceinline__ void eval_small_body(const ExactState& a, const Ctl* 
             const uint32_t oc = __shfl_xor_sync(0xFFFFFFFFu, best_c, o);
             if (better_pos(od, oc, best_d, best_c)) { best_d = od; best_c = oc; }
         }
-        if (tiny && j == 0) {
-            if (!act) record(a, r, u, 0, d, 0.0);
-            else if (!stays && best_d > 0.0 && best_c != kNone && best_c != d) record(a, r, u, 1, best_c, best_d);
-            else record(a, r, u, 1, d, 0.0);
+        if (redo && j == 0) {
+            if (act && !stays && best_d > 0.0 && best_c != kNone && best_c != d) record(a, r, u, d, best_c, best_d);
+            else record(a, r, u, d, kNoMove, 0.0);
         }
         // Rows of degree 9..32: the whole warp, one row at a time.
 #pragma unroll 1
@@ -1213,11 +1336,12 @@ __device__ __forceinline__ void eval_big_body(const ExactState& a, const Ctl* c)
         if (any) s_any = 1;
         __syncthreads();
         if (!s_any) {
-            if (tid == 0) record(a, r, u, 0, d, 0.0);
+            if (tid == 0) record(a, r, u, d, kNoMove, 0.0);
             __syncthreads();
             continue;
         }
         const double ku = (double)deg;
+        const CommRec rd = load_rec(a, d);
         const uint32_t kud = table_get(tk, tv, mask, d);
         // Compact the candidates (c != d); their order does not matter, the
         // selection is a total order.
@@ -1244,8 +1368,9 @@ __device__ __forceinline__ void eval_big_body(const ExactState& a, const Ctl* c)
             const uint32_t i = i0 + tid;
             const uint32_t cc[2] = {i < cnt ? cand_c[i] : kNone, d};
             const bool vv[2] = {i < cnt, i0 == 0};
+            const CommRec rr[2] = {vv[0] ? load_rec(a, cc[0]) : rd, rd};
             long long sg[2];
-            sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, u, sg);
+            sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, rr, u, sg);
             if (i0 == 0) sd = sg[1];
             if (vv[0]) {
                 const double dl = delta_qi(a.dq, cand_w[i], kud, deg, sg[0], sd);
@@ -1261,8 +1386,8 @@ __device__ __forceinline__ void eval_big_body(const ExactState& a, const Ctl* c)
             uint32_t bc = red_c[0];
             for (int k = 1; k < (int)(blockDim.x / 32); ++k)
                 if (better_pos(red_d[k], red_c[k], bd, bc)) { bd = red_d[k]; bc = red_c[k]; }
-            if (!refine_stays(a, (double)sd, ku) && bd > 0.0 && bc != kNone && bc != d) record(a, r, u, 1, bc, bd);
-            else record(a, r, u, 1, d, 0.0);
+            if (!refine_stays(a, (double)sd, ku) && bd > 0.0 && bc != kNone && bc != d) record(a, r, u, d, bc, bd);
+            else record(a, r, u, d, kNoMove, 0.0);
         }
         __syncthreads();
     }
@@ -1392,6 +1517,7 @@ __device__ __forceinline__ void hub_select_body(const ExactState& a, const Ctl* 
         const uint32_t d = a.vcom[h];
         const long long ku = a.rp[h + 1] - a.rp[h];
         const uint32_t kud = a.hub_kud[j];
+        const CommRec rd = load_rec(a, d);
         double best_d = 0.0;
         uint32_t best_c = kNone;
         // Segment `part` covers occupied-list positions [s0, s0 + kTabSeg):
@@ -1406,8 +1532,9 @@ __device__ __forceinline__ void hub_select_body(const ExactState& a, const Ctl* 
                 const uint32_t c0 = i < s1 ? tk[slot] : kNone, w0 = i < s1 ? tv[slot] : 0;
                 const uint32_t cc[2] = {c0, d};
                 const bool vv[2] = {c0 != kNone && c0 != d, i0 == s0};
+                const CommRec rr[2] = {vv[0] ? load_rec(a, c0) : rd, rd};
                 long long sgm[2];
-                sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, h, sgm);
+                sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, rr, h, sgm);
                 if (i0 == s0) sd = sgm[1];
                 if (vv[0]) {
                     const double dl = delta_qi(a.dq, w0, kud, ku, sgm[0], sd);
@@ -1454,13 +1581,13 @@ __device__ __forceinline__ void hub_select_body(const ExactState& a, const Ctl* 
                 if (a.vcob) {
                     const uint32_t cc[1] = {d};
                     const bool vv[1] = {true};
+                    const CommRec rr[1] = {rd};
                     long long o[1];
-                    sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, h, o);
+                    sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, rr, h, o);
                     stays = refine_stays(a, (double)o[0], ku);
                 }
-                if (!act) record(a, r, h, 0, d, 0.0);
-                else if (!stays && bd > 0.0 && bc != kNone && bc != d) record(a, r, h, 1, bc, bd);
-                else record(a, r, h, 1, d, 0.0);
+                if (act && !stays && bd > 0.0 && bc != kNone && bc != d) record(a, r, h, d, bc, bd);
+                else record(a, r, h, d, kNoMove, 0.0);
                 a.hub_done[j] = 0;
                 a.hub_any[j] = 0;
                 a.hub_kud[j] = 0;
@@ -1491,34 +1618,29 @@ __device__ __forceinline__ long long commit_end(const ExactState& a, const Ctl* 
 // round's "previous" buffers.
 struct CommitView {
     long long P, x;
-    const uint8_t* act;
-    const uint32_t* best;
-    const double* delta;
+    const uint32_t* dec;
 };
 
 __device__ __forceinline__ CommitView commit_view(const ExactState& a, const Ctl* ct) {
     CommitView c;
     c.P = ct->cP;
     c.x = ct->cX;
-    const int par = (int)(ct->round & 1);
-    c.act = a.act[par];
-    c.best = a.best[par];
-    c.delta = a.delta[par];
+    c.dec = a.dec[ct->round & 1];
     return c;
 }
 
 // Commit [cP, cX]: totals and memberships of movers, final deltas, processed
 // flags cleared, move flags for the affected-flag kernels; and the decided
 // window's hub tables cleared for the next round.
-// Adds (or, with neg, subtracts) v to total[key] once per distinct key of the
+// Adds (or, with neg, subtracts) v to the key's total once per distinct key of the
 // warp (kNone = no update); every lane of the warp calls it.  Degrees are
 // below 2^31, so the 16-bit halves of 32 of them sum without overflow.
-__device__ __forceinline__ void warp_add_total(unsigned long long* total, uint32_t key, uint32_t v, bool neg) {
+__device__ __forceinline__ void warp_add_total(CommRec* rec, uint32_t key, uint32_t v, bool neg) {
     const unsigned peers = __match_any_sync(0xFFFFFFFFu, key);
     const unsigned lo = __reduce_add_sync(peers, v & 0xFFFFu), hi = __reduce_add_sync(peers, v >> 16);
     if (key != kNone && (threadIdx.x & 31) == __ffs(peers) - 1) {
         const long long sum = ((long long)hi << 16) + (long long)lo;
-        if (sum) atomicAdd(&total[key], (unsigned long long)(neg ? -sum : sum));
+        if (sum) atomicAdd(&rec[key].total, (unsigned long long)(neg ? -sum : sum));
     }
 }
 
@@ -1539,19 +1661,19 @@ __device__ __forceinline__ void commit_a_body(const ExactState& a, const Ctl* ct
         if (u <= c.x) {
             double dl = 0.0;
             cur = a.vcom[u];
-            nb = c.best[u];
-            moves = c.act[u] == 1 && nb != cur;
+            nb = c.dec[u] & kNoMove;
+            moves = nb != kNoMove;
             if (moves) {
                 deg = (uint32_t)(a.rp[u + 1] - a.rp[u]);
-                dl = c.delta[u];
+                dl = a.delta[u];
                 a.vcom[u] = nb;
             }
             a.mv[u] = moves;
             a.final_delta[u] = dl;
             a.vaff[u] = 0;
         }
-        warp_add_total(a.ctot, moves ? cur : kNone, deg, true);
-        warp_add_total(a.ctot, moves ? nb : kNone, deg, false);
+        warp_add_total(a.rec, moves ? cur : kNone, deg, true);
+        warp_add_total(a.rec, moves ? nb : kNone, deg, false);
     }
     const long long q0 = ct->c_ts0, q1 = ct->c_ts1;
     __shared__ int s_last;
@@ -1751,8 +1873,8 @@ __device__ __forceinline__ void advance_ctl(const ExactState& a, Ctl* c, long lo
     const long long x = commit_end(a, c);
     const long long nP = x + 1, nE = min(n, nP + B);
     const int par = (int)(c->round & 1);
-    uint8_t* next_prev_act = a.act[par ^ 1];
-    for (long long u = E + tid0; u < nE; u += tstride) next_prev_act[u] = kUnknown;
+    uint32_t* next_dec = a.dec[par ^ 1];
+    for (long long u = E + tid0; u < nE; u += tstride) next_dec[u] = kNoMove;
     if (threadIdx.x == 0) {
         c->c_es0 = c->es0;
         c->c_es1 = c->es1;
@@ -1763,11 +1885,22 @@ __device__ __forceinline__ void advance_ctl(const ExactState& a, Ctl* c, long lo
     }
     __syncthreads();
     window_ranges(a, c, nP, nE);
+    // Designated communities: their records point the next table's lookups at
+    // the dense rows, and count as changed -- the old set's too, which a
+    // change of the set moves between the dense rows and the sorted table.
+    const uint32_t ntag = (uint32_t)c->tag + 1u;
+    if (threadIdx.x < c->nz) a.rec[c->zc[threadIdx.x]].cver = ntag;
     designate(a, c);
+    if (threadIdx.x < c->nz) {
+        CommRec* z = a.rec + c->zc[threadIdx.x];
+        z->cver = ntag;
+        z->slotw = ntag << kSlotwTagShift | kSlotwDesig | threadIdx.x;
+    }
     if (threadIdx.x == 0) {
         const long long rnd = c->round + 1;
         c->cP = P;
         c->cX = x;
+        c->pE = E;
         c->evals = c->evals + (E - P);
         c->P = nP;
         c->E = nE;
@@ -1794,7 +1927,7 @@ __global__ void __launch_bounds__(1024) k_ex_advance(ExactState a) {
 __device__ __forceinline__ void init_ctl(const ExactState& a, Ctl* c, long long tid0, long long tstride) {
     const long long n = c->n, B = c->B;
     const long long E = min(n, B);
-    for (long long u = tid0; u < E; u += tstride) a.act[0][u] = kUnknown;
+    for (long long u = tid0; u < E; u += tstride) a.dec[0][u] = kNoMove;
     window_ranges(a, c, 0, E);
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1802,8 +1935,9 @@ __device__ __forceinline__ void init_ctl(const ExactState& a, Ctl* c, long long 
         c->E = E;
         c->round = 0;
         c->evals = 0;
-        c->cP = 1;
+        c->cP = n;   // no window before: nothing to commit, nothing changed
         c->cX = 0;
+        c->pE = 0;
         c->tag = c->tag + 1;
         for (int j = 0; j < kZMax; ++j) c->zcount[j] = 0;
     }
@@ -1850,6 +1984,16 @@ __global__ void k_sum_serial(const double* __restrict__ d, int64_t n, double* __
         for (int64_t i = 0; i < n; ++i) s += d[i];
         *out = s;
     }
+}
+
+__global__ void k_rec_from_totals(const unsigned long long* __restrict__ ctot, int64_t n, CommRec* __restrict__ rec) {
+    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
+        rec[c] = CommRec{ctot[c], 0u, 0u};
+}
+
+__global__ void k_totals_from_rec(const CommRec* __restrict__ rec, int64_t n, unsigned long long* __restrict__ ctot) {
+    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
+        ctot[c] = rec[c].total;
 }
 
 __global__ void k_hub_degrees(const int64_t* __restrict__ rp, const uint32_t* __restrict__ hubs, int64_t nh,
@@ -1967,9 +2111,11 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     }
 
     // ---- round state ----
-    DevBuf<uint32_t> best0(n, s), best1(n, s);
-    DevBuf<uint8_t> act0(n, s), act1(n, s);
-    DevBuf<double> delta0(n, s), delta1(n, s), final_delta(n, s);
+    DevBuf<uint32_t> dec0(n, s), dec1(n, s);
+    DevBuf<double> delta(n, s), final_delta(n, s);
+    DevBuf<CommRec> rec(n, s);
+    k_rec_from_totals<<<grid_for(n, kT), kT, 0, s>>>(ctx.ctot, n, rec);
+    GB_LAUNCH_CHECK();
     DevBuf<uint8_t> mv(n, s);
     DevBuf<SlotMeta> slots(kTableSlots, s);
     GB_CUDA(cudaMemsetAsync(slots, 0xFF, kTableSlots * sizeof(SlotMeta), s));   // no generation yet
@@ -1999,17 +2145,14 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     a.rp = ctx.g.row_ptr;
     a.col = ctx.g.col;
     a.vcom = ctx.vcom;
-    a.ctot = ctx.ctot;
+    a.rec = rec.get();
     a.vaff = ctx.vaff;
     a.vcob = ctx.vcob;
     a.mv = mv.get();
     a.ctl = ctl.get();
-    a.best[0] = best0.get();
-    a.best[1] = best1.get();
-    a.act[0] = act0.get();
-    a.act[1] = act1.get();
-    a.delta[0] = delta0.get();
-    a.delta[1] = delta1.get();
+    a.dec[0] = dec0.get();
+    a.dec[1] = dec1.get();
+    a.delta = delta.get();
     a.final_delta = final_delta.get();
     a.slots = slots.get();
     a.tb_s0 = tb_s0.get();
@@ -2304,6 +2447,9 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
         nl += 2;
         if (stop) break;
     }
+    k_totals_from_rec<<<grid_for(n, kT), kT, 0, s>>>(rec, n, ctx.ctot);
+    GB_LAUNCH_CHECK();
+    nl += 2;
     cudaFreeHost(hctl);
     if (launches) *launches += nl;
     if (rounds_out) *rounds_out += rounds;
