@@ -13,6 +13,7 @@
 // (<= 2048) or one 1024-thread CTA (<= 16384) with a shared-memory LSD radix
 // sort, and a global radix sort of (row, new id) keys for the few longer
 // rows.  The three middle classes run concurrently on forked streams.
+#include "gb_chunks.cuh"
 #include "gb_common.cuh"
 #include "gb_stages.h"
 
@@ -284,12 +285,20 @@ __global__ void k_set_last(int64_t* p, int64_t n, int64_t v) { p[n] = v; }
 // Squished-CSR check: offsets non-decreasing from 0, neighbour ids in range,
 // rows strictly increasing (sorted, no duplicates).  bad[0]: offsets,
 // bad[1]: ids out of range, bad[2]: unsorted or duplicate.
-// Row offsets: rp[0] == 0, non-decreasing, rp[n] == nnz.
-__global__ void k_check_rows(const int64_t* __restrict__ rp, int64_t n, int64_t nnz, int32_t* __restrict__ bad) {
+// Row offsets: rp[0] == 0, non-decreasing, rp[n] == nnz.  The pass also notes the
+// row that holds each chunk's first entry (a serial search per chunk in the pass
+// below took most of its time: 114 us for 33 M entries).
+__global__ void k_check_rows(const int64_t* __restrict__ rp, int64_t n, int64_t nnz, int32_t* __restrict__ bad,
+                             int32_t* __restrict__ chunk_row) {
     for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u <= n; u += (int64_t)gridDim.x * blockDim.x) {
         const int64_t b = rp[u];
         const bool ok = b >= 0 && b <= nnz && (u == 0 ? b == 0 : rp[u - 1] <= b) && (u != n || b == nnz);
         if (!ok) atomicOr(&bad[0], 1);
+        const int64_t e = u < n ? rp[u + 1] : 0;
+        // (malformed offsets can overlap without end: stop once one is found)
+        if (ok && e <= nnz)
+            for (int64_t c = (b + kEdgeChunk - 1) / kEdgeChunk; c * kEdgeChunk < e && !*(volatile int32_t*)bad; ++c)
+                chunk_row[c] = (int32_t)u;
     }
 }
 
@@ -297,37 +306,29 @@ __global__ void k_check_rows(const int64_t* __restrict__ rp, int64_t n, int64_t 
 // starts that fall inside a chunk are marked in a shared bitmap, and every
 // entry that is not a row start must exceed its predecessor.  Runs only on
 // valid row offsets (bad[0] clear), so every entry lies in exactly one row.
-constexpr int kCheckChunk = 4096;
+constexpr int kCheckChunk = kEdgeChunk;
 constexpr int kCheckThreads = 256;
 
 __global__ void __launch_bounds__(kCheckThreads)
 k_check_cols(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, int64_t n, int64_t nnz,
-             int32_t* __restrict__ bad) {
+             const int32_t* __restrict__ chunk_row, int32_t* __restrict__ bad) {
     if (*(volatile int32_t*)&bad[0]) return;
     __shared__ uint32_t starts[kCheckChunk / 32];
-    __shared__ int64_t s_u0;
     const int64_t chunks = (nnz + kCheckChunk - 1) / kCheckChunk;
     int range_bad = 0, order_bad = 0;
     for (int64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
         const int64_t e0 = c * kCheckChunk;
         const int64_t e1 = min(nnz, e0 + kCheckChunk);
+        const int64_t u0 = chunk_row[c];
         for (int w = threadIdx.x; w < kCheckChunk / 32; w += blockDim.x) starts[w] = 0;
-        if (threadIdx.x == 0) {
-            // Largest u with rp[u] <= e0: the row holding entry e0.
-            int64_t lo = 0, hi = n;
-            while (hi - lo > 1) {
-                const int64_t mid = (lo + hi) >> 1;
-                if (rp[mid] <= e0) lo = mid; else hi = mid;
-            }
-            s_u0 = lo;
-        }
         __syncthreads();
-        for (int64_t u = s_u0 + threadIdx.x; u <= n; u += blockDim.x) {
+        for (int64_t u = u0 + threadIdx.x; u <= n; u += blockDim.x) {
             const int64_t r = rp[u];
             if (r >= e1) break;
             if (r >= e0) atomicOr(&starts[(r - e0) >> 5], 1u << ((r - e0) & 31));
         }
         __syncthreads();
+#pragma unroll 8
         for (int64_t i = e0 + threadIdx.x; i < e1; i += blockDim.x) {
             const int32_t v = col[i];
             range_bad |= (v < 0 || (int64_t)v >= n);
@@ -346,11 +347,12 @@ void check_graph_device(const DeviceCSR& g, cudaStream_t s) {
     if (g.n == 0) return;
     DevBuf<int32_t> bad(3, s);
     GB_CUDA(cudaMemsetAsync(bad, 0, 3 * sizeof(int32_t), s));
-    k_check_rows<<<grid_for(g.n + 1, 256), 256, 0, s>>>(g.row_ptr, g.n, g.nnz, bad);
+    DevBuf<int32_t> chunk_row(std::max<int64_t>(1, edge_chunks(g.nnz)), s);
+    k_check_rows<<<grid_for(g.n + 1, 256), 256, 0, s>>>(g.row_ptr, g.n, g.nnz, bad, chunk_row);
     GB_LAUNCH_CHECK();
     if (g.nnz > 0) {
         k_check_cols<<<grid_for(ceil_div(g.nnz, kCheckChunk), 1), kCheckThreads, 0, s>>>(g.row_ptr, g.col, g.n,
-                                                                                       g.nnz, bad);
+                                                                                       g.nnz, chunk_row, bad);
         GB_LAUNCH_CHECK();
     }
     int32_t h[3];

@@ -53,3 +53,45 @@ def test_gorder_by_community_size(ctx, sizes, window):
     np.testing.assert_array_equal(ids, expect)
     assert [st["gorder_communities"], st["gorder_vertices"], st["gorder_max_community"]] == \
         [ost.gorder_communities, ost.gorder_vertices, ost.gorder_max_community]
+
+
+def _kernel_graph(kind, size):
+    if kind == "star":        # one row at the edge of the segmented rows, and a path hanging off it
+        edges = [(0, i) for i in range(1, size + 1)] + [(size + i, size + i + 1) for i in range(40)]
+        return gg.from_edges(size + 60, edges)
+    if kind == "stars":       # several long rows and bridges between them
+        edges = [(h * size, h * size + i) for h in range(4) for i in range(1, size)]
+        return gg.from_edges(4 * size + 3, edges + [(size - 1, size), (3 * size, 2 * size + 5)])
+    if kind == "path":        # as many levels as vertices
+        return gg.from_edges(size, [(i, i + 1) for i in range(size - 1)])
+    if kind == "grid":        # frontiers on both sides of the one-CTA limit
+        return gg.grid(size, 60000 // size + 3, 0.02, seed=size)
+    return gg.uniform(size, 8, seed=size)
+
+
+@pytest.mark.parametrize("kind,size", [("star", 7), ("star", 8), ("star", 9), ("star", 64), ("star", 65),
+                                       ("star", 1023), ("star", 1024), ("star", 1025), ("star", 40000),
+                                       ("stars", 2049), ("stars", 9000), ("path", 2), ("path", 33), ("path", 3001),
+                                       ("grid", 3), ("grid", 245), ("uniform", 5), ("uniform", 13), ("uniform", 17)])
+def test_kernels_by_row_length_and_frontier(ctx, kind, size):
+    rp, col = (t.numpy() for t in _kernel_graph(kind, size))
+    n = len(rp) - 1
+    for source in {0, n // 2, int(np.argmax(np.diff(rp)))}:
+        np.testing.assert_array_equal(ctx.bfs(rp, col, source)[0], po.bfs_depths(rp, col, source))
+    np.testing.assert_array_equal(ctx.connected_components(rp, col)[0], po.cc_min_labels(rp, col))
+    # Seven Jacobi sweeps in float64.  A float32 row sum of d terms in lanes and a
+    # tree has a relative error below (d / 256 + 10) 2^-24 for the longest rows
+    # here (40,000: 1e-5), and a sweep passes 0.85 of the error on.
+    score = np.full(n, 1.0 / n)
+    degree = np.diff(rp)
+    row = np.repeat(np.arange(n), degree)
+    for _ in range(7):
+        share = np.where(degree > 0, score / np.maximum(degree, 1), 0.0)
+        score = 0.15 / n + 0.85 * np.bincount(row, weights=share[col], minlength=n)
+    got, sweeps, _ = ctx.pagerank(rp, col, max_iters=7, epsilon=0.0)
+    assert sweeps == 7
+    np.testing.assert_allclose(got, score, rtol=6e-5)
+    # A converged run stops at the sweep whose change is below epsilon.
+    _, stop, _ = ctx.pagerank(rp, col, max_iters=100, epsilon=1e-3)
+    _, one_less, _ = ctx.pagerank(rp, col, max_iters=max(1, stop - 1), epsilon=1e-3)
+    assert stop <= 100 and one_less == max(1, stop - 1)
