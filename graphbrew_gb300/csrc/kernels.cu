@@ -83,18 +83,23 @@ __device__ __forceinline__ double pr_put(const PrArgs& a, int64_t u, float s, in
 // One Jacobi sweep, score[u] = base + damp * sum contrib_in[v], over chunks of
 // kEdgeChunk entries: a CTA gathers its chunk's contributions into shared
 // memory (coalesced neighbour reads, sixteen gathers a thread in flight whatever
-// the row lengths), then adds up the rows in it, short ones by a thread, longer
-// ones by a warp.  Rows that cross chunks leave partial sums to k_pr_join.
+// the row lengths), then adds up the rows in it by a thread, eight lanes or a
+// warp.  Rows that cross chunks leave partial sums to k_pr_join.
 // Bound by the gather of contributions from L2, 4 bytes wanted of each 32-byte
 // sector.  RMAT scale 20, 33 M entries: a warp per row 1.43 ms a sweep (nearly
 // all of it the largest row's), lanes, warps and CTAs by row length 0.48 ms.
 // Rows without entries keep the score that k_pr_isolated gives them.
-constexpr int kPrOwn = 24;    // rows up to this long by a thread
+constexpr int kPrOwn = 24;      // rows up to this long by a thread
+constexpr int kPrOctet = 256;   // up to this long by eight lanes, longer ones by a warp
 
 __global__ void __launch_bounds__(kT, 6) k_pr_sweep(PrArgs a, int it) {
     if (pr_done(a.err, it, a.epsilon)) return;
     __shared__ float val[kEdgeChunkPadded];
-    __shared__ int32_t s_more;
+    __shared__ int32_t s_more, s_listed;
+    __shared__ int sb[kT], se[kT];
+    __shared__ float sums[kT];
+    __shared__ uint8_t list[kT];   // rows left to more lanes
+    static_assert(kT <= 256, "list entries");
     const int t = threadIdx.x, lane = t & 31;
     double err = 0.0;
     const int64_t chunks = (a.nnz + kEdgeChunk - 1) / kEdgeChunk;
@@ -109,7 +114,10 @@ __global__ void __launch_bounds__(kT, 6) k_pr_sweep(PrArgs a, int it) {
             for (int k = 0; k < kEdgeChunk / kT; ++k)
                 if (v[k] >= 0) val[chunk_pad(k * kT + t)] = a.cin[v[k]];
         }
-        if (t == 0) a.tail_row[c] = -1;
+        if (t == 0) {
+            a.tail_row[c] = -1;
+            s_listed = 0;
+        }
         __syncthreads();
         // Rows from the one that holds entry e0, 256 at a time, until one starts past the chunk.
         for (int64_t u0 = a.chunk_row[c];; u0 += kT) {
@@ -118,18 +126,34 @@ __global__ void __launch_bounds__(kT, 6) k_pr_sweep(PrArgs a, int it) {
             const int b = (int)(max(rb, e0) - e0), e = rb < e1 ? (int)(min(re, e1) - e0) : b;
             if (t == kT - 1) s_more = rb < e1;
             float s = 0.f;
-            if (e - b <= kPrOwn)
+            if (e - b <= kPrOwn) {
                 for (int i = b; i < e; ++i) s += val[chunk_pad(i)];
-            unsigned todo = __ballot_sync(kFull, e - b > kPrOwn);
-            while (todo) {
-                const int src = __ffs(todo) - 1;
-                todo &= todo - 1;
-                const int es = __shfl_sync(kFull, e, src);
-                float x = 0.f;
-                for (int i = __shfl_sync(kFull, b, src) + lane; i < es; i += 32) x += val[chunk_pad(i)];
-                for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
-                if (lane == src) s = x;
+            } else {
+                list[atomicAdd(&s_listed, 1)] = (uint8_t)t;
+                sb[t] = b;
+                se[t] = e;
             }
+            __syncthreads();
+            const int listed = s_listed;
+            for (int q = t >> 3; q - (t >> 3) < listed; q += kT / 8) {
+                const int w = q < listed ? list[q] : 0;
+                const bool mine = q < listed && se[w] - sb[w] <= kPrOctet;
+                float x = 0.f;
+                if (mine)
+                    for (int i = sb[w] + (lane & 7); i < se[w]; i += 8) x += val[chunk_pad(i)];
+                for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
+                if (mine && (lane & 7) == 0) sums[w] = x;
+            }
+            for (int q = t >> 5; q < listed; q += kT / 32) {
+                const int w = list[q];
+                if (se[w] - sb[w] <= kPrOctet) continue;
+                float x = 0.f;
+                for (int i = sb[w] + lane; i < se[w]; i += 32) x += val[chunk_pad(i)];
+                for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
+                if (lane == 0) sums[w] = x;
+            }
+            __syncthreads();
+            if (e - b > kPrOwn) s = sums[t];
             if (e > b) {
                 if (rb < e0) a.head[c] = s;
                 else if (re > e1) {
@@ -137,8 +161,8 @@ __global__ void __launch_bounds__(kT, 6) k_pr_sweep(PrArgs a, int it) {
                     a.tail_row[c] = (int32_t)u;
                 } else err += pr_put(a, u, s, re - rb);
             }
-            __syncthreads();
             const bool more = s_more;
+            if (t == 0) s_listed = 0;
             __syncthreads();
             if (!more) break;
         }
@@ -587,11 +611,13 @@ __global__ void k_cc_flatten(int64_t n, int32_t* parent) {
     }
 }
 
-// Joins every vertex with its second and its last neighbour: on graphs with a
-// giant component nearly all of it is one tree before the pass over all entries.
-__global__ void k_cc_sample(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, int64_t n,
+// Joins every step-th vertex with its second and its last neighbour: on graphs
+// with a giant component nearly all of it is one tree before the pass over all
+// entries.
+__global__ void k_cc_sample(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, int64_t n, int step,
                             int32_t* parent) {
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t v = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * step; v < n;
+         v += (int64_t)gridDim.x * blockDim.x * step) {
         const int64_t b = rp[v], e = rp[v + 1];
         if (e - b < 2) continue;
         cc_union(parent, (int32_t)v, col[b + 1]);
@@ -600,7 +626,7 @@ __global__ void k_cc_sample(const int64_t* __restrict__ rp, const int32_t* __res
 }
 
 // All entries, in chunks with their rows known: coalesced neighbour reads and
-// sixteen parent gathers a thread in flight.  The parents come through L1: a
+// eight pairs of parent reads a thread in flight.  The parents come through L1: a
 // stale one is still an ancestor, and only sends its entry to the union.
 __global__ void __launch_bounds__(kT)
 k_cc_link(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, int64_t n, int64_t nnz,
@@ -811,8 +837,12 @@ double cc_device(const DeviceCSR& g, int32_t* comp, cudaStream_t s) {
     k_cc_flatten<false><<<grid_for(n, kT), kT, 0, s>>>(n, comp);
     GB_LAUNCH_CHECK();
     if (g.nnz > 0) {
-        k_cc_sample<<<grid_for(n, kT), kT, 0, s>>>(g.row_ptr, g.col, n, comp);
-        k_cc_flatten<false><<<grid_for(n, kT), kT, 0, s>>>(n, comp);
+        // Every 32nd vertex first: the large trees meet with few threads asking
+        // for the same roots (all vertices at once: 0.56 ms on RMAT scale 20).
+        for (const int step : {32, 1}) {
+            k_cc_sample<<<grid_for(ceil_div(n, step), kT), kT, 0, s>>>(g.row_ptr, g.col, n, step, comp);
+            k_cc_flatten<false><<<grid_for(n, kT), kT, 0, s>>>(n, comp);
+        }
         GB_LAUNCH_CHECK();
         const int64_t chunks = edge_chunks(g.nnz);
         DevBuf<int32_t> chunk_row(chunks, s);
