@@ -14,6 +14,8 @@
 // log end-to-end times of the three arms (GraphBrew algorithm 12, DBG, original
 // order).  Forward, backward (mean squared error) and Adam are hand-written
 // kernels with a fixed summation order per output element.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -194,13 +196,19 @@ __global__ void k_mse(const float* __restrict__ Y, const float* __restrict__ T, 
     row_loss[r] = l;
 }
 
+__device__ __forceinline__ void adam_step(float& p, float g, float& m, float& v, float lr, float b1, float b2,
+                                          float eps, float c1, float c2) {
+    // Contracted by name: the same rounding in every kernel that steps.
+    m = fmaf(b1, m, (1.f - b1) * g);
+    v = fmaf(b2, v, (1.f - b2) * g * g);
+    p -= lr * (m / c1) / (sqrtf(v / c2) + eps);
+}
+
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                        float* __restrict__ v, int n, float lr, float b1, float b2, float eps, float c1, float c2) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    m[i] = b1 * m[i] + (1.f - b1) * g[i];
-    v[i] = b2 * v[i] + (1.f - b2) * g[i] * g[i];
-    p[i] -= lr * (m[i] / c1) / (sqrtf(v[i] / c2) + eps);
+    adam_step(p[i], g[i], m[i], v[i], lr, b1, b2, eps, c1, c2);
 }
 
 __global__ void k_gather_rows(const float* __restrict__ src, const int32_t* __restrict__ idx, int rows, int cols,
@@ -208,6 +216,302 @@ __global__ void k_gather_rows(const float* __restrict__ src, const int32_t* __re
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= rows * cols) return;
     dst[t] = src[(int64_t)idx[t / cols] * cols + t % cols];
+}
+
+// ---------------------------------------------------------------------------
+// One epoch of training in one launch.
+//
+// A minibatch of 128 rows is 1.9 M multiply-adds, so as a dozen launches with a
+// copy back and a wait each it was all latency: 98 us a minibatch.  Here one
+// cluster of eight CTAs runs the epoch's minibatches with two cluster barriers
+// each: every CTA takes an eighth of the rows through the forward pass and the
+// activations' gradients (weights in its shared memory), then owns a block of
+// the weights: it fetches the activation columns that those need from the
+// others' shared memory, forms their gradients and Adam steps with parameter and
+// moments in registers, and writes the new weights into all eight copies.
+//
+// Every sum runs in the order of the kernels above (inputs, outputs or rows
+// ascending, one fused multiply-add each), so the parameters are the same bit for
+// bit: training amplifies a changed rounding some thousandfold.
+// ---------------------------------------------------------------------------
+constexpr int kTrCtas = 8;
+constexpr int kTrThreads = 512;
+constexpr int kTrMaxIn = 32;      // the single-output threads cover in * 8 + 67 outputs
+constexpr int kTrMaxBatch = 256;  // activations and column copies in shared memory
+constexpr int kTrW2Stride = kMlpHidden + 1;   // W2 is read along both axes
+
+struct TrainArgs {
+    float *params, *m, *v;
+    const float *X, *T;
+    const int32_t* order;     // this epoch's rows
+    const float2* corr;       // per minibatch: Adam's 1 - b1^t, 1 - b2^t
+    float* row_loss;
+    int n, in, batch;
+    float lr, b1, b2, eps;
+};
+
+// Offsets (floats) into a CTA's shared memory.
+struct TrainLayout {
+    int w1, b1, w2, b2, w3, b3;             // weights
+    int x, h1, h2, d2, d1, dy;              // this CTA's rows
+    int cx, ch1, ch2, cd2, cd1, cdy;        // columns of all rows
+    int total;
+};
+
+__host__ __device__ inline TrainLayout train_layout(int in, int batch) {
+    const int rows = (batch + kTrCtas - 1) / kTrCtas, all = rows * kTrCtas;
+    TrainLayout l;
+    int at = 0;
+    auto take = [&](int floats) {
+        const int here = at;
+        at += (floats + 3) & ~3;
+        return here;
+    };
+    l.w1 = take(in * kMlpHidden);
+    l.b1 = take(kMlpHidden);
+    l.w2 = take(kMlpHidden * kTrW2Stride);
+    l.b2 = take(kMlpHidden);
+    l.w3 = take(kMlpHidden * kMlpOut);
+    l.b3 = take(kMlpOut);
+    l.x = take(rows * in);
+    l.h1 = take(rows * kMlpHidden);
+    l.h2 = take(rows * kMlpHidden);
+    l.d2 = take(rows * kMlpHidden);
+    l.d1 = take(rows * kMlpHidden);
+    l.dy = take(rows * 4);
+    l.cx = take(all * in);
+    l.ch1 = take(all * 16);
+    l.ch2 = take(all * 8);
+    l.cd2 = take(all * 32);
+    l.cd1 = take(all * 8);
+    l.cdy = take(all * 4);
+    l.total = at;
+    return l;
+}
+
+__global__ void __cluster_dims__(kTrCtas, 1, 1) __launch_bounds__(kTrThreads) k_mlp_epoch(TrainArgs a) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    extern __shared__ __align__(16) float sm[];
+    constexpr int H = kMlpHidden, O = kMlpOut;
+    const int t = threadIdx.x, rank = (int)cluster.block_rank(), in = a.in;
+    const TrainLayout L = train_layout(in, a.batch);
+    // Packed parameters -> shared memory.
+    const int gw1 = 0, gb1 = in * H, gw2 = gb1 + H, gb2 = gw2 + H * H, gw3 = gb2 + H, gb3 = gw3 + H * O;
+    for (int i = t; i < in * H; i += kTrThreads) sm[L.w1 + i] = a.params[gw1 + i];
+    for (int i = t; i < H * H; i += kTrThreads) sm[L.w2 + (i / H) * kTrW2Stride + i % H] = a.params[gw2 + i];
+    for (int i = t; i < H * O; i += kTrThreads) sm[L.w3 + i] = a.params[gw3 + i];
+    if (t < H) {
+        sm[L.b1 + t] = a.params[gb1 + t];
+        sm[L.b2 + t] = a.params[gb2 + t];
+    }
+    if (t < O) sm[L.b3 + t] = a.params[gb3 + t];
+    // Parameters that this thread owns: the first 128 threads a 1 x 4 piece of
+    // the CTA's 16 x 32 block of W2, each other thread one of the rest.
+    const int bi = (rank >> 1) * 16, bo = (rank & 1) * 32;
+    const int wi = t >> 3, wo = (t & 7) * 4;
+    const int q = t - 128;
+    int own = 0, pg = 0, ps = 0;            // how many, packed index, shared index
+    int kind = -1, ka = 0, kb = 0;          // what its gradient sums: two columns
+    if (q < 0) {
+        own = 4;
+        pg = gw2 + (bi + wi) * H + bo + wo;
+        ps = L.w2 + (bi + wi) * kTrW2Stride + bo + wo;
+    } else if (q < in * 8) {
+        kind = 0, ka = q >> 3, kb = q & 7, own = 1;
+        pg = gw1 + ka * H + rank * 8 + kb;
+        ps = L.w1 + ka * H + rank * 8 + kb;
+    } else if (q < in * 8 + 8) {
+        kind = 1, kb = q - in * 8, own = 1;
+        pg = gb1 + rank * 8 + kb;
+        ps = L.b1 + rank * 8 + kb;
+    } else if (q < in * 8 + 32) {
+        const int j = q - in * 8 - 8;
+        kind = 2, ka = j / O, kb = j % O, own = 1;
+        pg = gw3 + (rank * 8 + ka) * O + kb;
+        ps = L.w3 + (rank * 8 + ka) * O + kb;
+    } else if (q < in * 8 + 64 && rank < 2) {   // bo = rank * 32 for these
+        kind = 3, kb = q - in * 8 - 32, own = 1;
+        pg = gb2 + bo + kb;
+        ps = L.b2 + bo + kb;
+    } else if (q >= in * 8 + 64 && q < in * 8 + 64 + O && rank == 0) {
+        kind = 4, kb = q - in * 8 - 64, own = 1;
+        pg = gb3 + kb;
+        ps = L.b3 + kb;
+    }
+    float p[4], m[4], v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        p[k] = m[k] = v[k] = 0.f;
+        if (k < own) {
+            p[k] = a.params[pg + k];
+            m[k] = a.m[pg + k];
+            v[k] = a.v[pg + k];
+        }
+    }
+    const int o = t & (H - 1), rg = t >> 6;   // column and row group of the row phase
+    // A minibatch's inputs and this thread's target are read a minibatch ahead:
+    // the row number and the row are two round trips.
+    constexpr int kXPer = kTrMaxBatch / kTrCtas * kTrMaxIn / kTrThreads;
+    float nx[kXPer], ntarget = 0.f;
+    auto read_ahead = [&](int b0) {
+        const int B = min(a.batch, a.n - b0), R = (B + kTrCtas - 1) / kTrCtas;
+        const int r0 = rank * R, rows = max(0, min(R, B - r0));
+#pragma unroll
+        for (int k = 0; k < kXPer; ++k) {
+            const int i = t + k * kTrThreads;
+            nx[k] = i < rows * in ? a.X[(int64_t)a.order[b0 + r0 + i / in] * in + i % in] : 0.f;
+        }
+        if (t < rows * 4 && (t & 3) < O) ntarget = a.T[(int64_t)a.order[b0 + r0 + (t >> 2)] * O + (t & 3)];
+    };
+    read_ahead(0);
+    for (int b0 = 0, step = 0; b0 < a.n; b0 += a.batch, ++step) {
+        const int B = min(a.batch, a.n - b0), R = (B + kTrCtas - 1) / kTrCtas;
+        const int r0 = rank * R, rows = max(0, min(R, B - r0));
+        const float2 corr = a.corr[step];
+        const float target = ntarget;
+#pragma unroll
+        for (int k = 0; k < kXPer; ++k) {
+            const int i = t + k * kTrThreads;
+            if (i < rows * in) sm[L.x + i] = nx[k];
+        }
+        __syncthreads();
+        // ---- this CTA's rows: forward (rows rg, rg + 8, ..., two at a time) ----
+        for (int r = rg; r < rows; r += 16) {
+            const int r2 = r + 8 < rows ? r + 8 : r;
+            float x = sm[L.b1 + o], y = x;
+            for (int i = 0; i < in; ++i) {
+                const float w = sm[L.w1 + i * H + o];
+                x = fmaf(sm[L.x + r * in + i], w, x);
+                y = fmaf(sm[L.x + r2 * in + i], w, y);
+            }
+            sm[L.h1 + r * H + o] = fmaxf(x, 0.f);
+            sm[L.h1 + r2 * H + o] = fmaxf(y, 0.f);
+        }
+        __syncthreads();
+        for (int r = rg; r < rows; r += 16) {
+            const int r2 = r + 8 < rows ? r + 8 : r;
+            float x = sm[L.b2 + o], y = x;
+#pragma unroll 4
+            for (int i = 0; i < H; i += 4) {
+                const float4 f = *reinterpret_cast<const float4*>(&sm[L.h1 + r * H + i]);
+                const float4 g = *reinterpret_cast<const float4*>(&sm[L.h1 + r2 * H + i]);
+                const float w0 = sm[L.w2 + i * kTrW2Stride + o], w1 = sm[L.w2 + (i + 1) * kTrW2Stride + o];
+                const float w2 = sm[L.w2 + (i + 2) * kTrW2Stride + o], w3 = sm[L.w2 + (i + 3) * kTrW2Stride + o];
+                x = fmaf(f.w, w3, fmaf(f.z, w2, fmaf(f.y, w1, fmaf(f.x, w0, x))));
+                y = fmaf(g.w, w3, fmaf(g.z, w2, fmaf(g.y, w1, fmaf(g.x, w0, y))));
+            }
+            sm[L.h2 + r * H + o] = fmaxf(x, 0.f);
+            sm[L.h2 + r2 * H + o] = fmaxf(y, 0.f);
+        }
+        __syncthreads();
+        // Outputs: four threads a row, three of them with an output; the mean
+        // squared error's gradient and the row's loss.
+        if (t < rows * 4) {
+            const int r = t >> 2, c = t & 3;
+            const int cc = c < O ? c : 0;
+            float y = sm[L.b3 + cc];
+#pragma unroll 8
+            for (int i = 0; i < H; ++i) y = fmaf(sm[L.h2 + r * H + i], sm[L.w3 + i * O + cc], y);
+            const float d = y - target;
+            if (c < O) sm[L.dy + r * 4 + c] = 2.f * d / (float)(B * O);
+            const unsigned mask = __activemask();
+            const int q0 = (t & 31) & ~3;
+            const float d0 = __shfl_sync(mask, d, q0), d1 = __shfl_sync(mask, d, q0 + 1),
+                        d2 = __shfl_sync(mask, d, q0 + 2);
+            if (c == 0) a.row_loss[b0 + r0 + r] = fmaf(d2, d2, fmaf(d1, d1, fmaf(d0, d0, 0.f)));
+        }
+        __syncthreads();
+        // Gradients of the activations.
+        for (int r = rg; r < rows; r += 8) {
+            float x = 0.f;
+#pragma unroll
+            for (int c = 0; c < O; ++c) x = fmaf(sm[L.dy + r * 4 + c], sm[L.w3 + o * O + c], x);
+            sm[L.d2 + r * H + o] = sm[L.h2 + r * H + o] > 0.f ? x : 0.f;
+        }
+        __syncthreads();
+        for (int r = rg; r < rows; r += 16) {
+            const int r2 = r + 8 < rows ? r + 8 : r;
+            float x = 0.f, y = 0.f;
+#pragma unroll 4
+            for (int c = 0; c < H; c += 4) {
+                const float4 f = *reinterpret_cast<const float4*>(&sm[L.d2 + r * H + c]);
+                const float4 g = *reinterpret_cast<const float4*>(&sm[L.d2 + r2 * H + c]);
+                const float* w = &sm[L.w2 + o * kTrW2Stride + c];
+                x = fmaf(f.w, w[3], fmaf(f.z, w[2], fmaf(f.y, w[1], fmaf(f.x, w[0], x))));
+                y = fmaf(g.w, w[3], fmaf(g.z, w[2], fmaf(g.y, w[1], fmaf(g.x, w[0], y))));
+            }
+            sm[L.d1 + r * H + o] = sm[L.h1 + r * H + o] > 0.f ? x : 0.f;
+            sm[L.d1 + r2 * H + o] = sm[L.h1 + r2 * H + o] > 0.f ? y : 0.f;
+        }
+        cluster.sync();
+        // ---- columns of all rows that this CTA's parameters need ----
+        auto fetch = [&](int from, int stride, int col, int to, int width4) {   // width4 float4s a row
+            for (int i = t; i < B * width4; i += kTrThreads) {
+                const int r = i / width4, c = i % width4, src = r / R;
+                const float* base = cluster.map_shared_rank(sm, src);
+                reinterpret_cast<float4*>(&sm[to])[i] =
+                    *reinterpret_cast<const float4*>(&base[from + (r - src * R) * stride + col + 4 * c]);
+            }
+        };
+        fetch(L.h1, H, bi, L.ch1, 4);
+        fetch(L.d2, H, bo, L.cd2, 8);
+        fetch(L.h2, H, rank * 8, L.ch2, 2);
+        fetch(L.d1, H, rank * 8, L.cd1, 2);
+        fetch(L.dy, 4, 0, L.cdy, 1);
+        for (int i = t; i < B * in; i += kTrThreads) {
+            const int r = i / in, src = r / R;
+            sm[L.cx + i] = cluster.map_shared_rank(sm, src)[L.x + (r - src * R) * in + i % in];
+        }
+        if (b0 + a.batch < a.n) read_ahead(b0 + a.batch);
+        __syncthreads();
+        // ---- gradients, rows ascending ----
+        float g[4] = {0.f, 0.f, 0.f, 0.f};
+        if (q < 0) {
+#pragma unroll 8
+            for (int r = 0; r < B; ++r) {
+                const float h = sm[L.ch1 + r * 16 + wi];
+                const float4 d = *reinterpret_cast<const float4*>(&sm[L.cd2 + r * 32 + wo]);
+                g[0] = fmaf(h, d.x, g[0]);
+                g[1] = fmaf(h, d.y, g[1]);
+                g[2] = fmaf(h, d.z, g[2]);
+                g[3] = fmaf(h, d.w, g[3]);
+            }
+        } else if (kind == 0) {
+#pragma unroll 8
+            for (int r = 0; r < B; ++r) g[0] = fmaf(sm[L.cx + r * in + ka], sm[L.cd1 + r * 8 + kb], g[0]);
+        } else if (kind == 1) {
+#pragma unroll 8
+            for (int r = 0; r < B; ++r) g[0] += sm[L.cd1 + r * 8 + kb];
+        } else if (kind == 2) {
+#pragma unroll 8
+            for (int r = 0; r < B; ++r) g[0] = fmaf(sm[L.ch2 + r * 8 + ka], sm[L.cdy + r * 4 + kb], g[0]);
+        } else if (kind == 3) {
+#pragma unroll 8
+            for (int r = 0; r < B; ++r) g[0] += sm[L.cd2 + r * 32 + kb];
+        } else if (kind == 4) {
+#pragma unroll 8
+            for (int r = 0; r < B; ++r) g[0] += sm[L.cdy + r * 4 + kb];
+        }
+        // ---- Adam, and the new weights into every CTA's copy ----
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < own) adam_step(p[k], g[k], m[k], v[k], a.lr, a.b1, a.b2, a.eps, corr.x, corr.y);
+        for (int to = 0; to < kTrCtas; ++to) {
+            float* base = cluster.map_shared_rank(sm, to);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (k < own) base[ps + k] = p[k];
+        }
+        cluster.sync();
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (k < own) {
+            a.params[pg + k] = p[k];
+            a.m[pg + k] = m[k];
+            a.v[pg + k] = v[k];
+        }
 }
 
 inline int blocks(int64_t work) { return (int)((work + 255) / 256); }
@@ -313,6 +617,60 @@ float mlp_train_device(float* params, const float* X, const float* T, int n, int
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     int t = 0;
     float last = 0.f;
+    // Minibatches and inputs that the fused kernel's shared memory holds take
+    // one launch an epoch (the next epoch is shuffled meanwhile).
+    if (in <= kTrMaxIn && batch <= kTrMaxBatch) {
+        const int nb = (int)ceil_div(n, batch), smem = train_layout(in, batch).total * (int)sizeof(float);
+        GB_CUDA(cudaFuncSetAttribute(k_mlp_epoch, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     train_layout(kTrMaxIn, kTrMaxBatch).total * (int)sizeof(float)));
+        DevBuf<int32_t> rows(n, s);
+        DevBuf<float2> corr(nb, s);
+        DevBuf<float> row_loss(n, s);
+        // Two staging copies, reused once their transfer is over.
+        struct Stage {
+            std::vector<int32_t> rows;
+            std::vector<float2> corr;
+            cudaEvent_t done = nullptr;
+            ~Stage() {
+                if (done) cudaEventDestroy(done);
+            }
+        } stage[2];
+        for (Stage& st : stage) {
+            st.corr.resize(nb);
+            GB_CUDA(cudaEventCreateWithFlags(&st.done, cudaEventDisableTiming));
+        }
+        for (int ep = 0; ep < epochs; ++ep) {
+            Stage& st = stage[ep & 1];
+            for (int i = n - 1; i > 0; --i) std::swap(order[i], order[next() % (uint64_t)(i + 1)]);
+            GB_CUDA(cudaEventSynchronize(st.done));
+            st.rows = order;
+            for (float2& c : st.corr) {
+                ++t;
+                c = make_float2(1.f - std::pow(b1, (float)t), 1.f - std::pow(b2, (float)t));
+            }
+            GB_CUDA(cudaMemcpyAsync(rows, st.rows.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+            GB_CUDA(cudaMemcpyAsync(corr, st.corr.data(), nb * sizeof(float2), cudaMemcpyHostToDevice, s));
+            GB_CUDA(cudaEventRecord(st.done, s));
+            k_mlp_epoch<<<kTrCtas, kTrThreads, smem, s>>>(
+                TrainArgs{params, m, v, X, T, rows, corr, row_loss, n, in, batch, lr, b1, b2, eps});
+            GB_LAUNCH_CHECK();
+        }
+        if (epochs > 0) {
+            std::vector<float> rl(n);
+            GB_CUDA(cudaMemcpyAsync(rl.data(), row_loss.get(), n * sizeof(float), cudaMemcpyDeviceToHost, s));
+            GB_CUDA(cudaStreamSynchronize(s));
+            double ep_loss = 0.0;
+            for (int b0 = 0; b0 < n; b0 += batch) {
+                const int B = std::min(batch, n - b0);
+                double tot = 0.0;
+                for (int r = 0; r < B; ++r) tot += rl[b0 + r];
+                ep_loss += (float)(tot / ((double)B * kMlpOut));
+            }
+            last = (float)(ep_loss / std::max(1, nb));
+        }
+        GB_CUDA(cudaStreamSynchronize(s));
+        return last;
+    }
     for (int ep = 0; ep < epochs; ++ep) {
         for (int i = n - 1; i > 0; --i) std::swap(order[i], order[next() % (uint64_t)(i + 1)]);
         double ep_loss = 0.0;

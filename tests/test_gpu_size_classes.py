@@ -95,3 +95,40 @@ def test_kernels_by_row_length_and_frontier(ctx, kind, size):
     _, stop, _ = ctx.pagerank(rp, col, max_iters=100, epsilon=1e-3)
     _, one_less, _ = ctx.pagerank(rp, col, max_iters=max(1, stop - 1), epsilon=1e-3)
     assert stop <= 100 and one_less == max(1, stop - 1)
+
+
+@pytest.mark.parametrize("rows,in_dim,batch", [(1, 1, 1), (7, 12, 8), (9, 12, 8), (64, 3, 64), (129, 12, 128),
+                                               (300, 32, 256), (513, 12, 100), (300, 33, 256), (300, 12, 257)])
+def test_training_by_batch_and_inputs(ctx, rows, in_dim, batch):
+    # One launch per epoch up to 32 inputs and minibatches of 256 rows, one per
+    # kernel above: two epochs of Adam against float64 steps on the same shuffle.
+    rng = np.random.default_rng(rows * 1000 + in_dim)
+    count = ctx.mlp_param_count(in_dim)
+    start = rng.normal(0, 0.3, count).astype(np.float32)
+    x = rng.normal(0, 1, (rows, in_dim)).astype(np.float32)
+    t = rng.normal(0, 1, (rows, 3)).astype(np.float32)
+    seed, mask = 11, (1 << 64) - 1
+    got, loss = ctx.mlp_train(start, x, t, epochs=2, batch=batch, lr=1e-3, seed=seed)
+    p, m, v = start.astype(np.float64), np.zeros(count), np.zeros(count)
+    order, word, step = list(range(rows)), (seed ^ 0x9E3779B97F4A7C15) & mask, 0
+    for _ in range(2):
+        for i in range(rows - 1, 0, -1):
+            word = (word + 0x9E3779B97F4A7C15) & mask
+            z = ((word ^ (word >> 30)) * 0xBF58476D1CE4E5B9) & mask
+            z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & mask
+            j = (z ^ (z >> 31)) % (i + 1)
+            order[i], order[j] = order[j], order[i]
+        losses = []
+        for at in range(0, rows, batch):
+            pick = order[at:at + batch]
+            l, g, _ = po.mlp_loss_grad(p, x[pick].astype(np.float64), t[pick].astype(np.float64))
+            losses.append(l)
+            step += 1
+            m, v = 0.9 * m + 0.1 * g, 0.999 * v + 0.001 * g * g
+            p = p - 1e-3 * (m / (1 - 0.9 ** step)) / (np.sqrt(v / (1 - 0.999 ** step)) + 1e-8)
+    # Adam's step is at most lr whatever the gradient's size, so a gradient near
+    # the rounding of its own sum can move a parameter by up to lr either way a
+    # step; the others agree to the gradients' 1e-4.
+    assert np.abs(got - p).max() <= 2 * step * 1e-3
+    assert np.mean(np.abs(got - p) > 2e-3 * 1e-3 * step) < 0.02
+    np.testing.assert_allclose(loss, np.mean(losses), rtol=1e-3)
