@@ -8,11 +8,11 @@
 //
 // Relabel follows RelabelByMapping's undirected branch (builder.h:1168-1206):
 // new row x = sorted { new_ids[v] : v in N(old(x)) }.  Remap and sort are
-// fused per row; rows are bucketed by length: one thread (<= 16 entries),
-// one warp with a shared-memory bitonic sort (<= 256), one 256-thread CTA
-// (<= 2048) or one 1024-thread CTA (<= 16384) with a shared-memory LSD radix
-// sort, and a global radix sort of (row, new id) keys for the few longer
-// rows.  The three middle classes run concurrently on forked streams.
+// fused per row; rows are bucketed by length: eight lanes (<= 8 entries) or a
+// warp (<= 1024) with a bitonic sort in registers, one 256-thread CTA (<= 2048)
+// or one 1024-thread CTA (<= 16384) with a shared-memory LSD radix sort, and a
+// global radix sort of (row, new id) keys for the few longer rows.  The classes
+// above 32 entries run concurrently on forked streams.
 #include "gb_chunks.cuh"
 #include "gb_common.cuh"
 #include "gb_stages.h"
@@ -52,72 +52,163 @@ __global__ void k_new_degrees(const int64_t* __restrict__ rp, const int32_t* __r
     }
 }
 
-constexpr int kThreadRowMax = 16;
+constexpr int kTinyRowMax = 8;
+constexpr int kSmallRowMax = 32;
 constexpr int kWarpRowMax = 256;
+constexpr int kLongRowMax = 1024;
 constexpr int kMidRowMax = 2048;      // 256-thread CTA, 24 KB shared memory
 constexpr int kBlockRowMax = 16384;   // 1024-thread CTA, 160 KB shared memory
-constexpr int kRowLists = 4;          // warp, mid-CTA, CTA, huge
+constexpr int kRowLists = 5;          // warp, long warp, mid-CTA, CTA, huge
 
-__global__ void k_relabel_rows_small(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
-                                     const int32_t* __restrict__ new_ids, const int32_t* __restrict__ inv,
-                                     const int64_t* __restrict__ out_rp, int32_t* __restrict__ out_col,
-                                     int64_t n, int32_t* __restrict__ lists, int32_t* __restrict__ counts) {
-    // counts[0..3]: warp, mid-CTA, CTA, huge list sizes; lists: 4 x n entries.
-    for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t u = inv[x];
-        const int64_t b = rp[u], d = rp[u + 1] - b;
-        if (d <= kThreadRowMax) {
-            int32_t a[kThreadRowMax];
-            for (int i = 0; i < d; ++i) {
-                const int32_t v = new_ids[col[b + i]];
-                int j = i - 1;
-                while (j >= 0 && a[j] > v) { a[j + 1] = a[j]; --j; }
-                a[j + 1] = v;
+// Compare-exchange with the lane at distance j; the lower lane keeps the
+// smaller value where asc.
+__device__ __forceinline__ int32_t lane_exchange(int32_t v, int j, bool asc) {
+    const int32_t o = __shfl_xor_sync(0xFFFFFFFFu, v, j);
+    return ((((int)threadIdx.x & j) == 0) == asc) ? min(v, o) : max(v, o);
+}
+
+// Ascending bitonic sort of 32 E values by one warp, value e * 32 + lane in v[e].
+// Distances below 32 are shuffles, the others between a lane's own registers.
+// (In shared memory, with a barrier a step, the 33..256-entry rows of RMAT scale
+// 21 took 0.71 ms; rows up to 1,024 took a CTA with a radix sort, bound by its
+// seven barriers a pass.)
+template <int E>
+__device__ __forceinline__ void warp_sort(int32_t (&v)[E]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int k = 2; k <= 32; k <<= 1) {
+#pragma unroll 1
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const bool up = (lane & k) == 0;   // k = 32: by the register, below
+#pragma unroll
+            for (int e = 0; e < E; ++e) v[e] = lane_exchange(v[e], j, k == 32 ? (e & 1) == 0 : up);
+        }
+    }
+#pragma unroll
+    for (int q = 2; q <= E; q <<= 1) {   // runs of 32 q values
+#pragma unroll
+        for (int h = q >> 1; h > 0; h >>= 1) {
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                if (e & h) continue;
+                const int32_t x = v[e], y = v[e | h];
+                const bool asc = (e & q) == 0;
+                v[e] = asc ? min(x, y) : max(x, y);
+                v[e | h] = asc ? max(x, y) : min(x, y);
             }
-            const int64_t o = out_rp[x];
-            for (int i = 0; i < d; ++i) out_col[o + i] = a[i];
-        } else {
-            const int which = d <= kWarpRowMax ? 0 : (d <= kMidRowMax ? 1 : (d <= kBlockRowMax ? 2 : 3));
-            const int32_t slot = atomicAdd(&counts[which], 1);
-            lists[(int64_t)which * n + slot] = (int32_t)x;
+        }
+#pragma unroll 1
+        for (int j = 16; j > 0; j >>= 1) {
+#pragma unroll
+            for (int e = 0; e < E; ++e) v[e] = lane_exchange(v[e], j, (e & q) == 0);
         }
     }
 }
 
-__global__ void k_relabel_rows_warp(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
-                                    const int32_t* __restrict__ new_ids, const int32_t* __restrict__ inv,
-                                    const int64_t* __restrict__ out_rp, int32_t* __restrict__ out_col,
-                                    const int32_t* __restrict__ list, const int32_t* __restrict__ count) {
-    constexpr int kWarps = 8;
-    __shared__ int32_t sh[kWarps][kWarpRowMax];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int32_t* s = sh[w];
+// One row of at most 32 E entries.
+template <int E>
+__device__ __forceinline__ void warp_row(const int32_t* __restrict__ col, const int32_t* __restrict__ new_ids,
+                                         int d, int32_t* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    int32_t v[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = e * 32 + lane < d ? col[e * 32 + lane] : -1;
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = v[e] >= 0 ? new_ids[v[e]] : kIntMax;
+    warp_sort<E>(v);
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+        if (e * 32 + lane < d) out[e * 32 + lane] = v[e];
+}
+
+// Four consecutive new rows a warp: rows of up to 8 entries by eight lanes each,
+// together; rows of 9..32 then by the warp, their reads issued together; longer
+// ones go to their class's list, one atomic a class and warp.
+__global__ void __launch_bounds__(256)
+k_relabel_rows_small(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
+                     const int32_t* __restrict__ new_ids, const int32_t* __restrict__ inv,
+                     const int64_t* __restrict__ out_rp, int32_t* __restrict__ out_col, int64_t n,
+                     int32_t* __restrict__ lists, int32_t* __restrict__ counts) {
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31, g = lane >> 3, j = lane & 7;
+    const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t x0 = 4 * w0; x0 < n; x0 += 4 * nw) {
+        const int64_t x = x0 + g;
+        int64_t b = 0, o = 0;
+        int d = 0;
+        if (x < n) {
+            const int32_t u = inv[x];
+            b = rp[u];
+            d = (int)(rp[u + 1] - b);
+            o = out_rp[x];
+        }
+        // Reads of the short rows (v) and of the warp's rows (r) together.
+        int32_t v = j < d && d <= kTinyRowMax ? col[b + j] : -1;
+        int32_t r[4];
+        int dk[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            dk[k] = __shfl_sync(kFull, d, 8 * k);
+            const int64_t bk = __shfl_sync(kFull, b, 8 * k);
+            const bool mine = dk[k] > kTinyRowMax && dk[k] <= kSmallRowMax && lane < dk[k];
+            r[k] = mine ? col[bk + lane] : -1;
+        }
+        v = v >= 0 ? new_ids[v] : kIntMax;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) r[k] = r[k] >= 0 ? new_ids[r[k]] : kIntMax;
+#pragma unroll
+        for (int k = 2; k <= 8; k <<= 1)
+#pragma unroll
+            for (int h = k >> 1; h > 0; h >>= 1) v = lane_exchange(v, h, k == 8 || (lane & k) == 0);
+        if (j < d && d <= kTinyRowMax) out_col[o + j] = v;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (dk[k] <= kTinyRowMax || dk[k] > kSmallRowMax) continue;   // the same in every lane
+            int32_t one[1] = {r[k]};
+            warp_sort<1>(one);
+            const int64_t ok = __shfl_sync(kFull, o, 8 * k);
+            if (lane < dk[k]) out_col[ok + lane] = one[0];
+        }
+        const int which = d <= kSmallRowMax || j != 0 ? -1
+                          : d <= kWarpRowMax         ? 0
+                          : d <= kLongRowMax         ? 1
+                          : d <= kMidRowMax          ? 2
+                          : d <= kBlockRowMax        ? 3 : 4;
+        if (__any_sync(kFull, which >= 0)) {
+            const unsigned peers = __match_any_sync(kFull, which);
+            const int leader = __ffs(peers) - 1;
+            int32_t slot = 0;
+            if (which >= 0 && lane == leader) slot = atomicAdd(&counts[which], __popc(peers));
+            slot = __shfl_sync(kFull, slot, leader) + __popc(peers & ((1u << lane) - 1u));
+            if (which >= 0) lists[(int64_t)which * n + slot] = (int32_t)x;
+        }
+    }
+}
+
+// A warp per listed row: kLong rows of 257..1024 entries, else 33..256.
+template <bool kLong>
+__global__ void __launch_bounds__(256)
+k_relabel_rows_warp(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
+                    const int32_t* __restrict__ new_ids, const int32_t* __restrict__ inv,
+                    const int64_t* __restrict__ out_rp, int32_t* __restrict__ out_col,
+                    const int32_t* __restrict__ list, const int32_t* __restrict__ count) {
     const int32_t total = *count;
-    for (int64_t r = (int64_t)blockIdx.x * kWarps + w; r < total; r += (int64_t)gridDim.x * kWarps) {
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < total; r += nw) {
         const int32_t x = list[r];
         const int32_t u = inv[x];
         const int64_t b = rp[u];
         const int d = (int)(rp[u + 1] - b);
-        int p = 32;
-        while (p < d) p <<= 1;
-        for (int i = lane; i < p; i += 32) s[i] = i < d ? new_ids[col[b + i]] : kIntMax;
-        __syncwarp();
-        for (int k = 2; k <= p; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int i = lane; i < p; i += 32) {
-                    const int ixj = i ^ j;
-                    if (ixj > i) {
-                        const int32_t a = s[i], c = s[ixj];
-                        const bool asc = (i & k) == 0;
-                        if ((a > c) == asc) { s[i] = c; s[ixj] = a; }
-                    }
-                }
-                __syncwarp();
-            }
+        int32_t* out = out_col + out_rp[x];
+        if (kLong) {
+            if (d <= 512) warp_row<16>(col + b, new_ids, d, out);
+            else warp_row<32>(col + b, new_ids, d, out);
+        } else {
+            if (d <= 64) warp_row<2>(col + b, new_ids, d, out);
+            else if (d <= 128) warp_row<4>(col + b, new_ids, d, out);
+            else warp_row<8>(col + b, new_ids, d, out);
         }
-        const int64_t o = out_rp[x];
-        for (int i = lane; i < d; i += 32) out_col[o + i] = s[i];
-        __syncwarp();
     }
 }
 
@@ -412,11 +503,11 @@ void relabel_csr_device(const DeviceCSR& g, const int32_t* new_ids, const int32_
     DevBuf<int32_t> lists(kRowLists * n, s);
     DevBuf<int32_t> counts(kRowLists, s);
     GB_CUDA(cudaMemsetAsync(counts, 0, kRowLists * sizeof(int32_t), s));
-    k_relabel_rows_small<<<grid_for(n, 256), 256, 0, s>>>(g.row_ptr, g.col, new_ids, inv, out_rp, out_col, n,
-                                                          lists, counts);
+    k_relabel_rows_small<<<grid_for(n * 8, 256), 256, 0, s>>>(g.row_ptr, g.col, new_ids, inv, out_rp, out_col, n,
+                                                              lists, counts);
     GB_LAUNCH_CHECK();
-    // The warp, 256-thread and 1,024-thread classes write disjoint rows: they
-    // run concurrently on two forked streams beside s.
+    // The longer classes write disjoint rows: they run concurrently on two
+    // forked streams beside s.
     struct Fork {
         cudaStream_t s1 = nullptr, s2 = nullptr;
         cudaEvent_t ev[3] = {};
@@ -439,24 +530,27 @@ void relabel_csr_device(const DeviceCSR& g, const int32_t* new_ids, const int32_
     GB_CUDA(cudaFuncSetAttribute(k_relabel_rows_block<1024, kBlockRowMax>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, block_smem));
     k_relabel_rows_block<1024, kBlockRowMax><<<kNumSMs, 1024, block_smem, fk.s2>>>(
-        g.row_ptr, g.col, new_ids, inv, out_rp, out_col, lists.get() + 2 * n, counts.get() + 2, vbits);
+        g.row_ptr, g.col, new_ids, inv, out_rp, out_col, lists.get() + 3 * n, counts.get() + 3, vbits);
     GB_LAUNCH_CHECK();
     k_relabel_rows_block<256, kMidRowMax><<<kNumSMs * 8, 256, mid_smem, fk.s1>>>(
-        g.row_ptr, g.col, new_ids, inv, out_rp, out_col, lists.get() + n, counts.get() + 1, vbits);
+        g.row_ptr, g.col, new_ids, inv, out_rp, out_col, lists.get() + 2 * n, counts.get() + 2, vbits);
     GB_LAUNCH_CHECK();
-    k_relabel_rows_warp<<<kNumSMs * 8, 256, 0, s>>>(g.row_ptr, g.col, new_ids, inv, out_rp, out_col, lists.get(),
-                                                    counts.get());
+    k_relabel_rows_warp<true><<<kNumSMs * 4, 256, 0, s>>>(g.row_ptr, g.col, new_ids, inv, out_rp, out_col,
+                                                          lists.get() + n, counts.get() + 1);
+    GB_LAUNCH_CHECK();
+    k_relabel_rows_warp<false><<<kNumSMs * 8, 256, 0, s>>>(g.row_ptr, g.col, new_ids, inv, out_rp, out_col,
+                                                           lists.get(), counts.get());
     GB_LAUNCH_CHECK();
     GB_CUDA(cudaEventRecord(fk.ev[1], fk.s1));
     GB_CUDA(cudaEventRecord(fk.ev[2], fk.s2));
     GB_CUDA(cudaStreamWaitEvent(s, fk.ev[1], 0));
     GB_CUDA(cudaStreamWaitEvent(s, fk.ev[2], 0));
-    nl += 4;
+    nl += 5;
     int32_t huge = 0;
-    GB_CUDA(cudaMemcpyAsync(&huge, counts.get() + 3, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    GB_CUDA(cudaMemcpyAsync(&huge, counts.get() + 4, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     GB_CUDA(cudaStreamSynchronize(s));
     if (huge > 0) {
-        const int32_t* hlist = lists.get() + 3 * n;
+        const int32_t* hlist = lists.get() + 4 * n;
         DevBuf<int64_t> hoff(huge + 1, s);
         k_huge_degrees<<<grid_for(huge, 256), 256, 0, s>>>(g.row_ptr, inv, hlist, huge, hoff);
         GB_LAUNCH_CHECK();

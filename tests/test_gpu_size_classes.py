@@ -132,3 +132,21 @@ def test_training_by_batch_and_inputs(ctx, rows, in_dim, batch):
     assert np.abs(got - p).max() <= 2 * step * 1e-3
     assert np.mean(np.abs(got - p) > 2e-3 * 1e-3 * step) < 0.02
     np.testing.assert_allclose(loss, np.mean(losses), rtol=1e-3)
+
+
+@pytest.mark.parametrize("lengths", [(0, 1, 2, 7, 8, 9, 31, 32, 33), (63, 64, 65, 127, 128, 129, 255, 256, 257),
+                                     (511, 512, 513, 1023, 1024, 1025), (2047, 2048, 2049)])
+def test_relabel_by_row_length(ctx, lengths):
+    rng = np.random.default_rng(sum(lengths))
+    n, hubs = 6000, 4 * len(lengths)
+    edges = []
+    for h in range(hubs):
+        edges += [(h, int(w)) for w in hubs + rng.choice(n - hubs, lengths[h % len(lengths)], replace=False)]
+    rp, col = (t.numpy() for t in gg.from_edges(n, edges))
+    assert set(np.diff(rp)[:hubs]) == set(lengths)
+    ids = rng.permutation(n).astype(np.int32)
+    new_rp, new_col, old = ctx.relabel_by_mapping(rp, col, ids)
+    expect_rp, expect_col = po.relabel(rp, col, ids)
+    np.testing.assert_array_equal(new_rp, expect_rp)
+    np.testing.assert_array_equal(new_col, expect_col)
+    np.testing.assert_array_equal(ids[old], np.arange(n))
