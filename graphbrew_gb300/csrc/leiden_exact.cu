@@ -371,6 +371,36 @@ __device__ __forceinline__ uint32_t comm_at(const ExactState& a, const Round& r,
     return a.vcom[v];
 }
 
+// Totals of each candidate lane's community c and of the group's own community
+// d, one lookup per lane: a lane without a candidate (`idle`: those of the
+// group; the same in its lanes) looks d up beside the others.  Only groups that
+// have none take a second turn.  Every lane of the warp calls; `group` is the
+// lane's group.
+__device__ __forceinline__ void sigma_with_own(const ExactState& a, const Round& r, uint32_t u, bool cand, uint32_t c,
+                                               const CommRec& rc, uint32_t d, const CommRec& rd, unsigned idle,
+                                               unsigned group, long long& sc, long long& sd) {
+    const int lane = threadIdx.x & 31;
+    const int own = __ffs(idle ? idle : group) - 1;
+    const bool first = idle != 0 && lane == own && d != kNone;
+    long long o[1];
+    {
+        const uint32_t cc[1] = {cand ? c : d};
+        const bool vv[1] = {cand || first};
+        const CommRec rr[1] = {cand ? rc : rd};
+        sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, rr, u, o);
+        sc = o[0];
+    }
+    long long mine = sc;
+    if (__any_sync(0xFFFFFFFFu, idle == 0)) {
+        const uint32_t cc[1] = {d};
+        const bool vv[1] = {idle == 0 && lane == own};
+        const CommRec rr[1] = {rd};
+        sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, rr, u, o);
+        if (vv[0]) mine = o[0];
+    }
+    sd = __shfl_sync(0xFFFFFFFFu, mine, own);
+}
+
 // Whether the events of a community differ from the round before's (a mark of
 // this round for the next may be there already: then once too often).
 __device__ __forceinline__ bool comm_changed(const Round& r, const CommRec& rec) { return rec.cver >= (uint32_t)r.tag; }
@@ -1059,13 +1089,12 @@ __device__ __forceinline__ void eval_vertex(const ExactState& a, const Round& r,
         }
         const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
         const int kud = __popc(__ballot_sync(0xFFFFFFFFu, c == d));
-        if (c != kNone && c != d && lane == __ffs(peers) - 1) {
-            const uint32_t cc[2] = {c, d};
-            const bool vv[2] = {true, true};
-            const CommRec rr[2] = {rc, rd};
-            long long sg[2];
-            sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, rr, (uint32_t)u, sg);
-            const double dl = delta_qi(a.dq, __popc(peers), kud, deg, sg[0], sg[1]);
+        const bool cand = c != kNone && c != d && lane == __ffs(peers) - 1;
+        const unsigned idle = ~__ballot_sync(0xFFFFFFFFu, cand);
+        long long sc = 0, sd = 0;
+        sigma_with_own(a, r, (uint32_t)u, cand, c, rc, d, rd, idle, 0xFFFFFFFFu, sc, sd);
+        if (cand) {
+            const double dl = delta_qi(a.dq, __popc(peers), kud, deg, sc, sd);
             if (dpos(dl)) { best_d = dl; best_c = c; }
         }
     } else {
@@ -1123,7 +1152,7 @@ __device__ __forceinline__ void eval_vertex(const ExactState& a, const Round& r,
         __syncwarp();
         const uint32_t kud = table_get(tk, tv, mask, d);
         // Compact the candidate communities (c != d) to the front of the
-        // table, so the selection runs ceil(candidates / 32) lookup rounds.
+        // table, so the selection runs ceil((candidates + 1) / 32) lookup rounds.
         uint32_t cnt = 0;
         for (uint32_t i0 = 0; i0 < H; i0 += 32) {
             const uint32_t c = tk[i0 + lane], v = tv[i0 + lane];
@@ -1138,23 +1167,25 @@ __device__ __forceinline__ void eval_vertex(const ExactState& a, const Round& r,
             cnt += __popc(bal);
             __syncwarp();
         }
-        // One candidate per lane per step, its lookup interleaved with d's in
-        // the first step (wider interleaving costs registers, and occupancy
-        // matters more here: 64 registers, 28 warps per SM).
+        // One lookup per lane per step: lane 31 of the first step takes d's, the
+        // other 31 candidates; every later step 32 (a second lookup per lane, for
+        // d, doubled the step's instructions and registers).
         long long sd = 0;
         for (uint32_t i0 = 0;; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            const uint32_t cc[2] = {i < cnt ? tk[i] : kNone, d};
-            const bool vv[2] = {i < cnt, i0 == 0};
-            const CommRec rr[2] = {vv[0] ? load_rec(a, cc[0]) : rd, rd};
-            long long sg[2];
-            sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, rr, (uint32_t)u, sg);
-            if (i0 == 0) sd = sg[1];
-            if (vv[0]) {
+            const bool own = i0 == 0 && lane == 31;
+            const uint32_t i = i0 == 0 ? lane : i0 - 1 + lane;
+            const bool valid = !own && i < cnt;
+            const uint32_t cc[1] = {valid ? tk[i] : d};
+            const bool vv[1] = {valid || own};
+            const CommRec rr[1] = {valid ? load_rec(a, cc[0]) : rd};
+            long long sg[1];
+            sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, rr, (uint32_t)u, sg);
+            if (i0 == 0) sd = __shfl_sync(0xFFFFFFFFu, sg[0], 31);
+            if (valid) {
                 const double dl = delta_qi(a.dq, tv[i], kud, deg, sg[0], sd);
                 if (dpos(dl) && better_pos(dl, cc[0], best_d, best_c)) { best_d = dl; best_c = cc[0]; }
             }
-            if (i0 + 32 >= cnt) break;
+            if (i0 + 31 >= cnt) break;
         }
         __syncwarp();
         if (refine_stays(a, (double)sd, ku)) best_c = kNone;   // every lane holds the same sd
@@ -1245,13 +1276,12 @@ __device__ __forceinline__ void eval_small_body(const ExactState& a, const Ctl* 
         if (dirtyb) {
             const unsigned peers = __match_any_sync(0xFFFFFFFFu, ((unsigned long long)g << 32) | c);
             const unsigned eqd = __ballot_sync(0xFFFFFFFFu, act && c != kNone && c == d) & gmask;
-            if (act && c != kNone && c != d && lane == __ffs(peers) - 1) {
-                const uint32_t cc[2] = {c, d};
-                const bool vv[2] = {true, true};
-                const CommRec rr[2] = {rc, rd};
-                long long sg[2];
-                sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, rr, (uint32_t)u, sg);
-                const double dl = delta_qi(a.dq, __popc(peers), __popc(eqd), deg, sg[0], sg[1]);
+            const bool cand = act && c != kNone && c != d && lane == __ffs(peers) - 1;
+            const unsigned idle = ~__ballot_sync(0xFFFFFFFFu, cand) & gmask;
+            long long sc = 0, sd = 0;
+            sigma_with_own(a, r, (uint32_t)u, cand, c, rc, act ? d : kNone, rd, act ? idle : gmask, gmask, sc, sd);
+            if (cand) {
+                const double dl = delta_qi(a.dq, __popc(peers), __popc(eqd), deg, sc, sd);
                 if (dpos(dl)) { best_d = dl; best_c = c; }
             }
         }
@@ -1290,10 +1320,11 @@ __device__ __forceinline__ void eval_big_body(const ExactState& a, const Ctl* c)
     extern __shared__ uint32_t big_smem[];
     uint32_t* tk = big_smem;                      // kBigSlots keys
     uint32_t* tv = tk + kBigSlots;                // kBigSlots counts
-    uint32_t* cand_c = tv + kBigSlots;            // kBigMaxDeg compacted candidates
-    uint32_t* cand_w = cand_c + kBigMaxDeg;
+    uint32_t* cand_c = tv + kBigSlots;            // d and up to kBigMaxDeg compacted candidates
+    uint32_t* cand_w = cand_c + kBigMaxDeg + 1;
     __shared__ int s_any;
     __shared__ uint32_t s_cnt;
+    __shared__ long long s_own;
     __shared__ double red_d[32];
     __shared__ uint32_t red_c[32];
     const Round r = round_view(a, c);
@@ -1311,7 +1342,8 @@ __device__ __forceinline__ void eval_big_body(const ExactState& a, const Ctl* c)
         for (uint32_t i = tid; i < H; i += blockDim.x) { tk[i] = kNone; tv[i] = 0; }
         if (tid == 0) {
             s_any = a.vaff[u] != 0;
-            s_cnt = 0;
+            s_cnt = 1;
+            cand_c[0] = d;
         }
         __syncthreads();
         bool any = false;
@@ -1341,10 +1373,9 @@ __device__ __forceinline__ void eval_big_body(const ExactState& a, const Ctl* c)
             continue;
         }
         const double ku = (double)deg;
-        const CommRec rd = load_rec(a, d);
         const uint32_t kud = table_get(tk, tv, mask, d);
-        // Compact the candidates (c != d); their order does not matter, the
-        // selection is a total order.
+        // Compact the candidates (c != d) behind d itself; their order does not
+        // matter, the selection is a total order.
         for (uint32_t i0 = 0; i0 < H; i0 += blockDim.x) {
             const uint32_t i = i0 + tid;
             const uint32_t c = i < H ? tk[i] : kNone;
@@ -1366,13 +1397,18 @@ __device__ __forceinline__ void eval_big_body(const ExactState& a, const Ctl* c)
         long long sd = 0;
         for (uint32_t i0 = 0;; i0 += blockDim.x) {
             const uint32_t i = i0 + tid;
-            const uint32_t cc[2] = {i < cnt ? cand_c[i] : kNone, d};
-            const bool vv[2] = {i < cnt, i0 == 0};
-            const CommRec rr[2] = {vv[0] ? load_rec(a, cc[0]) : rd, rd};
-            long long sg[2];
-            sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, rr, u, sg);
-            if (i0 == 0) sd = sg[1];
-            if (vv[0]) {
+            const uint32_t cc[1] = {i < cnt ? cand_c[i] : kNone};
+            const bool vv[1] = {i < cnt};
+            CommRec rr[1] = {CommRec{0ull, 0u, 0u}};
+            if (vv[0]) rr[0] = load_rec(a, cc[0]);
+            long long sg[1];
+            sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, rr, u, sg);
+            if (i0 == 0) {   // thread 0 looked d up
+                if (tid == 0) s_own = sg[0];
+                __syncthreads();
+                sd = s_own;
+            }
+            if (vv[0] && i > 0) {
                 const double dl = delta_qi(a.dq, cand_w[i], kud, deg, sg[0], sd);
                 if (dpos(dl) && better_pos(dl, cc[0], best_d, best_c)) { best_d = dl; best_c = cc[0]; }
             }
@@ -2226,7 +2262,7 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     };
     const int mid_grid = resident((const void*)k_ex_eval_mid, kMidWarpsPerBlock * 32, mid_smem);
     const int select_grid = resident((const void*)k_ex_hub_select, kHubThreads2, 0);
-    const int big_smem = (2 * kBigSlots + 2 * kBigMaxDeg) * (int)sizeof(uint32_t);
+    const int big_smem = (2 * kBigSlots + 2 * (kBigMaxDeg + 1)) * (int)sizeof(uint32_t);
     GB_CUDA(cudaFuncSetAttribute(k_ex_eval_big, cudaFuncAttributeMaxDynamicSharedMemorySize, big_smem));
     const int big_grid = resident((const void*)k_ex_eval_big, kBigThreads, big_smem);
     const int hub_grid = resident((const void*)k_ex_hub_accum, kHubThreads2, 0);
