@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "gb_common.cuh"
@@ -227,8 +228,10 @@ __global__ void k_gather_rows(const float* __restrict__ src, const int32_t* __re
 // each: every CTA takes an eighth of the rows through the forward pass and the
 // activations' gradients (weights in its shared memory), then owns a block of
 // the weights: it fetches the activation columns that those need from the
-// others' shared memory, forms their gradients and Adam steps with parameter and
-// moments in registers, and writes the new weights into all eight copies.
+// others through L2, forms their gradients and Adam steps with parameter and
+// moments in registers, and leaves the new weights in L2 for all eight.  (Through
+// distributed shared memory, element by element, the two exchanges were half of
+// a minibatch's 14.5 us.)
 //
 // Every sum runs in the order of the kernels above (inputs, outputs or rows
 // ascending, one fused multiply-add each), so the parameters are the same bit for
@@ -241,7 +244,8 @@ constexpr int kTrMaxBatch = 256;  // activations and column copies in shared mem
 constexpr int kTrW2Stride = kMlpHidden + 1;   // W2 is read along both axes
 
 struct TrainArgs {
-    float *params, *m, *v;
+    float *params, *m, *v;    // 16-byte aligned
+    float* act;               // a minibatch's activations and gradients, TrainExchange
     const float *X, *T;
     const int32_t* order;     // this epoch's rows
     const float2* corr;       // per minibatch: Adam's 1 - b1^t, 1 - b2^t
@@ -250,11 +254,29 @@ struct TrainArgs {
     float lr, b1, b2, eps;
 };
 
+// Offsets (floats) into the exchange buffer: row-major, a row per minibatch row.
+struct TrainExchange {
+    int h1, h2, d2, d1, dy, x, total;
+};
+
+__host__ __device__ inline TrainExchange train_exchange(int in, int batch) {
+    TrainExchange e;
+    e.h1 = 0;
+    e.h2 = e.h1 + batch * kMlpHidden;
+    e.d2 = e.h2 + batch * kMlpHidden;
+    e.d1 = e.d2 + batch * kMlpHidden;
+    e.dy = e.d1 + batch * kMlpHidden;
+    e.x = e.dy + batch * 4;
+    e.total = e.x + batch * in;
+    return e;
+}
+
 // Offsets (floats) into a CTA's shared memory.
 struct TrainLayout {
     int w1, b1, w2, b2, w3, b3;             // weights
     int x, h1, h2, d2, d1, dy;              // this CTA's rows
     int cx, ch1, ch2, cd2, cd1, cdy;        // columns of all rows
+    int one;                                // 1.0: the input of a bias
     int total;
 };
 
@@ -285,6 +307,7 @@ __host__ __device__ inline TrainLayout train_layout(int in, int batch) {
     l.cd2 = take(all * 32);
     l.cd1 = take(all * 8);
     l.cdy = take(all * 4);
+    l.one = take(1);
     l.total = at;
     return l;
 }
@@ -296,48 +319,53 @@ __global__ void __cluster_dims__(kTrCtas, 1, 1) __launch_bounds__(kTrThreads) k_
     constexpr int H = kMlpHidden, O = kMlpOut;
     const int t = threadIdx.x, rank = (int)cluster.block_rank(), in = a.in;
     const TrainLayout L = train_layout(in, a.batch);
-    // Packed parameters -> shared memory.
+    const TrainExchange E = train_exchange(in, a.batch);
     const int gw1 = 0, gb1 = in * H, gw2 = gb1 + H, gb2 = gw2 + H * H, gw3 = gb2 + H, gb3 = gw3 + H * O;
-    for (int i = t; i < in * H; i += kTrThreads) sm[L.w1 + i] = a.params[gw1 + i];
-    for (int i = t; i < H * H; i += kTrThreads) sm[L.w2 + (i / H) * kTrW2Stride + i % H] = a.params[gw2 + i];
-    for (int i = t; i < H * O; i += kTrThreads) sm[L.w3 + i] = a.params[gw3 + i];
-    if (t < H) {
-        sm[L.b1 + t] = a.params[gb1 + t];
-        sm[L.b2 + t] = a.params[gb2 + t];
-    }
-    if (t < O) sm[L.b3 + t] = a.params[gb3 + t];
+    // Packed parameters -> shared memory (read at L2: other CTAs write them).
+    auto load_weights = [&]() {
+        for (int i = 4 * t; i < gb3; i += 4 * kTrThreads) {   // every part but the last is a multiple of 4
+            const float4 w = __ldcg(reinterpret_cast<const float4*>(a.params + i));
+            const bool in_w2 = i >= gw2 && i < gb2;
+            const int at = in_w2 ? L.w2 + (i - gw2) / H * kTrW2Stride + (i - gw2) % H
+                           : i < gb1 ? L.w1 + i : i < gw2 ? L.b1 + i - gb1 : i < gw3 ? L.b2 + i - gb2 : L.w3 + i - gw3;
+            sm[at] = w.x;
+            sm[at + 1] = w.y;
+            sm[at + 2] = w.z;
+            sm[at + 3] = w.w;
+        }
+        if (t < O) sm[L.b3 + t] = __ldcg(a.params + gb3 + t);
+    };
+    load_weights();
+    if (t == 0) sm[L.one] = 1.f;
     // Parameters that this thread owns: the first 128 threads a 1 x 4 piece of
     // the CTA's 16 x 32 block of W2, each other thread one of the rest.
     const int bi = (rank >> 1) * 16, bo = (rank & 1) * 32;
     const int wi = t >> 3, wo = (t & 7) * 4;
     const int q = t - 128;
-    int own = 0, pg = 0, ps = 0;            // how many, packed index, shared index
-    int kind = -1, ka = 0, kb = 0;          // what its gradient sums: two columns
+    int own = 0, pg = 0;                    // how many, packed index
+    int ax = L.one, as = 0, bx = 0, bs = 0; // its gradient: sum over rows of sm[ax + r as] sm[bx + r bs]
     if (q < 0) {
         own = 4;
         pg = gw2 + (bi + wi) * H + bo + wo;
-        ps = L.w2 + (bi + wi) * kTrW2Stride + bo + wo;
     } else if (q < in * 8) {
-        kind = 0, ka = q >> 3, kb = q & 7, own = 1;
-        pg = gw1 + ka * H + rank * 8 + kb;
-        ps = L.w1 + ka * H + rank * 8 + kb;
+        own = 1, pg = gw1 + (q >> 3) * H + rank * 8 + (q & 7);
+        ax = L.cx + (q >> 3), as = in, bx = L.cd1 + (q & 7), bs = 8;
     } else if (q < in * 8 + 8) {
-        kind = 1, kb = q - in * 8, own = 1;
-        pg = gb1 + rank * 8 + kb;
-        ps = L.b1 + rank * 8 + kb;
+        const int j = q - in * 8;
+        own = 1, pg = gb1 + rank * 8 + j;
+        bx = L.cd1 + j, bs = 8;
     } else if (q < in * 8 + 32) {
         const int j = q - in * 8 - 8;
-        kind = 2, ka = j / O, kb = j % O, own = 1;
-        pg = gw3 + (rank * 8 + ka) * O + kb;
-        ps = L.w3 + (rank * 8 + ka) * O + kb;
+        own = 1, pg = gw3 + (rank * 8 + j / O) * O + j % O;
+        ax = L.ch2 + j / O, as = 8, bx = L.cdy + j % O, bs = 4;
     } else if (q < in * 8 + 64 && rank < 2) {   // bo = rank * 32 for these
-        kind = 3, kb = q - in * 8 - 32, own = 1;
-        pg = gb2 + bo + kb;
-        ps = L.b2 + bo + kb;
+        const int j = q - in * 8 - 32;
+        own = 1, pg = gb2 + bo + j;
+        bx = L.cd2 + j, bs = 32;
     } else if (q >= in * 8 + 64 && q < in * 8 + 64 + O && rank == 0) {
-        kind = 4, kb = q - in * 8 - 64, own = 1;
-        pg = gb3 + kb;
-        ps = L.b3 + kb;
+        const int j = q - in * 8 - 64;
+        own = 1, pg = gb3 + j;
+        bx = L.cdy + j, bs = 4;
     }
     float p[4], m[4], v[4];
 #pragma unroll
@@ -444,25 +472,31 @@ __global__ void __cluster_dims__(kTrCtas, 1, 1) __launch_bounds__(kTrThreads) k_
             sm[L.d1 + r * H + o] = sm[L.h1 + r * H + o] > 0.f ? x : 0.f;
             sm[L.d1 + r2 * H + o] = sm[L.h1 + r2 * H + o] > 0.f ? y : 0.f;
         }
+        // This CTA's rows to the exchange.
+        __syncthreads();
+        for (int i = t; i < rows * (H / 4); i += kTrThreads) {
+            const int at = (r0 * H) / 4 + i;
+            reinterpret_cast<float4*>(a.act + E.h1)[at] = reinterpret_cast<const float4*>(&sm[L.h1])[i];
+            reinterpret_cast<float4*>(a.act + E.h2)[at] = reinterpret_cast<const float4*>(&sm[L.h2])[i];
+            reinterpret_cast<float4*>(a.act + E.d2)[at] = reinterpret_cast<const float4*>(&sm[L.d2])[i];
+            reinterpret_cast<float4*>(a.act + E.d1)[at] = reinterpret_cast<const float4*>(&sm[L.d1])[i];
+        }
+        for (int i = t; i < rows * 4; i += kTrThreads) a.act[E.dy + r0 * 4 + i] = sm[L.dy + i];
+        for (int i = t; i < rows * in; i += kTrThreads) a.act[E.x + r0 * in + i] = sm[L.x + i];
         cluster.sync();
         // ---- columns of all rows that this CTA's parameters need ----
-        auto fetch = [&](int from, int stride, int col, int to, int width4) {   // width4 float4s a row
-            for (int i = t; i < B * width4; i += kTrThreads) {
-                const int r = i / width4, c = i % width4, src = r / R;
-                const float* base = cluster.map_shared_rank(sm, src);
-                reinterpret_cast<float4*>(&sm[to])[i] =
-                    *reinterpret_cast<const float4*>(&base[from + (r - src * R) * stride + col + 4 * c]);
-            }
+        auto fetch = [&](int from, int stride, int col, int to, auto width) {   // float4s a row
+            constexpr int kW = decltype(width)::value;
+            for (int i = t; i < B * kW; i += kTrThreads)
+                reinterpret_cast<float4*>(&sm[to])[i] = __ldcg(
+                    reinterpret_cast<const float4*>(a.act + from + (i / kW) * stride + col + 4 * (i % kW)));
         };
-        fetch(L.h1, H, bi, L.ch1, 4);
-        fetch(L.d2, H, bo, L.cd2, 8);
-        fetch(L.h2, H, rank * 8, L.ch2, 2);
-        fetch(L.d1, H, rank * 8, L.cd1, 2);
-        fetch(L.dy, 4, 0, L.cdy, 1);
-        for (int i = t; i < B * in; i += kTrThreads) {
-            const int r = i / in, src = r / R;
-            sm[L.cx + i] = cluster.map_shared_rank(sm, src)[L.x + (r - src * R) * in + i % in];
-        }
+        fetch(E.h1, H, bi, L.ch1, std::integral_constant<int, 4>{});
+        fetch(E.d2, H, bo, L.cd2, std::integral_constant<int, 8>{});
+        fetch(E.h2, H, rank * 8, L.ch2, std::integral_constant<int, 2>{});
+        fetch(E.d1, H, rank * 8, L.cd1, std::integral_constant<int, 2>{});
+        fetch(E.dy, 4, 0, L.cdy, std::integral_constant<int, 1>{});
+        for (int i = t; i < B * in; i += kTrThreads) sm[L.cx + i] = __ldcg(a.act + E.x + i);
         if (b0 + a.batch < a.n) read_ahead(b0 + a.batch);
         __syncthreads();
         // ---- gradients, rows ascending ----
@@ -477,38 +511,23 @@ __global__ void __cluster_dims__(kTrCtas, 1, 1) __launch_bounds__(kTrThreads) k_
                 g[2] = fmaf(h, d.z, g[2]);
                 g[3] = fmaf(h, d.w, g[3]);
             }
-        } else if (kind == 0) {
+        } else if (own) {
+            // A bias multiplies by 1: the product and so the sum are exact copies.
 #pragma unroll 8
-            for (int r = 0; r < B; ++r) g[0] = fmaf(sm[L.cx + r * in + ka], sm[L.cd1 + r * 8 + kb], g[0]);
-        } else if (kind == 1) {
-#pragma unroll 8
-            for (int r = 0; r < B; ++r) g[0] += sm[L.cd1 + r * 8 + kb];
-        } else if (kind == 2) {
-#pragma unroll 8
-            for (int r = 0; r < B; ++r) g[0] = fmaf(sm[L.ch2 + r * 8 + ka], sm[L.cdy + r * 4 + kb], g[0]);
-        } else if (kind == 3) {
-#pragma unroll 8
-            for (int r = 0; r < B; ++r) g[0] += sm[L.cd2 + r * 32 + kb];
-        } else if (kind == 4) {
-#pragma unroll 8
-            for (int r = 0; r < B; ++r) g[0] += sm[L.cdy + r * 4 + kb];
+            for (int r = 0; r < B; ++r) g[0] = fmaf(sm[ax + r * as], sm[bx + r * bs], g[0]);
         }
         // ---- Adam, and the new weights into every CTA's copy ----
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < own) adam_step(p[k], g[k], m[k], v[k], a.lr, a.b1, a.b2, a.eps, corr.x, corr.y);
-        for (int to = 0; to < kTrCtas; ++to) {
-            float* base = cluster.map_shared_rank(sm, to);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (k < own) base[ps + k] = p[k];
-        }
+        if (own == 4) *reinterpret_cast<float4*>(a.params + pg) = make_float4(p[0], p[1], p[2], p[3]);
+        else if (own) a.params[pg] = p[0];
         cluster.sync();
+        load_weights();   // the next minibatch's barrier follows its inputs
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k)
         if (k < own) {
-            a.params[pg + k] = p[k];
             a.m[pg + k] = m[k];
             a.v[pg + k] = v[k];
         }
@@ -625,7 +644,8 @@ float mlp_train_device(float* params, const float* X, const float* T, int n, int
                                      train_layout(kTrMaxIn, kTrMaxBatch).total * (int)sizeof(float)));
         DevBuf<int32_t> rows(n, s);
         DevBuf<float2> corr(nb, s);
-        DevBuf<float> row_loss(n, s);
+        DevBuf<float> row_loss(n, s), act(train_exchange(in, batch).total, s), own_params(P, s);
+        GB_CUDA(cudaMemcpyAsync(own_params, params, P * sizeof(float), cudaMemcpyDeviceToDevice, s));
         // Two staging copies, reused once their transfer is over.
         struct Stage {
             std::vector<int32_t> rows;
@@ -652,9 +672,10 @@ float mlp_train_device(float* params, const float* X, const float* T, int n, int
             GB_CUDA(cudaMemcpyAsync(corr, st.corr.data(), nb * sizeof(float2), cudaMemcpyHostToDevice, s));
             GB_CUDA(cudaEventRecord(st.done, s));
             k_mlp_epoch<<<kTrCtas, kTrThreads, smem, s>>>(
-                TrainArgs{params, m, v, X, T, rows, corr, row_loss, n, in, batch, lr, b1, b2, eps});
+                TrainArgs{own_params, m, v, act, X, T, rows, corr, row_loss, n, in, batch, lr, b1, b2, eps});
             GB_LAUNCH_CHECK();
         }
+        GB_CUDA(cudaMemcpyAsync(params, own_params, P * sizeof(float), cudaMemcpyDeviceToDevice, s));
         if (epochs > 0) {
             std::vector<float> rl(n);
             GB_CUDA(cudaMemcpyAsync(rl.data(), row_loss.get(), n * sizeof(float), cudaMemcpyDeviceToHost, s));
