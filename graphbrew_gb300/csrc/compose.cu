@@ -882,10 +882,18 @@ k_gorder_scan(const int32_t* __restrict__ list, const int64_t* __restrict__ offs
 // Exact-order BFS from the hub (intraBFSFromHub), level-synchronous over all
 // BFS communities at once.  Within one community the reference's FIFO order
 // is reproduced: a vertex is discovered by the earliest frontier vertex (queue
-// position) that reaches it and, within that parent, in row order.  Claims are
-// atomicMin of (frontier index << 32 | row offset); the children of a level
-// are then written in (frontier index, row offset) order by an exclusive scan
-// over per-edge flags.
+// position) that reaches it and, within that parent, in row order.
+//
+// claim[w] is 0 once w is visited, else 1 + the smallest frontier index that
+// has reached it in this level (all ones: none): the row offset within the
+// parent needs no place in it, as a row names w once.  So a pass over the
+// frontier's edges asks one 4-byte word per neighbour, and only a smaller
+// frontier index looks at the community and claims; the edge that finds its own
+// index there afterwards is w's.  Edges are dealt in runs of eight to a thread:
+// a run's discoveries are one byte of bits, the children's positions a scan of
+// the runs' counts.  (A 64-bit claim, a visited byte and the community per edge
+// in both passes and an offset per edge took 0.73, 0.83 and 0.27 ms over the
+// 21 levels of RCM on RMAT scale 19.)
 // ---------------------------------------------------------------------------
 __global__ void k_bfs_slots(const int32_t* __restrict__ list, const int32_t* __restrict__ count_p,
                             const uint32_t* __restrict__ order_v, const int64_t* __restrict__ offs,
@@ -902,37 +910,62 @@ __global__ void k_bfs_slots(const int32_t* __restrict__ list, const int32_t* __r
     }
 }
 
-// Hub = max degree, first in vertex-id (= position) order.
-__global__ void k_bfs_hubs(const int64_t* __restrict__ slot_base, const int64_t* __restrict__ slot_size, int32_t nslots,
-                           const uint32_t* __restrict__ order_v, const int64_t* __restrict__ rp,
-                           unsigned long long* __restrict__ hubkey) {
-    // grid-stride over (slot, position) flattened per slot: one block per slot chunk
-    for (int32_t j = blockIdx.y; j < nslots; j += gridDim.y) {
-        const int64_t b = slot_base[j], sz = slot_size[j];
-        unsigned long long best = 0;
-        for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < sz; k += (int64_t)gridDim.x * blockDim.x) {
-            const uint32_t u = order_v[b + k];
-            const uint64_t d = (uint64_t)(rp[u + 1] - rp[u]);
-            const unsigned long long key = (d << 32) | (0xFFFFFFFFull - (uint64_t)k);
-            best = key > best ? key : best;
+// Per slot the best (degree, tie) over its positions: the largest degree,
+// first in position order (kMin = false), or the smallest, ties to the smaller id
+// (kMin).  A thread per position; a block inside one community, as most are,
+// reduces before its one atomic.
+template <bool kMin>
+__global__ void __launch_bounds__(kT)
+k_slot_extreme(const uint32_t* __restrict__ order_v, int64_t nn, const uint32_t* __restrict__ memb,
+               const int32_t* __restrict__ slot_of_comm, const int64_t* __restrict__ slot_base,
+               const int64_t* __restrict__ rp, unsigned long long* __restrict__ key) {
+    __shared__ unsigned long long s_best;
+    __shared__ int32_t s_first;
+    const unsigned long long none = kMin ? ~0ull : 0ull;
+    auto better = [](unsigned long long x, unsigned long long y) { return kMin ? (x < y ? x : y) : (x > y ? x : y); };
+    for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x; p0 < nn; p0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t p = p0 + threadIdx.x;
+        int32_t j = -1;
+        unsigned long long k = none;
+        if (p < nn) {
+            const uint32_t u = order_v[p];
+            j = slot_of_comm[memb[u]];
+            if (j >= 0) {
+                const unsigned long long d = (unsigned long long)(rp[u + 1] - rp[u]);
+                k = kMin ? d << 32 | u : d << 32 | (0xFFFFFFFFull - (unsigned long long)(p - slot_base[j]));
+            }
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long t = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-            best = t > best ? t : best;
+        if (threadIdx.x == 0) {
+            s_first = j;
+            s_best = none;
         }
-        if ((threadIdx.x & 31) == 0) atomicMax(&hubkey[j], best);
+        __syncthreads();
+        const bool same = __syncthreads_and(j == s_first || p >= nn);
+        if (same) {
+            for (int o = 16; o > 0; o >>= 1) k = better(k, __shfl_xor_sync(0xFFFFFFFFu, k, o));
+            if ((threadIdx.x & 31) == 0) {
+                if (kMin) atomicMin(&s_best, k); else atomicMax(&s_best, k);
+            }
+            __syncthreads();
+            if (threadIdx.x == 0 && s_first >= 0) {
+                if (kMin) atomicMin(&key[s_first], s_best); else atomicMax(&key[s_first], s_best);
+            }
+        } else if (j >= 0) {
+            if (kMin) atomicMin(&key[j], k); else atomicMax(&key[j], k);
+        }
+        __syncthreads();
     }
 }
 
 __global__ void k_bfs_init(const unsigned long long* __restrict__ hubkey, const int64_t* __restrict__ slot_base,
                            int32_t nslots, const uint32_t* __restrict__ order_v, int32_t* __restrict__ frontier,
-                           uint8_t* __restrict__ visited, uint32_t* __restrict__ local, int64_t* __restrict__ qlen,
+                           uint32_t* __restrict__ claim, uint32_t* __restrict__ local, int64_t* __restrict__ qlen,
                            int64_t* __restrict__ fs, int64_t* __restrict__ fe) {
     for (int32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nslots; j += gridDim.x * blockDim.x) {
         const int64_t k = (int64_t)(0xFFFFFFFFull - (hubkey[j] & 0xFFFFFFFFull));
         const uint32_t hub = order_v[slot_base[j] + k];
         frontier[j] = (int32_t)hub;
-        visited[hub] = 1;
+        claim[hub] = 0;
         local[hub] = 0;
         qlen[j] = 1;
         fs[j] = j;
@@ -958,80 +991,125 @@ __device__ __forceinline__ int64_t upper_index(const int64_t* __restrict__ D, in
     return lo;
 }
 
-// Frontier edges in runs of kEdgeRun consecutive edge indices per thread:
-// one binary search for the run's first edge, then the owning frontier
-// vertex advances with the edge index.
+// Frontier edges in runs of kEdgeRun consecutive edge indices per thread: one
+// binary search for the run's first edge, then the owning frontier vertex
+// advances with the edge index.  fn(run, nbr, idx): the run's neighbours (-1
+// past the last edge) and their frontier indices, all read together.
 constexpr int kEdgeRun = 8;
 
-template <typename Fn>
-__device__ __forceinline__ void for_frontier_edges(const int64_t* __restrict__ D, int64_t nf, int64_t T, Fn&& fn) {
-    for (int64_t e0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * kEdgeRun; e0 < T;
-         e0 += (int64_t)gridDim.x * blockDim.x * kEdgeRun) {
-        int64_t i = upper_index(D, nf, e0);
-        int64_t next = D[i + 1];
-        const int64_t e1 = min(T, e0 + kEdgeRun);
-        for (int64_t e = e0; e < e1; ++e) {
-            while (e >= next) {
-                ++i;
-                next = D[i + 1];
+template <typename Skip, typename Fn>
+__device__ __forceinline__ void for_edge_runs(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D,
+                                              const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
+                                              Skip&& skip, Fn&& fn) {
+    const int64_t T = D[nf];
+    for (int64_t run = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; run * kEdgeRun < T;
+         run += (int64_t)gridDim.x * blockDim.x) {
+        if (skip(run)) continue;
+        const int64_t e0 = run * kEdgeRun;
+        int64_t i = upper_index(D, nf, e0), at = D[i], next = D[i + 1];
+        int64_t row = rp[F[i]] - at;
+        int32_t nbr[kEdgeRun], idx[kEdgeRun];
+#pragma unroll
+        for (int k = 0; k < kEdgeRun; ++k) {
+            const int64_t e = e0 + k;
+            nbr[k] = -1;
+            idx[k] = 0;
+            if (e < T) {
+                if (e >= next) {
+                    do {
+                        ++i;
+                        next = D[i + 1];
+                    } while (e >= next);
+                    row = rp[F[i]] - D[i];
+                }
+                nbr[k] = col[row + e];
+                idx[k] = (int32_t)i;
             }
-            fn(i, e - D[i], e);
         }
+        fn(run, nbr, idx);
     }
 }
 
 inline int edge_grid(int64_t T) { return grid_for(ceil_div(T, kEdgeRun), 256); }
 
-__global__ void k_bfs_claim(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D, int64_t T,
-                            const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
-                            const uint32_t* __restrict__ memb, const uint8_t* __restrict__ visited,
-                            unsigned long long* __restrict__ claim) {
-    for_frontier_edges(D, nf, T, [&](int64_t i, int64_t k, int64_t) {
-        const int32_t u = F[i];
-        const int32_t w = col[rp[u] + k];
-        if (memb[w] == memb[u] && !visited[w])
-            atomicMin(&claim[w], ((unsigned long long)i << 32) | (unsigned long long)k);
-    });
+__global__ void __launch_bounds__(256)
+k_bfs_claim(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D, const int64_t* __restrict__ rp,
+            const int32_t* __restrict__ col, const uint32_t* __restrict__ memb, uint32_t* __restrict__ claim) {
+    for_edge_runs(F, nf, D, rp, col, [](int64_t) { return false; },
+                  [&](int64_t, const int32_t* nbr, const int32_t* idx) {
+                      uint32_t c[kEdgeRun];
+#pragma unroll
+                      for (int k = 0; k < kEdgeRun; ++k) c[k] = nbr[k] >= 0 ? claim[nbr[k]] : 0u;
+#pragma unroll
+                      for (int k = 0; k < kEdgeRun; ++k)
+                          if (c[k] > (uint32_t)idx[k] + 1u && memb[nbr[k]] == memb[F[idx[k]]])
+                              atomicMin(&claim[nbr[k]], (uint32_t)idx[k] + 1u);
+                  });
 }
 
-__global__ void k_bfs_flag(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D, int64_t T,
-                           const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
-                           const uint32_t* __restrict__ memb, const uint8_t* __restrict__ visited,
-                           const unsigned long long* __restrict__ claim, uint8_t* __restrict__ flag) {
-    for_frontier_edges(D, nf, T, [&](int64_t i, int64_t k, int64_t e) {
-        const int32_t u = F[i];
-        const int32_t w = col[rp[u] + k];
-        flag[e] = (memb[w] == memb[u] && !visited[w] &&
-                   claim[w] == (((unsigned long long)i << 32) | (unsigned long long)k)) ? 1 : 0;
-    });
+// Runs past the frontier's last edge, up to `runs`, get no bits.
+__global__ void __launch_bounds__(256)
+k_bfs_flag(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D, const int64_t* __restrict__ rp,
+           const int32_t* __restrict__ col, const uint32_t* __restrict__ claim, int64_t runs,
+           uint8_t* __restrict__ bits, uint8_t* __restrict__ cnt) {
+    for_edge_runs(F, nf, D, rp, col, [](int64_t) { return false; },
+                  [&](int64_t run, const int32_t* nbr, const int32_t* idx) {
+                      uint32_t c[kEdgeRun], b = 0;
+#pragma unroll
+                      for (int k = 0; k < kEdgeRun; ++k) c[k] = nbr[k] >= 0 ? claim[nbr[k]] : 0u;
+#pragma unroll
+                      for (int k = 0; k < kEdgeRun; ++k)
+                          b |= c[k] == (uint32_t)idx[k] + 1u ? 1u << k : 0u;
+                      bits[run] = (uint8_t)b;
+                      cnt[run] = (uint8_t)__popc(b);
+                  });
+    const int64_t used = (D[nf] + kEdgeRun - 1) / kEdgeRun;
+    for (int64_t run = used + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; run < runs;
+         run += (int64_t)gridDim.x * blockDim.x) {
+        bits[run] = 0;
+        cnt[run] = 0;
+    }
+}
+
+// Children found by the edges before edge e.
+__device__ __forceinline__ int64_t children_before(int64_t e, const uint8_t* __restrict__ bits,
+                                                   const int64_t* __restrict__ P, int64_t runs) {
+    const int64_t run = e / kEdgeRun;
+    if (run >= runs) return P[runs];
+    return P[run] + __popc(bits[run] & ((1u << (e % kEdgeRun)) - 1u));
 }
 
 // Per community: where its children start in the next frontier this level.
 __global__ void k_bfs_bases(int32_t nslots, const int64_t* __restrict__ fs, const int64_t* __restrict__ fe,
-                            const int64_t* __restrict__ D, const int64_t* __restrict__ P,
-                            int64_t* __restrict__ base, int64_t* __restrict__ end) {
+                            const int64_t* __restrict__ D, const uint8_t* __restrict__ bits,
+                            const int64_t* __restrict__ P, int64_t runs, int64_t* __restrict__ base,
+                            int64_t* __restrict__ end) {
     for (int32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nslots; j += gridDim.x * blockDim.x) {
-        base[j] = P[D[fs[j]]];
-        end[j] = P[D[fe[j]]];
+        base[j] = children_before(D[fs[j]], bits, P, runs);
+        end[j] = children_before(D[fe[j]], bits, P, runs);
     }
 }
 
-__global__ void k_bfs_write(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D, int64_t T,
-                            const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
-                            const uint32_t* __restrict__ memb, const uint8_t* __restrict__ flag,
-                            const int64_t* __restrict__ P, const int32_t* __restrict__ slot_of_comm,
-                            const int64_t* __restrict__ qlen, const int64_t* __restrict__ base,
-                            int32_t* __restrict__ nextF, uint8_t* __restrict__ visited, uint32_t* __restrict__ local) {
-    for_frontier_edges(D, nf, T, [&](int64_t i, int64_t k, int64_t e) {
-        if (!flag[e]) return;
-        const int32_t u = F[i];
-        const int32_t w = col[rp[u] + k];
-        const int64_t p = P[e];
-        const int32_t j = slot_of_comm[memb[u]];
-        nextF[p] = w;
-        visited[w] = 1;
-        local[w] = (uint32_t)(qlen[j] + (p - base[j]));
-    });
+__global__ void __launch_bounds__(256)
+k_bfs_write(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D, const int64_t* __restrict__ rp,
+            const int32_t* __restrict__ col, const uint32_t* __restrict__ memb, const uint8_t* __restrict__ bits,
+            const int64_t* __restrict__ P, const int32_t* __restrict__ slot_of_comm,
+            const int64_t* __restrict__ qlen, const int64_t* __restrict__ base, int32_t* __restrict__ nextF,
+            uint32_t* __restrict__ claim, uint32_t* __restrict__ local) {
+    for_edge_runs(F, nf, D, rp, col, [&](int64_t run) { return bits[run] == 0; },
+                  [&](int64_t run, const int32_t* nbr, const int32_t*) {
+                      const uint32_t b = bits[run];
+                      int64_t p = P[run];
+#pragma unroll
+                      for (int k = 0; k < kEdgeRun; ++k) {
+                          if (!((b >> k) & 1u)) continue;
+                          const int32_t w = nbr[k], j = slot_of_comm[memb[w]];
+                          nextF[p] = w;
+                          claim[w] = 0;
+                          local[w] = (uint32_t)(qlen[j] + (p - base[j]));
+                          ++p;
+                      }
+                  });
 }
 
 __global__ void k_bfs_advance(int32_t nslots, int64_t* __restrict__ qlen, int64_t* __restrict__ fs,
@@ -1046,11 +1124,11 @@ __global__ void k_bfs_advance(int32_t nslots, int64_t* __restrict__ qlen, int64_
 
 // Unreached vertices of BFS communities, in vertex order after the BFS order.
 __global__ void k_bfs_left_flags(const uint32_t* __restrict__ order_v, int64_t nn, const uint32_t* __restrict__ memb,
-                                 const int32_t* __restrict__ slot_of_comm, const uint8_t* __restrict__ visited,
+                                 const int32_t* __restrict__ slot_of_comm, const uint32_t* __restrict__ claim,
                                  int32_t* __restrict__ flag) {
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < nn; p += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t v = order_v[p];
-        flag[p] = (slot_of_comm[memb[v]] >= 0 && !visited[v]) ? 1 : 0;
+        flag[p] = (slot_of_comm[memb[v]] >= 0 && claim[v] != 0) ? 1 : 0;
     }
 }
 
@@ -1080,29 +1158,10 @@ __global__ void k_bfs_left_assign(const uint32_t* __restrict__ order_v, int64_t 
 //     (parent, degree) finishes it;
 //   * the reached part is reversed, unreached vertices follow in id order.
 // ---------------------------------------------------------------------------
-__global__ void k_rcm_start(const int64_t* __restrict__ slot_base, const int64_t* __restrict__ slot_size,
-                            int32_t nslots, const uint32_t* __restrict__ order_v, const int64_t* __restrict__ rp,
-                            unsigned long long* __restrict__ key) {
-    for (int32_t j = blockIdx.y; j < nslots; j += gridDim.y) {
-        const int64_t b = slot_base[j], sz = slot_size[j];
-        unsigned long long best = ~0ull;
-        for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < sz; k += (int64_t)gridDim.x * blockDim.x) {
-            const uint32_t u = order_v[b + k];
-            const unsigned long long kk = ((unsigned long long)(rp[u + 1] - rp[u]) << 32) | u;
-            best = kk < best ? kk : best;
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long t = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-            best = t < best ? t : best;
-        }
-        if ((threadIdx.x & 31) == 0) atomicMin(&key[j], best);
-    }
-}
-
 // Frontier of a sweep: one start per participating slot, in slot order.
 __global__ void k_rcm_frontier(int32_t nslots, const int32_t* __restrict__ part, const int64_t* __restrict__ pos,
                                const uint32_t* __restrict__ start, int mark, int32_t* __restrict__ F,
-                               uint8_t* __restrict__ visited, int64_t* __restrict__ fs, int64_t* __restrict__ fe,
+                               uint32_t* __restrict__ claim, int64_t* __restrict__ fs, int64_t* __restrict__ fe,
                                int64_t* __restrict__ qlen, int32_t* __restrict__ ecc,
                                unsigned long long* __restrict__ cand) {
     for (int32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nslots; j += gridDim.x * blockDim.x) {
@@ -1113,24 +1172,36 @@ __global__ void k_rcm_frontier(int32_t nslots, const int32_t* __restrict__ part,
         cand[j] = ~0ull;
         if (part[j]) {
             F[pos[j]] = (int32_t)start[j];
-            if (mark) visited[start[j]] = 1;
+            if (mark) claim[start[j]] = 0;
         }
     }
 }
 
-// Children in (parent, row offset) order with their parent's frontier index.
-__global__ void k_rcm_write(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D, int64_t T,
-                            const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
-                            const uint8_t* __restrict__ flag, const int64_t* __restrict__ P,
-                            int32_t* __restrict__ nextF, int64_t* __restrict__ parent, uint8_t* __restrict__ visited) {
-    for_frontier_edges(D, nf, T, [&](int64_t i, int64_t k, int64_t e) {
-        if (!flag[e]) return;
-        const int32_t w = col[rp[F[i]] + k];
-        const int64_t p = P[e];
-        nextF[p] = w;
-        parent[p] = i;
-        visited[w] = 1;
-    });
+// Children in (parent, row offset) order with their parent's frontier index,
+// and the largest of their degrees.
+__global__ void __launch_bounds__(256)
+k_rcm_write(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D, const int64_t* __restrict__ rp,
+            const int32_t* __restrict__ col, const uint8_t* __restrict__ bits, const int64_t* __restrict__ P,
+            int32_t* __restrict__ nextF, int32_t* __restrict__ parent, uint32_t* __restrict__ claim,
+            unsigned long long* __restrict__ max_deg) {
+    unsigned long long m = 0;
+    for_edge_runs(F, nf, D, rp, col, [&](int64_t run) { return bits[run] == 0; },
+                  [&](int64_t run, const int32_t* nbr, const int32_t* idx) {
+                      const uint32_t b = bits[run];
+                      int64_t p = P[run];
+#pragma unroll
+                      for (int k = 0; k < kEdgeRun; ++k) {
+                          if (!((b >> k) & 1u)) continue;
+                          const int32_t w = nbr[k];
+                          nextF[p] = w;
+                          parent[p] = idx[k];
+                          claim[w] = 0;
+                          m = max(m, (unsigned long long)(rp[w + 1] - rp[w]));
+                          ++p;
+                      }
+                  });
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(max_deg, m);
 }
 
 // Last level of a slot whose next level is empty: minimum degree, first in
@@ -1226,7 +1297,7 @@ __global__ void k_rcm_gl_step(int32_t nslots, int32_t* __restrict__ part, const 
     }
 }
 
-__global__ void k_rcm_keys(const int32_t* __restrict__ NF, const int64_t* __restrict__ parent, int64_t cnt,
+__global__ void k_rcm_keys(const int32_t* __restrict__ NF, const int32_t* __restrict__ parent, int64_t cnt,
                            const int64_t* __restrict__ rp, int degbits, uint64_t* __restrict__ keys,
                            uint32_t* __restrict__ vals) {
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < cnt; p += (int64_t)gridDim.x * blockDim.x) {
@@ -1250,12 +1321,12 @@ __global__ void k_rcm_assign(const uint32_t* __restrict__ sorted, int64_t cnt, c
 
 // Reverse the reached part: local = reached - 1 - Cuthill-McKee position.
 __global__ void k_rcm_reverse(const uint32_t* __restrict__ order_v, int64_t nn, const uint32_t* __restrict__ memb,
-                              const int32_t* __restrict__ slot_of_comm, const uint8_t* __restrict__ visited,
+                              const int32_t* __restrict__ slot_of_comm, const uint32_t* __restrict__ claim,
                               const int64_t* __restrict__ qlen, uint32_t* __restrict__ local) {
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < nn; p += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t v = order_v[p];
         const int32_t j = slot_of_comm[memb[v]];
-        if (j >= 0 && visited[v]) local[v] = (uint32_t)(qlen[j] - 1 - local[v]);
+        if (j >= 0 && claim[v] == 0) local[v] = (uint32_t)(qlen[j] - 1 - local[v]);
     }
 }
 
@@ -1313,13 +1384,57 @@ T read_dev(const T* p, cudaStream_t s) {
     return h;
 }
 
+// The discoveries of one BFS level, in device memory sized for the graph: the
+// host bounds the frontier's edges by its vertices and the largest degree, so a
+// level needs no look at the device before its kernels are enqueued, and one
+// after (two or three a level were a third of RCM's time).
+struct LevelBufs {
+    DevBuf<uint8_t> bits, cnt;
+    DevBuf<int64_t> P;
+    DevBuf<unsigned long long> out;   // children, the largest of their degrees
+    int64_t max_deg = 0, bound = 0, runs = 0;
+    LevelBufs(const DeviceCSR& g, int64_t nn, const int32_t* order_v, cudaStream_t s)
+        : bits(ceil_div(g.nnz, kEdgeRun), s), cnt(ceil_div(g.nnz, kEdgeRun), s), P(ceil_div(g.nnz, kEdgeRun) + 1, s),
+          out(2, s) {
+        GB_CUDA(cudaMemsetAsync(out, 0, 2 * sizeof(unsigned long long), s));
+        k_max_degree_of<<<grid_for(nn, kT), kT, 0, s>>>(order_v, nn, g.row_ptr, out);
+        GB_LAUNCH_CHECK();
+        max_deg = (int64_t)read_dev(out.get(), s);
+    }
+    unsigned long long* max_child() const { return out.get() + 1; }
+    // Claims and discovery bits of the frontier F[0, nf); D receives its edge offsets.
+    void find(const DeviceCSR& g, const int32_t* F, int64_t nf, int64_t* D, const uint32_t* memb, uint32_t* claim,
+              cudaStream_t s) {
+        bound = nf > g.nnz / std::max<int64_t>(max_deg, 1) ? g.nnz : nf * max_deg;
+        runs = ceil_div(bound, kEdgeRun);
+        GB_CUDA(cudaMemsetAsync(out, 0, 2 * sizeof(unsigned long long), s));
+        k_frontier_degrees<<<grid_for(nf, kT), kT, 0, s>>>(F, nf, g.row_ptr, D);
+        GB_LAUNCH_CHECK();
+        exclusive_scan_i64_total(D, D, nf, D + nf, s);
+        k_bfs_claim<<<edge_grid(bound), 256, 0, s>>>(F, nf, D, g.row_ptr, g.col, memb, claim);
+        GB_LAUNCH_CHECK();
+        k_bfs_flag<<<edge_grid(bound), 256, 0, s>>>(F, nf, D, g.row_ptr, g.col, claim, runs, bits, cnt);
+        GB_LAUNCH_CHECK();
+        exclusive_scan_u8_to_i64(cnt, P, runs, P.get() + runs, s);
+    }
+    // Children of the level (after the kernels that write them).
+    int64_t children(unsigned long long* max_child_deg, cudaStream_t s) {
+        GB_CUDA(cudaMemcpyAsync(out, P.get() + runs, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
+        unsigned long long h[2];
+        GB_CUDA(cudaMemcpyAsync(h, out.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+        GB_CUDA(cudaStreamSynchronize(s));
+        if (max_child_deg) *max_child_deg = h[1];
+        return (int64_t)h[0];
+    }
+};
+
 }  // namespace
 
 // Reverse Cuthill-McKee for the listed communities (see the kernels above).
 // Returns the number of BFS levels run.
 int64_t rcm_communities(const DeviceCSR& g, const uint32_t* memb, const int32_t* blist, const int32_t* count_p,
                         int32_t nslots, const uint32_t* order_v, const uint32_t* ranks, const int64_t* offs,
-                        const int64_t* ssize, int64_t C, int64_t nn, uint32_t largest, bool pp, uint32_t* local,
+                        const int64_t* ssize, int64_t C, int64_t nn, bool pp, uint32_t* local,
                         cudaStream_t s, int64_t* launches) {
     const int64_t n = g.n;
     DevBuf<int32_t> slot_of_comm(C, s);
@@ -1331,20 +1446,17 @@ int64_t rcm_communities(const DeviceCSR& g, const uint32_t* memb, const int32_t*
     GB_LAUNCH_CHECK();
     DevBuf<unsigned long long> key(nslots, s), cand(nslots, s);
     GB_CUDA(cudaMemsetAsync(key, 0xFF, nslots * sizeof(unsigned long long), s));
-    {
-        dim3 grid((unsigned)std::min<int64_t>(ceil_div(largest, kT), 64), (unsigned)std::min(nslots, 65535));
-        k_rcm_start<<<grid, kT, 0, s>>>(slot_base, slot_size, nslots, order_v, g.row_ptr, key);
-        GB_LAUNCH_CHECK();
-    }
+    k_slot_extreme<true><<<grid_for(nn, kT), kT, 0, s>>>(order_v, nn, memb, slot_of_comm, slot_base, g.row_ptr, key);
+    GB_LAUNCH_CHECK();
     DevBuf<uint32_t> start(nslots, s), last_node(nslots, s);
     DevBuf<int32_t> part(nslots, s), prev_ecc(nslots, s), ecc(nslots, s), still(1, s);
     k_rcm_init_slots<<<grid_for(nslots, kT), kT, 0, s>>>(nslots, slot_size, key, start, part, prev_ecc);
     GB_LAUNCH_CHECK();
     *launches += 4;
-    DevBuf<uint8_t> visited(n, s);
-    DevBuf<unsigned long long> claim(n, s);
-    DevBuf<int32_t> F(nn + 1, s), NF(nn + 1, s);
-    DevBuf<int64_t> D(nn + 1, s), parent(nn + 1, s);
+    DevBuf<uint32_t> claim(n, s);
+    DevBuf<int32_t> F(nn + 1, s), NF(nn + 1, s), parent(nn + 1, s);
+    DevBuf<int64_t> D(nn + 1, s);
+    LevelBufs lv(g, nn, reinterpret_cast<const int32_t*>(order_v), s);
     int64_t levels = 0;
     DevBuf<uint32_t> depth(pp ? n : 0, s);
     // One BFS over the participating slots: a George-Liu sweep, the
@@ -1352,10 +1464,9 @@ int64_t rcm_communities(const DeviceCSR& g, const uint32_t* memb, const int32_t*
     auto sweep = [&](bool cm, bool dep = false) -> void {
         exclusive_scan_i32_to_i64(part, pos, nslots, pos.get() + nslots, s);
         const int64_t np = read_dev(pos.get() + nslots, s);
-        GB_CUDA(cudaMemsetAsync(visited, 0, n, s));
-        GB_CUDA(cudaMemsetAsync(claim, 0xFF, n * sizeof(unsigned long long), s));
+        GB_CUDA(cudaMemsetAsync(claim, 0xFF, n * sizeof(uint32_t), s));
         k_rcm_frontier<<<grid_for(nslots, kT), kT, 0, s>>>(nslots, part, pos, start, (cm || dep) ? 1 : 0, F,
-                                                           visited, fs, fe, qlen, ecc, cand);
+                                                           claim, fs, fe, qlen, ecc, cand);
         GB_LAUNCH_CHECK();
         *launches += 4;
         if (cm) {
@@ -1379,29 +1490,14 @@ int64_t rcm_communities(const DeviceCSR& g, const uint32_t* memb, const int32_t*
                 ++*launches;
             }
             ++level;
-            k_frontier_degrees<<<grid_for(nf, kT), kT, 0, s>>>(F, nf, g.row_ptr, D);
+            lv.find(g, F, nf, D, memb, claim, s);
+            k_bfs_bases<<<grid_for(nslots, kT), kT, 0, s>>>(nslots, fs, fe, D, lv.bits, lv.P, lv.runs, bbase, bend);
             GB_LAUNCH_CHECK();
-            exclusive_scan_i64_total(D, D, nf, D.get() + nf, s);
-            const int64_t T = read_dev(D.get() + nf, s);
-            DevBuf<uint8_t> flag(T > 0 ? T : 1, s);
-            DevBuf<int64_t> P(T + 1, s);
-            if (T > 0) {
-                k_bfs_claim<<<edge_grid(T), 256, 0, s>>>(F, nf, D, T, g.row_ptr, g.col, memb, visited, claim);
-                GB_LAUNCH_CHECK();
-                k_bfs_flag<<<edge_grid(T), 256, 0, s>>>(F, nf, D, T, g.row_ptr, g.col, memb, visited, claim, flag);
-                GB_LAUNCH_CHECK();
-                exclusive_scan_u8_to_i64(flag, P, T, P.get() + T, s);
-            } else {
-                GB_CUDA(cudaMemsetAsync(P, 0, sizeof(int64_t), s));
-            }
-            k_bfs_bases<<<grid_for(nslots, kT), kT, 0, s>>>(nslots, fs, fe, D, P, bbase, bend);
+            k_rcm_write<<<edge_grid(lv.bound), 256, 0, s>>>(F, nf, D, g.row_ptr, g.col, lv.bits, lv.P, NF, parent, claim,
+                                                           lv.max_child());
             GB_LAUNCH_CHECK();
-            if (T > 0) {
-                k_rcm_write<<<edge_grid(T), 256, 0, s>>>(F, nf, D, T, g.row_ptr, g.col, flag, P, NF, parent,
-                                                           visited);
-                GB_LAUNCH_CHECK();
-            }
-            const int64_t next = T > 0 ? read_dev(P.get() + T, s) : 0;
+            unsigned long long md = 0;
+            const int64_t next = lv.children(&md, s);
             if (!cm && !dep) {
                 k_rcm_last_level<<<grid_for(nf, kT), kT, 0, s>>>(F, nf, g.row_ptr, memb, slot_of_comm, bbase, bend,
                                                                  pp ? 1 : 0, cand);
@@ -1411,14 +1507,6 @@ int64_t rcm_communities(const DeviceCSR& g, const uint32_t* memb, const int32_t*
                 GB_LAUNCH_CHECK();
             } else if (cm && next > 0) {
                 // Children of one parent by (degree, id): stable sort by (parent, degree).
-                unsigned long long md = 0;
-                {
-                    DevBuf<unsigned long long> mdd(1, s);
-                    GB_CUDA(cudaMemsetAsync(mdd, 0, sizeof(unsigned long long), s));
-                    k_max_degree_of<<<grid_for(next, kT), kT, 0, s>>>(NF, next, g.row_ptr, mdd);
-                    GB_LAUNCH_CHECK();
-                    md = read_dev(mdd.get(), s);
-                }
                 const int degbits = bits_for(md);
                 const int pbits = bits_for((uint64_t)(nf > 1 ? nf - 1 : 1));
                 DevBuf<uint64_t> keys(next, s);
@@ -1429,7 +1517,7 @@ int64_t rcm_communities(const DeviceCSR& g, const uint32_t* memb, const int32_t*
                 k_rcm_assign<<<grid_for(next, kT), kT, 0, s>>>(vals, next, memb, slot_of_comm, qlen, bbase, NF,
                                                                local);
                 GB_LAUNCH_CHECK();
-                *launches += 4 + 3 * ((degbits + pbits + 7) / 8);
+                *launches += 3 + 3 * ((degbits + pbits + 7) / 8);
             }
             k_bfs_advance<<<grid_for(nslots, kT), kT, 0, s>>>(nslots, qlen, fs, fe, bbase, bend);
             GB_LAUNCH_CHECK();
@@ -1503,11 +1591,11 @@ int64_t rcm_communities(const DeviceCSR& g, const uint32_t* memb, const int32_t*
     GB_LAUNCH_CHECK();
     sweep(true);
     // Reverse the reached part; unreached vertices follow in vertex order.
-    k_rcm_reverse<<<grid_for(nn, kT), kT, 0, s>>>(order_v, nn, memb, slot_of_comm, visited, qlen, local);
+    k_rcm_reverse<<<grid_for(nn, kT), kT, 0, s>>>(order_v, nn, memb, slot_of_comm, claim, qlen, local);
     GB_LAUNCH_CHECK();
     DevBuf<int32_t> lflag(nn, s);
     DevBuf<int64_t> R(nn + 1, s);
-    k_bfs_left_flags<<<grid_for(nn, kT), kT, 0, s>>>(order_v, nn, memb, slot_of_comm, visited, lflag);
+    k_bfs_left_flags<<<grid_for(nn, kT), kT, 0, s>>>(order_v, nn, memb, slot_of_comm, claim, lflag);
     GB_LAUNCH_CHECK();
     exclusive_scan_i32_to_i64(lflag, R, nn, R.get() + nn, s);
     k_bfs_left_assign<<<grid_for(nn, kT), kT, 0, s>>>(order_v, nn, memb, slot_of_comm, lflag, R, slot_base, qlen,
@@ -1703,7 +1791,7 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
     int64_t levels = 0;
     if (nbfs > 0 && (intra == kIntraRCM || intra == kIntraRCMpp)) {
         levels = rcm_communities(g, memb, lists.get() + kClsBfs * C, cc.get()->n + kClsBfs, nbfs, order_v, vkeys, offs, ssize, C,
-                                 nn, hc.largest, intra == kIntraRCMpp, local, s, &launches);
+                                 nn, intra == kIntraRCMpp, local, s, &launches);
     }
     // ---- sorted orders: every community ----
     if (sorted_intra) sorted_communities(g, memb, intra, order_v, vkeys, offs, ssize, nn, local, s, &launches);
@@ -1723,43 +1811,30 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
         GB_LAUNCH_CHECK();
         DevBuf<unsigned long long> hubkey(nbfs, s);
         GB_CUDA(cudaMemsetAsync(hubkey, 0, nbfs * sizeof(unsigned long long), s));
-        {
-            dim3 grid((unsigned)std::min<int64_t>(ceil_div(hc.largest, kT), 64), (unsigned)std::min(nbfs, 65535));
-            k_bfs_hubs<<<grid, kT, 0, s>>>(slot_base, slot_size, nbfs, order_v, g.row_ptr, hubkey);
-            GB_LAUNCH_CHECK();
-        }
-        DevBuf<uint8_t> visited(n, s);
-        GB_CUDA(cudaMemsetAsync(visited, 0, n, s));
-        DevBuf<unsigned long long> claim(n, s);
-        GB_CUDA(cudaMemsetAsync(claim, 0xFF, n * sizeof(unsigned long long), s));
-        DevBuf<int32_t> F(nn + 1, s), NF(nn + 1, s);
-        k_bfs_init<<<grid_for(nbfs, kT), kT, 0, s>>>(hubkey, slot_base, nbfs, order_v, F, visited, local, qlen, fs, fe);
+        k_slot_extreme<false><<<grid_for(nn, kT), kT, 0, s>>>(order_v, nn, memb, slot_of_comm, slot_base, g.row_ptr,
+                                                              hubkey);
         GB_LAUNCH_CHECK();
-        launches += 3;
+        DevBuf<uint32_t> claim(n, s);
+        GB_CUDA(cudaMemsetAsync(claim, 0xFF, n * sizeof(uint32_t), s));
+        DevBuf<int32_t> F(nn + 1, s), NF(nn + 1, s);
+        k_bfs_init<<<grid_for(nbfs, kT), kT, 0, s>>>(hubkey, slot_base, nbfs, order_v, F, claim, local, qlen, fs, fe);
+        GB_LAUNCH_CHECK();
+        launches += 4;
         int64_t nf = nbfs;
         DevBuf<int64_t> D(nn + 1, s);
+        LevelBufs lv(g, nn, reinterpret_cast<const int32_t*>(order_v.get()), s);
         while (nf > 0) {
             ++levels;
-            k_frontier_degrees<<<grid_for(nf, kT), kT, 0, s>>>(F, nf, g.row_ptr, D);
+            lv.find(g, F, nf, D, memb, claim, s);
+            if (lv.bound == 0) break;
+            k_bfs_bases<<<grid_for(nbfs, kT), kT, 0, s>>>(nbfs, fs, fe, D, lv.bits, lv.P, lv.runs, bbase, bend);
             GB_LAUNCH_CHECK();
-            exclusive_scan_i64_total(D, D, nf, D.get() + nf, s);
-            const int64_t T = read_dev(D.get() + nf, s);
-            if (T == 0) break;
-            DevBuf<uint8_t> flag(T, s);
-            DevBuf<int64_t> P(T + 1, s);
-            k_bfs_claim<<<edge_grid(T), 256, 0, s>>>(F, nf, D, T, g.row_ptr, g.col, memb, visited, claim);
-            GB_LAUNCH_CHECK();
-            k_bfs_flag<<<edge_grid(T), 256, 0, s>>>(F, nf, D, T, g.row_ptr, g.col, memb, visited, claim, flag);
-            GB_LAUNCH_CHECK();
-            exclusive_scan_u8_to_i64(flag, P, T, P.get() + T, s);
-            k_bfs_bases<<<grid_for(nbfs, kT), kT, 0, s>>>(nbfs, fs, fe, D, P, bbase, bend);
-            GB_LAUNCH_CHECK();
-            k_bfs_write<<<edge_grid(T), 256, 0, s>>>(F, nf, D, T, g.row_ptr, g.col, memb, flag, P, slot_of_comm,
-                                                       qlen, bbase, NF, visited, local);
+            k_bfs_write<<<edge_grid(lv.bound), 256, 0, s>>>(F, nf, D, g.row_ptr, g.col, memb, lv.bits, lv.P,
+                                                           slot_of_comm, qlen, bbase, NF, claim, local);
             GB_LAUNCH_CHECK();
             k_bfs_advance<<<grid_for(nbfs, kT), kT, 0, s>>>(nbfs, qlen, fs, fe, bbase, bend);
             GB_LAUNCH_CHECK();
-            const int64_t next = read_dev(P.get() + T, s);
+            const int64_t next = lv.children(nullptr, s);
             launches += 10;
             std::swap(F.ptr, NF.ptr);
             nf = next;
@@ -1767,7 +1842,7 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
         // Unreached vertices keep vertex order after the BFS order (:3978-3983).
         DevBuf<int32_t> lflag(nn, s);
         DevBuf<int64_t> R(nn + 1, s);
-        k_bfs_left_flags<<<grid_for(nn, kT), kT, 0, s>>>(order_v, nn, memb, slot_of_comm, visited, lflag);
+        k_bfs_left_flags<<<grid_for(nn, kT), kT, 0, s>>>(order_v, nn, memb, slot_of_comm, claim, lflag);
         GB_LAUNCH_CHECK();
         exclusive_scan_i32_to_i64(lflag, R, nn, R.get() + nn, s);
         k_bfs_left_assign<<<grid_for(nn, kT), kT, 0, s>>>(order_v, nn, memb, slot_of_comm, lflag, R, slot_base, qlen,
