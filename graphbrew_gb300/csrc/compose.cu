@@ -891,7 +891,7 @@ k_gorder_scan(const int32_t* __restrict__ list, const int64_t* __restrict__ offs
 // frontier index looks at the community and claims; the edge that finds its own
 // index there afterwards is w's.  Edges are dealt in runs of eight to a thread:
 // a run's discoveries are one byte of bits, the children's positions a scan of
-// the runs' counts.  (A 64-bit claim, a visited byte and the community per edge
+// the counts of 256 runs each.  (A 64-bit claim, a visited byte and the community per edge
 // in both passes and an offset per edge took 0.73, 0.83 and 0.27 ms over the
 // 21 levels of RCM on RMAT scale 19.)
 // ---------------------------------------------------------------------------
@@ -993,9 +993,35 @@ __device__ __forceinline__ int64_t upper_index(const int64_t* __restrict__ D, in
 
 // Frontier edges in runs of kEdgeRun consecutive edge indices per thread: one
 // binary search for the run's first edge, then the owning frontier vertex
-// advances with the edge index.  fn(run, nbr, idx): the run's neighbours (-1
-// past the last edge) and their frontier indices, all read together.
+// advances with the edge index.  nbr, idx: the run's neighbours (-1 past the last
+// edge, T) and their frontier indices, all read together.
 constexpr int kEdgeRun = 8;
+
+__device__ __forceinline__ void edge_run(int64_t run, const int32_t* __restrict__ F, int64_t nf,
+                                         const int64_t* __restrict__ D, int64_t T, const int64_t* __restrict__ rp,
+                                         const int32_t* __restrict__ col, int32_t (&nbr)[kEdgeRun],
+                                         int32_t (&idx)[kEdgeRun]) {
+    const int64_t e0 = run * kEdgeRun;
+    int64_t i = upper_index(D, nf, e0), next = D[i + 1];
+    int64_t row = rp[F[i]] - D[i];
+#pragma unroll
+    for (int k = 0; k < kEdgeRun; ++k) {
+        const int64_t e = e0 + k;
+        nbr[k] = -1;
+        idx[k] = 0;
+        if (e < T) {
+            if (e >= next) {
+                do {
+                    ++i;
+                    next = D[i + 1];
+                } while (e >= next);
+                row = rp[F[i]] - D[i];
+            }
+            nbr[k] = col[row + e];
+            idx[k] = (int32_t)i;
+        }
+    }
+}
 
 template <typename Skip, typename Fn>
 __device__ __forceinline__ void for_edge_runs(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D,
@@ -1005,27 +1031,8 @@ __device__ __forceinline__ void for_edge_runs(const int32_t* __restrict__ F, int
     for (int64_t run = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; run * kEdgeRun < T;
          run += (int64_t)gridDim.x * blockDim.x) {
         if (skip(run)) continue;
-        const int64_t e0 = run * kEdgeRun;
-        int64_t i = upper_index(D, nf, e0), at = D[i], next = D[i + 1];
-        int64_t row = rp[F[i]] - at;
         int32_t nbr[kEdgeRun], idx[kEdgeRun];
-#pragma unroll
-        for (int k = 0; k < kEdgeRun; ++k) {
-            const int64_t e = e0 + k;
-            nbr[k] = -1;
-            idx[k] = 0;
-            if (e < T) {
-                if (e >= next) {
-                    do {
-                        ++i;
-                        next = D[i + 1];
-                    } while (e >= next);
-                    row = rp[F[i]] - D[i];
-                }
-                nbr[k] = col[row + e];
-                idx[k] = (int32_t)i;
-            }
-        }
+        edge_run(run, F, nf, D, T, rp, col, nbr, idx);
         fn(run, nbr, idx);
     }
 }
@@ -1047,59 +1054,85 @@ k_bfs_claim(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict
                   });
 }
 
-// Runs past the frontier's last edge, up to `runs`, get no bits.
-__global__ void __launch_bounds__(256)
+// Discoveries of the frontier's edges.  A CTA takes kRunBlock runs at a time:
+// bits and first[run], the discoveries before the run within its block; count[]
+// gets the block's.  Blocks past the last edge count none.
+constexpr int kRunBlock = 256;
+
+struct Discoveries {
+    uint8_t* bits;      // per run: which of its edges discovered their neighbour
+    uint16_t* first;
+    int64_t* count;     // per block, then its exclusive scan (and the total behind)
+    int64_t blocks;
+};
+
+__global__ void __launch_bounds__(kRunBlock)
 k_bfs_flag(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D, const int64_t* __restrict__ rp,
-           const int32_t* __restrict__ col, const uint32_t* __restrict__ claim, int64_t runs,
-           uint8_t* __restrict__ bits, uint8_t* __restrict__ cnt) {
-    for_edge_runs(F, nf, D, rp, col, [](int64_t) { return false; },
-                  [&](int64_t run, const int32_t* nbr, const int32_t* idx) {
-                      uint32_t c[kEdgeRun], b = 0;
+           const int32_t* __restrict__ col, const uint32_t* __restrict__ claim, Discoveries d) {
+    __shared__ int wsum[kRunBlock / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t T = D[nf];
+    for (int64_t blk = blockIdx.x; blk < d.blocks; blk += gridDim.x) {
+        const int64_t run = blk * kRunBlock + threadIdx.x;
+        uint32_t b = 0;
+        if (run * kEdgeRun < T) {
+            int32_t nbr[kEdgeRun], idx[kEdgeRun];
+            edge_run(run, F, nf, D, T, rp, col, nbr, idx);
+            uint32_t c[kEdgeRun];
 #pragma unroll
-                      for (int k = 0; k < kEdgeRun; ++k) c[k] = nbr[k] >= 0 ? claim[nbr[k]] : 0u;
+            for (int k = 0; k < kEdgeRun; ++k) c[k] = nbr[k] >= 0 ? claim[nbr[k]] : 0u;
 #pragma unroll
-                      for (int k = 0; k < kEdgeRun; ++k)
-                          b |= c[k] == (uint32_t)idx[k] + 1u ? 1u << k : 0u;
-                      bits[run] = (uint8_t)b;
-                      cnt[run] = (uint8_t)__popc(b);
-                  });
-    const int64_t used = (D[nf] + kEdgeRun - 1) / kEdgeRun;
-    for (int64_t run = used + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; run < runs;
-         run += (int64_t)gridDim.x * blockDim.x) {
-        bits[run] = 0;
-        cnt[run] = 0;
+            for (int k = 0; k < kEdgeRun; ++k) b |= c[k] == (uint32_t)idx[k] + 1u ? 1u << k : 0u;
+        }
+        const int mine = __popc(b);
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += x;
+        }
+        if (lane == 31) wsum[w] = incl;
+        __syncthreads();
+        int before = 0;
+        for (int q = 0; q < w; ++q) before += wsum[q];
+        d.bits[run] = (uint8_t)b;
+        d.first[run] = (uint16_t)(before + incl - mine);
+        if (threadIdx.x == kRunBlock - 1) d.count[blk] = before + incl;
+        __syncthreads();
     }
 }
 
+__device__ __forceinline__ int64_t run_first(const Discoveries& d, int64_t run) {
+    return d.count[run / kRunBlock] + d.first[run];
+}
+
 // Children found by the edges before edge e.
-__device__ __forceinline__ int64_t children_before(int64_t e, const uint8_t* __restrict__ bits,
-                                                   const int64_t* __restrict__ P, int64_t runs) {
+__device__ __forceinline__ int64_t children_before(int64_t e, const Discoveries& d) {
     const int64_t run = e / kEdgeRun;
-    if (run >= runs) return P[runs];
-    return P[run] + __popc(bits[run] & ((1u << (e % kEdgeRun)) - 1u));
+    if (run >= d.blocks * kRunBlock) return d.count[d.blocks];
+    return run_first(d, run) + __popc(d.bits[run] & ((1u << (e % kEdgeRun)) - 1u));
 }
 
 // Per community: where its children start in the next frontier this level.
 __global__ void k_bfs_bases(int32_t nslots, const int64_t* __restrict__ fs, const int64_t* __restrict__ fe,
-                            const int64_t* __restrict__ D, const uint8_t* __restrict__ bits,
-                            const int64_t* __restrict__ P, int64_t runs, int64_t* __restrict__ base,
+                            const int64_t* __restrict__ D, Discoveries d, int64_t* __restrict__ base,
                             int64_t* __restrict__ end) {
     for (int32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nslots; j += gridDim.x * blockDim.x) {
-        base[j] = children_before(D[fs[j]], bits, P, runs);
-        end[j] = children_before(D[fe[j]], bits, P, runs);
+        base[j] = children_before(D[fs[j]], d);
+        end[j] = children_before(D[fe[j]], d);
     }
 }
 
 __global__ void __launch_bounds__(256)
 k_bfs_write(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D, const int64_t* __restrict__ rp,
-            const int32_t* __restrict__ col, const uint32_t* __restrict__ memb, const uint8_t* __restrict__ bits,
-            const int64_t* __restrict__ P, const int32_t* __restrict__ slot_of_comm,
+            const int32_t* __restrict__ col, const uint32_t* __restrict__ memb, Discoveries d,
+            const int32_t* __restrict__ slot_of_comm,
             const int64_t* __restrict__ qlen, const int64_t* __restrict__ base, int32_t* __restrict__ nextF,
             uint32_t* __restrict__ claim, uint32_t* __restrict__ local) {
-    for_edge_runs(F, nf, D, rp, col, [&](int64_t run) { return bits[run] == 0; },
+    for_edge_runs(F, nf, D, rp, col, [&](int64_t run) { return d.bits[run] == 0; },
                   [&](int64_t run, const int32_t* nbr, const int32_t*) {
-                      const uint32_t b = bits[run];
-                      int64_t p = P[run];
+                      const uint32_t b = d.bits[run];
+                      int64_t p = run_first(d, run);
 #pragma unroll
                       for (int k = 0; k < kEdgeRun; ++k) {
                           if (!((b >> k) & 1u)) continue;
@@ -1181,14 +1214,13 @@ __global__ void k_rcm_frontier(int32_t nslots, const int32_t* __restrict__ part,
 // and the largest of their degrees.
 __global__ void __launch_bounds__(256)
 k_rcm_write(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D, const int64_t* __restrict__ rp,
-            const int32_t* __restrict__ col, const uint8_t* __restrict__ bits, const int64_t* __restrict__ P,
-            int32_t* __restrict__ nextF, int32_t* __restrict__ parent, uint32_t* __restrict__ claim,
+            const int32_t* __restrict__ col, Discoveries d, int32_t* __restrict__ nextF, int32_t* __restrict__ parent, uint32_t* __restrict__ claim,
             unsigned long long* __restrict__ max_deg) {
     unsigned long long m = 0;
-    for_edge_runs(F, nf, D, rp, col, [&](int64_t run) { return bits[run] == 0; },
+    for_edge_runs(F, nf, D, rp, col, [&](int64_t run) { return d.bits[run] == 0; },
                   [&](int64_t run, const int32_t* nbr, const int32_t* idx) {
-                      const uint32_t b = bits[run];
-                      int64_t p = P[run];
+                      const uint32_t b = d.bits[run];
+                      int64_t p = run_first(d, run);
 #pragma unroll
                       for (int k = 0; k < kEdgeRun; ++k) {
                           if (!((b >> k) & 1u)) continue;
@@ -1389,37 +1421,42 @@ T read_dev(const T* p, cudaStream_t s) {
 // level needs no look at the device before its kernels are enqueued, and one
 // after (two or three a level were a third of RCM's time).
 struct LevelBufs {
-    DevBuf<uint8_t> bits, cnt;
-    DevBuf<int64_t> P;
+    DevBuf<uint8_t> bits;
+    DevBuf<uint16_t> first;
+    DevBuf<int64_t> count;
     DevBuf<unsigned long long> out;   // children, the largest of their degrees
-    int64_t max_deg = 0, bound = 0, runs = 0;
+    int64_t max_deg = 0, bound = 0, blocks = 0;
+    static int64_t blocks_for(int64_t edges) { return ceil_div(ceil_div(edges, kEdgeRun), kRunBlock); }
     LevelBufs(const DeviceCSR& g, int64_t nn, const int32_t* order_v, cudaStream_t s)
-        : bits(ceil_div(g.nnz, kEdgeRun), s), cnt(ceil_div(g.nnz, kEdgeRun), s), P(ceil_div(g.nnz, kEdgeRun) + 1, s),
-          out(2, s) {
+        : bits(blocks_for(g.nnz) * kRunBlock, s), first(blocks_for(g.nnz) * kRunBlock, s),
+          count(blocks_for(g.nnz) + 1, s), out(2, s) {
         GB_CUDA(cudaMemsetAsync(out, 0, 2 * sizeof(unsigned long long), s));
         k_max_degree_of<<<grid_for(nn, kT), kT, 0, s>>>(order_v, nn, g.row_ptr, out);
         GB_LAUNCH_CHECK();
         max_deg = (int64_t)read_dev(out.get(), s);
     }
     unsigned long long* max_child() const { return out.get() + 1; }
-    // Claims and discovery bits of the frontier F[0, nf); D receives its edge offsets.
+    Discoveries view() const { return {bits.get(), first.get(), count.get(), blocks}; }
+    // Claims and discoveries of the frontier F[0, nf); D receives its edge offsets.
     void find(const DeviceCSR& g, const int32_t* F, int64_t nf, int64_t* D, const uint32_t* memb, uint32_t* claim,
               cudaStream_t s) {
         bound = nf > g.nnz / std::max<int64_t>(max_deg, 1) ? g.nnz : nf * max_deg;
-        runs = ceil_div(bound, kEdgeRun);
+        blocks = blocks_for(bound);
         GB_CUDA(cudaMemsetAsync(out, 0, 2 * sizeof(unsigned long long), s));
         k_frontier_degrees<<<grid_for(nf, kT), kT, 0, s>>>(F, nf, g.row_ptr, D);
         GB_LAUNCH_CHECK();
         exclusive_scan_i64_total(D, D, nf, D + nf, s);
         k_bfs_claim<<<edge_grid(bound), 256, 0, s>>>(F, nf, D, g.row_ptr, g.col, memb, claim);
         GB_LAUNCH_CHECK();
-        k_bfs_flag<<<edge_grid(bound), 256, 0, s>>>(F, nf, D, g.row_ptr, g.col, claim, runs, bits, cnt);
-        GB_LAUNCH_CHECK();
-        exclusive_scan_u8_to_i64(cnt, P, runs, P.get() + runs, s);
+        if (blocks > 0) {
+            k_bfs_flag<<<grid_for(blocks, 1), kRunBlock, 0, s>>>(F, nf, D, g.row_ptr, g.col, claim, view());
+            GB_LAUNCH_CHECK();
+        }
+        exclusive_scan_i64_total(count, count, blocks, count.get() + blocks, s);
     }
     // Children of the level (after the kernels that write them).
     int64_t children(unsigned long long* max_child_deg, cudaStream_t s) {
-        GB_CUDA(cudaMemcpyAsync(out, P.get() + runs, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
+        GB_CUDA(cudaMemcpyAsync(out, count.get() + blocks, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
         unsigned long long h[2];
         GB_CUDA(cudaMemcpyAsync(h, out.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
         GB_CUDA(cudaStreamSynchronize(s));
@@ -1491,9 +1528,9 @@ int64_t rcm_communities(const DeviceCSR& g, const uint32_t* memb, const int32_t*
             }
             ++level;
             lv.find(g, F, nf, D, memb, claim, s);
-            k_bfs_bases<<<grid_for(nslots, kT), kT, 0, s>>>(nslots, fs, fe, D, lv.bits, lv.P, lv.runs, bbase, bend);
+            k_bfs_bases<<<grid_for(nslots, kT), kT, 0, s>>>(nslots, fs, fe, D, lv.view(), bbase, bend);
             GB_LAUNCH_CHECK();
-            k_rcm_write<<<edge_grid(lv.bound), 256, 0, s>>>(F, nf, D, g.row_ptr, g.col, lv.bits, lv.P, NF, parent, claim,
+            k_rcm_write<<<edge_grid(lv.bound), 256, 0, s>>>(F, nf, D, g.row_ptr, g.col, lv.view(), NF, parent, claim,
                                                            lv.max_child());
             GB_LAUNCH_CHECK();
             unsigned long long md = 0;
@@ -1827,9 +1864,9 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
             ++levels;
             lv.find(g, F, nf, D, memb, claim, s);
             if (lv.bound == 0) break;
-            k_bfs_bases<<<grid_for(nbfs, kT), kT, 0, s>>>(nbfs, fs, fe, D, lv.bits, lv.P, lv.runs, bbase, bend);
+            k_bfs_bases<<<grid_for(nbfs, kT), kT, 0, s>>>(nbfs, fs, fe, D, lv.view(), bbase, bend);
             GB_LAUNCH_CHECK();
-            k_bfs_write<<<edge_grid(lv.bound), 256, 0, s>>>(F, nf, D, g.row_ptr, g.col, memb, lv.bits, lv.P,
+            k_bfs_write<<<edge_grid(lv.bound), 256, 0, s>>>(F, nf, D, g.row_ptr, g.col, memb, lv.view(),
                                                            slot_of_comm, qlen, bbase, NF, claim, local);
             GB_LAUNCH_CHECK();
             k_bfs_advance<<<grid_for(nbfs, kT), kT, 0, s>>>(nbfs, qlen, fs, fe, bbase, bend);

@@ -3,6 +3,8 @@
 // All of these are bandwidth-bound integer passes: tiles of 2048 elements per
 // 256-thread CTA, coalesced loads, shared-memory staging, grid sizes set by
 // the element count.
+#include <algorithm>
+
 #include "gb_chunks.cuh"
 #include "gb_common.cuh"
 
@@ -93,6 +95,40 @@ __global__ void k_tile_scan(const Tin* __restrict__ in, int64_t* __restrict__ ou
     }
 }
 
+// Up to kScanOneMax values by one CTA, tile after tile with a running offset:
+// one launch of 3 to 7 us where reduce, scan of the partials and scan are three
+// launches of 4 us each and the gaps between them.  A tile's values are read
+// before any of it is written, so out may alias in.
+constexpr int kScanOneThreads = 512;   // block_excl_scan keeps a slot of its 32 for the total
+constexpr int kScanOneItems = 16;
+constexpr int kScanOneTile = kScanOneThreads * kScanOneItems;
+constexpr int64_t kScanOneMax = 4 * kScanOneTile;
+
+template <typename Tin>
+__global__ void __launch_bounds__(kScanOneThreads)
+k_scan_one(const Tin* __restrict__ in, int64_t* __restrict__ out, int64_t n, int64_t* __restrict__ total_out) {
+    int64_t carry = 0;
+    for (int64_t base = 0; base < n; base += kScanOneTile) {
+        int64_t v[kScanOneItems], sum = 0;
+#pragma unroll
+        for (int j = 0; j < kScanOneItems; ++j) {
+            const int64_t i = base + (int64_t)threadIdx.x * kScanOneItems + j;
+            v[j] = i < n ? (int64_t)in[i] : 0;
+            sum += v[j];
+        }
+        int64_t total;
+        int64_t run = carry + block_excl_scan(sum, &total);
+#pragma unroll
+        for (int j = 0; j < kScanOneItems; ++j) {
+            const int64_t i = base + (int64_t)threadIdx.x * kScanOneItems + j;
+            if (i < n) out[i] = run;
+            run += v[j];
+        }
+        carry += total;
+    }
+    if (total_out && threadIdx.x == 0) *total_out = carry;
+}
+
 template <typename Tin>
 void exclusive_scan_impl(const Tin* in, int64_t* out, int64_t n, int64_t* total_dev, cudaStream_t s) {
     if (n <= 0) {
@@ -102,6 +138,11 @@ void exclusive_scan_impl(const Tin* in, int64_t* out, int64_t n, int64_t* total_
     const int64_t tiles = ceil_div(n, kScanTile);
     if (tiles == 1) {
         k_tile_scan<Tin><<<1, kScanThreads, 0, s>>>(in, out, n, nullptr, total_dev);
+        GB_LAUNCH_CHECK();
+        return;
+    }
+    if (n <= kScanOneMax) {
+        k_scan_one<Tin><<<1, kScanOneThreads, 0, s>>>(in, out, n, total_dev);
         GB_LAUNCH_CHECK();
         return;
     }
@@ -200,10 +241,77 @@ __global__ void k_radix_scatter(const K* __restrict__ keys_in, const uint32_t* _
     }
 }
 
+// Up to kSmallSort pairs by one CTA: a bitonic sort in shared memory by (key,
+// input position), so it is stable too.  One launch of a few microseconds where a
+// radix sort takes three to five a pass and up to eight passes.
+constexpr int kSmallSort = 4096;
+constexpr int kSmallSortThreads = 1024;
+
+template <typename K, bool kHasValues>
+__global__ void __launch_bounds__(kSmallSortThreads)
+k_sort_small(K* __restrict__ keys, uint32_t* __restrict__ values, int n, int padded, K mask) {
+    extern __shared__ __align__(16) unsigned char sort_smem[];
+    K* k = reinterpret_cast<K*>(sort_smem);
+    uint16_t* at = reinterpret_cast<uint16_t*>(k + padded);
+    for (int i = threadIdx.x; i < padded; i += blockDim.x) {
+        k[i] = i < n ? keys[i] & mask : (K)~(K)0;   // the padding's positions are the largest, too
+        at[i] = (uint16_t)i;
+    }
+    __syncthreads();
+    for (int run = 2; run <= padded; run <<= 1) {
+        for (int d = run >> 1; d > 0; d >>= 1) {
+            for (int t = threadIdx.x; t < padded / 2; t += blockDim.x) {
+                const int i = 2 * t - (t & (d - 1)), j = i + d;
+                const K x = k[i], y = k[j];
+                const uint16_t p = at[i], q = at[j];
+                const bool after = x > y || (x == y && p > q);
+                if (after == ((i & run) == 0)) {
+                    k[i] = y;
+                    k[j] = x;
+                    at[i] = q;
+                    at[j] = p;
+                }
+            }
+            __syncthreads();
+        }
+    }
+    // Keys and values as given, moved: every read before the first write.
+    constexpr int kPer = kSmallSort / kSmallSortThreads;
+    K kk[kPer];
+    uint32_t vv[kPer];
+#pragma unroll
+    for (int r = 0; r < kPer; ++r) {
+        const int i = threadIdx.x + r * blockDim.x;
+        if (i < n) {
+            kk[r] = keys[at[i]];
+            if (kHasValues) vv[r] = values[at[i]];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kPer; ++r) {
+        const int i = threadIdx.x + r * blockDim.x;
+        if (i < n) {
+            keys[i] = kk[r];
+            if (kHasValues) values[i] = vv[r];
+        }
+    }
+}
+
 template <typename K, bool kHasValues>
 void radix_sort_impl(K* keys, uint32_t* values, int64_t n, int key_bits, cudaStream_t s) {
     if (n <= 1 || key_bits <= 0) return;
     const int passes = (key_bits + 7) / 8;
+    if (n <= kSmallSort) {
+        int padded = 2;
+        while (padded < n) padded <<= 1;
+        const K mask = 8 * passes >= (int)(8 * sizeof(K)) ? (K)~(K)0 : (((K)1 << (8 * passes)) - 1);
+        const int smem = padded * (int)(sizeof(K) + sizeof(uint16_t));
+        k_sort_small<K, kHasValues><<<1, std::min(kSmallSortThreads, std::max(32, padded / 2)), smem, s>>>(
+            keys, values, (int)n, padded, mask);
+        GB_LAUNCH_CHECK();
+        return;
+    }
     const int64_t tiles = ceil_div(n, kRadixTile);
     DevBuf<K> kbuf(n, s);
     DevBuf<uint32_t> vbuf(kHasValues ? n : 0, s);

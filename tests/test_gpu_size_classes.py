@@ -150,3 +150,21 @@ def test_relabel_by_row_length(ctx, lengths):
     np.testing.assert_array_equal(new_rp, expect_rp)
     np.testing.assert_array_equal(new_col, expect_col)
     np.testing.assert_array_equal(ids[old], np.arange(n))
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 33, 64, 65, 2047, 2048, 2049, 4095, 4096, 4097, 8192, 8193, 32767, 32768,
+                               32769])
+def test_sorts_and_scans_by_length(ctx, n):
+    # DBG is one stable sort of n small keys; the rebuilt offsets are one scan.
+    rp, col = (t.numpy() for t in _kernel_graph("stars", max(1, n // 4)) if n > 8) if n > 8 else \
+        (t.numpy() for t in gg.from_edges(n, [(i, i + 1) for i in range(n - 1)]))
+    n = len(rp) - 1
+    degree = np.diff(rp)
+    limits = (len(col) // n) * np.array([1, 2, 4, 8, 16, 32, 64]) // 2
+    order = np.argsort(-np.searchsorted(limits, degree, side="left"), kind="stable")
+    expect = np.empty(n, dtype=np.int32)
+    expect[order] = np.arange(n, dtype=np.int32)
+    ids, _ = ctx.dbg_mapping(rp, col)
+    np.testing.assert_array_equal(ids, expect)
+    new_rp, _, _ = ctx.relabel_by_mapping(rp, col, ids)
+    np.testing.assert_array_equal(new_rp, np.concatenate([[0], np.cumsum(degree[order])]))
