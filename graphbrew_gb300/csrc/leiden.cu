@@ -289,7 +289,8 @@ __global__ void k_super_weights(const int32_t* __restrict__ exists, const int64_
         if (exists[c]) sweight[cmap[c]] = (long long)ctot[c];
 }
 
-// Inter-community edges as keys (community(u) << 32 | community(v)), one
+// Inter-community edges as keys (community(u) << bits | community(v), bits the
+// width of a community id: no sort pass over empty bits between the two), one
 // entry-parallel pass: each CTA compacts its chunk's hits warp by warp and
 // reserves their slots with one atomic on the cursor.  The keys are sorted
 // next, so the order in which CTAs reserve does not reach the result.
@@ -297,7 +298,7 @@ constexpr int kInterThreads = 256;
 
 __global__ void __launch_bounds__(kInterThreads)
 k_inter_edges(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, const uint32_t* __restrict__ vcom,
-              int64_t n, int64_t nnz, const int32_t* __restrict__ chunk_row, uint64_t* __restrict__ keys,
+              int64_t n, int64_t nnz, const int32_t* __restrict__ chunk_row, int bits, uint64_t* __restrict__ keys,
               unsigned long long* __restrict__ cursor) {
     constexpr int kPer = kEdgeChunk / kInterThreads;
     __shared__ int32_t srow[kEdgeChunkPadded];
@@ -322,7 +323,7 @@ k_inter_edges(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, c
                 const uint32_t cu = vcom[srow[chunk_pad(i)]];
                 const uint32_t cv = vcom[col[e0 + i]];
                 hit = cu != cv;
-                key[k] = ((uint64_t)cu << 32) | cv;
+                key[k] = ((uint64_t)cu << bits) | cv;
             }
             hits[k] = __ballot_sync(0xFFFFFFFFu, hit);
             cnt += __popc(hits[k]);
@@ -347,20 +348,26 @@ k_inter_edges(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, c
 }
 
 // Run-length encode sorted keys: unique flags.
-__global__ void k_rle_flags(const uint64_t* __restrict__ keys, int64_t m, int32_t* __restrict__ flag) {
+__global__ void k_rle_flags(const uint64_t* __restrict__ keys, int64_t m, uint8_t* __restrict__ flag) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x)
         flag[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1 : 0;
 }
 
-__global__ void k_rle_emit(const uint64_t* __restrict__ keys, int64_t m, const int32_t* __restrict__ flag,
-                           const int64_t* __restrict__ pos, int64_t nuniq, uint32_t* __restrict__ snbr,
-                           uint32_t* __restrict__ sw, int32_t* __restrict__ sdeg, int64_t* __restrict__ start) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
-        if (!flag[i]) continue;
-        const int64_t p = pos[i];
-        snbr[p] = (uint32_t)(keys[i] & 0xFFFFFFFFull);
-        start[p] = i;
-        atomicAdd(&sdeg[keys[i] >> 32], 1);
+__global__ void k_rle_emit(const uint64_t* __restrict__ keys, int64_t m, const uint8_t* __restrict__ flag,
+                           const int64_t* __restrict__ pos, int bits, uint32_t* __restrict__ snbr,
+                           uint32_t* __restrict__ sdeg, int64_t* __restrict__ start) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; i0 < m;
+         i0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = i0 + lane;
+        const bool first = i < m && flag[i];
+        const uint64_t key = first ? keys[i] : 0;
+        if (first) {
+            const int64_t p = pos[i];
+            snbr[p] = (uint32_t)(key & ((1ull << bits) - 1ull));
+            start[p] = i;
+        }
+        warp_add_u32(sdeg, (uint32_t)(key >> bits), 1u, first);
     }
 }
 
@@ -1495,10 +1502,11 @@ void leiden_device(const DeviceCSR& g, const LeidenParams& p, uint32_t* vcom, gb
         // Super-graph adjacency (inter-community edges only, :2184-2224).
         DevBuf<uint64_t> ikeys(g.nnz > 0 ? g.nnz : 1, s);
         int64_t ninter = 0;
+        const int cb = std::max(1, bits_for((uint64_t)(C > 0 ? C - 1 : 0)));
         if (g.nnz > 0) {
             GB_CUDA(cudaMemsetAsync(inter_cursor, 0, sizeof(unsigned long long), s));
             k_inter_edges<<<grid_for(edge_chunks(g.nnz), 1), kInterThreads, 0, s>>>(
-                g.row_ptr, g.col, vcom, n, g.nnz, chunk_row, ikeys, inter_cursor);
+                g.row_ptr, g.col, vcom, n, g.nnz, chunk_row, cb, ikeys, inter_cursor);
             GB_LAUNCH_CHECK();
             ninter = (int64_t)read_dev(inter_cursor.get(), s);
             launches += 1;
@@ -1509,22 +1517,22 @@ void leiden_device(const DeviceCSR& g, const LeidenParams& p, uint32_t* vcom, gb
         DevBuf<uint32_t> snbr, sw;
         int64_t nuniq = 0;
         if (ninter > 0) {
-            const int cb = bits_for((uint64_t)(C > 0 ? C - 1 : 0));
-            radix_sort_keys_u64(ikeys, ninter, 32 + cb, s);
-            DevBuf<int32_t> uflag(ninter, s);
+            radix_sort_keys_u64(ikeys, ninter, 2 * cb, s);
+            DevBuf<uint8_t> uflag(ninter, s);
             DevBuf<int64_t> upos(ninter + 1, s);
             k_rle_flags<<<grid_for(ninter, kT), kT, 0, s>>>(ikeys, ninter, uflag);
             GB_LAUNCH_CHECK();
-            exclusive_scan_i32_to_i64(uflag, upos, ninter, upos.get() + ninter, s);
+            exclusive_scan_u8_to_i64(uflag, upos, ninter, upos.get() + ninter, s);
             nuniq = read_dev(upos.get() + ninter, s);
             snbr.alloc(nuniq, s);
             sw.alloc(nuniq, s);
             DevBuf<int64_t> ustart(nuniq, s);
-            k_rle_emit<<<grid_for(ninter, kT), kT, 0, s>>>(ikeys, ninter, uflag, upos, nuniq, snbr, sw, sdeg, ustart);
+            k_rle_emit<<<grid_for(ninter, kT), kT, 0, s>>>(ikeys, ninter, uflag, upos, cb, snbr,
+                                                           reinterpret_cast<uint32_t*>(sdeg.get()), ustart);
             GB_LAUNCH_CHECK();
             k_rle_weights<<<grid_for(nuniq, kT), kT, 0, s>>>(ustart, nuniq, ninter, sw);
             GB_LAUNCH_CHECK();
-            launches += 7 + 3 * ((32 + cb + 7) / 8);
+            launches += 7 + 3 * ((2 * cb + 7) / 8);
         }
         {
             // soff = exclusive scan of sdeg (int32 -> int64)
