@@ -168,3 +168,34 @@ def test_sorts_and_scans_by_length(ctx, n):
     np.testing.assert_array_equal(ids, expect)
     new_rp, _, _ = ctx.relabel_by_mapping(rp, col, ids)
     np.testing.assert_array_equal(new_rp, np.concatenate([[0], np.cumsum(degree[order])]))
+
+
+def _clustered_graph(kind, blocks, size):
+    """Blocks whose super-nodes have tied (cliques), nearly tied (copies with a few
+    extra edges) or many (a hub block) neighbours."""
+    rng = np.random.default_rng(blocks * 1000 + size)
+    edges = []
+    for b in range(blocks):
+        at = b * size
+        edges += [(at + i, at + j) for i in range(size) for j in range(i)]
+    between = [(b, (b + step) % blocks) for b in range(blocks) for step in (1, 2, 3)]
+    if kind == "hub":
+        between += [(0, b) for b in range(1, blocks)]
+    for a, b in between:
+        count = size if kind != "near" else size + int(rng.integers(0, 2))
+        edges += [(a * size + int(i), b * size + int(j))
+                  for i, j in zip(rng.permutation(size)[:count], rng.permutation(size)[:count])]
+    if kind == "near":
+        edges += [(int(a), int(b)) for a, b in rng.integers(0, blocks * size, (blocks // 3 + 1, 2)) if a != b]
+    return gg.from_edges(blocks * size, edges)
+
+
+@pytest.mark.parametrize("resolution", [1e-6, 0.3, 1.0, 1.7])
+@pytest.mark.parametrize("kind,blocks,size", [("ties", 9, 5), ("ties", 1500, 4), ("near", 40, 6), ("near", 1500, 4),
+                                              ("hub", 100, 5), ("hub", 300, 5), ("hub", 3000, 3)])
+def test_super_moves_with_close_candidates(ctx, kind, blocks, size, resolution):
+    rp, col = (t.numpy() for t in _clustered_graph(kind, blocks, size))
+    memb, st = ctx.run_graphbrew(rp, col, gb.DEFAULT_RECIPE, resolution)
+    expect, ost = po.leiden(rp, col, resolution)
+    np.testing.assert_array_equal(np.asarray(memb).view(np.uint32), expect)
+    assert [st["passes"], st["iterations"]] == [ost.passes, ost.iterations]
