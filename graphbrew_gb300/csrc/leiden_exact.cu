@@ -14,12 +14,12 @@
 //     exact prefix: all of [P, x] was evaluated from exact inputs (induction
 //     from P), so it is committed; the rest carries its new decisions forward.
 //
-// Community totals at time u come from an event table rebuilt every round by
-// one CTA: each speculative move contributes (old, -k) and (new, +k) at its
-// time; events are stably radix-sorted by community slot in shared memory and
-// prefix-summed, and a lookup binary-searches the community's events for the
-// last time before u.  All totals are exact integers, so every
-// Delta-modularity equals the serial one.
+// Community totals at time u come from an event table rebuilt every round:
+// each speculative move contributes (old, -k) and (new, +k) at its time, hashed
+// by community.  A lookup adds up the community's events before u; the few
+// communities with many events have theirs sorted by time and prefix-summed.
+// All totals are exact integers, so every Delta-modularity equals the serial
+// one whatever the order of the sums.
 //
 // Vertices above kWarpMaxDeg ("hubs") are split into 4096-edge segments, each
 // accumulated by its own CTA into the hub's global table, then scanned in
@@ -51,34 +51,35 @@ constexpr int kWindowMax = 65536;             // window vertices (events <= 2 x 
 constexpr int kEventsMax = 2 * kWindowMax;    // event index = 2 x window offset (+1)
 constexpr int kSlotBits = 18;
 constexpr int kTableSlots = 1 << kSlotBits;   // hash slots, >= 2 x events
-constexpr int kCoarseBits = 9;                // event grouping: 512 coarse buckets of slots
-constexpr int kCoarse = 1 << kCoarseBits;
-constexpr int kFineBits = kSlotBits - kCoarseBits;
-constexpr int kTbThreads = 1024;              // table insert / group: one window vertex per thread
-constexpr int kTbMinChunk = 512;            // smallest insert chunk (CTA size) the table kernels accept
-constexpr int kTbChunks = kWindowMax / kTbMinChunk;   // stride of the per-chunk histograms
-constexpr int kTbFinishThreads = 512;         // table finish: one CTA per coarse bucket, a thread per fine digit
+constexpr int kTbThreads = 256;               // table insert: one window vertex per thread
+constexpr int kSortThreads = 512;             // sorting of the slots with many events
+constexpr int kSortCtas = 2 * kNumSMs;
 constexpr uint32_t kPadSlot = 0xFFFFFFFFu;
-static_assert(kTableSlots >= 2 * kEventsMax, "hash load factor <= 1/2");
-static_assert(kCoarse <= kTbMinChunk, "one coarse bucket per grouping thread");
+// Events of a slot: up to kInline of them lie at the slot, in any order (their
+// sum is what a lookup wants), the others in blocks of kInline at slots of the
+// same table, under names of their own: 1 << 31 | slot << kBlockBits | block.
+constexpr int kInline = 16;
+constexpr int kBlockBits = 13;
+constexpr int kWarpSort = 64;                 // events of a slot that one warp sorts
+static_assert(kTableSlots >= 2 * (kEventsMax + kEventsMax / kInline) * 15 / 16, "hash load factor near 1/2");
+static_assert(kSlotBits + kBlockBits <= 31 && (kEventsMax / kInline) <= (1 << kBlockBits), "block names fit");
 // Slots with many events ("hot": a community that many window vertices join
-// or leave) get a time-bucket index: bidx[b] = first event at time >= P + 16 b,
-// so a lookup searches at most 16 events instead of the whole slot.
+// or leave) get an index by time: a bit per window offset that has an event,
+// and the events before each 32 offsets.
 constexpr int kHotMin = 128;                  // events that make a slot hot
-constexpr int kBucketV = 16;                  // window vertices per time bucket
-constexpr int kHotStride = kWindowMax / kBucketV + 1;
-constexpr int kHotMax = 2 * kEventsMax / kHotMin;
-constexpr int kEndBits = 18;                  // SlotMeta.endh: end | (hot id + 1) << kEndBits
+constexpr int kHotMax = kEventsMax / kHotMin;
+constexpr int kHotWords = kWindowMax / 32;
+constexpr int kBucketV = 16;                  // window vertices per bucket of a dense row
+constexpr int kBucketStride = kWindowMax / kBucketV + 1;
 // Designated communities: the few communities with the most events (on RMAT
-// the one most vertices join) leave the sorted table.  Each gets a dense row
+// the one most vertices join) leave the table.  Each gets a dense row
 // over the window (the signed degree of every window offset's move into or
 // out of it) and the prefix of its 16-offset bucket sums, so a lookup is one
-// prefix load plus one 64-byte read, and no bucket of the sorted table holds
-// a giant community.  Chosen each round from the previous table's counts.
+// prefix load plus one 64-byte read, and no slot of the table holds a giant
+// community.  Chosen each round from the previous table's counts.
 constexpr int kZMax = 8;                      // designated communities at most
 constexpr int kZKeep = 64;                    // events a designated community needs to stay / be chosen
-constexpr int kZCand = 128;                   // hot slots of the sorted table considered
-static_assert(kEventsMax < (1 << kEndBits), "event positions fit the end field");
+constexpr int kZCand = 128;                   // hot slots of the table considered
 // CommRec.slotw: where the community's events of the current table are -- low
 // bits of the table's generation, then a designated index or a hash slot.
 constexpr int kSlotwTagShift = kSlotBits + 1;
@@ -109,18 +110,26 @@ struct Ctl {
     long long error;          // nonzero: the round loop stopped without finishing
     unsigned long long tag;   // generation of the event table (slots of older tags are empty)
     unsigned int nhot;        // hot slots of the current table
-    unsigned long long tb_big; // largest coarse bucket: size << 32 | bucket (its CTA starts first)
-    unsigned int tb_ticket;    // insert CTAs done this round (the last one scans the histogram)
+    unsigned int nmany[2];     // slots with more than kInline / more than kWarpSort events
+    unsigned int sorted;       // events placed in the sorted arrays
     unsigned int nz;                 // designated communities of the current table
     unsigned int zc[kZMax];          // their ids
     unsigned int zcount[kZMax];      // events each received in the current table
 };
 
+// A slot's name, generation and count share one word, so that a claim is one
+// compare-and-swap and an event's place one add.  The generation is the
+// table's modulo 2^14 - 1, plus 1: the advance clears kClearSlots slots a round,
+// the whole table in a fraction of that cycle, and 0 is no generation.
+constexpr int kCountBits = 18;
+constexpr int kClearSlots = 128;
 struct __align__(16) SlotMeta {
-    unsigned long long tkey;  // table generation << 32 | community id
-    int32_t start;            // first sorted event of the slot
-    uint32_t endh;            // one past its last event | (hot index + 1) << kEndBits
+    unsigned long long word;  // community id << 32 | generation << kCountBits | events
+    int32_t start;            // more than kInline events: the first in the sorted arrays
+    uint32_t hot;             // hot index + 1, 0 = search by time
 };
+static_assert(kEventsMax < (1 << kCountBits), "counts fit");
+static_assert(2 * (kTableSlots / kClearSlots) < (1 << (32 - kCountBits)) - 1, "cleared before a generation returns");
 
 // What an evaluation needs of a community, in one 16-byte load: its committed
 // total, where its events of the current table are (if it has any) and the last
@@ -149,23 +158,18 @@ struct ExactState {
     double* delta;        // delta of the current decision (movers)
     double* final_delta;
     // event table
-    SlotMeta* slots;      // kTableSlots: community key and its sorted-event range
-    uint32_t* stime;      // event times (vertex ids), sorted by slot then time
+    SlotMeta* slots;      // kTableSlots
+    uint2* ev;            // kTableSlots x kInline events: window offset, signed degree
+    uint32_t* many[2];    // slots with more than kInline / more than kWarpSort events
+    uint32_t* stime;      // slots with more than kInline events: times (vertex ids), sorted by time within the slot
     long long* epre;      // inclusive prefix of the signed degrees within the slot
-    uint32_t* tb_s0;      // per window offset: slot of the departure event (kPadSlot: none)
-    uint32_t* tb_s1;      // slot of the arrival event
-    int32_t* wdeg;        // degree of a window mover, 0 otherwise
-    int32_t* tb_hist;     // coarse bucket x insert chunk counts
-    int32_t* tb_base;     // their exclusive prefix in bucket-major order: where a chunk's events of a bucket go
-    int32_t* tb_bstart;   // coarse bucket starts (kCoarse + 1)
-    unsigned long long* ev1;  // events grouped by coarse bucket: slot << 32 | event index
-    unsigned long long* ev2;  // events sorted by slot
-    int32_t* hot_bidx;        // kHotMax x kHotStride time-bucket starts of hot slots
-    uint8_t* zof;             // per community: designated index + 1, 0 = in the sorted table
+    int32_t* sdeg;        // signed degrees (slots sorted by a CTA)
+    uint2* hot_row;       // kHotMax x kHotWords: offsets with an event, events before the word
+    uint8_t* zof;             // per community: designated index + 1, 0 = in the table
     int32_t* zcontrib;        // [2 parities][kZMax][kWindowMax] signed degree per window offset
-    long long* zbsum;         // [2][kZMax][kHotStride] 16-offset bucket sums
-    long long* zpre;          // [2][kZMax][kHotStride] exclusive prefix of the bucket sums
-    unsigned long long* zcand;  // hot slots of the sorted table: events << 32 | community
+    long long* zbsum;         // [2][kZMax][kBucketStride] 16-offset bucket sums
+    long long* zpre;          // [2][kZMax][kBucketStride] exclusive prefix of the bucket sums
+    unsigned long long* zcand;  // hot slots of the table: events << 32 | community
     // hubs
     const uint32_t* hub_v;        // hub vertex ids (ascending)
     const int64_t* hub_toff;      // table offset
@@ -202,6 +206,12 @@ __device__ __forceinline__ uint32_t slot_hash(uint32_t c) {
     return (uint32_t)(((uint64_t)c * 0x9E3779B97F4A7C15ull) >> 40);
 }
 
+// The part of a slot's word above the count.
+__device__ __forceinline__ unsigned long long slot_name(unsigned long long tag, uint32_t id) {
+    constexpr uint32_t kCycle = (1u << (32 - kCountBits)) - 1u;
+    return (unsigned long long)id << (32 - kCountBits) | ((uint32_t)tag % kCycle + 1u);
+}
+
 __device__ __forceinline__ CommRec load_rec(const ExactState& a, uint32_t c) {
     const uint4 v = *reinterpret_cast<const uint4*>(a.rec + c);
     CommRec r;
@@ -216,16 +226,16 @@ __device__ __forceinline__ CommRec load_rec(const ExactState& a, uint32_t c) {
 // events in this table at all -- most candidates have none, and their total is
 // this one load (probing the hash for each cost a 16-byte read per candidate
 // more, and the total and the designated index one read each: uniform 2^23
-// took 225 us a round so) -- and where they are: a slot's time-sorted events,
-// binary-searched for the last before u, or a designated community's dense row.
+// took 225 us a round so) -- and where they are: a slot's few events, added up
+// where they lie before u; a slot's time-sorted events, the last before u found
+// by the hot index or by search; or a designated community's dense row.
 // The K chains advance in lockstep so their loads are in flight together.  The
 // record's generation is cut to its low bits, so what it points at is checked
-// against the full one.  valid[k] = false entries return 0.
+// against the slot's name.  valid[k] = false entries return 0.
 template <int K>
 __device__ __forceinline__ void sigma_at_k(const ExactState& a, unsigned long long tag, long long P, int par,
                                            const uint32_t (&c)[K], const bool (&valid)[K], const CommRec (&rec)[K],
                                            uint32_t u, long long (&out)[K]) {
-    uint32_t hot[K];
     int lo[K], l[K], r[K];
     int zd[K];
     SlotMeta sm[K];
@@ -244,35 +254,37 @@ __device__ __forceinline__ void sigma_at_k(const ExactState& a, unsigned long lo
 #pragma unroll
     for (int k = 0; k < K; ++k)
         if (slot[k]) sm[k] = a.slots[rec[k].slotw & (kTableSlots - 1)];
+    const uint32_t off = (uint32_t)((long long)u - P);
+    any = false;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         lo[k] = l[k] = r[k] = 0;
-        hot[k] = 0;
-        if (slot[k] && sm[k].tkey == (tag << 32 | c[k])) {
-            lo[k] = l[k] = sm[k].start;
-            r[k] = (int)(sm[k].endh & ((1u << kEndBits) - 1u));
-            hot[k] = sm[k].endh >> kEndBits;
-            if (hot[k] > (uint32_t)kHotMax) {   // never written by a finished table
-                a.ctl->error = 2;
-                hot[k] = 0;
+        if (slot[k] && sm[k].word >> kCountBits == slot_name(tag, c[k])) {
+            const int cnt = (int)(sm[k].word & ((1u << kCountBits) - 1u));
+            if (cnt <= kInline) {
+                const uint4* q = reinterpret_cast<const uint4*>(
+                    a.ev + (size_t)(rec[k].slotw & (kTableSlots - 1)) * kInline);
+#pragma unroll 1
+                for (int m = 0; m < cnt; m += 2) {
+                    const uint4 x = q[m >> 1];
+                    if (x.x < off) out[k] += (int32_t)x.y;
+                    if (m + 1 < cnt && x.z < off) out[k] += (int32_t)x.w;
+                }
+            } else {
+                lo[k] = sm[k].start;
+                if (sm[k].hot > (uint32_t)kHotMax) {   // never written by a finished table
+                    a.ctl->error = 2;
+                } else if (sm[k].hot) {
+                    const uint2 w = a.hot_row[(size_t)(sm[k].hot - 1) * kHotWords + (off >> 5)];
+                    l[k] = r[k] = lo[k] + (int)w.y + __popc(w.x & ((1u << (off & 31)) - 1u));
+                } else {
+                    l[k] = lo[k];
+                    r[k] = lo[k] + cnt;
+                    any = true;
+                }
             }
         }
         if (zd[k] >= 0 && (zd[k] >= (int)a.ctl->nz || a.ctl->zc[zd[k]] != c[k])) zd[k] = -1;
-    }
-    // Hot slots: narrow [l, r) to u's time bucket.
-    {
-        int bl[K], br[K];
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            if (hot[k]) {
-                const int32_t* bx = a.hot_bidx + (size_t)(hot[k] - 1) * kHotStride + (int)((u - P) / kBucketV);
-                bl[k] = bx[0];
-                br[k] = bx[1];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < K; ++k)
-            if (hot[k]) { l[k] = bl[k]; r[k] = br[k]; }
     }
     while (any) {
         uint32_t t[K];
@@ -295,13 +307,13 @@ __device__ __forceinline__ void sigma_at_k(const ExactState& a, unsigned long lo
     for (int k = 0; k < K; ++k)
         if (l[k] > lo[k]) out[k] += a.epre[l[k] - 1];
     // Designated communities: bucket prefix + the bucket's offsets before u.
-    const int off = (int)((long long)u - P), bk = off >> 4, rem = off & 15;
+    const int bk = (int)(off >> 4), rem = (int)(off & 15u);
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         if (zd[k] < 0) continue;
         const size_t row = (size_t)(par * kZMax + zd[k]);
         const int4* q = reinterpret_cast<const int4*>(a.zcontrib + row * kWindowMax + ((size_t)bk << 4));
-        long long sum = a.zpre[row * kHotStride + bk];
+        long long sum = a.zpre[row * kBucketStride + bk];
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
             const int4 v = q[m];
@@ -509,88 +521,112 @@ __device__ __forceinline__ void window_ranges(const ExactState& a, Ctl* c, long 
 // ---------------------------------------------------------------------------
 // Event table.  Each D_prev mover w of the window contributes two events at
 // time w: (old community, -deg w) and (new community, +deg w).  A lookup needs,
-// per community, its events in time order with inclusive prefix sums.  Built
-// in three kernels:
-//   insert: one thread per window vertex; movers insert both communities into
-//           the generation-tagged hash (no clearing between rounds) and count
-//           their events per coarse bucket (high slot bits) per chunk;
-//   group:  each chunk scatters its events, in time order, to its coarse
-//           buckets' ranges (a stable counting pass);
-//   finish: one CTA per coarse bucket sorts its events by the low slot bits
-//           (stable, so time order holds inside a slot) and runs the
-//           segmented prefix sum, filling each slot's event range.
+// per community, the sum of its events before a time: no order, unless there
+// are too many to read.  Built in two kernels:
+//   insert: one thread per window vertex; movers find both communities' slots
+//           in the generation-tagged hash (no clearing between rounds), take
+//           their events' numbers there by one add per slot and warp, and
+//           write the events to their places;
+//   sort:   slots with more than kInline events: a warp each up to kWarpSort,
+//           else a CTA, sorts them by time and prefix-sums them.
+// Chains of a few dependent L2 round trips, 65,536 threads of them, bound both.
+// (Grouping all events by slot first, stably, by a histogram, a scatter and a
+// sort per bucket of slots, took 37 us a round where this takes 10 on a grid and 13 on planted communities
+// of 300 K vertices.)
 // ---------------------------------------------------------------------------
-struct SegSum {
-    long long v;
-    int cnt;    // elements since the last segment start
-    int head;   // a segment starts inside this range
-};
-
-__device__ __forceinline__ SegSum seg_combine(SegSum a, SegSum b) {
-    return b.head ? b : SegSum{a.v + b.v, a.cnt + b.cnt, a.head};
-}
-
-__device__ __forceinline__ SegSum seg_shfl_up(SegSum x, int o) {
-    return SegSum{__shfl_up_sync(0xFFFFFFFFu, x.v, o), __shfl_up_sync(0xFFFFFFFFu, x.cnt, o),
-                  __shfl_up_sync(0xFFFFFFFFu, x.head, o)};
-}
-
-// Slot of community c in the generation-`tag` table, inserting it if absent;
-// the thread that inserts it notes the slot in the community's record.
-__device__ __forceinline__ uint32_t table_insert(const ExactState& a, unsigned long long tag, uint32_t c) {
-    SlotMeta* slots = a.slots;
-    const unsigned long long want = tag << 32 | c;
-    uint32_t h = slot_hash(c) & (kTableSlots - 1);
+// Slot of `name` in the table, claiming one if absent (`claimed`); h: where to
+// look first, cur: the word there.
+__device__ __forceinline__ uint32_t table_slot(const ExactState& a, unsigned long long name, uint32_t h,
+                                               unsigned long long cur, bool& claimed) {
+    constexpr unsigned long long kGen = (1ull << (32 - kCountBits)) - 1ull;
+    claimed = false;
     while (true) {
-        unsigned long long cur = ((volatile unsigned long long*)&slots[h].tkey)[0];
-        if (cur == want) return h;
-        if ((cur >> 32) != tag) {
-            const unsigned long long prev = atomicCAS(&slots[h].tkey, cur, want);
-            if (prev == cur) a.rec[c].slotw = (uint32_t)tag << kSlotwTagShift | h;
-            if (prev == cur || prev == want) return h;
-            continue;   // another community took the slot: look at it again
+        const unsigned long long at = cur >> kCountBits;
+        if (at == name) return h;
+        if ((at ^ name) & kGen) {   // of an older generation: free
+            const unsigned long long prev = atomicCAS(&a.slots[h].word, cur, name << kCountBits);
+            claimed = prev == cur;
+            if (claimed || prev >> kCountBits == name) return h;
+            cur = prev;             // another community took the slot
+        } else {
+            h = (h + 1) & (kTableSlots - 1);
+            cur = *(volatile unsigned long long*)&a.slots[h].word;
         }
-        h = (h + 1) & (kTableSlots - 1);
     }
 }
 
-// Window chunk `chunk` (blockDim.x consecutive window vertices).
-__device__ __forceinline__ void tb_insert_chunk(const ExactState& a, const Ctl* c, int chunk) {
-    __shared__ int32_t hist[kCoarse];
+__device__ __forceinline__ uint32_t home_slot(uint32_t id) { return slot_hash(id) & (kTableSlots - 1); }
+
+__device__ __forceinline__ uint32_t block_id(uint32_t slot, uint32_t number) {
+    return 0x80000000u | slot << kBlockBits | (number - kInline) / kInline;
+}
+
+// Numbers of a warp's events in their slots (kPadSlot: none): one add per slot.
+__device__ __forceinline__ uint32_t slot_number(const ExactState& a, uint32_t slot) {
+    const int lane = threadIdx.x & 31;
+    const unsigned peers = __match_any_sync(0xFFFFFFFFu, slot);
+    const int lead = __ffs(peers) - 1;
+    uint32_t first = 0;
+    if (slot != kPadSlot && lane == lead)
+        first = (uint32_t)atomicAdd(&a.slots[slot].word, (unsigned long long)__popc(peers)) & ((1u << kCountBits) - 1u);
+    first = __shfl_sync(0xFFFFFFFFu, first, lead);
+    return first + __popc(peers & ((1u << lane) - 1u));
+}
+
+__device__ __forceinline__ void put_event(const ExactState& a, unsigned long long tag, uint32_t slot, uint32_t number,
+                                          uint32_t off, int32_t sdeg) {
+    uint32_t at = slot;
+    if (number >= kInline) {
+        const uint32_t id = block_id(slot, number), h = home_slot(id);
+        bool claimed;
+        at = table_slot(a, slot_name(tag, id), h, *(volatile unsigned long long*)&a.slots[h].word, claimed);
+        if (number == kInline) a.many[0][atomicAdd(&a.ctl->nmany[0], 1u)] = slot;
+        if (number == kWarpSort) a.many[1][atomicAdd(&a.ctl->nmany[1], 1u)] = slot;
+    }
+    a.ev[(size_t)at * kInline + number % kInline] = make_uint2(off, (uint32_t)sdeg);
+}
+
+__global__ void __launch_bounds__(kTbThreads) k_tb_insert(ExactState a) {
+    const Ctl* c = a.ctl;
     const long long P = c->P, E = c->E;
+    if (P >= c->n) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->first_change = kNoChange;
     const Round r = round_view(a, c);
-    const int tid = threadIdx.x;
-    for (int b = tid; b < kCoarse; b += blockDim.x) hist[b] = 0;
-    __syncthreads();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int W = (int)(E - P);
-    const int i = chunk * blockDim.x + tid;
+    if ((i & ~31) >= W) return;   // whole warps
     const int nz = (int)c->nz;
     uint32_t z0 = 0, z1 = 0;   // designated index + 1 of the departure / arrival community
+    uint32_t s0 = kPadSlot, s1 = kPadSlot;
     int dg = 0;
     if (i < W) {
         const int64_t wv = P + i;
         const uint32_t pb = r.pdec[wv] & kNoMove, vc = a.vcom[wv];
         const int64_t r0 = a.rp[wv], r1 = a.rp[wv + 1];
-        uint32_t s0 = kPadSlot, s1 = kPadSlot;
         if (pb != kNoMove) {
             dg = (int)(r1 - r0);
+            const uint32_t h0 = home_slot(vc), h1 = home_slot(pb);
+            const unsigned long long w0 = *(volatile unsigned long long*)&a.slots[h0].word;
+            const unsigned long long w1 = *(volatile unsigned long long*)&a.slots[h1].word;
             if (nz) {
                 z0 = a.zof[vc];
                 z1 = a.zof[pb];
             }
+            // The thread that claims a slot notes it in the community's record.
+            bool claimed;
             if (!z0) {
-                s0 = table_insert(a, r.tag, vc);
-                atomicAdd(&hist[s0 >> kFineBits], 1);
+                s0 = table_slot(a, slot_name(r.tag, vc), h0, w0, claimed);
+                if (claimed) a.rec[vc].slotw = (uint32_t)r.tag << kSlotwTagShift | s0;
             }
             if (!z1) {
-                s1 = table_insert(a, r.tag, pb);
-                atomicAdd(&hist[s1 >> kFineBits], 1);
+                s1 = table_slot(a, slot_name(r.tag, pb), h1, w1, claimed);
+                if (claimed) a.rec[pb].slotw = (uint32_t)r.tag << kSlotwTagShift | s1;
             }
         }
-        a.tb_s0[i] = s0;
-        a.tb_s1[i] = s1;
-        a.wdeg[i] = dg;
     }
+    const uint32_t n0 = slot_number(a, s0), n1 = slot_number(a, s1);
+    if (s0 != kPadSlot) put_event(a, r.tag, s0, n0, (uint32_t)i, -dg);
+    if (s1 != kPadSlot) put_event(a, r.tag, s1, n1, (uint32_t)i, dg);
     // Dense rows: every window offset writes its signed degree for each
     // designated community (zero when it does not move into or out of it), and
     // each 16-offset bucket (a half-warp) its sum; warp-aggregated event counts.
@@ -601,424 +637,222 @@ __device__ __forceinline__ void tb_insert_chunk(const ExactState& a, const Ctl* 
         long long sum = v;
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-        if ((i & 15) == 0 && i < W) a.zbsum[row * kHotStride + (i >> 4)] = sum;
+        if ((i & 15) == 0 && i < W) a.zbsum[row * kBucketStride + (i >> 4)] = sum;
         const int evs = __popc(__ballot_sync(0xFFFFFFFFu, z0 == (uint32_t)j + 1)) +
                         __popc(__ballot_sync(0xFFFFFFFFu, z1 == (uint32_t)j + 1));
-        if ((tid & 31) == 0 && evs) atomicAdd(&a.ctl->zcount[j], (unsigned)evs);
+        if ((i & 31) == 0 && evs) atomicAdd(&a.ctl->zcount[j], (unsigned)evs);
     }
-    __syncthreads();
-    for (int b = tid; b < kCoarse; b += blockDim.x) a.tb_hist[b * kTbChunks + chunk] = hist[b];
-    __syncthreads();   // hist is reused by the CTA's next chunk
 }
 
-// Run by the last insert CTA of a round (chunks = the insert grid): exclusive
-// prefix of the (bucket, chunk) counts in bucket-major order -- the offset of
-// each chunk's events inside the grouped array -- plus the bucket starts and
-// the largest bucket.  Once per round instead of once per grouping CTA.  Warp
-// w owns buckets [w * kPerWarp, (w + 1) * kPerWarp); lane l holds chunks l and
-// l + 32 of each; all loads are issued before the scans.
-constexpr int kScanPerWarp = kCoarse / (kTbThreads / 32);
-static_assert(kCoarse % (kTbThreads / 32) == 0, "buckets split evenly over the insert CTA's warps");
-static_assert(kWindowMax / kTbThreads <= 64, "two insert chunks per lane");
-
-__device__ __forceinline__ void tb_scan_hist(const ExactState& a, int chunks) {
-    __shared__ int32_t bstart[kCoarse];
-    __shared__ int32_t wsum[32];
-    __shared__ unsigned long long wbig[32];
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    int v0[kScanPerWarp], v1[kScanPerWarp];
-#pragma unroll
-    for (int k = 0; k < kScanPerWarp; ++k) {
-        const int32_t* h = a.tb_hist + (size_t)(w * kScanPerWarp + k) * kTbChunks;
-        v0[k] = lane < chunks ? h[lane] : 0;
-        v1[k] = lane + 32 < chunks ? h[lane + 32] : 0;
-    }
-#pragma unroll
-    for (int k = 0; k < kScanPerWarp; ++k) {
-        int x0 = v0[k], x1 = v1[k];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y0 = __shfl_up_sync(0xFFFFFFFFu, x0, o), y1 = __shfl_up_sync(0xFFFFFFFFu, x1, o);
-            if (lane >= o) { x0 += y0; x1 += y1; }
+// Event `number` of a slot of the finished table.
+__device__ __forceinline__ uint2 get_event(const ExactState& a, unsigned long long tag, uint32_t slot,
+                                           uint32_t number) {
+    uint32_t at = slot;
+    if (number >= kInline) {
+        const uint32_t id = block_id(slot, number);
+        const unsigned long long name = slot_name(tag, id);
+        at = home_slot(id);
+        int steps = 0;
+        while (a.slots[at].word >> kCountBits != name && steps < kTableSlots) {
+            at = (at + 1) & (kTableSlots - 1);
+            ++steps;
         }
-        const int t0 = __shfl_sync(0xFFFFFFFFu, x0, 31), t1 = __shfl_sync(0xFFFFFFFFu, x1, 31);
-        v0[k] = x0 - v0[k];          // exclusive, inside the bucket
-        v1[k] = t0 + x1 - v1[k];
-        if (lane == 0) bstart[w * kScanPerWarp + k] = t0 + t1;   // bucket total for now
+        if (steps == kTableSlots) a.ctl->error = 2;   // never in a finished table
     }
-    __syncthreads();
-    // Exclusive scan of the bucket totals (kCoarse <= threads) and the largest bucket.
-    int tot = tid < kCoarse ? bstart[tid] : 0;
-    int incl = tot;
+    uint2 e = a.ev[(size_t)at * kInline + number % kInline];
+    e.x &= kWindowMax - 1;
+    return e;
+}
+
+template <typename T>
+__device__ __forceinline__ T warp_incl(T v) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += y;
+        const T y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if (lane >= o) v += y;
     }
-    unsigned long long big = tot ? ((unsigned long long)tot << 32) | (unsigned long long)tid : 0ull;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) big = max(big, __shfl_xor_sync(0xFFFFFFFFu, big, o));
-    if (lane == 31) wsum[w] = incl;
-    if (lane == 0) wbig[w] = big;
-    __syncthreads();
-    if (w == 0) {
-        const int v = wsum[lane];
-        int vi = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xFFFFFFFFu, vi, o);
-            if (lane >= o) vi += y;
-        }
-        wsum[lane] = vi - v;
-        unsigned long long bb = wbig[lane];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) bb = max(bb, __shfl_xor_sync(0xFFFFFFFFu, bb, o));
-        if (lane == 0) {
-            a.ctl->tb_big = bb;
-            a.ctl->tb_ticket = 0;
-        }
-    }
-    __syncthreads();
-    if (tid < kCoarse) {
-        const int excl = wsum[w] + incl - tot;
-        bstart[tid] = excl;
-        a.tb_bstart[tid] = excl;
-        if (tid == kCoarse - 1) a.tb_bstart[kCoarse] = excl + tot;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kScanPerWarp; ++k) {
-        const int b = w * kScanPerWarp + k;
-        int32_t* o = a.tb_base + (size_t)b * kTbChunks;
-        if (lane < chunks) o[lane] = bstart[b] + v0[k];
-        if (lane + 32 < chunks) o[lane + 32] = bstart[b] + v1[k];
-    }
+    return v;
 }
 
-__global__ void __launch_bounds__(kTbThreads) k_tb_insert(ExactState a) {
-    if (a.ctl->P >= a.ctl->n) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        a.ctl->first_change = kNoChange;
-        a.ctl->nhot = 0;
-    }
-    tb_insert_chunk(a, a.ctl, blockIdx.x);
-    // The last CTA to finish scans every CTA's histogram.
-    __shared__ bool s_last;
-    __threadfence();
+// Exclusive prefix of the CTA's values by thread; every thread calls.
+__device__ __forceinline__ long long cta_excl(long long v, long long* warp_sum) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long long incl = warp_incl(v);
     __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&a.ctl->tb_ticket, 1u) == gridDim.x - 1;
+    if (lane == 31) warp_sum[w] = incl;
     __syncthreads();
-    if (s_last) {
-        __threadfence();
-        tb_scan_hist(a, (int)gridDim.x);
-    }
+    long long before = 0;
+    for (int k = 0; k < w; ++k) before += warp_sum[k];
+    return before + incl - v;
 }
 
-// Stable scatter of each chunk's events to their coarse buckets.  Warp w of a
-// chunk owns its 32 consecutive vertices, i.e. 64 consecutive events.
-__device__ __forceinline__ void tb_group_chunk(const ExactState& a, const Ctl* c, int chunk, int chunks) {
-    __shared__ int32_t base[kCoarse];
-    extern __shared__ int32_t wcnt[];   // warps x kCoarse
-    const long long P = c->P, E = c->E;
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int nwarps = blockDim.x >> 5;
-    const int W = (int)(E - P);
-    (void)chunks;
-    // This chunk's offset inside each bucket (scanned by the last insert CTA).
-    for (int b = tid; b < kCoarse; b += blockDim.x) base[b] = a.tb_base[b * kTbChunks + chunk];
-    for (int k = tid; k < nwarps * kCoarse; k += blockDim.x) wcnt[k] = 0;
-    __syncthreads();
-    // Count per warp, then turn counts into per-warp offsets (exclusive over warps).
-    const int v0 = chunk * (int)blockDim.x + w * 32;   // first window offset of this warp
-    uint32_t sl[2];
+// Up to kWarpSort events of a slot by one warp: each lane counts the events
+// before its two.
+__device__ __forceinline__ void sort_slot_warp(const ExactState& a, const Round& r, uint32_t slot, int cnt,
+                                               uint2* buf) {
+    const int lane = threadIdx.x & 31;
+    uint2 e[2];
+    int pos[2] = {0, 0};
 #pragma unroll
-    for (int st = 0; st < 2; ++st) {
-        const int e = 2 * v0 + st * 32 + lane;    // event index (time order)
-        const int i = e >> 1;
-        sl[st] = i < W ? ((e & 1) ? a.tb_s1[i] : a.tb_s0[i]) : kPadSlot;
-        const int b = sl[st] == kPadSlot ? kCoarse : (int)(sl[st] >> kFineBits);
-        const unsigned peers = __match_any_sync(0xFFFFFFFFu, b);
-        if (b < kCoarse && lane == __ffs(peers) - 1) wcnt[w * kCoarse + b] += __popc(peers);
-        __syncwarp();
+    for (int k = 0; k < 2; ++k)
+        e[k] = lane + 32 * k < cnt ? get_event(a, r.tag, slot, lane + 32 * k) : make_uint2(0xFFFFFFFFu, 0u);
+    int start = 0;
+    if (lane == 0) start = (int)atomicAdd(&a.ctl->sorted, (unsigned)cnt);
+    start = __shfl_sync(0xFFFFFFFFu, start, 0);
+#pragma unroll 8
+    for (int j = 0; j < 32; ++j) {
+        const uint32_t x = __shfl_sync(0xFFFFFFFFu, e[0].x, j), y = __shfl_sync(0xFFFFFFFFu, e[1].x, j);
+        pos[0] += (x < e[0].x) + (y < e[0].x);
+        pos[1] += (x < e[1].x) + (y < e[1].x);
     }
-    __syncthreads();
-    for (int b = tid; b < kCoarse; b += blockDim.x) {
-        int acc = base[b];
-        for (int ww = 0; ww < nwarps; ++ww) {
-            const int t = wcnt[ww * kCoarse + b];
-            wcnt[ww * kCoarse + b] = acc;
-            acc += t;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        if (lane + 32 * k < cnt) buf[pos[k]] = e[k];   // a vertex is in a slot once
+    __syncwarp();
+    long long before = 0;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int i = lane + 32 * k;
+        const uint2 x = i < cnt ? buf[i] : make_uint2(0u, 0u);
+        const long long incl = before + warp_incl((long long)(int32_t)x.y);
+        if (i < cnt) {
+            a.stime[start + i] = (uint32_t)(r.P + x.x);
+            a.epre[start + i] = incl;
+        }
+        before = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    }
+    if (lane == 0) {
+        a.slots[slot].start = start;
+        a.slots[slot].hot = 0;
+    }
+    __syncwarp();
+}
+
+// Any number of events of a slot by one CTA: offsets with an event set their
+// bit, and an event's place is the bits before its own.
+__device__ __forceinline__ void sort_slot_cta(const ExactState& a, const Round& r, int words, uint32_t slot, int cnt,
+                                              uint32_t* bits, uint32_t* before, long long* warp_sum) {
+    __shared__ int s_start;
+    __shared__ uint32_t s_hot;
+    const int tid = threadIdx.x;
+    constexpr int kPer = kHotWords / kSortThreads;
+    for (int k = tid; k < words; k += kSortThreads) bits[k] = 0;
+    if (tid == 0) {
+        s_start = (int)atomicAdd(&a.ctl->sorted, (unsigned)cnt);
+        s_hot = 0;
+        if (cnt >= kHotMin) {
+            const unsigned id = atomicAdd(&a.ctl->nhot, 1u);
+            if (id < (unsigned)kHotMax) s_hot = id + 1;
+            if (id < (unsigned)kZCand)
+                a.zcand[id] = (unsigned long long)cnt << 32 | (uint32_t)(a.slots[slot].word >> 32);
         }
     }
     __syncthreads();
-#pragma unroll
-    for (int st = 0; st < 2; ++st) {
-        const int e = 2 * v0 + st * 32 + lane;
-        const int b = sl[st] == kPadSlot ? kCoarse : (int)(sl[st] >> kFineBits);
-        const unsigned peers = __match_any_sync(0xFFFFFFFFu, b);
-        int pos = 0;
-        if (b < kCoarse) pos = wcnt[w * kCoarse + b] + __popc(peers & ((1u << lane) - 1u));
-        __syncwarp();
-        if (b < kCoarse) {
-            a.ev1[pos] = (unsigned long long)sl[st] << 32 | (unsigned)e;
-            if (lane == __ffs(peers) - 1) wcnt[w * kCoarse + b] += __popc(peers);
-        }
-        __syncwarp();
+#pragma unroll 4
+    for (int k = tid; k < cnt; k += kSortThreads) {
+        const uint32_t off = get_event(a, r.tag, slot, k).x;
+        atomicOr(&bits[off >> 5], 1u << (off & 31));
     }
-    __syncthreads();   // shared arrays are reused by the CTA's next chunk
+    __syncthreads();
+    uint32_t own = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+        if (tid * kPer + k < words) own += __popc(bits[tid * kPer + k]);
+    uint32_t run = (uint32_t)cta_excl(own, warp_sum);
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+        if (tid * kPer + k < words) {
+            before[tid * kPer + k] = run;
+            run += __popc(bits[tid * kPer + k]);
+        }
+    __syncthreads();
+    const int start = s_start;
+    const uint32_t hot = s_hot;
+#pragma unroll 4
+    for (int k = tid; k < cnt; k += kSortThreads) {
+        const uint2 e = get_event(a, r.tag, slot, k);
+        const int at = start + (int)before[e.x >> 5] + __popc(bits[e.x >> 5] & ((1u << (e.x & 31)) - 1u));
+        a.stime[at] = (uint32_t)(r.P + e.x);
+        a.sdeg[at] = (int32_t)e.y;
+    }
+    if (hot)
+        for (int k = tid; k < words; k += kSortThreads)
+            a.hot_row[(size_t)(hot - 1) * kHotWords + k] = make_uint2(bits[k], before[k]);
+    if (tid == 0) {
+        a.slots[slot].start = start;
+        a.slots[slot].hot = hot;
+    }
+    __syncthreads();
+    long long carry = 0;
+    for (int k0 = 0; k0 < cnt; k0 += 4 * kSortThreads) {
+        int v[4];
+        long long sum = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int k = k0 + 4 * tid + j;
+            v[j] = k < cnt ? a.sdeg[start + k] : 0;
+            sum += v[j];
+        }
+        const long long ex = cta_excl(sum, warp_sum);
+        long long x = carry + ex;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int k = k0 + 4 * tid + j;
+            x += v[j];
+            if (k < cnt) a.epre[start + k] = x;
+        }
+        for (int k = 0; k < kSortThreads / 32; ++k) carry += warp_sum[k];
+    }
+    __syncthreads();
 }
 
-__global__ void __launch_bounds__(kTbThreads) k_tb_group(ExactState a) {
-    if (a.ctl->P >= a.ctl->n) return;
-    tb_group_chunk(a, a.ctl, blockIdx.x, gridDim.x);
-}
-
-// One CTA per coarse bucket: stable pass on the fine slot bits, then the
-// segmented inclusive scan of signed degrees; writes times, prefixes and the
-// slots' event ranges.
-// Coarse bucket number `vb` (after swapping the largest bucket to 0); the
-// CTA has at least kFine threads.
-__device__ __forceinline__ void tb_finish_bucket(const ExactState& a, const Ctl* c, int vb) {
-    constexpr int kFine = 1 << kFineBits;
-    constexpr int kRow = kFine + 1;          // padded row of per-warp digit counts
-    extern __shared__ int32_t wcnt[];   // warps x kRow per-warp digit counts (dynamic: > 48 KB)
-    __shared__ int32_t digit[kFine];
-    __shared__ long long warp_v[32];
-    __shared__ int warp_h[32];
-    const long long P = c->P;
-    if (vb >= kCoarse) {
-        // Designated community j = vb - kCoarse: exclusive prefix of its
-        // bucket sums (one extra entry holds the total).
-        const int j = vb - kCoarse;
+// Grid: kZMax designated-community prefixes, then kSortCtas over the slots with
+// many events.
+__global__ void __launch_bounds__(kSortThreads) k_tb_sort(ExactState a) {
+    __shared__ uint32_t bits[kHotWords], before[kHotWords];
+    __shared__ uint2 buf[kSortThreads / 32][kWarpSort];
+    __shared__ long long warp_sum[kSortThreads / 32];
+    static_assert(kHotWords % kSortThreads == 0, "bitmap words split evenly");
+    const Ctl* c = a.ctl;
+    if (c->P >= c->n) return;
+    const Round r = round_view(a, c);
+    const int tid = threadIdx.x, w = tid >> 5;
+    if (blockIdx.x < kZMax) {
+        // Designated community j: exclusive prefix of its bucket sums (one
+        // extra entry holds the total).
+        const int j = blockIdx.x;
         if (j >= (int)c->nz) return;
-        const int nbk = (int)((c->E - P + kBucketV - 1) / kBucketV);
-        const size_t row = ((size_t)(c->round & 1) * kZMax + j) * kHotStride;
-        const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nwarps = blockDim.x >> 5;
-        const int per = (nbk + blockDim.x - 1) / blockDim.x;
-        const int b0 = min(nbk, tid * per), b1 = min(nbk, b0 + per);
-        long long own = 0;
-        for (int b = b0; b < b1; ++b) own += a.zbsum[row + b];
-        long long inc = own;
-        for (int o = 1; o < 32; o <<= 1) {
-            const long long y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-            if (lane >= o) inc += y;
+        const int nbk = (int)((r.E - r.P + kBucketV - 1) / kBucketV);
+        const size_t row = ((size_t)r.par * kZMax + j) * kBucketStride;
+        constexpr int kPer = kWindowMax / kBucketV / kSortThreads;
+        long long v[kPer], own = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            v[k] = tid * kPer + k < nbk ? a.zbsum[row + tid * kPer + k] : 0;
+            own += v[k];
         }
-        if (lane == 31) warp_v[w] = inc;
-        __syncthreads();
-        if (w == 0) {
-            const long long x = lane < nwarps ? warp_v[lane] : 0;
-            long long xi = x;
-            for (int o = 1; o < 32; o <<= 1) {
-                const long long y = __shfl_up_sync(0xFFFFFFFFu, xi, o);
-                if (lane >= o) xi += y;
-            }
-            if (lane < nwarps) warp_v[lane] = xi - x;
+        long long run = cta_excl(own, warp_sum);
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            if (tid * kPer + k < nbk) a.zpre[row + tid * kPer + k] = run;
+            run += v[k];
         }
-        __syncthreads();
-        long long run = warp_v[w] + inc - own;
-        for (int b = b0; b < b1; ++b) {
-            a.zpre[row + b] = run;
-            run += a.zbsum[row + b];
-        }
-        if (tid == (int)blockDim.x - 1) a.zpre[row + nbk] = run;
-        __syncthreads();
+        if (tid == kSortThreads - 1) a.zpre[row + nbk] = run;
         return;
     }
-    // The largest bucket (the one holding a community many window vertices
-    // join) goes first (CTA 0 / virtual bucket 0).
-    const int big = (int)(a.ctl->tb_big & 0xFFFFFFFFull);
-    const int bucket = vb == 0 ? big : (vb == big ? 0 : vb);
-    const int bs = a.tb_bstart[bucket], be = a.tb_bstart[bucket + 1];
-    const int cnt = be - bs;
-    if (cnt == 0) return;
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int nwarps = blockDim.x >> 5;
-    static_assert(kFine % 32 == 0 && kFine <= kTbMinChunk && kFine <= kTbFinishThreads,
-                  "digit scan layout: one thread per fine digit");
-    for (int k = tid; k < nwarps * kRow; k += blockDim.x) wcnt[k] = 0;
-    __syncthreads();
-    // Stable pass on the fine slot bits: warp w owns a contiguous range; the
-    // next 32 keys are loaded while the current ones are ranked.
-    const int chunk = (cnt + nwarps - 1) / nwarps;
-    const int c0 = bs + min(cnt, w * chunk), c1 = bs + min(cnt, (w + 1) * chunk);
-    {
-        unsigned long long nxt = c0 + lane < c1 ? a.ev1[c0 + lane] : 0ull;
-        for (int base = c0; base < c1; base += 32) {
-            const int idx = base + lane;
-            const unsigned long long key = nxt;
-            if (base + 32 + lane < c1) nxt = a.ev1[base + 32 + lane];
-            const int d = idx < c1 ? (int)((key >> 32) & (kFine - 1)) : kFine;
-            const unsigned peers = __match_any_sync(0xFFFFFFFFu, d);
-            if (d < kFine && lane == __ffs(peers) - 1) wcnt[w * kRow + d] += __popc(peers);
-            __syncwarp();
-        }
+    const int words = (int)((r.E - r.P + 31) / 32);
+    const unsigned n1 = c->nmany[1], n0 = c->nmany[0];
+    const unsigned cta = blockIdx.x - kZMax, ctas = gridDim.x - kZMax;
+    for (unsigned q = cta; q < n1; q += ctas) {
+        const uint32_t slot = a.many[1][q];
+        sort_slot_cta(a, r, words, slot, (int)(a.slots[slot].word & ((1u << kCountBits) - 1u)), bits, before, warp_sum);
     }
-    __syncthreads();
-    if (tid < kFine) {
-        int acc = 0;
-        for (int ww = 0; ww < nwarps; ++ww) {
-            const int t = wcnt[ww * kRow + tid];
-            wcnt[ww * kRow + tid] = acc;
-            acc += t;
-        }
-        digit[tid] = acc;
+    for (unsigned q = w * ctas + cta; q < n0; q += ctas * (kSortThreads / 32)) {
+        const uint32_t slot = a.many[0][q];
+        const int cnt = (int)(a.slots[slot].word & ((1u << kCountBits) - 1u));
+        if (cnt <= kWarpSort) sort_slot_warp(a, r, slot, cnt, buf[w]);
     }
-    __syncthreads();
-    if (w == 0) {
-        constexpr int kPer = kFine / 32;
-        int v[kPer], t = 0;
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) { v[k] = digit[lane * kPer + k]; t += v[k]; }
-        int incl = t;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        int run = incl - t;
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) { digit[lane * kPer + k] = run; run += v[k]; }
-    }
-    __syncthreads();
-    {
-        unsigned long long nxt = c0 + lane < c1 ? a.ev1[c0 + lane] : 0ull;
-        for (int base = c0; base < c1; base += 32) {
-            const int idx = base + lane;
-            const unsigned long long key = nxt;
-            if (base + 32 + lane < c1) nxt = a.ev1[base + 32 + lane];
-            const int d = idx < c1 ? (int)((key >> 32) & (kFine - 1)) : kFine;
-            const unsigned peers = __match_any_sync(0xFFFFFFFFu, d);
-            int before = 0;
-            if (d < kFine) before = wcnt[w * kRow + d];
-            __syncwarp();
-            if (d < kFine) a.ev2[bs + digit[d] + before + __popc(peers & ((1u << lane) - 1u))] = key;
-            if (d < kFine && lane == __ffs(peers) - 1) wcnt[w * kRow + d] = before + __popc(peers);
-            __syncwarp();
-        }
-    }
-    __syncthreads();
-    // Segmented inclusive scan over ev2[bs, be), each thread a contiguous
-    // range read eight events at a time (keys, then degrees, in flight
-    // together).  The tail of each slot knows the slot's length from the scan
-    // and marks it hot.
-    __shared__ int s_cnt_w[32];
-    const int per = (cnt + blockDim.x - 1) / blockDim.x;
-    const int b0 = bs + min(cnt, tid * per), b1 = bs + min(cnt, tid * per + per);
-    SegSum own{0, 0, 0};
-    {
-        uint32_t psl = b0 > bs ? (uint32_t)(a.ev2[b0 - 1] >> 32) : kPadSlot;
-        for (int k0 = b0; k0 < b1; k0 += 8) {
-            unsigned long long key[8];
-            int32_t dg[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) key[j] = k0 + j < b1 ? a.ev2[k0 + j] : 0ull;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) dg[j] = k0 + j < b1 ? a.wdeg[(uint32_t)key[j] >> 1] : 0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (k0 + j >= b1) break;
-                const uint32_t sl = (uint32_t)(key[j] >> 32), e = (uint32_t)key[j];
-                const long long v = (e & 1) ? dg[j] : -(long long)dg[j];
-                own = seg_combine(own, SegSum{v, 1, sl != psl});
-                psl = sl;
-            }
-        }
-    }
-    SegSum inc = own;
-    for (int o = 1; o < 32; o <<= 1) {
-        const SegSum y = seg_shfl_up(inc, o);
-        if (lane >= o) inc = seg_combine(y, inc);
-    }
-    if (lane == 31) { warp_v[w] = inc.v; s_cnt_w[w] = inc.cnt; warp_h[w] = inc.head; }
-    __syncthreads();
-    if (w == 0) {
-        const SegSum x = lane < nwarps ? SegSum{warp_v[lane], s_cnt_w[lane], warp_h[lane]} : SegSum{0, 0, 0};
-        SegSum xi = x;
-        for (int o = 1; o < 32; o <<= 1) {
-            const SegSum y = seg_shfl_up(xi, o);
-            if (lane >= o) xi = seg_combine(y, xi);
-        }
-        SegSum ex = seg_shfl_up(xi, 1);
-        if (lane == 0) ex = SegSum{0, 0, 0};
-        if (lane < nwarps) { warp_v[lane] = ex.v; s_cnt_w[lane] = ex.cnt; warp_h[lane] = ex.head; }
-    }
-    __syncthreads();
-    SegSum ex_thread = seg_shfl_up(inc, 1);
-    if (lane == 0) ex_thread = SegSum{0, 0, 0};
-    const SegSum carry = seg_combine(SegSum{warp_v[w], s_cnt_w[w], warp_h[w]}, ex_thread);
-    {
-        long long run = carry.v;
-        int runc = carry.cnt;
-        uint32_t psl = b0 > bs ? (uint32_t)(a.ev2[b0 - 1] >> 32) : kPadSlot;
-        for (int k0 = b0; k0 < b1; k0 += 8) {
-            unsigned long long key[9];
-            int32_t dg[8];
-#pragma unroll
-            for (int j = 0; j < 9; ++j) key[j] = k0 + j < be ? a.ev2[k0 + j] : ~0ull;   // one past for the tail test
-#pragma unroll
-            for (int j = 0; j < 8; ++j) dg[j] = k0 + j < b1 ? a.wdeg[(uint32_t)key[j] >> 1] : 0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int k = k0 + j;
-                if (k >= b1) break;
-                const uint32_t sl = (uint32_t)(key[j] >> 32), e = (uint32_t)key[j];
-                const long long v = (e & 1) ? dg[j] : -(long long)dg[j];
-                const bool head = sl != psl;
-                run = head ? v : run + v;
-                runc = head ? 1 : runc + 1;
-                psl = sl;
-                a.stime[k] = (uint32_t)(P + (e >> 1));
-                a.epre[k] = run;
-                if (head) a.slots[sl].start = k;
-                if (k == be - 1 || (uint32_t)(key[j + 1] >> 32) != sl) {
-                    uint32_t endh = (uint32_t)(k + 1);
-                    if (runc >= kHotMin) {
-                        const unsigned id = atomicAdd(&a.ctl->nhot, 1u);
-                        if (id < (unsigned)kHotMax) endh |= (id + 1) << kEndBits;
-                        if (id < (unsigned)kZCand)
-                            a.zcand[id] = (unsigned long long)runc << 32 | (uint32_t)a.slots[sl].tkey;
-                    }
-                    a.slots[sl].endh = endh;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    // Hot slots: their time-bucket starts (bidx[b] = first event at a time
-    // >= P + kBucketV * b).
-    const int nb = (int)((c->E - P + kBucketV - 1) / kBucketV);
-    for (int k0 = b0; k0 < b1; k0 += 8) {
-        unsigned long long key[8];
-        uint32_t eh[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) key[j] = k0 + j < b1 ? a.ev2[k0 + j] : 0ull;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) eh[j] = k0 + j < b1 ? a.slots[(uint32_t)(key[j] >> 32)].endh : 0u;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int k = k0 + j;
-            const uint32_t hid = eh[j] >> kEndBits;
-            if (k >= b1 || !hid) continue;
-            if (hid > (uint32_t)kHotMax) {   // never written by a finished table
-                a.ctl->error = 2;
-                continue;
-            }
-            const uint32_t sl = (uint32_t)(key[j] >> 32), e = (uint32_t)key[j];
-            const int end = (int)(eh[j] & ((1u << kEndBits) - 1u));
-            int32_t* bx = a.hot_bidx + (size_t)(hid - 1) * kHotStride;
-            const int bk = (int)(e >> 1) / kBucketV;
-            const int bprev = k == a.slots[sl].start ? -1 : (int)((uint32_t)a.ev2[k - 1] >> 1) / kBucketV;
-            for (int b = bprev + 1; b <= bk; ++b) bx[b] = k;
-            if (k == end - 1)
-                for (int b = bk + 1; b <= nb; ++b) bx[b] = end;
-        }
-    }
-    __syncthreads();   // shared arrays are reused by the CTA's next bucket
-}
-
-// Grid: kCoarse buckets + kZMax designated-community prefixes.
-__global__ void __launch_bounds__(kTbFinishThreads) k_tb_finish(ExactState a) {
-    if (a.ctl->P >= a.ctl->n) return;
-    tb_finish_bucket(a, a.ctl, blockIdx.x);
 }
 
 constexpr int kMidWarpsPerBlock = 4;
@@ -1817,9 +1651,9 @@ __device__ __forceinline__ void commit_hub_body(const ExactState& a, const Ctl* 
 __global__ void __launch_bounds__(kHubThreads2) k_ex_commit_hub(ExactState a) { commit_hub_body(a, a.ctl); }
 
 // Re-choose the designated communities of the next table from the counts of
-// the table just used: the designated ones' event counts and the sorted
-// table's hot slots, largest first, at least kZKeep events each.  Keeps the
-// set when nothing in the sorted table was hot and every member kept its
+// the table just used: the designated ones' event counts and the table's
+// hot slots, largest first, at least kZKeep events each.  Keeps the
+// set when nothing in the table was hot and every member kept its
 // events.  Called by every thread of one CTA.
 __device__ __forceinline__ void designate(const ExactState& a, Ctl* c) {
     __shared__ unsigned long long cand[kZMax + kZCand];
@@ -1923,8 +1757,11 @@ __device__ __forceinline__ void advance_ctl(const ExactState& a, Ctl* c, long lo
     window_ranges(a, c, nP, nE);
     // Designated communities: their records point the next table's lookups at
     // the dense rows, and count as changed -- the old set's too, which a
-    // change of the set moves between the dense rows and the sorted table.
+    // change of the set moves between the dense rows and the table.
     const uint32_t ntag = (uint32_t)c->tag + 1u;
+    // This round's table is done with.
+    if (threadIdx.x < kClearSlots)
+        a.slots[((uint32_t)c->tag * kClearSlots + threadIdx.x) & (kTableSlots - 1)].word = 0;
     if (threadIdx.x < c->nz) a.rec[c->zc[threadIdx.x]].cver = ntag;
     designate(a, c);
     if (threadIdx.x < c->nz) {
@@ -1942,6 +1779,7 @@ __device__ __forceinline__ void advance_ctl(const ExactState& a, Ctl* c, long lo
         c->E = nE;
         c->round = rnd;
         c->tag = c->tag + 1;
+        c->nmany[0] = c->nmany[1] = c->sorted = c->nhot = 0;
         // Every round commits at least vertex P, so the loop ends within n
         // rounds; the bound only guards against a broken invariant.
         bool more = nP < n;
@@ -1975,6 +1813,7 @@ __device__ __forceinline__ void init_ctl(const ExactState& a, Ctl* c, long long 
         c->cX = 0;
         c->pE = 0;
         c->tag = c->tag + 1;
+        c->nmany[0] = c->nmany[1] = c->sorted = c->nhot = 0;
         for (int j = 0; j < kZMax; ++j) c->zcount[j] = 0;
     }
     __syncthreads();
@@ -2154,17 +1993,15 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     GB_LAUNCH_CHECK();
     DevBuf<uint8_t> mv(n, s);
     DevBuf<SlotMeta> slots(kTableSlots, s);
-    GB_CUDA(cudaMemsetAsync(slots, 0xFF, kTableSlots * sizeof(SlotMeta), s));   // no generation yet
-    DevBuf<uint32_t> stime(kEventsMax, s), tb_s0(kWindowMax, s), tb_s1(kWindowMax, s);
+    GB_CUDA(cudaMemsetAsync(slots, 0, kTableSlots * sizeof(SlotMeta), s));   // no generation yet
+    DevBuf<uint2> ev((size_t)kTableSlots * kInline, s), hot_row((size_t)kHotMax * kHotWords, s);
+    DevBuf<uint32_t> many0(kEventsMax / kInline, s), many1(kEventsMax / kWarpSort, s), stime(kEventsMax, s);
     DevBuf<long long> epre(kEventsMax, s);
-    DevBuf<int32_t> wdeg(kWindowMax, s), tb_hist(kCoarse * kTbChunks, s), tb_base(kCoarse * kTbChunks, s),
-        tb_bstart(kCoarse + 1, s);
-    DevBuf<unsigned long long> ev1(kEventsMax, s), ev2(kEventsMax, s);
-    DevBuf<int32_t> hot_bidx((size_t)kHotMax * kHotStride, s);
+    DevBuf<int32_t> sdeg(kEventsMax, s);
     DevBuf<uint8_t> zof(n > 0 ? n : 1, s);
     GB_CUDA(cudaMemsetAsync(zof, 0, (n > 0 ? n : 1), s));
     DevBuf<int32_t> zcontrib((size_t)2 * kZMax * kWindowMax, s);
-    DevBuf<long long> zbsum((size_t)2 * kZMax * kHotStride, s), zpre((size_t)2 * kZMax * kHotStride, s);
+    DevBuf<long long> zbsum((size_t)2 * kZMax * kBucketStride, s), zpre((size_t)2 * kZMax * kBucketStride, s);
     DevBuf<unsigned long long> zcand(kZCand, s);
     DevBuf<Ctl> ctl(1, s);
     Ctl* hctl = nullptr;
@@ -2191,15 +2028,11 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     a.delta = delta.get();
     a.final_delta = final_delta.get();
     a.slots = slots.get();
-    a.tb_s0 = tb_s0.get();
-    a.tb_s1 = tb_s1.get();
-    a.wdeg = wdeg.get();
-    a.tb_hist = tb_hist.get();
-    a.tb_base = tb_base.get();
-    a.tb_bstart = tb_bstart.get();
-    a.ev1 = ev1.get();
-    a.ev2 = ev2.get();
-    a.hot_bidx = hot_bidx.get();
+    a.ev = ev.get();
+    a.many[0] = many0.get();
+    a.many[1] = many1.get();
+    a.sdeg = sdeg.get();
+    a.hot_row = hot_row.get();
     a.zof = zof.get();
     a.zcontrib = zcontrib.get();
     a.zbsum = zbsum.get();
@@ -2236,16 +2069,10 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     a.R = ctx.R;
     a.dq = ctx.dq;
 
-    static_assert(kEventsMax + 32 * 257 <= kTableSlots + kEventsMax, "sort scratch fits the hash area");
-    const int group_smem = 32 * kCoarse * (int)sizeof(int32_t);
-    GB_CUDA(cudaFuncSetAttribute(k_tb_group, cudaFuncAttributeMaxDynamicSharedMemorySize, group_smem));
     const int tb_grid = (int)ceil_div(B, kTbThreads);
-    const int finish_smem = (kTbFinishThreads / 32) * ((1 << kFineBits) + 1) * (int)sizeof(int32_t);
-    GB_CUDA(cudaFuncSetAttribute(k_tb_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, finish_smem));
     auto enqueue_table = [&](cudaStream_t st) {
         k_tb_insert<<<tb_grid, kTbThreads, 0, st>>>(a);
-        k_tb_group<<<tb_grid, kTbThreads, group_smem, st>>>(a);
-        k_tb_finish<<<kCoarse + kZMax, kTbFinishThreads, finish_smem, st>>>(a);
+        k_tb_sort<<<kZMax + kSortCtas, kSortThreads, 0, st>>>(a);
     };
     const int mid_smem = kMidWarpsPerBlock * 2 * kWarpHash * (int)sizeof(uint32_t);
     GB_CUDA(cudaFuncSetAttribute(k_ex_eval_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, mid_smem));
@@ -2268,9 +2095,9 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     const int hub_grid = resident((const void*)k_ex_hub_accum, kHubThreads2, 0);
     const int commit_grid = (int)std::max<int64_t>(1, ceil_div(B, kT));
     const int commit_b_grid = (int)std::max<int64_t>(1, ceil_div(B, kT));
-    // eval_small, advance, 3 table kernels, commit_a, commit_b; eval_mid;
+    // eval_small, advance, 2 table kernels, commit_a, commit_b; eval_mid;
     // eval_big; hub_select + hub_accum; commit_hub (hubs or big rows).
-    const int per_round = 7 + (n_mid ? 1 : 0) + (n_big ? 1 : 0) + (nh ? 2 : 0) + ((nh || n_big) ? 1 : 0);
+    const int per_round = 6 + (n_mid ? 1 : 0) + (n_big ? 1 : 0) + (nh ? 2 : 0) + ((nh || n_big) ? 1 : 0);
     const int commit_a_grid = std::max(commit_grid, nh ? hub_grid : 0);
     // Side streams and events for the fork/join shape of a captured round:
     struct Fork {
@@ -2419,8 +2246,7 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
                 GB_CUDA(cudaGraphKernelNodeGetParams(nd, &kp));
                 const void* f = kp.func;
                 int pr = mid;
-                if (f == (const void*)k_tb_insert || f == (const void*)k_tb_group || f == (const void*)k_tb_finish ||
-                    f == (const void*)k_ex_advance)
+                if (f == (const void*)k_tb_insert || f == (const void*)k_tb_sort || f == (const void*)k_ex_advance)
                     pr = greatest;
                 else if (f == (const void*)k_ex_commit_b || f == (const void*)k_ex_commit_hub ||
                          f == (const void*)k_ex_hub_accum)
@@ -2455,7 +2281,7 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
             throw Error(GBGPU_E_CUDA, "serial-order local moving: event table slot with an invalid hot index");
         if (hctl->error)
             throw Error(GBGPU_E_CUDA, "serial-order local moving: round loop stopped without progress");
-        nl += 4 + (nh ? 1 : 0) + hctl->round * per_round;
+        nl += 3 + (nh ? 1 : 0) + hctl->round * per_round;
         rounds += hctl->round;
         evals += hctl->evals;
         ++iterations;

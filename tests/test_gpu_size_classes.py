@@ -199,3 +199,30 @@ def test_super_moves_with_close_candidates(ctx, kind, blocks, size, resolution):
     expect, ost = po.leiden(rp, col, resolution)
     np.testing.assert_array_equal(np.asarray(memb).view(np.uint32), expect)
     assert [st["passes"], st["iterations"]] == [ost.passes, ost.iterations]
+
+
+@pytest.mark.parametrize("sizes", [(1, 7, 8, 15), (16, 17, 18, 31, 32, 33), (48, 49, 63, 64, 65, 66),
+                                   (127, 128, 129, 511, 512, 513, 1024), (2048, 2049, 4100, 40, 40),
+                                   (20000, 33, 17, 300), (70000, 16, 65)])
+def test_local_moving_by_moves_per_community(ctx, sizes):
+    # Stars whose leaves join the centre's community in one window, the leaves'
+    # ids shuffled; every fifth leaf also sees a leaf of the next star.
+    rng = np.random.default_rng(sum(sizes))
+    copies = max(1, 400 // sum(sizes))
+    stars = [k for k in sizes for _ in range(copies)]
+    n = sum(stars) + len(stars)
+    ids = np.concatenate([np.arange(len(stars)), len(stars) + rng.permutation(sum(stars))])
+    at, leaves, edges = len(stars), [], []
+    for c, k in enumerate(stars):
+        leaves.append(ids[at:at + k])
+        at += k
+        edges += [(c, int(v)) for v in leaves[-1]]
+    for c in range(len(stars)):
+        nxt = leaves[(c + 1) % len(stars)]
+        edges += [(int(v), int(nxt[i % len(nxt)])) for i, v in enumerate(leaves[c][::5])]
+    rp, col = (t.numpy() for t in gg.from_edges(n, [e for e in edges if e[0] != e[1]]))
+    for resolution in (0.1, 1.0):
+        memb, st = ctx.run_graphbrew(rp, col, gb.DEFAULT_RECIPE, resolution)
+        expect, ost = po.leiden(rp, col, resolution)
+        np.testing.assert_array_equal(np.asarray(memb).view(np.uint32), expect)
+        assert [st["passes"], st["iterations"]] == [ost.passes, ost.iterations]
