@@ -226,3 +226,27 @@ def test_local_moving_by_moves_per_community(ctx, sizes):
         expect, ost = po.leiden(rp, col, resolution)
         np.testing.assert_array_equal(np.asarray(memb).view(np.uint32), expect)
         assert [st["passes"], st["iterations"]] == [ost.passes, ost.iterations]
+
+
+@pytest.mark.parametrize("parts", [("grid", "uniform", "grid"), ("uniform", "grid", "uniform")])
+def test_local_moving_window_grows_and_shrinks(ctx, parts):
+    # Consecutive id ranges that commit a window at once and in many rounds.
+    at, edges = 0, []
+    for i, kind in enumerate(parts):
+        rp_t, col_t = gg.grid(300, 300, 0.05, seed=50 + i) if kind == "grid" else gg.uniform(17, 8, seed=50 + i)
+        rp, col = rp_t.numpy(), col_t.numpy()
+        src = np.repeat(np.arange(len(rp) - 1), np.diff(rp))
+        keep = src < col
+        edges.append(np.stack([src[keep], col[keep]], axis=1) + at)
+        if at:
+            edges.append(np.array([[at - 1, at]]))
+        at += len(rp) - 1
+    e = np.concatenate(edges)
+    src, dst = np.concatenate([e[:, 0], e[:, 1]]), np.concatenate([e[:, 1], e[:, 0]])
+    order = np.lexsort((dst, src))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=at))]).astype(np.int64)
+    col = dst[order].astype(np.int32)
+    memb, st = ctx.run_graphbrew(rp, col, gb.DEFAULT_RECIPE, 1.0)
+    expect, ost = po.leiden(rp, col, 1.0)
+    np.testing.assert_array_equal(np.asarray(memb).view(np.uint32), expect)
+    assert [st["passes"], st["iterations"]] == [ost.passes, ost.iterations]
