@@ -85,9 +85,11 @@ constexpr int kZCand = 128;                   // hot slots of the table consider
 constexpr int kSlotwTagShift = kSlotBits + 1;
 constexpr uint32_t kSlotwDesig = 1u << kSlotBits;
 constexpr int kHubThreads2 = 256;             // threads of the hub kernels
+constexpr int kSmallMaxDeg = 32;              // rows up to this: a lane per neighbour
+constexpr int kMidMaxDeg = 128;               // rows above that up to this: one warp each
+constexpr int kLongThreads = 128;             // rows above that up to kWarpMaxDeg: one CTA of this size each
 constexpr int kBigMaxDeg = 2048;              // rows above kWarpMaxDeg up to this: one CTA each
 constexpr int kBigThreads = 256;
-constexpr int kBigSlots = 2 * kBigMaxDeg;     // shared table of a big row
 constexpr int kHubSeg = 4 * kHubThreads2;     // edges per hub-accumulation CTA (4 per thread)
 constexpr int kTabSeg = 4 * kHubThreads2;     // table slots per hub-selection CTA (4 per thread)
 constexpr unsigned long long kNoChange = ~0ull;
@@ -100,6 +102,7 @@ struct Ctl {
     long long es0, es1;       // hub edge-segment range of the window
     long long ts0, ts1;       // hub table-segment range of the window
     long long ms0, ms1;       // mid-degree list range of the window
+    long long ls0, ls1;       // long-row list range of the window
     long long bs0, bs1;       // big-row list range of the window
     long long c_bs0, c_bs1;   // big-row range of the last decided window
     long long round;
@@ -194,8 +197,10 @@ struct ExactState {
     int32_t* hub_clr;             // per hub: table segments cleared this round
     double* part_d;               // per table segment
     uint32_t* part_c;
-    const uint32_t* mid_v;        // vertices with 32 < degree <= kWarpMaxDeg (ascending)
+    const uint32_t* mid_v;        // vertices with kSmallMaxDeg < degree <= kMidMaxDeg (ascending)
     long long n_mid;
+    const uint32_t* long_v;       // vertices with kMidMaxDeg < degree <= kWarpMaxDeg (ascending)
+    long long n_long;
     const uint32_t* big_v;        // vertices with kWarpMaxDeg < degree <= kBigMaxDeg (ascending)
     long long n_big;
     cudaGraphConditionalHandle cond;  // while-node condition (graph-driven rounds)
@@ -498,13 +503,13 @@ __device__ __forceinline__ long long warp_lower_bound_u32(const uint32_t* a, lon
     return b ? lo + (__ffs(b) - 1) : hi;
 }
 
-// Window ranges of the hub segment lists, the mid-degree list and the
-// big-row list for the window [P, E): eight searches on warps 0-7.
+// Window ranges of the hub segment lists and the mid, long and big-row lists
+// for the window [P, E): ten searches on warps 0-9.
 __device__ __forceinline__ void window_ranges(const ExactState& a, Ctl* c, long long P, long long E) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (w >= 8) return;
-    const uint32_t* arr = w < 2 ? a.eseg_v : (w < 4 ? a.tseg_v : (w < 6 ? a.mid_v : a.big_v));
-    const long long len = w < 2 ? a.n_eseg : (w < 4 ? a.n_tseg : (w < 6 ? a.n_mid : a.n_big));
+    if (w >= 10) return;
+    const uint32_t* arr = w < 2 ? a.eseg_v : (w < 4 ? a.tseg_v : (w < 6 ? a.mid_v : (w < 8 ? a.big_v : a.long_v)));
+    const long long len = w < 2 ? a.n_eseg : (w < 4 ? a.n_tseg : (w < 6 ? a.n_mid : (w < 8 ? a.n_big : a.n_long)));
     const long long pos = warp_lower_bound_u32(arr, len, (uint32_t)((w & 1) ? E : P), lane);
     if (lane == 0) {
         switch (w) {
@@ -515,7 +520,9 @@ __device__ __forceinline__ void window_ranges(const ExactState& a, Ctl* c, long 
             case 4: c->ms0 = pos; break;
             case 5: c->ms1 = pos; break;
             case 6: c->bs0 = pos; break;
-            default: c->bs1 = pos; break;
+            case 7: c->bs1 = pos; break;
+            case 8: c->ls0 = pos; break;
+            default: c->ls1 = pos; break;
         }
     }
 }
@@ -859,172 +866,42 @@ __global__ void __launch_bounds__(kSortThreads) k_tb_sort(ExactState a) {
 
 constexpr int kMidWarpsPerBlock = 4;
 constexpr int kSmallWarpsPerBlock = 8;
-constexpr int kSmallMaxDeg = 32;
 
-// One window vertex by one warp.  Small rows (deg <= 32) hold one neighbour
-// per lane and rank communities with __match_any_sync; mid rows
-// (32 < deg <= kWarpMaxDeg) accumulate into the warp's shared-memory table.
-template <bool kMid>
-__device__ __forceinline__ void eval_vertex(const ExactState& a, const Round& r, int64_t u, int lane, uint32_t* tk,
-                                            uint32_t* tv) {
-    const int64_t rb = a.rp[u];
-    const int deg = (int)(a.rp[u + 1] - rb);
-    bool act = a.vaff[u] != 0;
-    if (!act) {
-        bool any = false;
-        for (int i = lane; i < deg && !any; i += 32) {
-            const int32_t v = a.col[rb + i];
-            any = (v >= r.P && v < u && prev_mover(a, r, v));
-        }
-        act = __any_sync(0xFFFFFFFFu, any);
-    }
-    const uint32_t d = a.vcom[u];
-    if (!act) {
-        if (lane == 0) record(a, r, u, d, kNoMove, 0.0);
-        return;
-    }
-    const bool known = u < r.pE;
+// Row of up to 32 neighbours by a warp: c is the lane's neighbour's community
+// (kNone: none that counts), d the vertex's own; lanes of a community are ranked by
+// __match_any_sync.
+__device__ __forceinline__ void decide_small(const ExactState& a, const Round& r, int64_t u, int deg, uint32_t d,
+                                             uint32_t c) {
+    const int lane = threadIdx.x & 31;
     const CommRec rd = load_rec(a, d);
-    const double ku = (double)deg;
-    const uint32_t ub = bound_of(a, (uint32_t)u);
-    double best_d = 0.0;
-    uint32_t best_c = kNone;
-    if (!kMid) {
-        uint32_t c = kNone;
-        CommRec rc = rd;
-        bool dirty = !known || comm_changed(r, rd);
-        if (lane < deg) {
-            const int32_t v = a.col[rb + lane];
-            const Seen sv = see(a, r, v, u);
-            if (counts(a, v, (uint32_t)u, ub)) {
-                c = sv.c;
-                rc = load_rec(a, c);
-                dirty = dirty || comm_changed(r, rc);
-            }
-            dirty = dirty || sv.changed;
+    const CommRec rc = c != kNone ? load_rec(a, c) : rd;
+    if (a.vcob) {
+        long long sg1 = 0;
+        if (lane == 0) {
+            const uint32_t cc[1] = {d};
+            const bool vv[1] = {true};
+            const CommRec rr[1] = {rd};
+            long long o[1];
+            sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, rr, (uint32_t)u, o);
+            sg1 = o[0];
         }
-        if (!__any_sync(0xFFFFFFFFu, dirty)) {
-            if (lane == 0) keep_decision(r, u);
+        sg1 = __shfl_sync(0xFFFFFFFFu, sg1, 0);
+        if (refine_stays(a, (double)sg1, (double)deg)) {
+            if (lane == 0) record(a, r, u, d, kNoMove, 0.0);
             return;
         }
-        if (a.vcob) {
-            long long sg1 = 0;
-            if (lane == 0) {
-                const uint32_t cc[1] = {d};
-                const bool vv[1] = {true};
-                const CommRec rr[1] = {rd};
-                long long o[1];
-                sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, rr, (uint32_t)u, o);
-                sg1 = o[0];
-            }
-            sg1 = __shfl_sync(0xFFFFFFFFu, sg1, 0);
-            if (refine_stays(a, (double)sg1, ku)) {
-                if (lane == 0) record(a, r, u, d, kNoMove, 0.0);
-                return;
-            }
-        }
-        const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
-        const int kud = __popc(__ballot_sync(0xFFFFFFFFu, c == d));
-        const bool cand = c != kNone && c != d && lane == __ffs(peers) - 1;
-        const unsigned idle = ~__ballot_sync(0xFFFFFFFFu, cand);
-        long long sc = 0, sd = 0;
-        sigma_with_own(a, r, (uint32_t)u, cand, c, rc, d, rd, idle, 0xFFFFFFFFu, sc, sd);
-        if (cand) {
-            const double dl = delta_qi(a.dq, __popc(peers), kud, deg, sc, sd);
-            if (dpos(dl)) { best_d = dl; best_c = c; }
-        }
-    } else {
-        // Has anything changed that the vertex sees?  Asked of rows of up to 128
-        // entries (longer ones see a community that changes every round), in a
-        // gather of its own: with the question inside the accumulation below
-        // its loads no longer overlapped (RMAT-22: 143 -> 188 us a round).
-        if (known && deg <= 128 && !comm_changed(r, rd)) {
-            bool dirty = false;
-            uint32_t c[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int e = 32 * k + lane;
-                c[k] = d;
-                if (e < deg) {
-                    const Seen sv = see(a, r, a.col[rb + e], u);
-                    dirty |= sv.changed;
-                    c[k] = sv.c;
-                }
-            }
-            uint32_t ver[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) ver[k] = 32 * k < deg ? a.rec[c[k]].cver : 0u;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) dirty |= ver[k] >= (uint32_t)r.tag;
-            if (!__any_sync(0xFFFFFFFFu, dirty)) {
-                if (lane == 0) keep_decision(r, u);
-                return;
-            }
-        }
-        uint32_t H = 64;
-        while (H < 2u * (uint32_t)deg) H <<= 1;
-        const uint32_t mask = H - 1;
-        for (uint32_t i = lane; i < H; i += 32) { tk[i] = kNone; tv[i] = 0; }
-        __syncwarp();
-        // Neighbour communities, four 32-edge batches in flight per step.
-        for (int base = 0; base < deg; base += 128) {
-            uint32_t c[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int e = base + 32 * k + lane;
-                c[k] = kNone;
-                if (e < deg) {
-                    const int32_t v = a.col[rb + e];
-                    if (counts(a, v, (uint32_t)u, ub)) c[k] = comm_at(a, r, v, u);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const unsigned peers = __match_any_sync(0xFFFFFFFFu, c[k]);
-                if (c[k] != kNone && lane == __ffs(peers) - 1)
-                    table_add(tk, tv, mask, c[k], (uint32_t)__popc(peers));
-            }
-        }
-        __syncwarp();
-        const uint32_t kud = table_get(tk, tv, mask, d);
-        // Compact the candidate communities (c != d) to the front of the
-        // table, so the selection runs ceil((candidates + 1) / 32) lookup rounds.
-        uint32_t cnt = 0;
-        for (uint32_t i0 = 0; i0 < H; i0 += 32) {
-            const uint32_t c = tk[i0 + lane], v = tv[i0 + lane];
-            const bool occ = c != kNone && c != d;
-            const unsigned bal = __ballot_sync(0xFFFFFFFFu, occ);
-            __syncwarp();
-            if (occ) {
-                const uint32_t pos = cnt + __popc(bal & ((1u << lane) - 1u));
-                tk[pos] = c;
-                tv[pos] = v;
-            }
-            cnt += __popc(bal);
-            __syncwarp();
-        }
-        // One lookup per lane per step: lane 31 of the first step takes d's, the
-        // other 31 candidates; every later step 32 (a second lookup per lane, for
-        // d, doubled the step's instructions and registers).
-        long long sd = 0;
-        for (uint32_t i0 = 0;; i0 += 32) {
-            const bool own = i0 == 0 && lane == 31;
-            const uint32_t i = i0 == 0 ? lane : i0 - 1 + lane;
-            const bool valid = !own && i < cnt;
-            const uint32_t cc[1] = {valid ? tk[i] : d};
-            const bool vv[1] = {valid || own};
-            const CommRec rr[1] = {valid ? load_rec(a, cc[0]) : rd};
-            long long sg[1];
-            sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, rr, (uint32_t)u, sg);
-            if (i0 == 0) sd = __shfl_sync(0xFFFFFFFFu, sg[0], 31);
-            if (valid) {
-                const double dl = delta_qi(a.dq, tv[i], kud, deg, sg[0], sd);
-                if (dpos(dl) && better_pos(dl, cc[0], best_d, best_c)) { best_d = dl; best_c = cc[0]; }
-            }
-            if (i0 + 31 >= cnt) break;
-        }
-        __syncwarp();
-        if (refine_stays(a, (double)sd, ku)) best_c = kNone;   // every lane holds the same sd
+    }
+    const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
+    const int kud = __popc(__ballot_sync(0xFFFFFFFFu, c == d));
+    const bool cand = c != kNone && c != d && lane == __ffs(peers) - 1;
+    const unsigned idle = ~__ballot_sync(0xFFFFFFFFu, cand);
+    long long sc = 0, sd = 0;
+    sigma_with_own(a, r, (uint32_t)u, cand, c, rc, d, rd, idle, 0xFFFFFFFFu, sc, sd);
+    double best_d = 0.0;
+    uint32_t best_c = kNone;
+    if (cand) {
+        const double dl = delta_qi(a.dq, __popc(peers), kud, deg, sc, sd);
+        if (dpos(dl)) { best_d = dl; best_c = c; }
     }
     warp_argmax_pos(best_d, best_c);
     if (lane == 0) {
@@ -1033,10 +910,117 @@ __device__ __forceinline__ void eval_vertex(const ExactState& a, const Round& r,
     }
 }
 
-// Small rows, no shared memory.  A warp takes four consecutive window
-// vertices: rows of degree <= 8 are evaluated together by four 8-lane groups
-// (one neighbour per lane), rows of degree 9..32 then one at a time by the
-// whole warp.
+// Mid row (kSmallMaxDeg < degree <= kMidMaxDeg) by one warp: its neighbours'
+// communities in one gather of up to four a lane, which also says whether anything
+// that the vertex sees has changed; then a count per community in the warp's shared
+// table.  One warp's chain of dependent loads bounds it, so the tables are small
+// enough (2 KB) for the registers to limit the warps in flight, and longer rows go
+// to CTAs: with 8 KB tables, up to three gathers and rows of up to 512, R-MAT-22's
+// rounds spent 90 us here, now 33, and 26 on the longer rows beside it.
+constexpr int kMidSlots = 2 * kMidMaxDeg;
+__device__ __forceinline__ void eval_mid(const ExactState& a, const Round& r, int64_t u, int lane, uint32_t* tk,
+                                         uint32_t* tv) {
+    const int64_t rb = a.rp[u];
+    const int deg = (int)(a.rp[u + 1] - rb);
+    const bool aff = a.vaff[u] != 0;
+    const uint32_t d = a.vcom[u], ub = bound_of(a, (uint32_t)u);
+    int32_t v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = 32 * k + lane < deg ? a.col[rb + 32 * k + lane] : -1;
+    const CommRec rd = load_rec(a, d);
+    bool dirty = u >= r.pE || comm_changed(r, rd), moved = false;
+    uint32_t c[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        c[k] = kNone;
+        if (v[k] >= 0) {
+            const Seen sv = see(a, r, v[k], u);
+            moved |= sv.moved;
+            dirty |= sv.changed;
+            if (counts(a, v[k], (uint32_t)u, ub)) c[k] = sv.c;
+        }
+    }
+    if (!__any_sync(0xFFFFFFFFu, dirty)) {
+        uint32_t ver[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) ver[k] = c[k] != kNone ? a.rec[c[k]].cver : 0u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) dirty |= ver[k] >= (uint32_t)r.tag;
+        if (!__any_sync(0xFFFFFFFFu, dirty)) {
+            if (lane == 0) keep_decision(r, u);
+            return;
+        }
+    }
+    if (!aff && !__any_sync(0xFFFFFFFFu, moved)) {
+        if (lane == 0) record(a, r, u, d, kNoMove, 0.0);
+        return;
+    }
+    uint32_t H = 64;
+    while (H < 2u * (uint32_t)deg) H <<= 1;
+    const uint32_t mask = H - 1;
+    for (uint32_t i = lane; i < H; i += 32) { tk[i] = kNone; tv[i] = 0; }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (32 * k >= deg) break;
+        const unsigned peers = __match_any_sync(0xFFFFFFFFu, c[k]);
+        if (c[k] != kNone && lane == __ffs(peers) - 1) table_add(tk, tv, mask, c[k], (uint32_t)__popc(peers));
+    }
+    __syncwarp();
+    const uint32_t kud = table_get(tk, tv, mask, d);
+    // The candidate communities (c != d) to the front of the table, so that the
+    // selection takes ceil((candidates + 1) / 32) lookup steps.
+    uint32_t cnt = 0;
+    for (uint32_t i0 = 0; i0 < H; i0 += 32) {
+        const uint32_t x = tk[i0 + lane], y = tv[i0 + lane];
+        const bool occ = x != kNone && x != d;
+        const unsigned bal = __ballot_sync(0xFFFFFFFFu, occ);
+        __syncwarp();
+        if (occ) {
+            const uint32_t pos = cnt + __popc(bal & ((1u << lane) - 1u));
+            tk[pos] = x;
+            tv[pos] = y;
+        }
+        cnt += __popc(bal);
+        __syncwarp();
+    }
+    // One lookup per lane per step: lane 31 of the first step takes d's, the
+    // other 31 candidates; every later step 32 (a second lookup per lane, for
+    // d, doubled the step's instructions and registers).
+    long long sd = 0;
+    double best_d = 0.0;
+    uint32_t best_c = kNone;
+    for (uint32_t i0 = 0;; i0 += 32) {
+        const bool own = i0 == 0 && lane == 31;
+        const uint32_t i = i0 == 0 ? lane : i0 - 1 + lane;
+        const bool valid = !own && i < cnt;
+        const uint32_t cc[1] = {valid ? tk[i] : d};
+        const bool vv[1] = {valid || own};
+        const CommRec rr[1] = {valid ? load_rec(a, cc[0]) : rd};
+        long long sg[1];
+        sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, rr, (uint32_t)u, sg);
+        if (i0 == 0) sd = __shfl_sync(0xFFFFFFFFu, sg[0], 31);
+        if (valid) {
+            const double dl = delta_qi(a.dq, tv[i], kud, deg, sg[0], sd);
+            if (dpos(dl) && better_pos(dl, cc[0], best_d, best_c)) { best_d = dl; best_c = cc[0]; }
+        }
+        if (i0 + 31 >= cnt) break;
+    }
+    __syncwarp();
+    if (refine_stays(a, (double)sd, (double)deg)) best_c = kNone;   // every lane holds the same sd
+    warp_argmax_pos(best_d, best_c);
+    if (lane == 0) {
+        if (best_d > 0.0 && best_c != kNone && best_c != d) record(a, r, u, d, best_c, best_d);
+        else record(a, r, u, d, kNoMove, 0.0);
+    }
+}
+
+// Small rows.  A warp takes four consecutive window vertices: rows of degree
+// <= 8 are evaluated together by four 8-lane groups (one neighbour per lane).
+// Of rows of degree 9..32 the neighbours' communities are gathered for all four at
+// once, a lane per neighbour, and those that see a change are then decided one
+// after another by the whole warp.  (Gathered one after another, with the change to mid
+// rows: 8 M uniform vertices 268 ms, now 220.)
 constexpr int kTinyDeg = 8;
 
 __device__ __forceinline__ void eval_small_body(const ExactState& a, const Ctl* c) {
@@ -1045,6 +1029,7 @@ __device__ __forceinline__ void eval_small_body(const ExactState& a, const Ctl* 
     const int g = lane >> 3, j = lane & 7;
     const unsigned gmask = 0xFFu << (g * 8);
     const int wpb = (int)(blockDim.x >> 5);
+    __shared__ uint32_t wide_c[kSmallWarpsPerBlock][4][32];
     const int64_t nw = (int64_t)gridDim.x * wpb;
     for (int64_t u0 = r.P + 4 * ((int64_t)blockIdx.x * wpb + w); u0 < r.E; u0 += 4 * nw) {
         const int64_t u = u0 + g;
@@ -1055,27 +1040,28 @@ __device__ __forceinline__ void eval_small_body(const ExactState& a, const Ctl* 
             rb = a.rp[u];
             deg = (int)(a.rp[u + 1] - rb);
         }
-        const bool tiny = inwin && deg <= kTinyDeg;
+        const bool tiny = inwin && deg <= kTinyDeg, wide = inwin && !tiny && deg <= kSmallMaxDeg;
         // One load round for the row and its vertex state, one for its
         // neighbours' states, one for the communities they are in.
         int32_t v = -1;
         uint32_t d = kNone;
         bool aff = false;
         uint32_t ub = 0;
-        if (tiny) {
-            if (j < deg) v = a.col[rb + j];
+        if (tiny || wide) {
+            if (tiny && j < deg) v = a.col[rb + j];
             d = a.vcom[u];
             aff = a.vaff[u] != 0;
             ub = bound_of(a, (uint32_t)u);
         }
-        bool dirty = tiny && u >= r.pE;
+        bool fresh = u >= r.pE;
         bool pm = false;
         uint32_t cv = kNone;
         CommRec rc{0ull, 0u, 0u}, rd = rc;
-        if (tiny) {
+        if (tiny || wide) {
             rd = load_rec(a, d);
-            dirty = dirty || comm_changed(r, rd);
+            fresh = fresh || comm_changed(r, rd);
         }
+        bool dirty = tiny && fresh;
         if (v >= 0) {
             const Seen sv = see(a, r, v, u);
             pm = sv.moved;
@@ -1131,13 +1117,47 @@ __device__ __forceinline__ void eval_small_body(const ExactState& a, const Ctl* 
             if (act && !stays && best_d > 0.0 && best_c != kNone && best_c != d) record(a, r, u, d, best_c, best_d);
             else record(a, r, u, d, kNoMove, 0.0);
         }
-        // Rows of degree 9..32: the whole warp, one row at a time.
+        // Rows of degree 9..32.
+        if (!__any_sync(0xFFFFFFFFu, wide)) continue;
+        uint32_t ck[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int dk = __shfl_sync(0xFFFFFFFFu, wide ? deg : 0, k * 8);
+            const int64_t rk = __shfl_sync(0xFFFFFFFFu, rb, k * 8);
+            ck[k] = lane < dk ? (uint32_t)a.col[rk + lane] : kNone;
+        }
+        unsigned flags = 0;   // bit k: a neighbour of row k moved; bit 4 + k: something it sees changed
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (ck[k] == kNone) continue;
+            const int32_t vk = (int32_t)ck[k];
+            const int64_t uk = u0 + k;
+            const Seen sv = see(a, r, vk, uk);
+            flags |= (sv.moved ? 1u << k : 0u) | (sv.changed ? 16u << k : 0u);
+            ck[k] = counts(a, vk, (uint32_t)uk, bound_of(a, (uint32_t)uk)) ? sv.c : kNone;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (ck[k] != kNone && a.rec[ck[k]].cver >= (uint32_t)r.tag) flags |= 16u << k;
+            wide_c[w][k][lane] = ck[k];
+        }
+        __syncwarp();
+        flags = __reduce_or_sync(0xFFFFFFFFu, flags);
 #pragma unroll 1
         for (int k = 0; k < 4; ++k) {
-            const int dk = __shfl_sync(0xFFFFFFFFu, deg, k * 8);
-            const int ik = __shfl_sync(0xFFFFFFFFu, (int)inwin, k * 8);
-            if (ik && dk > kTinyDeg && dk <= kSmallMaxDeg) eval_vertex<false>(a, r, u0 + k, lane, nullptr, nullptr);
+            const int dk = __shfl_sync(0xFFFFFFFFu, wide ? deg : 0, k * 8);
+            const bool freshk = __shfl_sync(0xFFFFFFFFu, fresh, k * 8), affk = __shfl_sync(0xFFFFFFFFu, aff, k * 8);
+            const uint32_t dcom = __shfl_sync(0xFFFFFFFFu, d, k * 8);
+            if (dk == 0) continue;
+            if (!freshk && !(flags >> (4 + k) & 1u)) {
+                if (lane == 0) keep_decision(r, u0 + k);
+            } else if (!affk && !(flags >> k & 1u)) {
+                if (lane == 0) record(a, r, u0 + k, dcom, kNoMove, 0.0);
+            } else {
+                decide_small(a, r, u0 + k, dk, dcom, wide_c[w][k][lane]);
+            }
         }
+        __syncwarp();
     }
 }
 
@@ -1148,26 +1168,30 @@ __global__ void __launch_bounds__(kSmallWarpsPerBlock * 32, 4) k_ex_eval_small(E
     eval_small_body(a, a.ctl);
 }
 
-// Big rows (kWarpMaxDeg < degree <= kBigMaxDeg): one CTA per row, table in
-// shared memory, candidates compacted, one candidate per thread per step (its
+// Long and big rows (kMidMaxDeg < degree <= kWarpMaxDeg, up to kBigMaxDeg): one
+// CTA per row, table in shared memory, candidates compacted, one candidate per thread per step (its
 // lookup interleaved with d's in the first step; wider interleaving spilled
 // under the register cap).  Three CTAs per SM (registers capped near 80).
-__device__ __forceinline__ void eval_big_body(const ExactState& a, const Ctl* c) {
+template <int kMaxDeg>
+constexpr int row_smem() { return (2 * 2 * kMaxDeg + 2 * (kMaxDeg + 1)) * (int)sizeof(uint32_t); }
+
+template <int kMaxDeg>
+__device__ __forceinline__ void eval_row_cta(const ExactState& a, const Ctl* c, const uint32_t* rows, long long b0,
+                                             long long b1) {
     extern __shared__ uint32_t big_smem[];
-    uint32_t* tk = big_smem;                      // kBigSlots keys
-    uint32_t* tv = tk + kBigSlots;                // kBigSlots counts
-    uint32_t* cand_c = tv + kBigSlots;            // d and up to kBigMaxDeg compacted candidates
-    uint32_t* cand_w = cand_c + kBigMaxDeg + 1;
+    uint32_t* tk = big_smem;                      // 2 kMaxDeg keys
+    uint32_t* tv = tk + 2 * kMaxDeg;              // 2 kMaxDeg counts
+    uint32_t* cand_c = tv + 2 * kMaxDeg;          // d and up to kMaxDeg compacted candidates
+    uint32_t* cand_w = cand_c + kMaxDeg + 1;
     __shared__ int s_any;
     __shared__ uint32_t s_cnt;
     __shared__ long long s_own;
     __shared__ double red_d[32];
     __shared__ uint32_t red_c[32];
     const Round r = round_view(a, c);
-    const long long b0 = c->bs0, b1 = c->bs1;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     for (long long bi = b0 + blockIdx.x; bi < b1; bi += gridDim.x) {
-        const uint32_t u = a.big_v[bi];
+        const uint32_t u = rows[bi];
         const int64_t rb = a.rp[u], re = a.rp[u + 1];
         const int deg = (int)(re - rb);
         const uint32_t d = a.vcom[u];
@@ -1267,7 +1291,12 @@ __device__ __forceinline__ void eval_big_body(const ExactState& a, const Ctl* c)
 
 __global__ void __launch_bounds__(kBigThreads, 3) k_ex_eval_big(ExactState a) {
     if (a.ctl->P >= a.ctl->n) return;
-    eval_big_body(a, a.ctl);
+    eval_row_cta<kBigMaxDeg>(a, a.ctl, a.big_v, a.ctl->bs0, a.ctl->bs1);
+}
+
+__global__ void __launch_bounds__(kLongThreads, 8) k_ex_eval_long(ExactState a) {
+    if (a.ctl->P >= a.ctl->n) return;
+    eval_row_cta<kWarpMaxDeg>(a, a.ctl, a.long_v, a.ctl->ls0, a.ctl->ls1);
 }
 
 // Mid rows of the window (from the ascending list of mid-degree vertices).
@@ -1277,11 +1306,11 @@ __device__ __forceinline__ void eval_mid_body(const ExactState& a, const Ctl* c)
     const long long m0 = c->ms0, m1 = c->ms1;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int wpb = (int)(blockDim.x >> 5);
-    uint32_t* tk = ex_smem + (size_t)w * 2 * kWarpHash;
-    uint32_t* tv = tk + kWarpHash;
+    uint32_t* tk = ex_smem + (size_t)w * 2 * kMidSlots;
+    uint32_t* tv = tk + kMidSlots;
     const long long nw = (long long)gridDim.x * wpb;
     for (long long i = m0 + (long long)blockIdx.x * wpb + w; i < m1; i += nw)
-        eval_vertex<true>(a, r, a.mid_v[i], lane, tk, tv);
+        eval_mid(a, r, a.mid_v[i], lane, tk, tv);
 }
 
 __global__ void __launch_bounds__(kMidWarpsPerBlock * 32) k_ex_eval_mid(ExactState a) {
@@ -1289,15 +1318,16 @@ __global__ void __launch_bounds__(kMidWarpsPerBlock * 32) k_ex_eval_mid(ExactSta
     eval_mid_body(a, a.ctl);
 }
 
-__global__ void k_mid_flags(const int64_t* __restrict__ rp, int64_t n, int32_t* __restrict__ flag) {
+__global__ void k_degree_flags(const int64_t* __restrict__ rp, int64_t n, int64_t above, int64_t most,
+                               int32_t* __restrict__ flag) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
         const int64_t d = rp[v + 1] - rp[v];
-        flag[v] = d > kSmallMaxDeg && d <= kWarpMaxDeg;
+        flag[v] = d > above && d <= most;
     }
 }
 
-__global__ void k_mid_scatter(const int32_t* __restrict__ flag, const int64_t* __restrict__ pos, int64_t n,
-                              uint32_t* __restrict__ out) {
+__global__ void k_degree_scatter(const int32_t* __restrict__ flag, const int64_t* __restrict__ pos, int64_t n,
+                                 uint32_t* __restrict__ out) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
         if (flag[v]) out[pos[v]] = (uint32_t)v;
 }
@@ -1988,21 +2018,26 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     DevBuf<double> part_d(tseg.empty() ? 1 : tseg.size(), s);
     DevBuf<uint32_t> part_c(tseg.empty() ? 1 : tseg.size(), s);
 
-    // ---- mid-degree list (ascending vertex ids) ----
-    int64_t n_mid = 0;
-    DevBuf<uint32_t> mid_v;
+    // ---- mid and long rows (ascending vertex ids) ----
+    int64_t n_mid = 0, n_long = 0;
+    DevBuf<uint32_t> mid_v, long_v;
     {
         DevBuf<int32_t> flag(n, s);
         DevBuf<int64_t> pos(n, s), tot(1, s);
-        k_mid_flags<<<grid_for(n, kT), kT, 0, s>>>(ctx.g.row_ptr, n, flag);
-        GB_LAUNCH_CHECK();
-        exclusive_scan_i32_to_i64(flag, pos, n, tot, s);
-        n_mid = read_dev(tot.get(), s);
-        mid_v.alloc(n_mid > 0 ? n_mid : 1, s);
-        if (n_mid) {
-            k_mid_scatter<<<grid_for(n, kT), kT, 0, s>>>(flag, pos, n, mid_v);
+        auto list = [&](int64_t above, int64_t most, DevBuf<uint32_t>& out) {
+            k_degree_flags<<<grid_for(n, kT), kT, 0, s>>>(ctx.g.row_ptr, n, above, most, flag);
             GB_LAUNCH_CHECK();
-        }
+            exclusive_scan_i32_to_i64(flag, pos, n, tot, s);
+            const int64_t count = read_dev(tot.get(), s);
+            out.alloc(count > 0 ? count : 1, s);
+            if (count) {
+                k_degree_scatter<<<grid_for(n, kT), kT, 0, s>>>(flag, pos, n, out);
+                GB_LAUNCH_CHECK();
+            }
+            return count;
+        };
+        n_mid = list(kSmallMaxDeg, kMidMaxDeg, mid_v);
+        n_long = list(kMidMaxDeg, kWarpMaxDeg, long_v);
     }
 
     // ---- round state ----
@@ -2087,6 +2122,8 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     a.part_c = part_c.get();
     a.mid_v = mid_v.get();
     a.n_mid = n_mid;
+    a.long_v = long_v.get();
+    a.n_long = n_long;
     a.M = ctx.M;
     a.R = ctx.R;
     a.dq = ctx.dq;
@@ -2096,7 +2133,7 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
         k_tb_insert<<<tb_grid, kTbThreads, 0, st>>>(a);
         k_tb_sort<<<kZMax + kSortCtas, kSortThreads, 0, st>>>(a);
     };
-    const int mid_smem = kMidWarpsPerBlock * 2 * kWarpHash * (int)sizeof(uint32_t);
+    const int mid_smem = kMidWarpsPerBlock * 2 * kMidSlots * (int)sizeof(uint32_t);
     GB_CUDA(cudaFuncSetAttribute(k_ex_eval_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, mid_smem));
     const int small_grid = (int)std::max<int64_t>(1, ceil_div(B, 4 * kSmallWarpsPerBlock));
     // Grid-stride kernels: one resident wave (blocks per SM from the occupancy
@@ -2111,50 +2148,59 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     };
     const int mid_grid = resident((const void*)k_ex_eval_mid, kMidWarpsPerBlock * 32, mid_smem);
     const int select_grid = resident((const void*)k_ex_hub_select, kHubThreads2, 0);
-    const int big_smem = (2 * kBigSlots + 2 * (kBigMaxDeg + 1)) * (int)sizeof(uint32_t);
+    const int big_smem = row_smem<kBigMaxDeg>(), long_smem = row_smem<kWarpMaxDeg>();
     GB_CUDA(cudaFuncSetAttribute(k_ex_eval_big, cudaFuncAttributeMaxDynamicSharedMemorySize, big_smem));
     const int big_grid = resident((const void*)k_ex_eval_big, kBigThreads, big_smem);
+    const int long_grid = resident((const void*)k_ex_eval_long, kLongThreads, long_smem);
     const int hub_grid = resident((const void*)k_ex_hub_accum, kHubThreads2, 0);
     const int commit_grid = (int)std::max<int64_t>(1, ceil_div(B, kT));
     const int commit_b_grid = (int)std::max<int64_t>(1, ceil_div(B, kT));
     // eval_small, advance, 2 table kernels, commit_a, commit_b; eval_mid;
-    // eval_big; hub_select + hub_accum; commit_hub (hubs or big rows).
-    const int per_round = 6 + (n_mid ? 1 : 0) + (n_big ? 1 : 0) + (nh ? 2 : 0) + ((nh || n_big) ? 1 : 0);
+    // eval_long; eval_big; hub_select + hub_accum; commit_hub (hubs or big rows).
+    const int per_round = 6 + (n_mid ? 1 : 0) + (n_long ? 1 : 0) + (n_big ? 1 : 0) + (nh ? 2 : 0) + ((nh || n_big) ? 1 : 0);
     const int commit_a_grid = std::max(commit_grid, nh ? hub_grid : 0);
     // Side streams and events for the fork/join shape of a captured round:
     struct Fork {
-        cudaStream_t s1 = nullptr, s2 = nullptr, s3 = nullptr;
-        cudaEvent_t ev[9] = {};
+        cudaStream_t s1 = nullptr, s2 = nullptr, s3 = nullptr, s4 = nullptr;
+        cudaEvent_t ev[10] = {};
         ~Fork() {
             for (cudaEvent_t e : ev)
                 if (e) cudaEventDestroy(e);
             if (s1) cudaStreamDestroy(s1);
             if (s2) cudaStreamDestroy(s2);
             if (s3) cudaStreamDestroy(s3);
+            if (s4) cudaStreamDestroy(s4);
         }
     } fk;
     // One round: decide the window, advance, then prepare the next window
     // while this one commits.  Forked shape (graph capture):
-    //   { eval_small | eval_mid | hub_select } -> advance
+    //   { eval_small | eval_mid | eval_long | eval_big | hub_select } -> advance
     //   -> { table(next) | commit_a -> { commit_b | commit_hub | hub_accum(next) } }
     // hub_accum needs the committed memberships but no event table; the
     // round before the first needs the first window's table and accumulation.
     auto enqueue_round = [&](cudaStream_t st, bool fork) {
-        cudaStream_t sm = fork ? fk.s1 : st, sh = fork ? fk.s2 : st, sa = fork ? fk.s3 : st;
+        cudaStream_t sm = fork ? fk.s1 : st, sh = fork ? fk.s2 : st, sa = fork ? fk.s3 : st,
+                     sl = fork ? fk.s4 : st;
         if (fork) {
             GB_CUDA(cudaEventRecord(fk.ev[0], st));
             GB_CUDA(cudaStreamWaitEvent(sm, fk.ev[0], 0));
             GB_CUDA(cudaStreamWaitEvent(sh, fk.ev[0], 0));
         }
         if (fork) GB_CUDA(cudaStreamWaitEvent(sa, fk.ev[0], 0));
+        if (fork && n_long) GB_CUDA(cudaStreamWaitEvent(sl, fk.ev[0], 0));
         k_ex_eval_small<<<small_grid, kSmallWarpsPerBlock * 32, 0, st>>>(a);
         if (n_mid) k_ex_eval_mid<<<mid_grid, kMidWarpsPerBlock * 32, mid_smem, sm>>>(a);
         if (nh) k_ex_hub_select<<<select_grid, kHubThreads2, 0, sh>>>(a);
+        if (n_long) k_ex_eval_long<<<long_grid, kLongThreads, long_smem, sl>>>(a);
         if (n_big) k_ex_eval_big<<<big_grid, kBigThreads, big_smem, sa>>>(a);
         if (fork) {
             GB_CUDA(cudaEventRecord(fk.ev[1], sm));
             GB_CUDA(cudaEventRecord(fk.ev[2], sh));
             GB_CUDA(cudaEventRecord(fk.ev[8], sa));
+            if (n_long) {
+                GB_CUDA(cudaEventRecord(fk.ev[9], sl));
+                GB_CUDA(cudaStreamWaitEvent(st, fk.ev[9], 0));
+            }
             GB_CUDA(cudaStreamWaitEvent(st, fk.ev[1], 0));
             GB_CUDA(cudaStreamWaitEvent(st, fk.ev[2], 0));
             GB_CUDA(cudaStreamWaitEvent(st, fk.ev[8], 0));
@@ -2242,6 +2288,7 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
         GB_CUDA(cudaStreamCreateWithFlags(&fk.s1, cudaStreamNonBlocking));
         GB_CUDA(cudaStreamCreateWithFlags(&fk.s2, cudaStreamNonBlocking));
         GB_CUDA(cudaStreamCreateWithFlags(&fk.s3, cudaStreamNonBlocking));
+        GB_CUDA(cudaStreamCreateWithFlags(&fk.s4, cudaStreamNonBlocking));
         for (cudaEvent_t& e : fk.ev) GB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         GB_CUDA(cudaStreamBeginCaptureToGraph(gg.cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
         enqueue_round(gg.cs, true);
