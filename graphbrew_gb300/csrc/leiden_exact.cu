@@ -89,9 +89,9 @@ constexpr int kSmallMaxDeg = 32;              // rows up to this: a lane per nei
 constexpr int kMidMaxDeg = 128;               // rows above that up to this: one warp each
 constexpr int kLongThreads = 128;             // rows above that up to kWarpMaxDeg: one CTA of this size each
 constexpr int kBigMaxDeg = 2048;              // rows above kWarpMaxDeg up to this: one CTA each
-constexpr int kBigThreads = 256;
+constexpr int kBigThreads = 512;
 constexpr int kHubSeg = 4 * kHubThreads2;     // edges per hub-accumulation CTA (4 per thread)
-constexpr int kTabSeg = 4 * kHubThreads2;     // table slots per hub-selection CTA (4 per thread)
+constexpr int kTabSeg = 2 * kHubThreads2;     // table slots per hub-selection CTA (2 per thread)
 constexpr unsigned long long kNoChange = ~0ull;
 
 struct Ctl {
@@ -1289,7 +1289,7 @@ __device__ __forceinline__ void eval_row_cta(const ExactState& a, const Ctl* c, 
     }
 }
 
-__global__ void __launch_bounds__(kBigThreads, 3) k_ex_eval_big(ExactState a) {
+__global__ void __launch_bounds__(kBigThreads, 2) k_ex_eval_big(ExactState a) {
     if (a.ctl->P >= a.ctl->n) return;
     eval_row_cta<kBigMaxDeg>(a, a.ctl, a.big_v, a.ctl->bs0, a.ctl->bs1);
 }
@@ -1333,7 +1333,9 @@ __global__ void k_degree_scatter(const int32_t* __restrict__ flag, const int64_t
 }
 
 // Hub accumulation: one CTA per kHubSeg-edge segment of a window hub, four
-// edges per thread in flight.  Needs no event table: it runs while the
+// edges per thread in flight, and their first probes (one edge after another took
+// R-MAT-22's rounds 38 us here, now 21; counting a segment in shared memory first
+// costs more than it saves, as most keys are different).  Needs no event table: it runs while the
 // previous window commits its affected flags and the event table is built.
 __device__ __forceinline__ void hub_accum_body(const ExactState& a, const Ctl* c) {
     const Round r = round_view(a, c);
@@ -1366,25 +1368,42 @@ __device__ __forceinline__ void hub_accum_body(const ExactState& a, const Ctl* c
                 if (counts(a, v, h, ub)) c[k] = comm_at(a, r, v, h);
             }
         }
+        // Insert-or-add, the four first probes in flight together; keys that are
+        // new also go on the hub's occupied list, one reservation per warp.
         uint32_t own = 0;
+        uint32_t at[4], prev[4], cnt[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const unsigned peers = __match_any_sync(0xFFFFFFFFu, c[k]);
-            if (c[k] != kNone && lane == __ffs(peers) - 1) {
-                // insert-or-add; a new key also goes on the hub's occupied list
-                uint32_t hh = hash_u32(c[k]) & mask;
-                while (true) {
-                    const uint32_t prev = atomicCAS(&tk[hh], kNone, c[k]);
-                    if (prev == kNone) occ[atomicAdd(occn, 1u)] = hh;
-                    if (prev == kNone || prev == c[k]) {
-                        atomicAdd(&tv[hh], (uint32_t)__popc(peers));
-                        break;
-                    }
-                    hh = (hh + 1) & mask;
-                }
-            }
             own += __popc(__ballot_sync(0xFFFFFFFFu, c[k] == d));
+            cnt[k] = c[k] != kNone && lane == __ffs(peers) - 1 ? (uint32_t)__popc(peers) : 0u;
+            at[k] = hash_u32(c[k]) & mask;
+            if (cnt[k]) prev[k] = atomicCAS(&tk[at[k]], kNone, c[k]);
         }
+        unsigned fresh = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (!cnt[k]) continue;
+            while (prev[k] != kNone && prev[k] != c[k]) {
+                at[k] = (at[k] + 1) & mask;
+                prev[k] = atomicCAS(&tk[at[k]], kNone, c[k]);
+            }
+            atomicAdd(&tv[at[k]], cnt[k]);
+            if (prev[k] == kNone) fresh |= 1u << k;
+        }
+        const int nfresh = __popc(fresh);
+        int incl = nfresh;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        uint32_t pos = 0;
+        if (lane == 31 && incl) pos = atomicAdd(occn, (uint32_t)incl);
+        pos = __shfl_sync(0xFFFFFFFFu, pos, 31) + (uint32_t)(incl - nfresh);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (fresh >> k & 1u) occ[pos++] = at[k];
         if (lane == 0 && own) atomicAdd(&a.hub_kud[sg.hub], own);
         if (any) s_any = 1;
         __syncthreads();
