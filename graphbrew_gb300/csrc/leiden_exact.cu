@@ -91,7 +91,7 @@ constexpr int kLongThreads = 128;             // rows above that up to kWarpMaxD
 constexpr int kBigMaxDeg = 2048;              // rows above kWarpMaxDeg up to this: one CTA each
 constexpr int kBigThreads = 512;
 constexpr int kHubSeg = 4 * kHubThreads2;     // edges per hub-accumulation CTA (4 per thread)
-constexpr int kTabSeg = 2 * kHubThreads2;     // table slots per hub-selection CTA (2 per thread)
+constexpr int kTabSeg = 2 * kHubThreads2 - 1; // occupied slots per hub-selection CTA (2 per thread, one for the hub's own)
 constexpr unsigned long long kNoChange = ~0ull;
 
 struct Ctl {
@@ -1417,8 +1417,8 @@ __global__ void __launch_bounds__(kHubThreads2) k_ex_hub_accum(ExactState a) {
     hub_accum_body(a, a.ctl);
 }
 
-// Hub selection: one CTA per kTabSeg-slot segment of a window hub's table,
-// one slot per thread; the last CTA of a hub reduces the partial maxima and
+// Hub selection: one CTA per kTabSeg occupied slots of a window hub's table, two
+// per thread, in flight together; the last CTA of a hub reduces the partial maxima and
 // records the decision.  Three CTAs per SM, as for the big rows.
 __device__ __forceinline__ void hub_select_body(const ExactState& a, const Ctl* c) {
     const Round r = round_view(a, c);
@@ -1427,6 +1427,7 @@ __device__ __forceinline__ void hub_select_body(const ExactState& a, const Ctl* 
     __shared__ double red_d[32];
     __shared__ uint32_t red_c[32];
     __shared__ int s_last;
+    __shared__ long long s_own;
     for (long long q = q0 + blockIdx.x; q < q1; q += gridDim.x) {
         const HubSeg sg = a.tseg[q];
         const int j = sg.hub;
@@ -1435,33 +1436,43 @@ __device__ __forceinline__ void hub_select_body(const ExactState& a, const Ctl* 
         const uint32_t* tv = a.tvals + a.hub_toff[j];
         const uint32_t* occ = a.hub_occ + a.hub_toff[j];
         const uint32_t nocc = a.hub_occn[j];
+        const int parts = max(1, (int)((nocc + kTabSeg - 1) / kTabSeg));
+        if (sg.part >= parts) continue;   // block-uniform
         const uint32_t d = a.vcom[h];
         const long long ku = a.rp[h + 1] - a.rp[h];
         const uint32_t kud = a.hub_kud[j];
-        const CommRec rd = load_rec(a, d);
         double best_d = 0.0;
         uint32_t best_c = kNone;
-        // Segment `part` covers occupied-list positions [s0, s0 + kTabSeg):
-        // one per thread per step, the first step's lookup interleaved with
-        // the one for d.
+        // Occupied slots [s0, s0 + kTabSeg); thread 0's first lookup is d's.
+        uint32_t cc[2], wt[2], slot[2];
+        bool vv[2];
+        CommRec rr[2];
         const uint32_t s0 = (uint32_t)sg.part * kTabSeg, s1 = min(nocc, s0 + kTabSeg);
-        if (s0 < s1) {
-            long long sd = 0;
-            for (uint32_t i0 = s0; i0 < s1; i0 += blockDim.x) {
-                const uint32_t i = i0 + threadIdx.x;
-                const uint32_t slot = i < s1 ? occ[i] : 0u;
-                const uint32_t c0 = i < s1 ? tk[slot] : kNone, w0 = i < s1 ? tv[slot] : 0;
-                const uint32_t cc[2] = {c0, d};
-                const bool vv[2] = {c0 != kNone && c0 != d, i0 == s0};
-                const CommRec rr[2] = {vv[0] ? load_rec(a, c0) : rd, rd};
-                long long sgm[2];
-                sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, rr, h, sgm);
-                if (i0 == s0) sd = sgm[1];
-                if (vv[0]) {
-                    const double dl = delta_qi(a.dq, w0, kud, ku, sgm[0], sd);
-                    if (dpos(dl) && better_pos(dl, c0, best_d, best_c)) { best_d = dl; best_c = c0; }
-                }
-            }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const uint32_t i = s0 + k * kHubThreads2 + threadIdx.x - 1u;
+            vv[k] = (k > 0 || threadIdx.x > 0) && i < s1;
+            slot[k] = vv[k] ? occ[i] : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            cc[k] = vv[k] ? tk[slot[k]] : d;
+            wt[k] = vv[k] ? tv[slot[k]] : 0u;
+            vv[k] = vv[k] && cc[k] != d;
+        }
+        vv[0] = vv[0] || threadIdx.x == 0;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) rr[k] = vv[k] ? load_rec(a, cc[k]) : CommRec{0ull, 0u, 0u};
+        long long sgm[2];
+        sigma_at_k<2>(a, r.tag, r.P, r.par, cc, vv, rr, h, sgm);
+        if (threadIdx.x == 0) s_own = sgm[0];
+        __syncthreads();
+        const long long sd = s_own;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (!vv[k] || cc[k] == d) continue;
+            const double dl = delta_qi(a.dq, wt[k], kud, ku, sgm[k], sd);
+            if (dpos(dl) && better_pos(dl, cc[k], best_d, best_c)) { best_d = dl; best_c = cc[k]; }
         }
         warp_argmax_pos(best_d, best_c);
         if (lane == 0) { red_d[w] = best_d; red_c[w] = best_c; }
@@ -1474,7 +1485,7 @@ __device__ __forceinline__ void hub_select_body(const ExactState& a, const Ctl* 
             a.part_d[q] = bd;
             a.part_c[q] = bc;
             __threadfence();
-            s_last = atomicAdd(&a.hub_done[j], 1) == a.hub_tcount[j] - 1;
+            s_last = atomicAdd(&a.hub_done[j], 1) == parts - 1;
         }
         __syncthreads();
         if (s_last) {
@@ -1482,8 +1493,8 @@ __device__ __forceinline__ void hub_select_body(const ExactState& a, const Ctl* 
             __threadfence();
             double bd = 0.0;
             uint32_t bc = kNone;
-            const int f = a.hub_tfirst[j], nt = a.hub_tcount[j];
-            for (int k = threadIdx.x; k < nt; k += blockDim.x) {
+            const int f = a.hub_tfirst[j];
+            for (int k = threadIdx.x; k < parts; k += blockDim.x) {
                 const double pd = ((volatile double*)a.part_d)[f + k];
                 const uint32_t pc = ((volatile uint32_t*)a.part_c)[f + k];
                 if (better_pos(pd, pc, bd, bc)) { bd = pd; bc = pc; }
@@ -1498,15 +1509,7 @@ __device__ __forceinline__ void hub_select_body(const ExactState& a, const Ctl* 
                 for (int k = 1; k < (int)(blockDim.x / 32); ++k)
                     if (better_pos(red_d[k], red_c[k], bd, bc)) { bd = red_d[k]; bc = red_c[k]; }
                 const bool act = a.vaff[h] != 0 || ((volatile int32_t*)a.hub_any)[j] != 0;
-                bool stays = false;
-                if (a.vcob) {
-                    const uint32_t cc[1] = {d};
-                    const bool vv[1] = {true};
-                    const CommRec rr[1] = {rd};
-                    long long o[1];
-                    sigma_at_k<1>(a, r.tag, r.P, r.par, cc, vv, rr, h, o);
-                    stays = refine_stays(a, (double)o[0], ku);
-                }
+                const bool stays = refine_stays(a, (double)sd, (double)ku);
                 if (act && !stays && bd > 0.0 && bc != kNone && bc != d) record(a, r, h, d, bc, bd);
                 else record(a, r, h, d, kNoMove, 0.0);
                 a.hub_done[j] = 0;
