@@ -93,6 +93,8 @@ constexpr int kBigThreads = 512;
 constexpr int kHubSeg = 4 * kHubThreads2;     // edges per hub-accumulation CTA (4 per thread)
 constexpr int kTabSeg = 2 * kHubThreads2 - 1; // occupied slots per hub-selection CTA (2 per thread, one for the hub's own)
 constexpr unsigned long long kNoChange = ~0ull;
+constexpr int kIndexV = 64;                   // vertices per entry of the lists' index
+constexpr int kIndexLists = 5;
 
 struct Ctl {
     long long P, E, n;
@@ -201,6 +203,8 @@ struct ExactState {
     long long n_mid;
     const uint32_t* long_v;       // vertices with kMidMaxDeg < degree <= kWarpMaxDeg (ascending)
     long long n_long;
+    const int32_t* list_index;    // per list of window_ranges: entries before each kIndexV-th vertex
+    long long index_len;
     const uint32_t* big_v;        // vertices with kWarpMaxDeg < degree <= kBigMaxDeg (ascending)
     long long n_big;
     cudaGraphConditionalHandle cond;  // while-node condition (graph-driven rounds)
@@ -382,8 +386,14 @@ __device__ __forceinline__ bool prev_mover(const ExactState& a, const Round& r, 
     return (r.pdec[v] & kNoMove) != kNoMove;
 }
 
+// Vertices that enter with this window (from pE on) have no decision yet: the
+// insert kernel marks them, beside the hub accumulation.
+__device__ __forceinline__ bool decided_before(const Round& r, int64_t v, int64_t u) {
+    return v >= r.P && v < u && v < r.pE;
+}
+
 __device__ __forceinline__ uint32_t comm_at(const ExactState& a, const Round& r, int64_t v, int64_t u) {
-    if (v >= r.P && v < u) {
+    if (decided_before(r, v, u)) {
         const uint32_t to = r.pdec[v] & kNoMove;
         if (to != kNoMove) return to;
     }
@@ -504,13 +514,21 @@ __device__ __forceinline__ long long warp_lower_bound_u32(const uint32_t* a, lon
 }
 
 // Window ranges of the hub segment lists and the mid, long and big-row lists
-// for the window [P, E): ten searches on warps 0-9.
+// for the window [P, E): ten searches on warps 0-9, within the entries of a block of
+// kIndexV vertices (over the whole lists they took five dependent loads each, of an
+// advance that every round waits for).
 __device__ __forceinline__ void window_ranges(const ExactState& a, Ctl* c, long long P, long long E) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (w >= 10) return;
     const uint32_t* arr = w < 2 ? a.eseg_v : (w < 4 ? a.tseg_v : (w < 6 ? a.mid_v : (w < 8 ? a.big_v : a.long_v)));
+    const long long v = (w & 1) ? E : P;
     const long long len = w < 2 ? a.n_eseg : (w < 4 ? a.n_tseg : (w < 6 ? a.n_mid : (w < 8 ? a.n_big : a.n_long)));
-    const long long pos = warp_lower_bound_u32(arr, len, (uint32_t)((w & 1) ? E : P), lane);
+    long long pos = 0;
+    if (len) {
+        const int32_t* ix = a.list_index + (size_t)(w >> 1) * a.index_len + (v / kIndexV);
+        const long long lo = ix[0], hi = ix[1];
+        pos = lo + warp_lower_bound_u32(arr + lo, hi - lo, (uint32_t)v, lane);
+    }
     if (lane == 0) {
         switch (w) {
             case 0: c->es0 = pos; break;
@@ -610,7 +628,9 @@ __global__ void __launch_bounds__(kTbThreads) k_tb_insert(ExactState a) {
     int dg = 0;
     if (i < W) {
         const int64_t wv = P + i;
-        const uint32_t pb = r.pdec[wv] & kNoMove, vc = a.vcom[wv];
+        const bool enters = wv >= r.pE;
+        if (enters) a.dec[r.par][wv] = kNoMove;
+        const uint32_t pb = enters ? kNoMove : r.pdec[wv] & kNoMove, vc = a.vcom[wv];
         const int64_t r0 = a.rp[wv], r1 = a.rp[wv + 1];
         if (pb != kNoMove) {
             dg = (int)(r1 - r0);
@@ -1215,7 +1235,7 @@ __device__ __forceinline__ void eval_row_cta(const ExactState& a, const Ctl* c, 
                 c[k] = kNone;
                 if (e < re) {
                     const int32_t v = a.col[e];
-                    any = any || (v >= r.P && v < (int64_t)u && prev_mover(a, r, v));
+                    any = any || (decided_before(r, v, u) && prev_mover(a, r, v));
                     if (counts(a, v, u, ub)) c[k] = comm_at(a, r, v, u);
                 }
             }
@@ -1332,6 +1352,13 @@ __global__ void k_degree_scatter(const int32_t* __restrict__ flag, const int64_t
         if (flag[v]) out[pos[v]] = (uint32_t)v;
 }
 
+// Entries of an ascending list before each kIndexV-th vertex; the last one: all.
+__global__ void k_list_index(const uint32_t* __restrict__ list, int64_t len, int64_t entries,
+                             int32_t* __restrict__ out) {
+    for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < entries; b += (int64_t)gridDim.x * blockDim.x)
+        out[b] = (int32_t)(b == entries - 1 ? len : lower_bound_u32(list, len, (uint32_t)(b * kIndexV)));
+}
+
 // Hub accumulation: one CTA per kHubSeg-edge segment of a window hub, four
 // edges per thread in flight, and their first probes (one edge after another took
 // R-MAT-22's rounds 38 us here, now 21; counting a segment in shared memory first
@@ -1364,7 +1391,7 @@ __device__ __forceinline__ void hub_accum_body(const ExactState& a, const Ctl* c
             c[k] = kNone;
             if (e < e1) {
                 const int32_t v = a.col[e];
-                any = any || (v >= r.P && v < (int64_t)h && prev_mover(a, r, v));
+                any = any || (decided_before(r, v, h) && prev_mover(a, r, v));
                 if (counts(a, v, h, ub)) c[k] = comm_at(a, r, v, h);
             }
         }
@@ -1789,14 +1816,11 @@ __device__ __forceinline__ long long window_length(const Ctl* c, long long progr
 }
 
 // After the window's decisions: fix the committed prefix [P, x] for the commit
-// kernels, slide the window (the new decisions become D_prev; entering
-// vertices are unknown) and tell the graph's loop whether to go on.  The next
+// kernels, slide the window (the new decisions become D_prev) and tell the graph's loop whether to go on.  The next
 // window's event table and this window's commits then run concurrently: they
-// touch disjoint vertices.  `c` is the control block this CTA works on; the
-// entering vertices' marks are written by threads (tid0, tid0 + tstride, ...).
-// Ends with a CTA barrier, so every thread sees the updated block.
-__device__ __forceinline__ void advance_ctl(const ExactState& a, Ctl* c, long long tid0, long long tstride,
-                                            bool set_cond) {
+// touch disjoint vertices.  Ends with a CTA barrier, so every thread sees the
+// updated block.
+__device__ __forceinline__ void advance_ctl(const ExactState& a, Ctl* c, bool set_cond) {
     const long long P = c->P, E = c->E, n = c->n;
     if (P >= n) {
         __syncthreads();
@@ -1813,9 +1837,6 @@ __device__ __forceinline__ void advance_ctl(const ExactState& a, Ctl* c, long lo
     const long long progress = c->progress + (64 * (nP - P) - c->progress) / 16;
     // May end before E: what is dropped enters again as new.
     const long long nE = min(n, nP + window_length(c, progress));
-    const int par = (int)(c->round & 1);
-    uint32_t* next_dec = a.dec[par ^ 1];
-    for (long long u = E + tid0; u < nE; u += tstride) next_dec[u] = kNoMove;
     if (threadIdx.x == 0) {
         c->c_es0 = c->es0;
         c->c_es1 = c->es1;
@@ -1866,14 +1887,13 @@ __device__ __forceinline__ void advance_ctl(const ExactState& a, Ctl* c, long lo
 }
 
 __global__ void __launch_bounds__(1024) k_ex_advance(ExactState a) {
-    advance_ctl(a, a.ctl, threadIdx.x, blockDim.x, a.use_cond != 0);
+    advance_ctl(a, a.ctl, a.use_cond != 0);
 }
 
-// The first window of an iteration; same split of the marks as advance_ctl.
-__device__ __forceinline__ void init_ctl(const ExactState& a, Ctl* c, long long tid0, long long tstride) {
+// The first window of an iteration.
+__device__ __forceinline__ void init_ctl(const ExactState& a, Ctl* c) {
     const long long n = c->n;
     const long long E = min(n, window_length(c, c->progress));
-    for (long long u = tid0; u < E; u += tstride) a.dec[0][u] = kNoMove;
     window_ranges(a, c, 0, E);
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1892,7 +1912,7 @@ __device__ __forceinline__ void init_ctl(const ExactState& a, Ctl* c, long long 
 }
 
 __global__ void __launch_bounds__(1024) k_ex_init_iter(ExactState a) {
-    init_ctl(a, a.ctl, threadIdx.x, blockDim.x);
+    init_ctl(a, a.ctl);
 }
 
 // Deterministic tree sum of the iteration's committed deltas (and count).
@@ -2062,6 +2082,18 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
         n_long = list(kMidMaxDeg, kWarpMaxDeg, long_v);
     }
 
+    const int64_t index_len = n / kIndexV + 2;
+    DevBuf<int32_t> list_index(kIndexLists * index_len, s);
+    {
+        const uint32_t* lists[kIndexLists] = {d_eseg_v.get(), d_tseg_v.get(), mid_v.get(), d_big_v.get(), long_v.get()};
+        const int64_t lens[kIndexLists] = {(int64_t)eseg_v.size(), (int64_t)tseg_v.size(), n_mid, n_big, n_long};
+        for (int k = 0; k < kIndexLists; ++k) {
+            k_list_index<<<grid_for(index_len, kT), kT, 0, s>>>(lists[k], lens[k], index_len,
+                                                               list_index.get() + k * index_len);
+            GB_LAUNCH_CHECK();
+        }
+    }
+
     // ---- round state ----
     DevBuf<uint32_t> dec0(n, s), dec1(n, s);
     DevBuf<double> delta(n, s), final_delta(n, s);
@@ -2146,6 +2178,8 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     a.n_mid = n_mid;
     a.long_v = long_v.get();
     a.n_long = n_long;
+    a.list_index = list_index.get();
+    a.index_len = index_len;
     a.M = ctx.M;
     a.R = ctx.R;
     a.dq = ctx.dq;
