@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cmath>
+#include <memory>
 #include <vector>
 
 #include "gb_common.cuh"
@@ -192,10 +193,13 @@ struct LocalMoveContext {
     uint32_t* hub_gk = nullptr;           // per-CTA global tables for very large hubs
     uint32_t* hub_gv = nullptr;
     int64_t hub_gcap = 0;
+    std::shared_ptr<struct RowLists> rows;   // local_move_exact's lists of the graph's rows by length
 };
 
-// Serial-order local moving (leiden_exact.cu).  Returns the iterations run.
-int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iterations, int64_t window,
+// Serial-order local moving (leiden_exact.cu).  Returns the iterations run.  The
+// first call on a context lists its graph's rows; the mapping's later passes use
+// the lists again.
+int local_move_exact(LocalMoveContext& ctx, double tolerance, int max_iterations, int64_t window,
                      cudaStream_t s, int64_t* launches, int64_t* rounds_out, int64_t* evals_out);
 
 }  // namespace gb

@@ -1986,12 +1986,24 @@ DevBuf<T> upload(const std::vector<T>& v, cudaStream_t s) {
 
 }  // namespace
 
-int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iterations, int64_t window,
-                     cudaStream_t s, int64_t* launches, int64_t* rounds_out, int64_t* evals_out) {
-    const int64_t n = ctx.g.n;
-    const int64_t B = std::max<int64_t>(32, std::min<int64_t>(std::min<int64_t>(window, kWindowMax), n));
+// A graph's rows above kSmallMaxDeg by length, with the segments of the longest:
+// what local moving needs to know of the graph, the same in every pass (R-MAT-22:
+// 1 ms of host work and copies).
+struct RowLists {
+    int64_t nh = 0, n_big = 0, n_mid = 0, n_long = 0, n_eseg = 0, n_tseg = 0;
+    int64_t pool = 0;        // slots of the hubs' tables
+    int64_t index_len = 0;
+    DevBuf<int64_t> toff;
+    DevBuf<uint32_t> tcap;
+    DevBuf<int32_t> tfirst, tcount, index;
+    DevBuf<HubSeg> eseg, tseg;
+    DevBuf<uint32_t> eseg_v, tseg_v, hub_v, big_v, mid_v, long_v;
+};
 
-    // ---- hub segment tables (once per call) ----
+static std::shared_ptr<RowLists> list_rows(const LocalMoveContext& ctx, cudaStream_t s) {
+    const int64_t n = ctx.g.n;
+    auto rows = std::make_shared<RowLists>();
+    RowLists& L = *rows;
     // Rows above kWarpMaxDeg: up to kBigMaxDeg one CTA each ("big"), above
     // that segmented over CTAs ("hubs").
     const int64_t nh_all = (int64_t)ctx.hubs_h.size();
@@ -2013,19 +2025,20 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
             hdeg.push_back(hdeg_all[j]);
         }
     }
-    const int64_t nh = (int64_t)hub_h.size(), n_big = (int64_t)big_h.size();
+    const int64_t nh = (int64_t)hub_h.size();
+    L.nh = nh;
+    L.n_big = (int64_t)big_h.size();
     std::vector<int64_t> toff(nh);
     std::vector<uint32_t> tcap(nh);
     std::vector<int32_t> tfirst(nh), tcount(nh);
     std::vector<HubSeg> eseg, tseg;
     std::vector<uint32_t> eseg_v, tseg_v;
-    int64_t pool = 0;
     for (int64_t j = 0; j < nh; ++j) {
         uint32_t cap = 64;
         while ((int64_t)cap < 2 * hdeg[j]) cap <<= 1;
         tcap[j] = cap;
-        toff[j] = pool;
-        pool += cap;
+        toff[j] = L.pool;
+        L.pool += cap;
         const int ne = (int)ceil_div(hdeg[j], kHubSeg);
         for (int k = 0; k < ne; ++k) {
             eseg.push_back({(int32_t)j, k});
@@ -2039,12 +2052,67 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
             tseg_v.push_back(hub_h[j]);
         }
     }
-    DevBuf<int64_t> d_toff = upload(toff, s);
-    DevBuf<uint32_t> d_tcap = upload(tcap, s);
-    DevBuf<int32_t> d_tfirst = upload(tfirst, s), d_tcount = upload(tcount, s);
-    DevBuf<HubSeg> d_eseg = upload(eseg, s), d_tseg = upload(tseg, s);
-    DevBuf<uint32_t> d_eseg_v = upload(eseg_v, s), d_tseg_v = upload(tseg_v, s);
-    DevBuf<uint32_t> d_hub_v = upload(hub_h, s), d_big_v = upload(big_h, s);
+    L.toff = upload(toff, s);
+    L.tcap = upload(tcap, s);
+    L.tfirst = upload(tfirst, s);
+    L.tcount = upload(tcount, s);
+    L.eseg = upload(eseg, s);
+    L.tseg = upload(tseg, s);
+    L.eseg_v = upload(eseg_v, s);
+    L.tseg_v = upload(tseg_v, s);
+    L.hub_v = upload(hub_h, s);
+    L.big_v = upload(big_h, s);
+    L.n_eseg = (int64_t)eseg.size();
+    L.n_tseg = (int64_t)tseg.size();
+
+    // Mid and long rows: both counts in one look at the device.
+    {
+        DevBuf<int32_t> flag(2 * n, s);
+        DevBuf<int64_t> pos(2 * n, s), tot(2, s);
+        const int64_t above[2] = {kSmallMaxDeg, kMidMaxDeg}, most[2] = {kMidMaxDeg, kWarpMaxDeg};
+        for (int k = 0; k < 2; ++k) {
+            k_degree_flags<<<grid_for(n, kT), kT, 0, s>>>(ctx.g.row_ptr, n, above[k], most[k], flag.get() + k * n);
+            GB_LAUNCH_CHECK();
+            exclusive_scan_i32_to_i64(flag.get() + k * n, pos.get() + k * n, n, tot.get() + k, s);
+        }
+        int64_t counts[2];
+        GB_CUDA(cudaMemcpyAsync(counts, tot.get(), sizeof(counts), cudaMemcpyDeviceToHost, s));
+        GB_CUDA(cudaStreamSynchronize(s));
+        DevBuf<uint32_t>* out[2] = {&L.mid_v, &L.long_v};
+        for (int k = 0; k < 2; ++k) {
+            out[k]->alloc(counts[k] > 0 ? counts[k] : 1, s);
+            if (counts[k] == 0) continue;
+            k_degree_scatter<<<grid_for(n, kT), kT, 0, s>>>(flag.get() + k * n, pos.get() + k * n, n, out[k]->get());
+            GB_LAUNCH_CHECK();
+        }
+        L.n_mid = counts[0];
+        L.n_long = counts[1];
+    }
+
+    L.index_len = n / kIndexV + 2;
+    L.index.alloc(kIndexLists * L.index_len, s);
+    const uint32_t* lists[kIndexLists] = {L.eseg_v.get(), L.tseg_v.get(), L.mid_v.get(), L.big_v.get(),
+                                          L.long_v.get()};
+    const int64_t lens[kIndexLists] = {L.n_eseg, L.n_tseg, L.n_mid, L.n_big, L.n_long};
+    for (int k = 0; k < kIndexLists; ++k) {
+        if (lens[k] == 0) continue;   // window_ranges does not look
+        k_list_index<<<grid_for(L.index_len, kT), kT, 0, s>>>(lists[k], lens[k], L.index_len,
+                                                             L.index.get() + k * L.index_len);
+        GB_LAUNCH_CHECK();
+    }
+    return rows;
+}
+
+int local_move_exact(LocalMoveContext& ctx, double tolerance, int max_iterations, int64_t window,
+                     cudaStream_t s, int64_t* launches, int64_t* rounds_out, int64_t* evals_out) {
+    const int64_t n = ctx.g.n;
+    const int64_t B = std::max<int64_t>(32, std::min<int64_t>(std::min<int64_t>(window, kWindowMax), n));
+
+    if (!ctx.rows) ctx.rows = list_rows(ctx, s);
+    const RowLists& L = *ctx.rows;
+    const int64_t nh = L.nh, n_big = L.n_big, n_mid = L.n_mid, n_long = L.n_long, pool = L.pool;
+
+    // ---- hub tables ----
     DevBuf<uint32_t> tkeys(pool > 0 ? pool : 1, s), tvals(pool > 0 ? pool : 1, s);
     GB_CUDA(cudaMemsetAsync(tkeys, 0xFF, (pool > 0 ? pool : 1) * sizeof(uint32_t), s));
     GB_CUDA(cudaMemsetAsync(tvals, 0, (pool > 0 ? pool : 1) * sizeof(uint32_t), s));
@@ -2057,42 +2125,8 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     GB_CUDA(cudaMemsetAsync(hub_occn, 0, (nh > 0 ? nh : 1) * sizeof(uint32_t), s));
     GB_CUDA(cudaMemsetAsync(hub_clr, 0, (nh > 0 ? nh : 1) * sizeof(int32_t), s));
     GB_CUDA(cudaMemsetAsync(hub_kud, 0, (nh > 0 ? nh : 1) * sizeof(uint32_t), s));
-    DevBuf<double> part_d(tseg.empty() ? 1 : tseg.size(), s);
-    DevBuf<uint32_t> part_c(tseg.empty() ? 1 : tseg.size(), s);
-
-    // ---- mid and long rows (ascending vertex ids) ----
-    int64_t n_mid = 0, n_long = 0;
-    DevBuf<uint32_t> mid_v, long_v;
-    {
-        DevBuf<int32_t> flag(n, s);
-        DevBuf<int64_t> pos(n, s), tot(1, s);
-        auto list = [&](int64_t above, int64_t most, DevBuf<uint32_t>& out) {
-            k_degree_flags<<<grid_for(n, kT), kT, 0, s>>>(ctx.g.row_ptr, n, above, most, flag);
-            GB_LAUNCH_CHECK();
-            exclusive_scan_i32_to_i64(flag, pos, n, tot, s);
-            const int64_t count = read_dev(tot.get(), s);
-            out.alloc(count > 0 ? count : 1, s);
-            if (count) {
-                k_degree_scatter<<<grid_for(n, kT), kT, 0, s>>>(flag, pos, n, out);
-                GB_LAUNCH_CHECK();
-            }
-            return count;
-        };
-        n_mid = list(kSmallMaxDeg, kMidMaxDeg, mid_v);
-        n_long = list(kMidMaxDeg, kWarpMaxDeg, long_v);
-    }
-
-    const int64_t index_len = n / kIndexV + 2;
-    DevBuf<int32_t> list_index(kIndexLists * index_len, s);
-    {
-        const uint32_t* lists[kIndexLists] = {d_eseg_v.get(), d_tseg_v.get(), mid_v.get(), d_big_v.get(), long_v.get()};
-        const int64_t lens[kIndexLists] = {(int64_t)eseg_v.size(), (int64_t)tseg_v.size(), n_mid, n_big, n_long};
-        for (int k = 0; k < kIndexLists; ++k) {
-            k_list_index<<<grid_for(index_len, kT), kT, 0, s>>>(lists[k], lens[k], index_len,
-                                                               list_index.get() + k * index_len);
-            GB_LAUNCH_CHECK();
-        }
-    }
+    DevBuf<double> part_d(L.n_tseg > 0 ? L.n_tseg : 1, s);
+    DevBuf<uint32_t> part_c(L.n_tseg > 0 ? L.n_tseg : 1, s);
 
     // ---- round state ----
     DevBuf<uint32_t> dec0(n, s), dec1(n, s);
@@ -2151,19 +2185,19 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     a.zcand = zcand.get();
     a.stime = stime.get();
     a.epre = epre.get();
-    a.hub_v = d_hub_v.get();
-    a.big_v = d_big_v.get();
+    a.hub_v = L.hub_v.get();
+    a.big_v = L.big_v.get();
     a.n_big = n_big;
-    a.hub_toff = d_toff.get();
-    a.hub_tcap = d_tcap.get();
-    a.hub_tfirst = d_tfirst.get();
-    a.hub_tcount = d_tcount.get();
-    a.eseg = d_eseg.get();
-    a.eseg_v = d_eseg_v.get();
-    a.n_eseg = (long long)eseg.size();
-    a.tseg = d_tseg.get();
-    a.tseg_v = d_tseg_v.get();
-    a.n_tseg = (long long)tseg.size();
+    a.hub_toff = L.toff.get();
+    a.hub_tcap = L.tcap.get();
+    a.hub_tfirst = L.tfirst.get();
+    a.hub_tcount = L.tcount.get();
+    a.eseg = L.eseg.get();
+    a.eseg_v = L.eseg_v.get();
+    a.n_eseg = L.n_eseg;
+    a.tseg = L.tseg.get();
+    a.tseg_v = L.tseg_v.get();
+    a.n_tseg = L.n_tseg;
     a.tkeys = tkeys.get();
     a.tvals = tvals.get();
     a.hub_any = hub_any.get();
@@ -2174,12 +2208,12 @@ int local_move_exact(const LocalMoveContext& ctx, double tolerance, int max_iter
     a.hub_done = hub_done.get();
     a.part_d = part_d.get();
     a.part_c = part_c.get();
-    a.mid_v = mid_v.get();
+    a.mid_v = L.mid_v.get();
     a.n_mid = n_mid;
-    a.long_v = long_v.get();
+    a.long_v = L.long_v.get();
     a.n_long = n_long;
-    a.list_index = list_index.get();
-    a.index_len = index_len;
+    a.list_index = L.index.get();
+    a.index_len = L.index_len;
     a.M = ctx.M;
     a.R = ctx.R;
     a.dq = ctx.dq;
