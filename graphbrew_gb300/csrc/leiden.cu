@@ -496,11 +496,13 @@ struct SmArgs {
 // relative error 2^-24, A carries three such errors, a product with it five, so
 // y is within 12 x 2^-24 (w(e) + A s(e) + w(d) + rem) of the real value, and the
 // double evaluation within 2^-48 of the same sum; E is 2^-19 of the largest such
-// sum, more than twice both.  If all candidates within 2 E of the largest score
-// are communities other than d with the same w and s, their exact deltas are
-// equal and above all others': the smallest id among them is the exact winner;
-// if the largest score is further than E from 0, its sign is certain as well.
-// Everything else takes the exact evaluation.  A mapping of 300 K vertices in
+// sum, more than twice both.  The exact winner is among the candidates within
+// 2 E of the largest score.  If those are communities other than d with the same
+// w, it is the one with the smallest s, then the smallest id: the deltas fall with
+// s, and a step of one in s, worth A, is far above the double evaluation's error
+// (A >= 2^-11 E is asked where their s differ; a super-graph of a uniform graph has
+// many candidates of weight 1 and nearly the same s).  A largest score above 3 E or
+// below -E makes the sign certain.  Everything else takes the exact evaluation.  A mapping of 300 K vertices in
 // planted communities: 25.2 to 23.1 ms.
 struct FilterScore {
     float A, rem, wd;
@@ -518,8 +520,18 @@ struct FilterScore {
     __device__ __forceinline__ float bound(float max_mag) const {
         return 1.9073486e-6f * (max_mag + wd + fabsf(rem));   // 2^-19
     }
+    __device__ __forceinline__ bool tells_totals(float E) const { return A >= 4.8828125e-4f * E; }   // 2^-11
 };
 constexpr float kNoScore = -3.402823466e38f;
+constexpr unsigned long long kMaxTotal = 0x7FFFFFFFFFFFFFFFull;
+
+// Largest value of a warp (no NaN), compared as integers of the same order.
+__device__ __forceinline__ float warp_max(float x) {
+    int i = __float_as_int(x);
+    i ^= (i >> 31) & 0x7FFFFFFF;
+    i = __reduce_max_sync(0xFFFFFFFFu, i);
+    return __int_as_float(i ^ ((i >> 31) & 0x7FFFFFFF));
+}
 
 constexpr int kSmSmall = 256;     // per-warp shared table slots
 
@@ -610,6 +622,57 @@ __device__ void super_propose_cached(const SmArgs& a, uint32_t c, uint32_t* tk, 
     }
     __syncwarp();
     const uint32_t own_w = table_get(k, v, mask, d);
+    out.c = c;
+    out.d = d;
+    out.kc = kcl;
+    {
+        const FilterScore f(a, kcl, (long long)sd_raw, own_w);
+        float top = own_w ? f.own() : kNoScore, mag = 0.f;
+        for (uint32_t i = lane; i < H; i += 32) {
+            const uint32_t ek = k[i];
+            if (ek == kNone || ek == d) continue;
+            const long long se = (long long)(shared ? tt[i] : a.sctot[ek]);
+            top = fmaxf(top, f.score(v[i], se));
+            mag = fmaxf(mag, f.mag(v[i], se));
+        }
+        top = warp_max(top);
+        mag = warp_max(mag);
+        const float E = f.bound(mag);
+        const bool own_near = own_w && f.own() >= top - 2.f * E;
+        bool near = false, one_w = true, one_s = true;
+        uint32_t w0 = 0, id = kNone;
+        unsigned long long s0 = kMaxTotal;
+        for (uint32_t i = lane; i < H; i += 32) {
+            const uint32_t ek = k[i];
+            if (ek == kNone || ek == d) continue;
+            const unsigned long long se = shared ? tt[i] : a.sctot[ek];
+            if (f.score(v[i], (long long)se) < top - 2.f * E) continue;
+            one_w = one_w && (!near || v[i] == w0);
+            one_s = one_s && (!near || se == s0);
+            if (se < s0 || (se == s0 && ek < id)) {
+                s0 = se;
+                id = ek;
+            }
+            near = true;
+            w0 = v[i];
+        }
+        // The smallest total, then the smallest id (totals are not negative).
+        const uint32_t hi = __reduce_min_sync(0xFFFFFFFFu, (uint32_t)(s0 >> 32));
+        const uint32_t lo = __reduce_min_sync(0xFFFFFFFFu, (uint32_t)(s0 >> 32) == hi ? (uint32_t)s0 : 0xFFFFFFFFu);
+        const unsigned long long least = (unsigned long long)hi << 32 | lo;
+        const uint32_t best = __reduce_min_sync(0xFFFFFFFFu, s0 == least ? id : kNone);
+        const unsigned nb = __ballot_sync(0xFFFFFFFFu, near);
+        const uint32_t ws = __shfl_sync(0xFFFFFFFFu, w0, nb ? __ffs(nb) - 1 : 0);
+        const bool all_w = !__any_sync(0xFFFFFFFFu, near && (!one_w || w0 != ws));
+        const bool all_s = !__any_sync(0xFFFFFFFFu, near && (!one_s || s0 != least));
+        const bool stays = nb == 0 || top < -E;
+        if (E <= 1e30f && (stays || (all_w && (all_s || f.tells_totals(E)) && !own_near && top > 3.f * E))) {
+            out.best = stays ? d : best;
+            out.delta = stays ? 0.0 : 1.0;
+            __syncwarp();
+            return;
+        }
+    }
     // Occupied slots to the front, in slot order: the scoring loop then takes
     // ceil(occupied / 32) full-warp steps instead of H / 32 mostly idle ones
     // (an FP64 instruction costs the same with one lane active or 32).
@@ -628,54 +691,6 @@ __device__ void super_propose_cached(const SmArgs& a, uint32_t c, uint32_t* tk, 
         }
         __syncwarp();
         occ += (uint32_t)__popc(m);
-    }
-    out.c = c;
-    out.d = d;
-    out.kc = kcl;
-    {
-        const FilterScore f(a, kcl, (long long)sd_raw, own_w);
-        float top = own_w ? f.own() : kNoScore, mag = 0.f;
-        for (uint32_t i = lane; i < occ; i += 32) {
-            if (k[i] == d) continue;
-            const long long se = (long long)(shared ? tt[i] : a.sctot[k[i]]);
-            top = fmaxf(top, f.score(v[i], se));
-            mag = fmaxf(mag, f.mag(v[i], se));
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
-            mag = fmaxf(mag, __shfl_xor_sync(0xFFFFFFFFu, mag, o));
-        }
-        const float E = f.bound(mag);
-        const bool own_near = own_w && f.own() >= top - 2.f * E;
-        bool near = false, same = true;
-        uint32_t w0 = 0, id = kNone;
-        long long s0 = 0;
-        for (uint32_t i = lane; i < occ; i += 32) {
-            if (k[i] == d) continue;
-            const long long se = (long long)(shared ? tt[i] : a.sctot[k[i]]);
-            if (f.score(v[i], se) < top - 2.f * E) continue;
-            if (!near) {
-                near = true;
-                w0 = v[i];
-                s0 = se;
-            }
-            same = same && v[i] == w0 && se == s0;
-            id = min(id, k[i]);
-        }
-        const unsigned nb = __ballot_sync(0xFFFFFFFFu, near);
-        const int src = nb ? __ffs(nb) - 1 : 0;
-        const uint32_t ws = __shfl_sync(0xFFFFFFFFu, w0, src);
-        const long long ss = __shfl_sync(0xFFFFFFFFu, s0, src);
-        const bool one = !__any_sync(0xFFFFFFFFu, near && (!same || w0 != ws || s0 != ss));
-        const uint32_t best = __reduce_min_sync(0xFFFFFFFFu, id);
-        const bool stays = nb == 0 || top < -E;
-        if (E <= 1e30f && (nb == 0 || (one && !own_near && fabsf(top) > E))) {
-            out.best = stays ? d : best;
-            out.delta = stays ? 0.0 : 1.0;
-            __syncwarp();
-            return;
-        }
     }
     const double kc_to_d = (double)own_w;
     const double kc = (double)kcl;
@@ -814,22 +829,24 @@ __device__ void super_propose_light(const SmArgs& a, uint32_t c, SmProposal& out
         }
         const float E = f.bound(mag);
         const bool own_near = kc_to_d_w && f.own() >= top - 2.f * E;
-        bool any = false, one = true;
+        bool any = false, one_w = true, one_s = true;
         uint32_t id = kNone, w0 = 0;
-        unsigned long long s0 = 0;
+        long long s0 = (long long)kMaxTotal;
 #pragma unroll
         for (int k = 0; k < kLightDeg; ++k) {
             if (key[k] == kNone || key[k] == d || y[k] < top - 2.f * E) continue;
-            if (!any) {
-                w0 = wsum[k];
-                s0 = se_raw[k];
+            const long long se = (long long)se_raw[k];
+            one_w = one_w && (!any || wsum[k] == w0);
+            one_s = one_s && (!any || se == s0);
+            if (se < s0 || (se == s0 && key[k] < id)) {
+                s0 = se;
+                id = key[k];
             }
             any = true;
-            one = one && wsum[k] == w0 && se_raw[k] == s0;
-            id = min(id, key[k]);
+            w0 = wsum[k];
         }
-        if (E <= 1e30f && (!any || (one && !own_near && fabsf(top) > E))) {
-            const bool stays = !any || top < -E;
+        const bool stays = !any || top < -E;
+        if (E <= 1e30f && (stays || (one_w && (one_s || f.tells_totals(E)) && !own_near && top > 3.f * E))) {
             out.best = stays ? d : id;
             out.delta = stays ? 0.0 : 1.0;
             return;
