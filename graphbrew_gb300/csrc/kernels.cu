@@ -89,8 +89,20 @@ __device__ __forceinline__ double pr_put(const PrArgs& a, int64_t u, float s, in
 // sector.  RMAT scale 20, 33 M entries: a warp per row 1.43 ms a sweep (nearly
 // all of it the largest row's), lanes, warps and CTAs by row length 0.48 ms.
 // Rows without entries keep the score that k_pr_isolated gives them.
+// A lane adds its entries up with the rounding errors kept beside the sum (Knuth's
+// two-sum), so that 24 of them in a row are no further off than a tree over a warp.
 constexpr int kPrOwn = 24;      // rows up to this long by a thread
 constexpr int kPrOctet = 256;   // up to this long by eight lanes, longer ones by a warp
+
+struct PrSum {
+    float s = 0.f, c = 0.f;
+    __device__ __forceinline__ void add(float x) {
+        const float t = __fadd_rn(s, x), z = __fsub_rn(t, s);
+        c = __fadd_rn(c, __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(x, z)));
+        s = t;
+    }
+    __device__ __forceinline__ float value() const { return s + c; }
+};
 
 __global__ void __launch_bounds__(kT, 6) k_pr_sweep(PrArgs a, int it) {
     if (pr_done(a.err, it, a.epsilon)) return;
@@ -127,7 +139,9 @@ __global__ void __launch_bounds__(kT, 6) k_pr_sweep(PrArgs a, int it) {
             if (t == kT - 1) s_more = rb < e1;
             float s = 0.f;
             if (e - b <= kPrOwn) {
-                for (int i = b; i < e; ++i) s += val[chunk_pad(i)];
+                PrSum x;
+                for (int i = b; i < e; ++i) x.add(val[chunk_pad(i)]);
+                s = x.value();
             } else {
                 list[atomicAdd(&s_listed, 1)] = (uint8_t)t;
                 sb[t] = b;
@@ -138,17 +152,19 @@ __global__ void __launch_bounds__(kT, 6) k_pr_sweep(PrArgs a, int it) {
             for (int q = t >> 3; q - (t >> 3) < listed; q += kT / 8) {
                 const int w = q < listed ? list[q] : 0;
                 const bool mine = q < listed && se[w] - sb[w] <= kPrOctet;
-                float x = 0.f;
+                PrSum p;
                 if (mine)
-                    for (int i = sb[w] + (lane & 7); i < se[w]; i += 8) x += val[chunk_pad(i)];
+                    for (int i = sb[w] + (lane & 7); i < se[w]; i += 8) p.add(val[chunk_pad(i)]);
+                float x = p.value();
                 for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
                 if (mine && (lane & 7) == 0) sums[w] = x;
             }
             for (int q = t >> 5; q < listed; q += kT / 32) {
                 const int w = list[q];
                 if (se[w] - sb[w] <= kPrOctet) continue;
-                float x = 0.f;
-                for (int i = sb[w] + lane; i < se[w]; i += 32) x += val[chunk_pad(i)];
+                PrSum p;
+                for (int i = sb[w] + lane; i < se[w]; i += 32) p.add(val[chunk_pad(i)]);
+                float x = p.value();
                 for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
                 if (lane == 0) sums[w] = x;
             }
@@ -183,8 +199,9 @@ __global__ void __launch_bounds__(kT) k_pr_join(PrArgs a, int it) {
         if (u < 0) continue;
         const int64_t rb = a.rp[u], re = a.rp[u + 1];
         const int64_t last = (re - 1) / kEdgeChunk;
-        float s = 0.f;
-        for (int64_t k = c + 1 + lane; k <= last; k += 32) s += a.head[k];
+        PrSum p;
+        for (int64_t k = c + 1 + lane; k <= last; k += 32) p.add(a.head[k]);
+        float s = p.value();
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
         if (lane == 0) err += pr_put(a, u, a.tail[c] + s, re - rb);
     }
