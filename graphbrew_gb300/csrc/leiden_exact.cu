@@ -21,11 +21,11 @@
 // All totals are exact integers, so every Delta-modularity equals the serial
 // one whatever the order of the sums.
 //
-// Vertices above kWarpMaxDeg ("hubs") are split into 4096-edge segments, each
-// accumulated by its own CTA into the hub's global table, then scanned in
-// 4096-slot segments; the last CTA of a hub reduces the partial maxima.  The
-// whole round reads its window bounds from a device control block, so the host
-// enqueues rounds without waiting and checks completion every few rounds.
+// Vertices above kBigMaxDeg ("hubs") are split into 1024-edge segments, each
+// accumulated by its own CTA into the hub's global table, whose occupied slots
+// are then scored in segments; the last CTA of a hub reduces the partial maxima.
+// The whole round reads its window bounds from a device control block, so an
+// iteration's rounds are one graph launch, or enqueued without waiting.
 //
 // The iteration's totalDelta decides the tolerance break; it is summed in a
 // fixed tree order with a rigorous error bound and re-summed serially in
