@@ -47,8 +47,8 @@ constexpr int kT = 256;
 // whether the last evaluation changed it (vertex ids are below 2^31 - 1).
 constexpr uint32_t kNoMove = 0x7FFFFFFFu;
 constexpr uint32_t kChanged = 0x80000000u;
-constexpr int kWindowMax = 65536;             // window vertices (events <= 2 x window)
-constexpr int kEventsMax = 2 * kWindowMax;    // event index = 2 x window offset (+1)
+constexpr int kWindowMax = 65536;             // window vertices
+constexpr int kEventsMax = 2 * kWindowMax;    // a departure and an arrival each
 constexpr int kSlotBits = 18;
 constexpr int kTableSlots = 1 << kSlotBits;   // hash slots, >= 2 x events
 constexpr int kTbThreads = 256;               // table insert: one window vertex per thread
