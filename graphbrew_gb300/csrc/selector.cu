@@ -434,7 +434,9 @@ __global__ void __cluster_dims__(kTrCtas, 1, 1) __launch_bounds__(kTrThreads) k_
         }
         __syncthreads();
         // Outputs: four threads a row, three of them with an output; the mean
-        // squared error's gradient and the row's loss.
+        // squared error's gradient and the row's loss.  The shuffles' lanes are named
+        // before any of them part.
+        const unsigned mask = __ballot_sync(0xFFFFFFFFu, t < rows * 4);
         if (t < rows * 4) {
             const int r = t >> 2, c = t & 3;
             const int cc = c < O ? c : 0;
@@ -443,7 +445,6 @@ __global__ void __cluster_dims__(kTrCtas, 1, 1) __launch_bounds__(kTrThreads) k_
             for (int i = 0; i < H; ++i) y = fmaf(sm[L.h2 + r * H + i], sm[L.w3 + i * O + cc], y);
             const float d = y - target;
             if (c < O) sm[L.dy + r * 4 + c] = 2.f * d / (float)(B * O);
-            const unsigned mask = __activemask();
             const int q0 = (t & 31) & ~3;
             const float d0 = __shfl_sync(mask, d, q0), d1 = __shfl_sync(mask, d, q0 + 1),
                         d2 = __shfl_sync(mask, d, q0 + 2);

@@ -134,6 +134,22 @@ def test_training_by_batch_and_inputs(ctx, rows, in_dim, batch):
     np.testing.assert_allclose(loss, np.mean(losses), rtol=1e-3)
 
 
+@pytest.mark.parametrize("rows,in_dim", [(1, 1), (2, 32), (7, 12), (8, 12), (9, 12), (15, 1), (63, 31), (65, 12),
+                                         (100, 12), (128, 12), (129, 32), (255, 12), (256, 1), (256, 32)])
+def test_training_epoch_kernel_equals_the_launches(ctx, rows, in_dim):
+    # A minibatch of all rows: `batch` up to 256 takes the one-launch epoch, 257 the
+    # kernels one by one.  The same sums in the same order: equal to the last bit.
+    rng = np.random.default_rng(rows * 1000 + in_dim)
+    start = rng.normal(0, 0.3, ctx.mlp_param_count(in_dim)).astype(np.float32)
+    x = rng.normal(0, 1, (rows, in_dim)).astype(np.float32)
+    t = rng.normal(0, 1, (rows, 3)).astype(np.float32)
+    expect, expect_loss = ctx.mlp_train(start, x, t, epochs=4, batch=257, lr=1e-3, seed=5)
+    for batch in {rows, 256}:
+        got, loss = ctx.mlp_train(start, x, t, epochs=4, batch=batch, lr=1e-3, seed=5)
+        np.testing.assert_array_equal(got, expect)
+        assert loss == expect_loss
+
+
 @pytest.mark.parametrize("lengths", [(0, 1, 2, 7, 8, 9, 31, 32, 33), (63, 64, 65, 127, 128, 129, 255, 256, 257),
                                      (511, 512, 513, 1023, 1024, 1025), (2047, 2048, 2049)])
 def test_relabel_by_row_length(ctx, lengths):
