@@ -1,4 +1,6 @@
 """Kernel variants chosen by size, at the edges of their ranges, against the oracle."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -148,6 +150,54 @@ def test_training_epoch_kernel_equals_the_launches(ctx, rows, in_dim):
         got, loss = ctx.mlp_train(start, x, t, epochs=4, batch=batch, lr=1e-3, seed=5)
         np.testing.assert_array_equal(got, expect)
         assert loss == expect_loss
+
+
+def _fmaf(a, b, c):
+    """a * b + c of float32 values, rounded once: the product is exact in float64, and
+    the sum's rounding error turns it to the odd neighbour before the last rounding."""
+    p, c = a.astype(np.float64) * b.astype(np.float64), c.astype(np.float64)
+    s = p + c
+    t = s - p
+    err = (p - (s - t)) + (c - t)
+    even = (s.view(np.int64) & 1) == 0
+    return np.where((err != 0) & even, np.nextafter(s, np.copysign(np.inf, err)), s).astype(np.float32)
+
+
+@pytest.mark.parametrize("rows,in_dim,batch", [(10, 12, 4), (129, 12, 64), (300, 12, 128), (300, 32, 256),
+                                               (300, 33, 128)])
+def test_training_steps_in_float32(ctx, rows, in_dim, batch):
+    # Two epochs of several minibatches: the gradients of the kernels one by one and
+    # Adam in float32, with its two fused multiply-adds.
+    powf = ctypes.CDLL("libm.so.6").powf
+    powf.restype, powf.argtypes = ctypes.c_float, [ctypes.c_float, ctypes.c_float]
+    rng = np.random.default_rng(rows * 1000 + in_dim)
+    p = rng.normal(0, 0.3, ctx.mlp_param_count(in_dim)).astype(np.float32)
+    x = rng.normal(0, 1, (rows, in_dim)).astype(np.float32)
+    t = rng.normal(0, 1, (rows, 3)).astype(np.float32)
+    seed, mask, f = 11, (1 << 64) - 1, np.float32
+    got, loss = ctx.mlp_train(p, x, t, epochs=2, batch=batch, lr=1e-3, seed=seed)
+    m, v = np.zeros_like(p), np.zeros_like(p)
+    b1, b2, one = f(0.9), f(0.999), f(1)
+    order, word, step = list(range(rows)), (seed ^ 0x9E3779B97F4A7C15) & mask, 0
+    for _ in range(2):
+        for i in range(rows - 1, 0, -1):
+            word = (word + 0x9E3779B97F4A7C15) & mask
+            z = ((word ^ (word >> 30)) * 0xBF58476D1CE4E5B9) & mask
+            z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & mask
+            j = (z ^ (z >> 31)) % (i + 1)
+            order[i], order[j] = order[j], order[i]
+        losses = []
+        for at in range(0, rows, batch):
+            pick = order[at:at + batch]
+            g, l = ctx.mlp_gradient(p, x[pick], t[pick])
+            losses.append(l)
+            step += 1
+            c1, c2 = one - f(powf(float(b1), step)), one - f(powf(float(b2), step))
+            m = _fmaf(np.full_like(m, b1), m, (one - b1) * g)
+            v = _fmaf(np.full_like(v, b2), v, (one - b2) * g * g)
+            p = p - f(1e-3) * (m / c1) / (np.sqrt(v / c2) + f(1e-8))
+    np.testing.assert_array_equal(got, p)
+    assert f(loss) == f(np.sum(np.array(losses, dtype=np.float64)) / len(losses))
 
 
 @pytest.mark.parametrize("lengths", [(0, 1, 2, 7, 8, 9, 31, 32, 33), (63, 64, 65, 127, 128, 129, 255, 256, 257),
