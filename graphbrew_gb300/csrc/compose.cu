@@ -196,7 +196,9 @@ __global__ void k_classify(const int64_t* __restrict__ ssize, int64_t C, int int
 
 // ---------------------------------------------------------------------------
 // Local adjacency for Gorder communities: for each position p, the local
-// indices of in-community neighbours in row order.
+// indices of in-community neighbours in row order.  A vertex is not its own
+// neighbour here: a placed vertex is never moved again, and the scan heap writes
+// its word while it bumps the rest of its row.
 // ---------------------------------------------------------------------------
 __global__ void k_mark_gorder_positions(const int32_t* __restrict__ list, const int32_t* __restrict__ count_p,
                                         const int64_t* __restrict__ offs, const int64_t* __restrict__ ssize,
@@ -226,21 +228,21 @@ __device__ __forceinline__ void for_marked_rows(const int64_t* __restrict__ rp, 
     for (int64_t p0 = 4 * w; p0 < nn; p0 += 4 * nw) {
         const int64_t p = p0 + g;
         int64_t b = 0, e = 0;
-        uint32_t cu = 0;
+        uint32_t u = 0, cu = 0;
         if (p < nn && mark[p]) {
-            const uint32_t u = order_v[p];
+            u = order_v[p];
             b = rp[u];
             e = rp[u + 1];
             cu = memb[u];
         }
         const bool is_long = e - b > kOctetRow;
-        short_row(p, b, is_long ? b : e, cu, is_long);
+        short_row(p, b, is_long ? b : e, u, cu, is_long);
         unsigned todo = __ballot_sync(0xFFFFFFFFu, is_long && (lane & 7) == 0);
         while (todo) {
             const int src = __ffs(todo) - 1;
             todo &= todo - 1;
             long_row(p0 + (src >> 3), __shfl_sync(0xFFFFFFFFu, b, src), __shfl_sync(0xFFFFFFFFu, e, src),
-                     __shfl_sync(0xFFFFFFFFu, cu, src));
+                     __shfl_sync(0xFFFFFFFFu, u, src), __shfl_sync(0xFFFFFFFFu, cu, src));
         }
     }
 }
@@ -249,19 +251,20 @@ __global__ void k_local_count(const int64_t* __restrict__ rp, const int32_t* __r
                               const uint32_t* __restrict__ memb, const uint32_t* __restrict__ order_v,
                               const uint8_t* __restrict__ mark, int64_t nn, int64_t* __restrict__ cnt) {
     const int lane = threadIdx.x & 31, j = lane & 7;
+    auto counts = [&](int32_t w, uint32_t u, uint32_t cu) { return memb[w] == cu && (uint32_t)w != u; };
     for_marked_rows(
         rp, memb, order_v, mark, nn,
-        [&](int64_t p, int64_t b, int64_t e, uint32_t cu, bool is_long) {
+        [&](int64_t p, int64_t b, int64_t e, uint32_t u, uint32_t cu, bool is_long) {
             int c = 0;
-            for (int64_t x = b + j; x < e; x += 8) c += memb[col[x]] == cu;
+            for (int64_t x = b + j; x < e; x += 8) c += counts(col[x], u, cu);
             c += __shfl_xor_sync(0xFFFFFFFFu, c, 4);
             c += __shfl_xor_sync(0xFFFFFFFFu, c, 2);
             c += __shfl_xor_sync(0xFFFFFFFFu, c, 1);
             if (j == 0 && p < nn && !is_long) cnt[p] = c;
         },
-        [&](int64_t p, int64_t b, int64_t e, uint32_t cu) {
+        [&](int64_t p, int64_t b, int64_t e, uint32_t u, uint32_t cu) {
             int c = 0;
-            for (int64_t x = b + lane; x < e; x += 32) c += memb[col[x]] == cu;
+            for (int64_t x = b + lane; x < e; x += 32) c += counts(col[x], u, cu);
             c = __reduce_add_sync(0xFFFFFFFFu, c);
             if (lane == 0) cnt[p] = c;
         });
@@ -279,22 +282,22 @@ __global__ void k_local_fill(const int64_t* __restrict__ rp, const int32_t* __re
     };
     for_marked_rows(
         rp, memb, order_v, mark, nn,
-        [&](int64_t p, int64_t b, int64_t e, uint32_t cu, bool) {
+        [&](int64_t p, int64_t b, int64_t e, uint32_t u, uint32_t cu, bool) {
             int64_t o = e > b ? loff[p] : 0;
             for (int64_t x = b + j; __any_sync(0xFFFFFFFFu, x < e); x += 8) {
                 const int32_t w = x < e ? col[x] : -1;
-                const bool keep = w >= 0 && memb[w] == cu;
+                const bool keep = w >= 0 && memb[w] == cu && (uint32_t)w != u;
                 const unsigned bal = (__ballot_sync(0xFFFFFFFFu, keep) >> (lane & 24)) & 0xFFu;
                 if (keep) put(o + __popc(bal & ((1u << j) - 1u)), w);
                 o += __popc(bal);
             }
         },
-        [&](int64_t p, int64_t b, int64_t e, uint32_t cu) {
+        [&](int64_t p, int64_t b, int64_t e, uint32_t u, uint32_t cu) {
             int64_t o = loff[p];
             for (int64_t x0 = b; x0 < e; x0 += 32) {
                 const int64_t x = x0 + lane;
                 const int32_t w = x < e ? col[x] : -1;
-                const bool keep = w >= 0 && memb[w] == cu;
+                const bool keep = w >= 0 && memb[w] == cu && (uint32_t)w != u;
                 const unsigned bal = __ballot_sync(0xFFFFFFFFu, keep);
                 if (keep) put(o + __popc(bal & ((1u << lane) - 1u)), w);
                 o += __popc(bal);

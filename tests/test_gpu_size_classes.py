@@ -57,6 +57,31 @@ def test_gorder_by_community_size(ctx, sizes, window):
         [ost.gorder_communities, ost.gorder_vertices, ost.gorder_max_community]
 
 
+@pytest.mark.parametrize("form", ["loops", "directed", "both"])
+@pytest.mark.parametrize("window", [1, 8])
+@pytest.mark.parametrize("sizes", [(20, 32, 33, 300, 1024), (1025, 4097, 16384), (16385, 40)])
+def test_gorder_with_loops_and_directed_rows(ctx, sizes, window, form):
+    # Rows that the input check lets through: every third vertex and each hub its own
+    # neighbour, every fifth entry without its reverse.
+    rp, col, memb = _communities(sizes, seed=sum(sizes) + window)
+    n = len(rp) - 1
+    src = np.repeat(np.arange(n), np.diff(rp))
+    dst = col.astype(np.int64)
+    if form != "loops":
+        keep = (src * 7 + dst * 3) % 5 != 0
+        src, dst = src[keep], dst[keep]
+    if form != "directed":
+        loops = np.union1d(np.arange(0, n, 3), np.argsort(np.diff(rp))[-2 * len(sizes):])
+        src, dst = np.concatenate([src, loops]), np.concatenate([dst, loops])
+    order = np.lexsort((dst, src))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int64)
+    col = dst[order].astype(np.int32)
+    recipe = gb.DEFAULT_RECIPE.replace("gw8", f"gw{window}").replace("gordf5000", "gordf100000")
+    ids, _ = ctx.order_compose(rp, col, memb, recipe)
+    expect, _ = po.compose(rp, col, memb, gorder_window=window, gorder_fallback=100000)
+    np.testing.assert_array_equal(ids, expect)
+
+
 def _kernel_graph(kind, size):
     if kind == "star":        # one row at the edge of the segmented rows, and a path hanging off it
         edges = [(0, i) for i in range(1, size + 1)] + [(size + i, size + i + 1) for i in range(40)]
