@@ -29,12 +29,36 @@ constexpr int kHubRow = 1024;   // frontier rows above this go to CTAs
 
 // ---- PageRank ----
 __global__ void k_pr_init(const int64_t* __restrict__ rp, int64_t n, float init, float* __restrict__ score,
-                          float* __restrict__ contrib, float* __restrict__ other) {
+                          float* __restrict__ contrib, float* __restrict__ other, uint8_t* __restrict__ full) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
         const int64_t d = rp[v + 1] - rp[v];
         score[v] = init;
         contrib[v] = d ? init / (float)d : 0.f;
         other[v] = 0.f;   // rows without entries are never written again
+        full[v] = d != 0;
+    }
+}
+
+// The rows with entries, in order: their offsets and ids.  The places behind them
+// hold nnz, so the offsets end as a CSR's whose last rows are empty.  And the rows
+// that hold each chunk's first and last entry.
+__global__ void k_pr_rows(const int64_t* __restrict__ rp, int64_t n, const int64_t* __restrict__ pos,
+                          int64_t* __restrict__ off, int32_t* __restrict__ id, int32_t* __restrict__ first,
+                          int32_t* __restrict__ last) {
+    const int64_t nnz = rp[n];
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t b = rp[v], e = rp[v + 1], p = pos[v];
+        if (b == e) {
+            off[n - (v - p)] = nnz;   // v - p empty rows before this one
+            continue;
+        }
+        off[p] = b;
+        id[p] = (int32_t)v;
+        if (e == nnz) off[p + 1] = nnz;
+        for (int64_t c = b / kEdgeChunk; c * kEdgeChunk < e; ++c) {
+            if (c * kEdgeChunk >= b) first[c] = (int32_t)v;
+            if (min((c + 1) * kEdgeChunk, nnz) <= e) last[c] = (int32_t)v;
+        }
     }
 }
 
@@ -60,7 +84,9 @@ struct PrArgs {
     const int64_t* rp;
     const int32_t* col;
     int64_t n, nnz;
-    const int32_t* chunk_row;
+    const int64_t* off;   // offsets of the rows with entries (k_pr_rows)
+    const int32_t* id;    // their vertices
+    const int32_t* chunk_row;   // row of the chunk's first entry, or the complement of its place in off
     float base, damp;
     const float* cin;
     float* cout;
@@ -72,7 +98,7 @@ struct PrArgs {
     double epsilon;
 };
 
-__device__ __forceinline__ double pr_put(const PrArgs& a, int64_t u, float s, int64_t d) {
+__device__ __forceinline__ double pr_put(const PrArgs& a, int32_t u, float s, int64_t d) {
     const float ns = a.base + a.damp * s;
     const double e = fabsf(ns - a.score[u]);
     a.score[u] = ns;
@@ -88,7 +114,7 @@ __device__ __forceinline__ double pr_put(const PrArgs& a, int64_t u, float s, in
 // Bound by the gather of contributions from L2, 4 bytes wanted of each 32-byte
 // sector.  RMAT scale 20, 33 M entries: a warp per row 1.43 ms a sweep (nearly
 // all of it the largest row's), lanes, warps and CTAs by row length 0.48 ms.
-// Rows without entries keep the score that k_pr_isolated gives them.
+// Rows without entries keep the score that k_pr_first gives them.
 // A lane adds its entries up with the rounding errors kept beside the sum (Knuth's
 // two-sum), so that 24 of them in a row are no further off than a tree over a warp.
 constexpr int kPrOwn = 24;      // rows up to this long by a thread
@@ -118,6 +144,7 @@ __global__ void __launch_bounds__(kT, 6) k_pr_sweep(PrArgs a, int it) {
     for (int64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
         const int64_t e0 = c * kEdgeChunk, e1 = min(a.nnz, e0 + kEdgeChunk);
         const int len = (int)(e1 - e0);
+        const int32_t row0 = a.chunk_row[c];
         {
             int32_t v[kEdgeChunk / kT];
 #pragma unroll
@@ -132,9 +159,12 @@ __global__ void __launch_bounds__(kT, 6) k_pr_sweep(PrArgs a, int it) {
         }
         __syncthreads();
         // Rows from the one that holds entry e0, 256 at a time, until one starts past the chunk.
-        for (int64_t u0 = a.chunk_row[c];; u0 += kT) {
+        const bool gaps = row0 < 0;
+        const int64_t* rp = gaps ? a.off : a.rp;
+        for (int64_t u0 = gaps ? ~row0 : row0;; u0 += kT) {
             const int64_t u = u0 + t;
-            const int64_t rb = u < a.n ? a.rp[u] : e1, re = u < a.n ? a.rp[u + 1] : e1;
+            const int64_t rb = u < a.n ? rp[u] : e1, re = u < a.n ? rp[u + 1] : e1;
+            const int32_t vertex = gaps && u < a.n ? a.id[u] : (int32_t)u;
             const int b = (int)(max(rb, e0) - e0), e = rb < e1 ? (int)(min(re, e1) - e0) : b;
             if (t == kT - 1) s_more = rb < e1;
             float s = 0.f;
@@ -174,8 +204,8 @@ __global__ void __launch_bounds__(kT, 6) k_pr_sweep(PrArgs a, int it) {
                 if (rb < e0) a.head[c] = s;
                 else if (re > e1) {
                     a.tail[c] = s;
-                    a.tail_row[c] = (int32_t)u;
-                } else err += pr_put(a, u, s, re - rb);
+                    a.tail_row[c] = vertex;
+                } else err += pr_put(a, vertex, s, re - rb);
             }
             const bool more = s_more;
             if (t == 0) s_listed = 0;
@@ -208,11 +238,24 @@ __global__ void __launch_bounds__(kT) k_pr_join(PrArgs a, int it) {
     pr_add_change(err, a.err + it);
 }
 
-// Rows without entries: the base score from the first sweep on.
-__global__ void __launch_bounds__(kT) k_pr_isolated(PrArgs a) {
+// Before the first sweep.  Rows without entries: the base score from here on.
+// Chunks: more than a fifth of the rows between the first and the last entry empty,
+// and the rows with entries are walked: first[c] becomes the complement of the
+// first one's place.  (By their ids a gap of 4 M in one chunk took 6.6 ms a sweep,
+// and R-MAT scale 20, where two ids in five are free, 34 us more; where there are
+// no gaps the ids are one more read, 4 us a sweep of a 517 x 1023 grid.)
+__global__ void __launch_bounds__(kT) k_pr_first(PrArgs a, const uint8_t* __restrict__ full,
+                                                 const int64_t* __restrict__ pos, const int32_t* __restrict__ last,
+                                                 int32_t* __restrict__ first) {
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t chunks = (a.nnz + kEdgeChunk - 1) / kEdgeChunk;
+    for (int64_t c = tid; c < chunks; c += stride) {
+        const int64_t rows = last[c] - first[c] + 1, place = pos[first[c]], held = pos[last[c]] - place + 1;
+        if (rows - held > rows / 5) first[c] = ~(int32_t)place;
+    }
     double err = 0.0;
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < a.n; v += (int64_t)gridDim.x * blockDim.x) {
-        if (a.rp[v] != a.rp[v + 1]) continue;
+    for (int64_t v = tid; v < a.n; v += stride) {
+        if (full[v]) continue;
         const float ns = a.base + a.damp * 0.f;
         err += fabsf(ns - a.score[v]);
         a.score[v] = ns;
@@ -709,26 +752,34 @@ double pagerank_device(const DeviceCSR& g, int max_iters, double epsilon, float*
     if (n == 0) return 0.0;
     constexpr int kBatch = 8;   // sweeps enqueued between two looks at the change
     const int64_t chunks = edge_chunks(g.nnz);
-    DevBuf<float> ca(n, s), cb(n, s), head(chunks, s), tail(chunks, s);
-    DevBuf<int32_t> chunk_row(chunks, s), tail_row(chunks, s);
+    // Few buffers: an allocation and its release are some 10 us of host time.
+    DevBuf<float> contrib(2 * n, s), sums(2 * chunks, s);
+    DevBuf<int64_t> places(2 * n + 1, s);
+    DevBuf<int32_t> rows(n + 3 * chunks, s);
+    DevBuf<uint8_t> full(n, s);
     DevBuf<double> err(kBatch, s);
+    float *ca = contrib.get(), *cb = ca + n, *head = sums.get(), *tail = head + chunks;
+    int64_t *pos = places.get(), *off = pos + n;
+    int32_t *id = rows.get(), *chunk_row = id + n, *chunk_last = chunk_row + chunks, *tail_row = chunk_last + chunks;
     cudaEvent_t e0, e1;
     GB_CUDA(cudaEventCreate(&e0));
     GB_CUDA(cudaEventCreate(&e1));
     GB_CUDA(cudaEventRecord(e0, s));
     const float init = 1.0f / (float)n, damp = 0.85f, base = (1.0f - damp) / (float)n;
-    k_pr_init<<<grid_for(n, kT), kT, 0, s>>>(g.row_ptr, n, init, score, ca, cb);
+    k_pr_init<<<grid_for(n, kT), kT, 0, s>>>(g.row_ptr, n, init, score, ca, cb, full);
     GB_LAUNCH_CHECK();
-    chunk_rows_device(g.row_ptr, n, g.nnz, chunk_row, s);
-    PrArgs a{g.row_ptr, g.col,  n,    g.nnz, chunk_row, base, damp,   ca,
-             cb,        score, head, tail,  tail_row,  err,  epsilon};
+    exclusive_scan_u8_to_i64(full, pos, n, nullptr, s);
+    k_pr_rows<<<grid_for(n, kT), kT, 0, s>>>(g.row_ptr, n, pos, off, id, chunk_row, chunk_last);
+    GB_LAUNCH_CHECK();
+    PrArgs a{g.row_ptr, g.col, n,    g.nnz, off,  id,       chunk_row, base,
+             damp,      ca,    cb,   score, head, tail,     tail_row,  err, epsilon};
     const int grid = grid_for(chunks, 1), join_grid = grid_for(chunks * 32, kT);
     int it = 0;
     for (bool done = false; it < max_iters && !done;) {
         const int count = std::min(kBatch, max_iters - it);
         GB_CUDA(cudaMemsetAsync(err, 0, kBatch * sizeof(double), s));
         for (int k = 0; k < count; ++k) {
-            if (it + k == 0) k_pr_isolated<<<grid_for(n, kT), kT, 0, s>>>(a);
+            if (it + k == 0) k_pr_first<<<grid_for(n, kT), kT, 0, s>>>(a, full, pos, chunk_last, chunk_row);
             if (chunks > 0) {
                 k_pr_sweep<<<grid, kT, 0, s>>>(a, k);
                 k_pr_join<<<join_grid, kT, 0, s>>>(a, k);
