@@ -22,19 +22,80 @@ constexpr int kEdgeChunkPadded = kEdgeChunk + kEdgeChunk / 32;
 
 __device__ __forceinline__ int chunk_pad(int i) { return i + (i >> 5); }
 
-// chunk_row has ceil(nnz / kEdgeChunk) entries.  The CSR must be valid
+// chunk_row has ceil(nnz / kEdgeChunk) entries, and so has chunk_last where it is
+// given: the row that holds the chunk's last entry.  The CSR must be valid
 // (row_ptr non-decreasing from 0 to nnz).
-void chunk_rows_device(const int64_t* row_ptr, int64_t n, int64_t nnz, int32_t* chunk_row, cudaStream_t s);
+void chunk_rows_device(const int64_t* row_ptr, int64_t n, int64_t nnz, int32_t* chunk_row, cudaStream_t s,
+                       int32_t* chunk_last = nullptr);
 
 inline int64_t edge_chunks(int64_t nnz) { return ceil_div(nnz, kEdgeChunk); }
 
+// fn(c) for the chunks c with entries of this lane's row, [b, e); a row of more than
+// a few chunks is the whole warp's, whose lanes all call (b == e: no row).  fn gets
+// the row's bounds and id with it, as they may be another lane's.
+template <typename Fn>
+__device__ __forceinline__ void for_row_chunks(int64_t b, int64_t e, int32_t u, Fn&& fn) {
+    constexpr int kOwn = 4;
+    const int lane = threadIdx.x & 31;
+    int64_t c0 = b / kEdgeChunk;
+    const int64_t c1 = b < e ? (e - 1) / kEdgeChunk + 1 : c0;
+    unsigned longer = __ballot_sync(0xFFFFFFFFu, c1 - c0 > kOwn);
+    if (c1 - c0 <= kOwn)
+        for (; c0 < c1; ++c0) fn(c0, b, e, u);
+    while (longer) {
+        const int src = __ffs(longer) - 1;
+        longer &= longer - 1;
+        const int64_t rb = __shfl_sync(0xFFFFFFFFu, b, src), re = __shfl_sync(0xFFFFFFFFu, e, src);
+        const int64_t end = __shfl_sync(0xFFFFFFFFu, c1, src);
+        const int32_t ru = __shfl_sync(0xFFFFFFFFu, u, src);
+        for (int64_t c = __shfl_sync(0xFFFFFFFFu, c0, src) + lane; c < end; c += 32) fn(c, rb, re, ru);
+    }
+}
+
+// Rows that a CTA walks between a chunk's first and last.  Where there are more,
+// nearly all of them empty, every entry's row is searched for instead: some 0.1 ms,
+// which is what a walk over 64 K rows takes (4 M isolated ids in one chunk: 3.1 ms).
+constexpr int64_t kChunkWalk = 65536;
+
+// srow[chunk_pad(i)] = the largest row of [u0, last] that begins at or before e0 + i.
+template <int kThreads>
+__device__ __forceinline__ void chunk_search_rows(const int64_t* __restrict__ rp, int32_t u0, int32_t last, int64_t e0,
+                                                  int64_t e1, int32_t* srow) {
+    constexpr int kStep = 4;   // searches of a thread in flight
+    const int len = (int)(e1 - e0);
+    int64_t top = 1;
+    while (top <= last - u0) top <<= 1;
+    for (int i0 = threadIdx.x; i0 < len; i0 += kStep * kThreads) {
+        int64_t u[kStep];
+#pragma unroll
+        for (int k = 0; k < kStep; ++k) u[k] = u0;
+        for (int64_t half = top >> 1; half > 0; half >>= 1) {
+#pragma unroll
+            for (int k = 0; k < kStep; ++k) {
+                const int64_t at = u[k] + half;
+                if (at <= last && rp[at] <= e0 + i0 + k * kThreads) u[k] = at;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kStep; ++k)
+            if (i0 + k * kThreads < len) srow[chunk_pad(i0 + k * kThreads)] = (int32_t)u[k];
+    }
+    __syncthreads();
+}
+
 // srow (kEdgeChunkPadded ints of shared memory) receives, at chunk_pad(i),
 // the row of entry e0 + i for i < e1 - e0.  warp_max: kThreads / 32 ints of
-// shared memory.  Every thread of the CTA calls it; it ends with a barrier.
+// shared memory; last: the row of entry e1 - 1, where it is known.  Every thread
+// of the CTA calls it; it ends with a barrier.
 template <int kThreads>
 __device__ __forceinline__ void chunk_entry_rows(const int64_t* __restrict__ rp, int64_t n, int32_t u0,
-                                                 int64_t e0, int64_t e1, int32_t* srow, int32_t* warp_max) {
+                                                 int64_t e0, int64_t e1, int32_t* srow, int32_t* warp_max,
+                                                 int32_t last = -1) {
     static_assert(kEdgeChunk % kThreads == 0 && kThreads % 32 == 0, "chunk / CTA shape");
+    if (last - u0 > kChunkWalk) {
+        chunk_search_rows<kThreads>(rp, u0, last, e0, e1, srow);
+        return;
+    }
     constexpr int kPer = kEdgeChunk / kThreads;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     for (int i = t; i < kEdgeChunk; i += kThreads) srow[chunk_pad(i)] = -1;

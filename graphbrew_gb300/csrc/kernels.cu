@@ -46,19 +46,22 @@ __global__ void k_pr_rows(const int64_t* __restrict__ rp, int64_t n, const int64
                           int64_t* __restrict__ off, int32_t* __restrict__ id, int32_t* __restrict__ first,
                           int32_t* __restrict__ last) {
     const int64_t nnz = rp[n];
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t b = rp[v], e = rp[v + 1], p = pos[v];
-        if (b == e) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t v0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; v0 < n;
+         v0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t v = v0 + lane;
+        const int64_t b = v < n ? rp[v] : 0, e = v < n ? rp[v + 1] : 0, p = v < n ? pos[v] : 0;
+        if (b < e) {
+            off[p] = b;
+            id[p] = (int32_t)v;
+            if (e == nnz) off[p + 1] = nnz;
+        } else if (v < n) {
             off[n - (v - p)] = nnz;   // v - p empty rows before this one
-            continue;
         }
-        off[p] = b;
-        id[p] = (int32_t)v;
-        if (e == nnz) off[p + 1] = nnz;
-        for (int64_t c = b / kEdgeChunk; c * kEdgeChunk < e; ++c) {
-            if (c * kEdgeChunk >= b) first[c] = (int32_t)v;
-            if (min((c + 1) * kEdgeChunk, nnz) <= e) last[c] = (int32_t)v;
-        }
+        for_row_chunks(b, e, (int32_t)v, [&](int64_t c, int64_t rb, int64_t re, int32_t row) {
+            if (c * kEdgeChunk >= rb) first[c] = row;
+            if (min((c + 1) * kEdgeChunk, nnz) <= re) last[c] = row;
+        });
     }
 }
 
@@ -690,14 +693,14 @@ __global__ void k_cc_sample(const int64_t* __restrict__ rp, const int32_t* __res
 // stale one is still an ancestor, and only sends its entry to the union.
 __global__ void __launch_bounds__(kT)
 k_cc_link(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, int64_t n, int64_t nnz,
-          const int32_t* __restrict__ chunk_row, int32_t* parent) {
+          const int32_t* __restrict__ chunk_row, const int32_t* __restrict__ chunk_last, int32_t* parent) {
     __shared__ int32_t srow[kEdgeChunkPadded], wmax[kT / 32];
     constexpr int kStep = 8;
     const int64_t chunks = (nnz + kEdgeChunk - 1) / kEdgeChunk;
     for (int64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
         const int64_t e0 = c * kEdgeChunk, e1 = min(nnz, e0 + kEdgeChunk);
         const int len = (int)(e1 - e0);
-        chunk_entry_rows<kT>(rp, n, chunk_row[c], e0, e1, srow, wmax);
+        chunk_entry_rows<kT>(rp, n, chunk_row[c], e0, e1, srow, wmax, chunk_last[c]);
         for (int i0 = threadIdx.x; i0 < len; i0 += kStep * kT) {
             int32_t u[kStep], v[kStep], pu[kStep], pv[kStep];
 #pragma unroll
@@ -913,9 +916,10 @@ double cc_device(const DeviceCSR& g, int32_t* comp, cudaStream_t s) {
         }
         GB_LAUNCH_CHECK();
         const int64_t chunks = edge_chunks(g.nnz);
-        DevBuf<int32_t> chunk_row(chunks, s);
-        chunk_rows_device(g.row_ptr, n, g.nnz, chunk_row, s);
-        k_cc_link<<<grid_for(chunks, 1), kT, 0, s>>>(g.row_ptr, g.col, n, g.nnz, chunk_row, comp);
+        DevBuf<int32_t> chunk_row(2 * chunks, s);
+        int32_t* chunk_last = chunk_row.get() + chunks;
+        chunk_rows_device(g.row_ptr, n, g.nnz, chunk_row, s, chunk_last);
+        k_cc_link<<<grid_for(chunks, 1), kT, 0, s>>>(g.row_ptr, g.col, n, g.nnz, chunk_row, chunk_last, comp);
         GB_LAUNCH_CHECK();
     }
     k_cc_flatten<false><<<grid_for(n, kT), kT, 0, s>>>(n, comp);

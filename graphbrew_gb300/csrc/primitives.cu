@@ -403,18 +403,26 @@ __global__ void k_degrees(const int64_t* __restrict__ rp, int64_t* __restrict__ 
         deg[i] = rp[i + 1] - rp[i];
 }
 
-__global__ void k_chunk_rows(const int64_t* __restrict__ rp, int64_t n, int32_t* __restrict__ chunk_row) {
-    for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t b = rp[u], e = rp[u + 1];
-        for (int64_t c = (b + kEdgeChunk - 1) / kEdgeChunk; c * kEdgeChunk < e; ++c) chunk_row[c] = (int32_t)u;
+__global__ void k_chunk_rows(const int64_t* __restrict__ rp, int64_t n, int64_t nnz, int32_t* __restrict__ chunk_row,
+                             int32_t* __restrict__ chunk_last) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t u0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; u0 < n;
+         u0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t u = u0 + lane;
+        const int64_t b = u < n ? rp[u] : 0, e = u < n ? rp[u + 1] : 0;
+        for_row_chunks(b, e, (int32_t)u, [&](int64_t c, int64_t rb, int64_t re, int32_t row) {
+            if (c * kEdgeChunk >= rb) chunk_row[c] = row;
+            if (chunk_last && min((c + 1) * kEdgeChunk, nnz) <= re) chunk_last[c] = row;
+        });
     }
 }
 
 }  // namespace
 
-void chunk_rows_device(const int64_t* row_ptr, int64_t n, int64_t nnz, int32_t* chunk_row, cudaStream_t s) {
+void chunk_rows_device(const int64_t* row_ptr, int64_t n, int64_t nnz, int32_t* chunk_row, cudaStream_t s,
+                       int32_t* chunk_last) {
     if (n <= 0 || nnz <= 0) return;
-    k_chunk_rows<<<grid_for(n, 256), 256, 0, s>>>(row_ptr, n, chunk_row);
+    k_chunk_rows<<<grid_for(n, 256), 256, 0, s>>>(row_ptr, n, nnz, chunk_row, chunk_last);
     GB_LAUNCH_CHECK();
 }
 
