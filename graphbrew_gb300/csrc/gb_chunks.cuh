@@ -30,26 +30,38 @@ void chunk_rows_device(const int64_t* row_ptr, int64_t n, int64_t nnz, int32_t* 
 
 inline int64_t edge_chunks(int64_t nnz) { return ceil_div(nnz, kEdgeChunk); }
 
-// fn(c) for the chunks c with entries of this lane's row, [b, e); a row of more than
-// a few chunks is the whole warp's, whose lanes all call (b == e: no row).  fn gets
-// the row's bounds and id with it, as they may be another lane's.
-template <typename Fn>
-__device__ __forceinline__ void for_row_chunks(int64_t b, int64_t e, int32_t u, Fn&& fn) {
-    constexpr int kOwn = 4;
+// fn(c, u) for the chunks c of [c0, c1), this lane's row u being what is noted in
+// them (c0 >= c1: nothing).  More than kOwn of them are the whole warp's work, whose
+// lanes all call; they are left out once stop() holds.
+template <typename Fn, typename Stop>
+__device__ __forceinline__ void for_chunks(int64_t c0, int64_t c1, int32_t u, Fn&& fn, Stop&& stop) {
+    constexpr int kOwn = 64;   // some 0.3 us of stores; the question of stop() alone is a read of L2
     const int lane = threadIdx.x & 31;
-    int64_t c0 = b / kEdgeChunk;
-    const int64_t c1 = b < e ? (e - 1) / kEdgeChunk + 1 : c0;
     unsigned longer = __ballot_sync(0xFFFFFFFFu, c1 - c0 > kOwn);
     if (c1 - c0 <= kOwn)
-        for (; c0 < c1; ++c0) fn(c0, b, e, u);
-    while (longer) {
+        for (int64_t c = c0; c < c1; ++c) fn(c, u);
+    while (longer && !__any_sync(0xFFFFFFFFu, stop())) {
         const int src = __ffs(longer) - 1;
         longer &= longer - 1;
-        const int64_t rb = __shfl_sync(0xFFFFFFFFu, b, src), re = __shfl_sync(0xFFFFFFFFu, e, src);
         const int64_t end = __shfl_sync(0xFFFFFFFFu, c1, src);
-        const int32_t ru = __shfl_sync(0xFFFFFFFFu, u, src);
-        for (int64_t c = __shfl_sync(0xFFFFFFFFu, c0, src) + lane; c < end; c += 32) fn(c, rb, re, ru);
+        const int32_t row = __shfl_sync(0xFFFFFFFFu, u, src);
+        for (int64_t c = __shfl_sync(0xFFFFFFFFu, c0, src) + lane; c < end; c += 32) fn(c, row);
     }
+}
+
+// first[c] = u for the chunks whose first entry is in [b, e), the entries of this
+// lane's row u (b == e: none); last[c] likewise for the last entry.
+template <typename Stop>
+__device__ __forceinline__ void note_chunk_first(int64_t b, int64_t e, int32_t u, int32_t* first, Stop&& stop) {
+    const uint64_t up = kEdgeChunk - 1;
+    for_chunks((int64_t)(((uint64_t)b + up) / kEdgeChunk), (int64_t)(((uint64_t)e + up) / kEdgeChunk), u,
+               [&](int64_t c, int32_t row) { first[c] = row; }, stop);
+}
+
+__device__ __forceinline__ void note_chunk_last(int64_t b, int64_t e, int32_t u, int64_t nnz, int32_t* last) {
+    const uint64_t up = b < e && e == nnz ? kEdgeChunk - 1 : 0;   // the last chunk may be a short one
+    for_chunks((int64_t)((uint64_t)b / kEdgeChunk), (int64_t)(((uint64_t)e + up) / kEdgeChunk), u,
+               [&](int64_t c, int32_t row) { last[c] = row; }, [] { return false; });
 }
 
 // Rows that a CTA walks between a chunk's first and last.  Where there are more,

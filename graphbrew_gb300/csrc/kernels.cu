@@ -58,10 +58,8 @@ __global__ void k_pr_rows(const int64_t* __restrict__ rp, int64_t n, const int64
         } else if (v < n) {
             off[n - (v - p)] = nnz;   // v - p empty rows before this one
         }
-        for_row_chunks(b, e, (int32_t)v, [&](int64_t c, int64_t rb, int64_t re, int32_t row) {
-            if (c * kEdgeChunk >= rb) first[c] = row;
-            if (min((c + 1) * kEdgeChunk, nnz) <= re) last[c] = row;
-        });
+        note_chunk_first(b, e, (int32_t)v, first, [] { return false; });
+        note_chunk_last(b, e, (int32_t)v, nnz, last);
     }
 }
 

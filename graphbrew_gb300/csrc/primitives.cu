@@ -410,10 +410,8 @@ __global__ void k_chunk_rows(const int64_t* __restrict__ rp, int64_t n, int64_t 
          u0 += (int64_t)gridDim.x * blockDim.x) {
         const int64_t u = u0 + lane;
         const int64_t b = u < n ? rp[u] : 0, e = u < n ? rp[u + 1] : 0;
-        for_row_chunks(b, e, (int32_t)u, [&](int64_t c, int64_t rb, int64_t re, int32_t row) {
-            if (c * kEdgeChunk >= rb) chunk_row[c] = row;
-            if (chunk_last && min((c + 1) * kEdgeChunk, nnz) <= re) chunk_last[c] = row;
-        });
+        note_chunk_first(b, e, (int32_t)u, chunk_row, [] { return false; });
+        if (chunk_last) note_chunk_last(b, e, (int32_t)u, nnz, chunk_last);
     }
 }
 

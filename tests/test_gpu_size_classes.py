@@ -185,6 +185,32 @@ def test_components_with_gaps_in_the_ids(ctx, gaps):
         5 * _least(lambda: ctx.connected_components(*dense)[1]) + 0.4
 
 
+def test_input_check_of_one_long_row(ctx):
+    # Every call checks its graph.  A row of 32 M entries is noted in 8,192 chunks: by a
+    # warp 256 steps, 0.1 ms at most; a quarter of the call and twice that allowed beside a
+    # path of the same size.
+    def call_ms(u, v, n):
+        rp, col = gg.squish(u, v, n)
+
+        def once():
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            begin.record()
+            ids, _ = ctx.dbg_mapping(rp, col)
+            end.record()
+            torch.cuda.synchronize()
+            return begin.elapsed_time(end)
+        return _least(once)
+
+    leaves = torch.arange(1, (1 << 25) + 1, device="cuda")
+    star = call_ms(torch.zeros_like(leaves), leaves, len(leaves) + 1)
+    path = call_ms(leaves - 1, leaves, len(leaves) + 1)
+    assert star <= 1.25 * path + 0.2
+    for offsets in ([0, 40000, 0, 40000, 40000], [0, 50000, 40000], [0, 30000, 60000, 40000], [-5, 20000, 40000]):
+        with pytest.raises(ValueError, match="row offsets"):
+            ctx.dbg_mapping(torch.tensor(offsets, device="cuda"), torch.zeros(40000, dtype=torch.int32, device="cuda"))
+
+
 @pytest.mark.parametrize("rows,in_dim,batch", [(1, 1, 1), (7, 12, 8), (9, 12, 8), (64, 3, 64), (129, 12, 128),
                                                (300, 32, 256), (513, 12, 100), (300, 33, 256), (300, 12, 257)])
 def test_training_by_batch_and_inputs(ctx, rows, in_dim, batch):
