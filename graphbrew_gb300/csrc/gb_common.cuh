@@ -127,6 +127,7 @@ struct DeviceCSR {
     int64_t nnz = 0;
     const int64_t* row_ptr = nullptr;
     const int32_t* col = nullptr;
+    bool gaps = false;   // a chunk of entries spans many more rows than it has entries (check_graph_device)
 };
 
 // -------------------------------------------------------------------------

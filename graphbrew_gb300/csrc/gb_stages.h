@@ -14,7 +14,7 @@ void relabel_csr_device(const DeviceCSR& g, const int32_t* new_ids, const int32_
                         int64_t* out_rp, int32_t* out_col, cudaStream_t s, int64_t* launches);
 // Rejects graphs that are not squished CSR (every kernel relies on in-range
 // ids; the Gorder heap relies on duplicate-free rows).
-void check_graph_device(const DeviceCSR& g, cudaStream_t s);
+void check_graph_device(DeviceCSR& g, cudaStream_t s);
 
 // ---- compose.cu ----
 struct ComposeParams {

@@ -28,38 +28,43 @@ constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr int kHubRow = 1024;   // frontier rows above this go to CTAs
 
 // ---- PageRank ----
+__global__ void k_pr_full(const int64_t* __restrict__ rp, int64_t n, uint8_t* __restrict__ full) {
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
+        full[v] = rp[v] != rp[v + 1];
+}
+
+// id: the rows with entries, in order, then n (n + 1 places in all); pos: how many
+// come before a row.  And the rows that hold each chunk's first and last entry, in
+// first and last, with their places in id.
+struct PrChunks {
+    int32_t *first, *last, *first_place, *last_place;
+};
+
+__global__ void k_pr_rows(const int64_t* __restrict__ rp, int64_t n, int64_t nnz, const int64_t* __restrict__ pos,
+                          int32_t* __restrict__ id, PrChunks chunk) {
+    const int lane = threadIdx.x & 31;
+    auto go_on = [] { return false; };
+    for (int64_t v0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; v0 < n;
+         v0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t v = v0 + lane;
+        const int64_t b = v < n ? rp[v] : 0, e = v < n ? rp[v + 1] : 0, p = v < n ? pos[v] : 0;
+        if (b < e) id[p] = (int32_t)v;
+        else if (v < n) id[n - (v - p)] = (int32_t)n;   // v - p empty rows before this one
+        if (v == n - 1) id[p + (b < e)] = (int32_t)n;   // the place behind the last row
+        note_chunk_first(b, e, (int32_t)v, chunk.first, go_on);
+        note_chunk_first(b, e, (int32_t)p, chunk.first_place, go_on);
+        note_chunk_last(b, e, (int32_t)v, nnz, chunk.last);
+        note_chunk_last(b, e, (int32_t)p, nnz, chunk.last_place);
+    }
+}
+
 __global__ void k_pr_init(const int64_t* __restrict__ rp, int64_t n, float init, float* __restrict__ score,
-                          float* __restrict__ contrib, float* __restrict__ other, uint8_t* __restrict__ full) {
+                          float* __restrict__ contrib, float* __restrict__ other) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
         const int64_t d = rp[v + 1] - rp[v];
         score[v] = init;
         contrib[v] = d ? init / (float)d : 0.f;
         other[v] = 0.f;   // rows without entries are never written again
-        full[v] = d != 0;
-    }
-}
-
-// The rows with entries, in order: their offsets and ids.  The places behind them
-// hold nnz, so the offsets end as a CSR's whose last rows are empty.  And the rows
-// that hold each chunk's first and last entry.
-__global__ void k_pr_rows(const int64_t* __restrict__ rp, int64_t n, const int64_t* __restrict__ pos,
-                          int64_t* __restrict__ off, int32_t* __restrict__ id, int32_t* __restrict__ first,
-                          int32_t* __restrict__ last) {
-    const int64_t nnz = rp[n];
-    const int lane = threadIdx.x & 31;
-    for (int64_t v0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; v0 < n;
-         v0 += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t v = v0 + lane;
-        const int64_t b = v < n ? rp[v] : 0, e = v < n ? rp[v + 1] : 0, p = v < n ? pos[v] : 0;
-        if (b < e) {
-            off[p] = b;
-            id[p] = (int32_t)v;
-            if (e == nnz) off[p + 1] = nnz;
-        } else if (v < n) {
-            off[n - (v - p)] = nnz;   // v - p empty rows before this one
-        }
-        note_chunk_first(b, e, (int32_t)v, first, [] { return false; });
-        note_chunk_last(b, e, (int32_t)v, nnz, last);
     }
 }
 
@@ -85,9 +90,8 @@ struct PrArgs {
     const int64_t* rp;
     const int32_t* col;
     int64_t n, nnz;
-    const int64_t* off;   // offsets of the rows with entries (k_pr_rows)
-    const int32_t* id;    // their vertices
-    const int32_t* chunk_row;   // row of the chunk's first entry, or the complement of its place in off
+    const int32_t* id;          // the rows with entries (k_pr_rows)
+    const int32_t* chunk_row;   // row of the chunk's first entry, or the complement of its place in id
     float base, damp;
     const float* cin;
     float* cout;
@@ -99,7 +103,7 @@ struct PrArgs {
     double epsilon;
 };
 
-__device__ __forceinline__ double pr_put(const PrArgs& a, int32_t u, float s, int64_t d) {
+__device__ __forceinline__ double pr_put(const PrArgs& a, int64_t u, float s, int64_t d) {
     const float ns = a.base + a.damp * s;
     const double e = fabsf(ns - a.score[u]);
     a.score[u] = ns;
@@ -161,11 +165,9 @@ __global__ void __launch_bounds__(kT, 6) k_pr_sweep(PrArgs a, int it) {
         __syncthreads();
         // Rows from the one that holds entry e0, 256 at a time, until one starts past the chunk.
         const bool gaps = row0 < 0;
-        const int64_t* rp = gaps ? a.off : a.rp;
         for (int64_t u0 = gaps ? ~row0 : row0;; u0 += kT) {
-            const int64_t u = u0 + t;
-            const int64_t rb = u < a.n ? rp[u] : e1, re = u < a.n ? rp[u + 1] : e1;
-            const int32_t vertex = gaps && u < a.n ? a.id[u] : (int32_t)u;
+            const int64_t u = gaps ? (int64_t)a.id[min(u0 + t, a.n)] : u0 + t;
+            const int64_t rb = u < a.n ? a.rp[u] : e1, re = u < a.n ? a.rp[u + 1] : e1;
             const int b = (int)(max(rb, e0) - e0), e = rb < e1 ? (int)(min(re, e1) - e0) : b;
             if (t == kT - 1) s_more = rb < e1;
             float s = 0.f;
@@ -205,8 +207,8 @@ __global__ void __launch_bounds__(kT, 6) k_pr_sweep(PrArgs a, int it) {
                 if (rb < e0) a.head[c] = s;
                 else if (re > e1) {
                     a.tail[c] = s;
-                    a.tail_row[c] = vertex;
-                } else err += pr_put(a, vertex, s, re - rb);
+                    a.tail_row[c] = (int32_t)u;
+                } else err += pr_put(a, u, s, re - rb);
             }
             const bool more = s_more;
             if (t == 0) s_listed = 0;
@@ -239,24 +241,22 @@ __global__ void __launch_bounds__(kT) k_pr_join(PrArgs a, int it) {
     pr_add_change(err, a.err + it);
 }
 
-// Before the first sweep.  Rows without entries: the base score from here on.
-// Chunks: more than a fifth of the rows between the first and the last entry empty,
-// and the rows with entries are walked: first[c] becomes the complement of the
-// first one's place.  (By their ids a gap of 4 M in one chunk took 6.6 ms a sweep,
-// and R-MAT scale 20, where two ids in five are free, 34 us more; where there are
-// no gaps the ids are one more read, 4 us a sweep of a 517 x 1023 grid.)
-__global__ void __launch_bounds__(kT) k_pr_first(PrArgs a, const uint8_t* __restrict__ full,
-                                                 const int64_t* __restrict__ pos, const int32_t* __restrict__ last,
-                                                 int32_t* __restrict__ first) {
+// Before the first sweep.  Rows without entries: the base score from here on.  In a
+// graph with gaps, chunks of which more than a fifth of the rows are empty walk the
+// rows with entries: first[c] becomes the complement of the first one's place.  (By
+// their ids a gap of 4 M in one chunk took 6.6 ms a sweep.  Graphs without gaps are
+// spared the list: 30 us for a 517 x 1023 grid.)
+__global__ void __launch_bounds__(kT) k_pr_first(PrArgs a, PrChunks chunk) {
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t chunks = (a.nnz + kEdgeChunk - 1) / kEdgeChunk;
-    for (int64_t c = tid; c < chunks; c += stride) {
-        const int64_t rows = last[c] - first[c] + 1, place = pos[first[c]], held = pos[last[c]] - place + 1;
-        if (rows - held > rows / 5) first[c] = ~(int32_t)place;
+    for (int64_t c = tid; chunk.first_place && c < chunks; c += stride) {
+        const int32_t place = chunk.first_place[c];
+        const int32_t rows = chunk.last[c] - chunk.first[c] + 1, held = chunk.last_place[c] - place + 1;
+        if (rows - held > rows / 5) chunk.first[c] = ~place;
     }
     double err = 0.0;
     for (int64_t v = tid; v < a.n; v += stride) {
-        if (full[v]) continue;
+        if (a.rp[v] != a.rp[v + 1]) continue;
         const float ns = a.base + a.damp * 0.f;
         err += fabsf(ns - a.score[v]);
         a.score[v] = ns;
@@ -753,34 +753,43 @@ double pagerank_device(const DeviceCSR& g, int max_iters, double epsilon, float*
     if (n == 0) return 0.0;
     constexpr int kBatch = 8;   // sweeps enqueued between two looks at the change
     const int64_t chunks = edge_chunks(g.nnz);
-    // Few buffers: an allocation and its release are some 10 us of host time.
     DevBuf<float> contrib(2 * n, s), sums(2 * chunks, s);
-    DevBuf<int64_t> places(2 * n + 1, s);
-    DevBuf<int32_t> rows(n + 3 * chunks, s);
-    DevBuf<uint8_t> full(n, s);
+    DevBuf<int32_t> rows(g.gaps ? n + 1 + 5 * chunks : 2 * chunks, s);
     DevBuf<double> err(kBatch, s);
     float *ca = contrib.get(), *cb = ca + n, *head = sums.get(), *tail = head + chunks;
-    int64_t *pos = places.get(), *off = pos + n;
-    int32_t *id = rows.get(), *chunk_row = id + n, *chunk_last = chunk_row + chunks, *tail_row = chunk_last + chunks;
+    int32_t *tail_row = rows.get(), *id = g.gaps ? tail_row + 5 * chunks : nullptr;
+    PrChunks chunk{tail_row + chunks, nullptr, nullptr, nullptr};
     cudaEvent_t e0, e1;
     GB_CUDA(cudaEventCreate(&e0));
     GB_CUDA(cudaEventCreate(&e1));
     GB_CUDA(cudaEventRecord(e0, s));
     const float init = 1.0f / (float)n, damp = 0.85f, base = (1.0f - damp) / (float)n;
-    k_pr_init<<<grid_for(n, kT), kT, 0, s>>>(g.row_ptr, n, init, score, ca, cb, full);
+    if (g.gaps) {
+        // The scores and contributions lend their place to the rows' flags and positions.
+        uint8_t* full = reinterpret_cast<uint8_t*>(score);
+        int64_t* pos = reinterpret_cast<int64_t*>(contrib.get());
+        chunk.last = chunk.first + chunks;
+        chunk.first_place = chunk.last + chunks;
+        chunk.last_place = chunk.first_place + chunks;
+        k_pr_full<<<grid_for(n, kT), kT, 0, s>>>(g.row_ptr, n, full);
+        GB_LAUNCH_CHECK();
+        exclusive_scan_u8_to_i64(full, pos, n, nullptr, s);
+        k_pr_rows<<<grid_for(n, kT), kT, 0, s>>>(g.row_ptr, n, g.nnz, pos, id, chunk);
+        GB_LAUNCH_CHECK();
+    } else {
+        chunk_rows_device(g.row_ptr, n, g.nnz, chunk.first, s);
+    }
+    k_pr_init<<<grid_for(n, kT), kT, 0, s>>>(g.row_ptr, n, init, score, ca, cb);
     GB_LAUNCH_CHECK();
-    exclusive_scan_u8_to_i64(full, pos, n, nullptr, s);
-    k_pr_rows<<<grid_for(n, kT), kT, 0, s>>>(g.row_ptr, n, pos, off, id, chunk_row, chunk_last);
-    GB_LAUNCH_CHECK();
-    PrArgs a{g.row_ptr, g.col, n,    g.nnz, off,  id,       chunk_row, base,
-             damp,      ca,    cb,   score, head, tail,     tail_row,  err, epsilon};
+    PrArgs a{g.row_ptr, g.col, n,    g.nnz, id,   chunk.first, base, damp,   ca,
+             cb,        score, head, tail,  tail_row, err,     epsilon};
     const int grid = grid_for(chunks, 1), join_grid = grid_for(chunks * 32, kT);
     int it = 0;
     for (bool done = false; it < max_iters && !done;) {
         const int count = std::min(kBatch, max_iters - it);
         GB_CUDA(cudaMemsetAsync(err, 0, kBatch * sizeof(double), s));
         for (int k = 0; k < count; ++k) {
-            if (it + k == 0) k_pr_first<<<grid_for(n, kT), kT, 0, s>>>(a, full, pos, chunk_last, chunk_row);
+            if (it + k == 0) k_pr_first<<<grid_for(n, kT), kT, 0, s>>>(a, chunk);
             if (chunks > 0) {
                 k_pr_sweep<<<grid, kT, 0, s>>>(a, k);
                 k_pr_join<<<join_grid, kT, 0, s>>>(a, k);

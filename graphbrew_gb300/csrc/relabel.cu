@@ -375,7 +375,8 @@ __global__ void k_set_last(int64_t* p, int64_t n, int64_t v) { p[n] = v; }
 
 // Squished-CSR check: offsets non-decreasing from 0, neighbour ids in range,
 // rows strictly increasing (sorted, no duplicates).  bad[0]: offsets,
-// bad[1]: ids out of range, bad[2]: unsorted or duplicate.
+// bad[1]: ids out of range, bad[2]: unsorted or duplicate; and bad[3], which is no
+// fault: a chunk of entries whose rows are far apart (DeviceCSR::gaps).
 // Row offsets: rp[0] == 0, non-decreasing, rp[n] == nnz.  The pass also notes the
 // row that holds each chunk's first entry (a serial search per chunk in the pass
 // below took most of its time: 114 us for 33 M entries).  Malformed offsets can
@@ -406,6 +407,7 @@ __global__ void k_check_rows(const int64_t* __restrict__ rp, int64_t n, int64_t 
 // valid row offsets (bad[0] clear), so every entry lies in exactly one row.
 constexpr int kCheckChunk = kEdgeChunk;
 constexpr int kCheckThreads = 256;
+constexpr int kGapSteps = 64;   // 16 K rows for 4,096 entries: three in four of them empty
 
 __global__ void __launch_bounds__(kCheckThreads)
 k_check_cols(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, int64_t n, int64_t nnz,
@@ -420,11 +422,13 @@ k_check_cols(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, in
         const int64_t u0 = chunk_row[c];
         for (int w = threadIdx.x; w < kCheckChunk / 32; w += blockDim.x) starts[w] = 0;
         __syncthreads();
-        for (int64_t u = u0 + threadIdx.x; u <= n; u += blockDim.x) {
+        int64_t u = u0 + threadIdx.x;
+        for (; u <= n; u += blockDim.x) {
             const int64_t r = rp[u];
             if (r >= e1) break;
             if (r >= e0) atomicOr(&starts[(r - e0) >> 5], 1u << ((r - e0) & 31));
         }
+        if (threadIdx.x == 0 && u - u0 > kGapSteps * kCheckThreads) bad[3] = 1;
         __syncthreads();
 #pragma unroll 8
         for (int64_t i = e0 + threadIdx.x; i < e1; i += blockDim.x) {
@@ -441,10 +445,10 @@ k_check_cols(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, in
 
 }  // namespace
 
-void check_graph_device(const DeviceCSR& g, cudaStream_t s) {
+void check_graph_device(DeviceCSR& g, cudaStream_t s) {
     if (g.n == 0) return;
-    DevBuf<int32_t> bad(3, s);
-    GB_CUDA(cudaMemsetAsync(bad, 0, 3 * sizeof(int32_t), s));
+    DevBuf<int32_t> bad(4, s);
+    GB_CUDA(cudaMemsetAsync(bad, 0, 4 * sizeof(int32_t), s));
     DevBuf<int32_t> chunk_row(std::max<int64_t>(1, edge_chunks(g.nnz)), s);
     k_check_rows<<<grid_for(g.n + 1, 256), 256, 0, s>>>(g.row_ptr, g.n, g.nnz, bad, chunk_row);
     GB_LAUNCH_CHECK();
@@ -453,12 +457,13 @@ void check_graph_device(const DeviceCSR& g, cudaStream_t s) {
                                                                                        g.nnz, chunk_row, bad);
         GB_LAUNCH_CHECK();
     }
-    int32_t h[3];
+    int32_t h[4];
     GB_CUDA(cudaMemcpyAsync(h, bad.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
     GB_CUDA(cudaStreamSynchronize(s));
     GB_REQUIRE(!h[0], GBGPU_E_INVALID, "row offsets are not a non-decreasing sequence from 0 to nnz");
     GB_REQUIRE(!h[1], GBGPU_E_INVALID, "neighbour id out of range");
     GB_REQUIRE(!h[2], GBGPU_E_INVALID, "rows must be sorted ascending without duplicates (squished CSR)");
+    g.gaps = h[3] != 0;
 }
 
 int validate_permutation_device(const int32_t* ids, int64_t n, int32_t* inv_out, cudaStream_t s,
