@@ -300,6 +300,7 @@ __device__ __forceinline__ void bfs_push(bool add, int32_t v, int64_t deg, int32
 constexpr int kSmallEdges = 32768;
 constexpr int kSmallT = 1024;
 constexpr int kSmallOwn = 8;         // rows up to this long by their own thread
+constexpr int kSmallPlain = 4096;    // frontiers of more entries ask for their rows' mean length
 constexpr int kBitsQ = 2048;         // queue beside a bitmap
 constexpr int kPlainQ = 4096;
 constexpr int64_t kBitsMax = 160 * 1024 * 8;   // vertices whose bitmap shared memory holds
@@ -322,10 +323,11 @@ k_bfs_small(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, int
     uint32_t* bits = reinterpret_cast<uint32_t*>(nxt + kSmallQ);
     __shared__ int s_n[2];
     __shared__ unsigned s_edges[2];   // degrees cut at 2^16, below 2^31 for kSmallEdges claims
+    __shared__ int s_warp[kSmallT / 32];
     const int tid = threadIdx.x, lane = tid & 31;
     int nf = ctl->nf, level = ctl->level;
-    unsigned long long edges = ctl->edges;
-    if (nf > kSmallQ || edges > (unsigned long long)kSmallEdges) return;
+    if (nf > kSmallQ || ctl->edges > (unsigned long long)kSmallEdges) return;
+    unsigned edges = (unsigned)ctl->edges;
     if (kBits) {
         for (int64_t w = tid; w < words; w += kSmallT) bits[w] = fresh ? 0u : visited[w];
         __syncthreads();
@@ -403,22 +405,125 @@ k_bfs_small(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, int
                 ++at;
             }
     };
-    while (nf > 0 && nf <= kSmallQ && edges <= (unsigned long long)kSmallEdges) {
-        for (int i0 = tid - lane; i0 < nf; i0 += kSmallT) {
-            const int i = i0 + lane;
-            SmallEntry u{0, 0, 0};
-            if (i < nf) u = cur[i];
-            const int own = u.deg <= kSmallOwn ? u.deg : 0;
-            for (int k = 0; __any_sync(kFull, k < own); k += 4) claim4(col + u.b + k, own - k, false);
-            unsigned todo = __ballot_sync(kFull, u.deg > kSmallOwn);
-            while (todo) {
-                const int src = __ffs(todo) - 1;
-                todo &= todo - 1;
-                const int64_t b = __shfl_sync(kFull, u.b, src);
-                const int d = __shfl_sync(kFull, u.deg, src);
-                for (int k = 0; k < d; k += 128) claim4(col + b + k + 4 * lane, d - k - 4 * lane, true);
+    // A level of rows above kSmallOwn entries on average: entries dealt to the lanes one
+    // by one, 192 a warp at a time, whatever the rows.  Degrees become their inclusive
+    // prefix, where an entry's row is searched for; the next frontier's rows are looked
+    // up once a level.  Row after row by a warp, 500 levels of 2,000 vertices with 16
+    // neighbours took 27.8 ms, where a launch and a look a level had taken 17.1; so
+    // 9.1.  Without a bitmap, 700 levels: 46.0, 24.3 and 17.7.
+    auto flat_level = [&]() {
+        constexpr int kPer = kSmallQ / kSmallT, kLane = 6, kRows = 2;
+        const int i0 = tid * kPer;
+        int sum = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) sum += i0 + k < nf ? cur[i0 + k].deg : 0;
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += x;
+        }
+        if (lane == 31) s_warp[tid >> 5] = incl;
+        __syncthreads();
+        int run = incl - sum + __reduce_add_sync(kFull, lane < tid >> 5 ? s_warp[lane] : 0);
+#pragma unroll
+        for (int k = 0; k < kPer; ++k)
+            if (i0 + k < nf) cur[i0 + k].deg = run += cur[i0 + k].deg;
+        __syncthreads();
+        const int total = cur[nf - 1].deg;
+        int top = 1;
+        while (top < nf) top <<= 1;
+        // The first entry's row by search, the later ones' by walking on: a search for
+        // each took most of the level's instructions.
+        auto fetch = [&](int k0, int32_t (&v)[kLane]) {
+            int at = 0;
+            for (int half = top >> 1; half > 0; half >>= 1)
+                if (at + half < nf && cur[at + half - 1].deg <= k0 + lane) at += half;
+#pragma unroll
+            for (int k = 0; k < kLane; ++k) {
+                const int e = k0 + 32 * k + lane;
+                v[k] = -1;
+                if (e < total) {
+                    while (cur[at].deg <= e) ++at;
+                    v[k] = col[cur[at].b + (e - (at ? cur[at - 1].deg : 0))];
+                }
+            }
+        };
+        int32_t ahead[kLane];
+        int k0 = (tid - lane) * kLane;
+        fetch(k0, ahead);
+        while (k0 < total) {
+            int32_t v[kLane];
+#pragma unroll
+            for (int k = 0; k < kLane; ++k) v[k] = ahead[k];
+            k0 += kSmallT * kLane;
+            if (k0 < total) fetch(k0, ahead);   // in flight during the claims
+            if (!kBits) {
+#pragma unroll
+                for (int k = 0; k < kLane; ++k)
+                    if (v[k] >= 0 && depth[v[k]] >= 0) v[k] = -1;
+            }
+            // Claims in flight together.
+            int32_t old[kLane];
+#pragma unroll
+            for (int k = 0; k < kLane; ++k) {
+                old[k] = 0;
+                if (v[k] < 0) continue;
+                if (kBits) old[k] = (int32_t)(atomicOr(&bits[v[k] >> 5], 1u << (v[k] & 31)) >> (v[k] & 31) & 1u) - 1;
+                else old[k] = atomicCAS(&depth[v[k]], -1, level + 1);
+            }
+            int mine = 0;
+#pragma unroll
+            for (int k = 0; k < kLane; ++k) {
+                if (old[k] != -1) continue;
+                if (kBits) depth[v[k]] = level + 1;
+                ++mine;
+            }
+            if (!__any_sync(kFull, mine != 0)) continue;
+            int put = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(kFull, put, o);
+                if (lane >= o) put += x;
+            }
+            int base = 0;
+            if (lane == 31) base = atomicAdd(&s_n[par], put);
+            put += __shfl_sync(kFull, base, 31) - mine;
+#pragma unroll
+            for (int k = 0; k < kLane; ++k)
+                if (old[k] == -1) {
+                    if (put < kSmallQ) nxt[put].v = v[k];
+                    else q[put] = v[k];
+                    ++put;
+                }
+        }
+        __syncthreads();
+        const int found = s_n[par];
+        unsigned deg = 0;
+        for (int i0 = tid; i0 < found; i0 += kRows * kSmallT) {
+            int32_t u[kRows];
+            int64_t b[kRows], e[kRows];
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) {
+                const int i = i0 + k * kSmallT;
+                u[k] = i < min(found, kSmallQ) ? nxt[i].v : i < found ? q[i] : -1;
+            }
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) {
+                b[k] = u[k] >= 0 ? rp[u[k]] : 0;
+                e[k] = u[k] >= 0 ? rp[u[k] + 1] : 0;
+            }
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) {
+                const int i = i0 + k * kSmallT;
+                if (i < min(found, kSmallQ)) nxt[i] = SmallEntry{b[k], (int32_t)(e[k] - b[k]), u[k]};
+                deg += (unsigned)min(e[k] - b[k], (int64_t)65536);
             }
         }
+        deg = __reduce_add_sync(kFull, deg);
+        if (lane == 0) atomicAdd(&s_edges[par], deg);
+    };
+    auto next_level = [&]() {
         __syncthreads();
         nf = s_n[par];
         edges = s_edges[par];
@@ -432,6 +537,33 @@ k_bfs_small(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, int
         cur = nxt;
         nxt = t;
         __syncthreads();
+    };
+    while (nf > 0 && nf <= kSmallQ && edges <= (unsigned)kSmallEdges) {
+        if (edges > (unsigned)(kSmallOwn * nf)) {
+            flat_level();
+            next_level();
+            continue;
+        }
+        // Asked again after a level of many entries; smaller ones go on without.
+        const unsigned most = edges <= (unsigned)kSmallPlain ? kSmallPlain : 0;
+        do {
+            for (int i0 = tid - lane; i0 < nf; i0 += kSmallT) {
+                const int i = i0 + lane;
+                SmallEntry u{0, 0, 0};
+                if (i < nf) u = cur[i];
+                const int own = u.deg <= kSmallOwn ? u.deg : 0;
+                for (int k = 0; __any_sync(kFull, k < own); k += 4) claim4(col + u.b + k, own - k, false);
+                unsigned todo = __ballot_sync(kFull, u.deg > kSmallOwn);
+                while (todo) {
+                    const int src = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    const int64_t b = __shfl_sync(kFull, u.b, src);
+                    const int d = __shfl_sync(kFull, u.deg, src);
+                    for (int k = 0; k < d; k += 128) claim4(col + b + k + 4 * lane, d - k - 4 * lane, true);
+                }
+            }
+            next_level();
+        } while (nf > 0 && nf <= kSmallQ && edges <= most);
     }
     for (int i = tid; i < min(nf, kSmallQ); i += kSmallT) q[i] = cur[i].v;
     if (tid == 0) {

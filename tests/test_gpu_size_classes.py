@@ -211,6 +211,45 @@ def test_input_check_of_one_long_row(ctx):
             ctx.dbg_mapping(torch.tensor(offsets, device="cuda"), torch.zeros(40000, dtype=torch.int32, device="cuda"))
 
 
+def _bfs_levels(rp, col, source):
+    """BFS depths, a level at a time over whole arrays."""
+    depth = torch.full((len(rp) - 1,), -1, dtype=torch.int32, device=rp.device)
+    depth[source] = 0
+    front, level = torch.tensor([source], device=rp.device), 0
+    while len(front):
+        degree = rp[front + 1] - rp[front]
+        first = torch.repeat_interleave(rp[front] - torch.cumsum(degree, 0) + degree, degree)
+        reached = col[first + torch.arange(len(first), device=rp.device)].long()
+        front = torch.unique(reached[depth[reached] < 0])
+        level += 1
+        depth[front] = level
+    return depth
+
+
+def _layers(width, fan, count):
+    """Layers of `width` vertices, each joined to `fan` random ones of the next."""
+    i = torch.arange(width * (count - 1), device="cuda").repeat_interleave(fan)
+    rng = np.random.default_rng(width + fan)
+    j = (i // width + 1) * width + torch.from_numpy(rng.integers(0, width, len(i))).cuda()
+    return gg.squish(i, j, width * count)
+
+
+@pytest.mark.parametrize("width,fan,count,most_us", [
+    # Levels of the one-CTA kernel: rows on both sides of 8 entries, frontiers on both
+    # sides of 2,048 vertices (4,096 above 1,310,720 vertices), 4,096 and 32,768 entries.
+    (1, 1, 60, 0), (3, 7, 60, 0), (40, 40, 40, 0), (512, 4, 60, 0), (513, 4, 60, 0), (1025, 2, 60, 0),
+    (2048, 8, 40, 0), (2049, 7, 40, 0), (1024, 16, 40, 0), (1024, 18, 40, 0), (33, 31, 60, 0),
+    # A level of some 30,000 entries takes 34 us as two launches and a look at the
+    # counters, and no longer by one CTA.
+    (1900, 8, 500, 34), (1900, 8, 720, 34)])
+def test_bfs_of_small_frontiers(ctx, width, fan, count, most_us):
+    rp, col = _layers(width, fan, count)
+    for source in {0, (width * count) // 2}:
+        assert torch.equal(ctx.bfs(rp, col, source)[0], _bfs_levels(rp, col, source))
+    if most_us:
+        assert _least(lambda: ctx.bfs(rp, col, 0)[1]) <= 1e-3 * most_us * count
+
+
 @pytest.mark.parametrize("rows,in_dim,batch", [(1, 1, 1), (7, 12, 8), (9, 12, 8), (64, 3, 64), (129, 12, 128),
                                                (300, 32, 256), (513, 12, 100), (300, 33, 256), (300, 12, 257)])
 def test_training_by_batch_and_inputs(ctx, rows, in_dim, batch):
