@@ -1126,12 +1126,19 @@ __global__ void k_bfs_bases(int32_t nslots, const int64_t* __restrict__ fs, cons
     }
 }
 
+__device__ __forceinline__ void warp_add_sum(unsigned long long* out, unsigned long long v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(out, v);
+}
+
+// degree_sum: the entries of the next frontier.
 __global__ void __launch_bounds__(256)
 k_bfs_write(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D, const int64_t* __restrict__ rp,
             const int32_t* __restrict__ col, const uint32_t* __restrict__ memb, Discoveries d,
             const int32_t* __restrict__ slot_of_comm,
             const int64_t* __restrict__ qlen, const int64_t* __restrict__ base, int32_t* __restrict__ nextF,
-            uint32_t* __restrict__ claim, uint32_t* __restrict__ local) {
+            uint32_t* __restrict__ claim, uint32_t* __restrict__ local, unsigned long long* __restrict__ degree_sum) {
+    unsigned long long sum = 0;
     for_edge_runs(F, nf, D, rp, col, [&](int64_t run) { return d.bits[run] == 0; },
                   [&](int64_t run, const int32_t* nbr, const int32_t*) {
                       const uint32_t b = d.bits[run];
@@ -1143,9 +1150,11 @@ k_bfs_write(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict
                           nextF[p] = w;
                           claim[w] = 0;
                           local[w] = (uint32_t)(qlen[j] + (p - base[j]));
+                          sum += (unsigned long long)(rp[w + 1] - rp[w]);
                           ++p;
                       }
                   });
+    warp_add_sum(degree_sum, sum);
 }
 
 __global__ void k_bfs_advance(int32_t nslots, int64_t* __restrict__ qlen, int64_t* __restrict__ fs,
@@ -1214,12 +1223,12 @@ __global__ void k_rcm_frontier(int32_t nslots, const int32_t* __restrict__ part,
 }
 
 // Children in (parent, row offset) order with their parent's frontier index,
-// and the largest of their degrees.
+// and the largest of their degrees and their sum.
 __global__ void __launch_bounds__(256)
 k_rcm_write(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict__ D, const int64_t* __restrict__ rp,
             const int32_t* __restrict__ col, Discoveries d, int32_t* __restrict__ nextF, int32_t* __restrict__ parent, uint32_t* __restrict__ claim,
-            unsigned long long* __restrict__ max_deg) {
-    unsigned long long m = 0;
+            unsigned long long* __restrict__ max_deg, unsigned long long* __restrict__ degree_sum) {
+    unsigned long long m = 0, sum = 0;
     for_edge_runs(F, nf, D, rp, col, [&](int64_t run) { return d.bits[run] == 0; },
                   [&](int64_t run, const int32_t* nbr, const int32_t* idx) {
                       const uint32_t b = d.bits[run];
@@ -1231,12 +1240,15 @@ k_rcm_write(const int32_t* __restrict__ F, int64_t nf, const int64_t* __restrict
                           nextF[p] = w;
                           parent[p] = idx[k];
                           claim[w] = 0;
-                          m = max(m, (unsigned long long)(rp[w + 1] - rp[w]));
+                          const unsigned long long deg = (unsigned long long)(rp[w + 1] - rp[w]);
+                          m = max(m, deg);
+                          sum += deg;
                           ++p;
                       }
                   });
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
     if ((threadIdx.x & 31) == 0 && m) atomicMax(max_deg, m);
+    warp_add_sum(degree_sum, sum);
 }
 
 // Last level of a slot whose next level is empty: minimum degree, first in
@@ -1419,33 +1431,39 @@ T read_dev(const T* p, cudaStream_t s) {
     return h;
 }
 
-// The discoveries of one BFS level, in device memory sized for the graph: the
-// host bounds the frontier's edges by its vertices and the largest degree, so a
-// level needs no look at the device before its kernels are enqueued, and one
-// after (two or three a level were a third of RCM's time).
+// The discoveries of one BFS level, in device memory sized for the graph.  A level
+// needs no look at the device before its kernels are enqueued, and one after (two or
+// three a level were a third of RCM's time): its number of edges comes with the
+// children of the level before.  A first level's is bounded by its vertices and the
+// largest degree; with that bound for every level, one hub had 1,500 levels of 40
+// vertices pass over all of 142 M entries' runs (196.7 ms, 134.9 with the looks).
 struct LevelBufs {
     DevBuf<uint8_t> bits;
     DevBuf<uint16_t> first;
     DevBuf<int64_t> count;
-    DevBuf<unsigned long long> out;   // children, the largest of their degrees
+    DevBuf<unsigned long long> out;   // children, the largest of their degrees, the degrees' sum
     int64_t max_deg = 0, bound = 0, blocks = 0;
+    int64_t edges = -1;               // the next frontier's entries, -1: not known
     static int64_t blocks_for(int64_t edges) { return ceil_div(ceil_div(edges, kEdgeRun), kRunBlock); }
     LevelBufs(const DeviceCSR& g, int64_t nn, const int32_t* order_v, cudaStream_t s)
         : bits(blocks_for(g.nnz) * kRunBlock, s), first(blocks_for(g.nnz) * kRunBlock, s),
-          count(blocks_for(g.nnz) + 1, s), out(2, s) {
-        GB_CUDA(cudaMemsetAsync(out, 0, 2 * sizeof(unsigned long long), s));
+          count(blocks_for(g.nnz) + 1, s), out(3, s) {
+        GB_CUDA(cudaMemsetAsync(out, 0, 3 * sizeof(unsigned long long), s));
         k_max_degree_of<<<grid_for(nn, kT), kT, 0, s>>>(order_v, nn, g.row_ptr, out);
         GB_LAUNCH_CHECK();
         max_deg = (int64_t)read_dev(out.get(), s);
     }
     unsigned long long* max_child() const { return out.get() + 1; }
+    unsigned long long* degree_sum() const { return out.get() + 2; }
     Discoveries view() const { return {bits.get(), first.get(), count.get(), blocks}; }
+    // A frontier that is not the last level's children comes next.
+    void restart() { edges = -1; }
     // Claims and discoveries of the frontier F[0, nf); D receives its edge offsets.
     void find(const DeviceCSR& g, const int32_t* F, int64_t nf, int64_t* D, const uint32_t* memb, uint32_t* claim,
               cudaStream_t s) {
-        bound = nf > g.nnz / std::max<int64_t>(max_deg, 1) ? g.nnz : nf * max_deg;
+        bound = edges >= 0 ? edges : nf > g.nnz / std::max<int64_t>(max_deg, 1) ? g.nnz : nf * max_deg;
         blocks = blocks_for(bound);
-        GB_CUDA(cudaMemsetAsync(out, 0, 2 * sizeof(unsigned long long), s));
+        GB_CUDA(cudaMemsetAsync(out, 0, 3 * sizeof(unsigned long long), s));
         k_frontier_degrees<<<grid_for(nf, kT), kT, 0, s>>>(F, nf, g.row_ptr, D);
         GB_LAUNCH_CHECK();
         exclusive_scan_i64_total(D, D, nf, D + nf, s);
@@ -1460,10 +1478,11 @@ struct LevelBufs {
     // Children of the level (after the kernels that write them).
     int64_t children(unsigned long long* max_child_deg, cudaStream_t s) {
         GB_CUDA(cudaMemcpyAsync(out, count.get() + blocks, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
-        unsigned long long h[2];
+        unsigned long long h[3];
         GB_CUDA(cudaMemcpyAsync(h, out.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
         GB_CUDA(cudaStreamSynchronize(s));
         if (max_child_deg) *max_child_deg = h[1];
+        edges = (int64_t)h[2];
         return (int64_t)h[0];
     }
 };
@@ -1522,6 +1541,7 @@ int64_t rcm_communities(const DeviceCSR& g, const uint32_t* memb, const int32_t*
         }
         int64_t nf = np;
         uint32_t level = 0;
+        lv.restart();
         while (nf > 0) {
             ++levels;
             if (dep) {
@@ -1534,7 +1554,7 @@ int64_t rcm_communities(const DeviceCSR& g, const uint32_t* memb, const int32_t*
             k_bfs_bases<<<grid_for(nslots, kT), kT, 0, s>>>(nslots, fs, fe, D, lv.view(), bbase, bend);
             GB_LAUNCH_CHECK();
             k_rcm_write<<<edge_grid(lv.bound), 256, 0, s>>>(F, nf, D, g.row_ptr, g.col, lv.view(), NF, parent, claim,
-                                                           lv.max_child());
+                                                           lv.max_child(), lv.degree_sum());
             GB_LAUNCH_CHECK();
             unsigned long long md = 0;
             const int64_t next = lv.children(&md, s);
@@ -1870,7 +1890,7 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
             k_bfs_bases<<<grid_for(nbfs, kT), kT, 0, s>>>(nbfs, fs, fe, D, lv.view(), bbase, bend);
             GB_LAUNCH_CHECK();
             k_bfs_write<<<edge_grid(lv.bound), 256, 0, s>>>(F, nf, D, g.row_ptr, g.col, memb, lv.view(),
-                                                           slot_of_comm, qlen, bbase, NF, claim, local);
+                                                           slot_of_comm, qlen, bbase, NF, claim, local, lv.degree_sum());
             GB_LAUNCH_CHECK();
             k_bfs_advance<<<grid_for(nbfs, kT), kT, 0, s>>>(nbfs, qlen, fs, fe, bbase, bend);
             GB_LAUNCH_CHECK();

@@ -250,6 +250,29 @@ def test_bfs_of_small_frontiers(ctx, width, fan, count, most_us):
         assert _least(lambda: ctx.bfs(rp, col, 0)[1]) <= 1e-3 * most_us * count
 
 
+@pytest.mark.parametrize("intra", ["intra_bfs", "intra_rcm"])
+def test_orders_of_long_paths_beside_a_hub(ctx, intra):
+    # One community: a hub of 4 M leaves, 40 of which begin a path of 1,500 vertices, and a
+    # uniform graph.  The levels along the paths cost what they do without the rest, but
+    # for some dozen levels of the uniform graph's 67 M entries (a millisecond each).
+    def order_ms(leaves, *extra):
+        p, i = torch.arange(60000, device="cuda"), torch.arange(1, leaves + 1, device="cuda")
+        u = [torch.zeros_like(i), torch.where(p % 1500 == 0, 1 + p // 1500, leaves + p)]
+        v, n = [i, leaves + 1 + p], leaves + 60001
+        if extra:
+            rp, col = gg.uniform(*extra, seed=5, device="cuda")
+            u += [torch.repeat_interleave(torch.arange(len(rp) - 1, device="cuda"), rp[1:] - rp[:-1]) + n]
+            v += [col.long() + n]
+            u, v, n = u + [torch.tensor([0], device="cuda")], v + [torch.tensor([n], device="cuda")], n + len(rp) - 1
+        rp, col = gg.squish(torch.cat(u), torch.cat(v), n)
+        memb = torch.zeros(n, dtype=torch.int32, device="cuda")
+        recipe = gb.DEFAULT_RECIPE.replace("intra_gorder", intra)
+        return _least(lambda: ctx.order_compose(rp, col, memb, recipe)[1]["intra_ms"], 3)
+
+    alone = order_ms(40)
+    assert order_ms(1 << 22, 21, 16) <= 1.25 * alone + (60 if intra == "intra_rcm" else 15)
+
+
 @pytest.mark.parametrize("rows,in_dim,batch", [(1, 1, 1), (7, 12, 8), (9, 12, 8), (64, 3, 64), (129, 12, 128),
                                                (300, 32, 256), (513, 12, 100), (300, 33, 256), (300, 12, 257)])
 def test_training_by_batch_and_inputs(ctx, rows, in_dim, batch):
