@@ -1573,11 +1573,10 @@ int64_t rcm_communities(const DeviceCSR& g, const uint32_t* memb, const int32_t*
                 DevBuf<uint32_t> vals(next, s);
                 k_rcm_keys<<<grid_for(next, kT), kT, 0, s>>>(NF, parent, next, g.row_ptr, degbits, keys, vals);
                 GB_LAUNCH_CHECK();
-                radix_sort_pairs_u64(keys, vals, next, degbits + pbits, s);
+                *launches += 3 + radix_sort_pairs_u64(keys, vals, next, degbits + pbits, s);
                 k_rcm_assign<<<grid_for(next, kT), kT, 0, s>>>(vals, next, memb, slot_of_comm, qlen, bbase, NF,
                                                                local);
                 GB_LAUNCH_CHECK();
-                *launches += 3 + 3 * ((degbits + pbits + 7) / 8);
             }
             k_bfs_advance<<<grid_for(nslots, kT), kT, 0, s>>>(nslots, qlen, fs, fe, bbase, bend);
             GB_LAUNCH_CHECK();
@@ -1616,10 +1615,9 @@ int64_t rcm_communities(const DeviceCSR& g, const uint32_t* memb, const int32_t*
                 k_rcmpp_keys<<<grid_for(nn, kT), kT, 0, s>>>(order_v, ranks, nn, g.row_ptr, depth.get(), low, max_depth,
                                                             by_depth, keys, sp);
                 GB_LAUNCH_CHECK();
-                radix_sort_pairs_u64(keys, sp, nn, low + rbits, s);
+                *launches += 2 + radix_sort_pairs_u64(keys, sp, nn, low + rbits, s);
                 k_rcmpp_rank<<<grid_for(nn, kT), kT, 0, s>>>(sp, ranks, offs, nn, score);
                 GB_LAUNCH_CHECK();
-                *launches += 2 + 3 * ((low + rbits + 7) / 8);
             }
             DevBuf<unsigned long long> best(nslots, s);
             GB_CUDA(cudaMemsetAsync(best, 0xFF, nslots * sizeof(unsigned long long), s));
@@ -1726,8 +1724,7 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
         int kbits = 0;
         if (co == kSizeDesc || co == kSizeAsc) kbits = bits_for(max_size);
         else if (co == kDegreeDesc || co == kDegreeAsc) kbits = bits_for(max_deg);
-        radix_sort_pairs_u64(keys, comm_order, C, kbits, s);
-        launches += 4 + 3 * ((kbits + 7) / 8);
+        launches += 4 + radix_sort_pairs_u64(keys, comm_order, C, kbits, s);
     }
     DevBuf<uint32_t> rank(C, s);
     DevBuf<int64_t> ssize(C, s);
@@ -1742,12 +1739,11 @@ void compose_device(const DeviceCSR& g, const uint32_t* memb, const ComposeParam
     k_vertex_keys<<<grid_for(n, kT), kT, 0, s>>>(g.row_ptr, memb, rank, n, (uint32_t)C, vkeys, order_v);
     GB_LAUNCH_CHECK();
     const int vbits = bits_for((uint64_t)C);
-    radix_sort_pairs_u32(vkeys, order_v, n, vbits, s);
+    launches += 6 + radix_sort_pairs_u32(vkeys, order_v, n, vbits, s);
     DevBuf<int64_t> pos_of(n, s);
     DevBuf<uint32_t> local(n, s);
     k_positions<<<grid_for(n, kT), kT, 0, s>>>(order_v, vkeys, offs, n, (uint32_t)C, pos_of, local);
     GB_LAUNCH_CHECK();
-    launches += 6 + 3 * ((vbits + 7) / 8);
 
     // Classify communities.
     DevBuf<int32_t> lists(kClasses * C, s);

@@ -1022,10 +1022,9 @@ void hilbert_perm(const DeviceCSR& g, const uint32_t* memb, const uint32_t* csiz
     DevBuf<uint32_t> ids(C, s);
     k_hilbert_keys<<<grid_for(C, kT), kT, 0, s>>>(csize, tot, C, mx, key, ids);
     GB_LAUNCH_CHECK();
-    radix_sort_pairs_u64(key, ids, C, 16, s);   // d < 2^16; stable: ties by id
+    *nl += 4 + radix_sort_pairs_u64(key, ids, C, 16, s);   // d < 2^16; stable: ties by id
     k_perm_from_order<<<grid_for(C, kT), kT, 0, s>>>(ids, C, perm);
     GB_LAUNCH_CHECK();
-    *nl += 4 + 3 * 2;
 }
 
 // The super-graph's maps (RG:5033-5072, one thread): sizes, offsets, the
@@ -1078,7 +1077,7 @@ void build_super_maps(const DeviceCSR& g, const uint32_t* memb, int64_t C, Super
         GB_LAUNCH_CHECK();
         *nl += 5;
         if (m0 > 0) {
-            radix_sort_pairs_u64(key, val, m0, 2 * cb, s);   // stable: entries ascending inside a pair
+            *nl += 7 + radix_sort_pairs_u64(key, val, m0, 2 * cb, s);   // stable: entries ascending inside a pair
             DevBuf<uint8_t> uflag(m0, s);
             DevBuf<int64_t> upos(m0 + 1, s);
             k_run_flags<<<grid_for(m0, kT), kT, 0, s>>>(key, m0, uflag);
@@ -1096,7 +1095,6 @@ void build_super_maps(const DeviceCSR& g, const uint32_t* memb, int64_t C, Super
             GB_LAUNCH_CHECK();
             k_unique_weights<<<grid_for(m, kT), kT, 0, s>>>(head, m, m0, sm.uw);
             GB_LAUNCH_CHECK();
-            *nl += 7 + 3 * ((2 * cb + 7) / 8);
         }
     }
     sm.m = m;
@@ -1110,10 +1108,9 @@ void build_super_maps(const DeviceCSR& g, const uint32_t* memb, int64_t C, Super
         rkey.alloc(mr > 0 ? mr : 1, s);
         k_reverse_emit<<<grid_for(m, kT), kT, 0, s>>>(key2, d2, m, eb, cb, rflag, rpos, rkey);
         GB_LAUNCH_CHECK();
-        if (mr > 0) radix_sort_keys_u64(rkey, mr, 2 * cb, s);
+        if (mr > 0) *nl += radix_sort_keys_u64(rkey, mr, 2 * cb, s);
         // Per-map insertion order: by community, then first entry.
-        radix_sort_pairs_u64(key2, d2, m, cb + eb, s);
-        *nl += 4 + 3 * ((2 * cb + 7) / 8) + 3 * ((cb + eb + 7) / 8);
+        *nl += 4 + radix_sort_pairs_u64(key2, d2, m, cb + eb, s);
     }
     sm.mr = mr;
     sm.moff.alloc(C + 1, s);

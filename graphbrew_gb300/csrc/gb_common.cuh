@@ -148,10 +148,11 @@ void exclusive_scan_u8_to_i64(const uint8_t* in, int64_t* out, int64_t n, int64_
 
 // Stable LSD radix sort of (key, value) pairs by the low `key_bits` bits of
 // the key.  keys/values are sorted in place (double-buffered through scratch).
-void radix_sort_pairs_u32(uint32_t* keys, uint32_t* values, int64_t n, int key_bits, cudaStream_t s);
-void radix_sort_pairs_u64(uint64_t* keys, uint32_t* values, int64_t n, int key_bits, cudaStream_t s);
+// The sorts return the kernels they launched.
+int radix_sort_pairs_u32(uint32_t* keys, uint32_t* values, int64_t n, int key_bits, cudaStream_t s);
+int radix_sort_pairs_u64(uint64_t* keys, uint32_t* values, int64_t n, int key_bits, cudaStream_t s);
 // Stable LSD radix sort of 64-bit keys alone.
-void radix_sort_keys_u64(uint64_t* keys, int64_t n, int key_bits, cudaStream_t s);
+int radix_sort_keys_u64(uint64_t* keys, int64_t n, int key_bits, cudaStream_t s);
 
 // Fill helpers.
 void fill_u32(uint32_t* p, uint32_t v, int64_t n, cudaStream_t s);

@@ -1655,7 +1655,7 @@ void leiden_device(const DeviceCSR& g, const LeidenParams& p, uint32_t* vcom, gb
         DevBuf<uint32_t> snbr, sw;
         int64_t nuniq = 0;
         if (ninter > 0) {
-            radix_sort_keys_u64(ikeys, ninter, 2 * cb, s);
+            launches += 7 + radix_sort_keys_u64(ikeys, ninter, 2 * cb, s);
             DevBuf<uint8_t> uflag(ninter, s);
             DevBuf<int64_t> upos(ninter + 1, s);
             k_rle_flags<<<grid_for(ninter, kT), kT, 0, s>>>(ikeys, ninter, uflag);
@@ -1670,7 +1670,6 @@ void leiden_device(const DeviceCSR& g, const LeidenParams& p, uint32_t* vcom, gb
             GB_LAUNCH_CHECK();
             k_rle_weights<<<grid_for(nuniq, kT), kT, 0, s>>>(ustart, nuniq, ninter, sw);
             GB_LAUNCH_CHECK();
-            launches += 7 + 3 * ((2 * cb + 7) / 8);
         }
         {
             // soff = exclusive scan of sdeg (int32 -> int64)

@@ -129,29 +129,31 @@ k_scan_one(const Tin* __restrict__ in, int64_t* __restrict__ out, int64_t n, int
     if (total_out && threadIdx.x == 0) *total_out = carry;
 }
 
+// Returns its kernel launches.
 template <typename Tin>
-void exclusive_scan_impl(const Tin* in, int64_t* out, int64_t n, int64_t* total_dev, cudaStream_t s) {
+int exclusive_scan_impl(const Tin* in, int64_t* out, int64_t n, int64_t* total_dev, cudaStream_t s) {
     if (n <= 0) {
         if (total_dev) GB_CUDA(cudaMemsetAsync(total_dev, 0, sizeof(int64_t), s));
-        return;
+        return 0;
     }
     const int64_t tiles = ceil_div(n, kScanTile);
     if (tiles == 1) {
         k_tile_scan<Tin><<<1, kScanThreads, 0, s>>>(in, out, n, nullptr, total_dev);
         GB_LAUNCH_CHECK();
-        return;
+        return 1;
     }
     if (n <= kScanOneMax) {
         k_scan_one<Tin><<<1, kScanOneThreads, 0, s>>>(in, out, n, total_dev);
         GB_LAUNCH_CHECK();
-        return;
+        return 1;
     }
     DevBuf<int64_t> partial(tiles, s);
     k_tile_reduce<Tin><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, partial);
     GB_LAUNCH_CHECK();
-    exclusive_scan_impl<int64_t>(partial, partial, tiles, nullptr, s);
+    const int partials = exclusive_scan_impl<int64_t>(partial, partial, tiles, nullptr, s);
     k_tile_scan<Tin><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, out, n, partial, total_dev);
     GB_LAUNCH_CHECK();
+    return 2 + partials;
 }
 
 // ---------------------------------------------------------------------------
@@ -343,8 +345,8 @@ k_sort_small(K* __restrict__ keys, uint32_t* __restrict__ values, int n, int pad
 }
 
 template <typename K, bool kHasValues>
-void radix_sort_impl(K* keys, uint32_t* values, int64_t n, int key_bits, cudaStream_t s) {
-    if (n <= 1 || key_bits <= 0) return;
+int radix_sort_impl(K* keys, uint32_t* values, int64_t n, int key_bits, cudaStream_t s) {
+    if (n <= 1 || key_bits <= 0) return 0;
     const int passes = (key_bits + 7) / 8;
     if (n <= kSmallSort) {
         int padded = 2;
@@ -354,7 +356,7 @@ void radix_sort_impl(K* keys, uint32_t* values, int64_t n, int key_bits, cudaStr
         k_sort_small<K, kHasValues><<<1, std::min(kSmallSortThreads, std::max(32, padded / 2)), smem, s>>>(
             keys, values, (int)n, padded, mask);
         GB_LAUNCH_CHECK();
-        return;
+        return 1;
     }
     const int64_t tiles = ceil_div(n, kRadixTile);
     constexpr int smem = radix_scatter_smem<K, kHasValues>();
@@ -368,11 +370,12 @@ void radix_sort_impl(K* keys, uint32_t* values, int64_t n, int key_bits, cudaStr
     K* kout = kbuf.get();
     uint32_t* vin = values;
     uint32_t* vout = vbuf.get();
+    int launches = 0;
     for (int p = 0; p < passes; ++p) {
         const int shift = 8 * p;
         k_radix_hist<K><<<(unsigned)tiles, kRadixThreads, 0, s>>>(kin, n, shift, tiles, hist);
         GB_LAUNCH_CHECK();
-        exclusive_scan_impl<int32_t>(hist, offs, 256 * tiles, nullptr, s);
+        launches += 2 + exclusive_scan_impl<int32_t>(hist, offs, 256 * tiles, nullptr, s);
         k_radix_scatter<K, kHasValues><<<(unsigned)tiles, kRadixThreads, smem, s>>>(
             kin, vin, kout, vout, n, shift, tiles, offs);
         GB_LAUNCH_CHECK();
@@ -384,6 +387,7 @@ void radix_sort_impl(K* keys, uint32_t* values, int64_t n, int key_bits, cudaStr
         if (kHasValues)
             GB_CUDA(cudaMemcpyAsync(values, vin, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
     }
+    return launches;
 }
 
 __global__ void k_fill_u32(uint32_t* p, uint32_t v, int64_t n) {
@@ -442,14 +446,14 @@ void exclusive_scan_u8_to_i64(const uint8_t* in, int64_t* out, int64_t n, int64_
     exclusive_scan_impl<uint8_t>(in, out, n, total_dev, s);
 }
 
-void radix_sort_pairs_u32(uint32_t* keys, uint32_t* values, int64_t n, int key_bits, cudaStream_t s) {
-    radix_sort_impl<uint32_t, true>(keys, values, n, key_bits, s);
+int radix_sort_pairs_u32(uint32_t* keys, uint32_t* values, int64_t n, int key_bits, cudaStream_t s) {
+    return radix_sort_impl<uint32_t, true>(keys, values, n, key_bits, s);
 }
-void radix_sort_pairs_u64(uint64_t* keys, uint32_t* values, int64_t n, int key_bits, cudaStream_t s) {
-    radix_sort_impl<uint64_t, true>(keys, values, n, key_bits, s);
+int radix_sort_pairs_u64(uint64_t* keys, uint32_t* values, int64_t n, int key_bits, cudaStream_t s) {
+    return radix_sort_impl<uint64_t, true>(keys, values, n, key_bits, s);
 }
-void radix_sort_keys_u64(uint64_t* keys, int64_t n, int key_bits, cudaStream_t s) {
-    radix_sort_impl<uint64_t, false>(keys, nullptr, n, key_bits, s);
+int radix_sort_keys_u64(uint64_t* keys, int64_t n, int key_bits, cudaStream_t s) {
+    return radix_sort_impl<uint64_t, false>(keys, nullptr, n, key_bits, s);
 }
 
 void fill_u32(uint32_t* p, uint32_t v, int64_t n, cudaStream_t s) {

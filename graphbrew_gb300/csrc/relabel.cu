@@ -575,10 +575,9 @@ void relabel_csr_device(const DeviceCSR& g, const int32_t* new_ids, const int32_
         k_huge_gather<<<grid_for(total, 256), 256, 0, s>>>(g.row_ptr, g.col, new_ids, inv, hlist, hoff, huge, vbits,
                                                            keys);
         GB_LAUNCH_CHECK();
-        radix_sort_keys_u64(keys, total, kbits, s);
+        nl += 6 + radix_sort_keys_u64(keys, total, kbits, s);
         k_huge_scatter<<<grid_for(total, 256), 256, 0, s>>>(hlist, hoff, out_rp, huge, vbits, keys, out_col);
         GB_LAUNCH_CHECK();
-        nl += 6 + 3 * ((kbits + 7) / 8);
     }
     if (launches) *launches += nl;
 }

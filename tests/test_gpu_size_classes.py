@@ -490,3 +490,16 @@ def test_local_moving_window_grows_and_shrinks(ctx, parts):
     expect, ost = po.leiden(rp, col, 1.0)
     np.testing.assert_array_equal(np.asarray(memb).view(np.uint32), expect)
     assert [st["passes"], st["iterations"]] == [ost.passes, ost.iterations]
+
+
+def test_launch_count_of_sorts(ctx):
+    # One community: the vertices' sort is one launch up to 4,096 of them, and above that
+    # a histogram, a scan and a scatter for its one digit; the call's other kernels are the
+    # same (scans of up to 32,768 values are one launch).
+    def launches(n):
+        rp, col = (t.numpy() for t in gg.from_edges(n, [(i, i + 1) for i in range(n - 1)]))
+        recipe = gb.DEFAULT_RECIPE.replace("gordf5000", "gordf100000")
+        return ctx.order_compose(rp, col, np.zeros(n, dtype=np.uint32), recipe)[1]["kernel_launches"]
+
+    assert launches(4096) == launches(4095)
+    assert launches(4097) == launches(4096) + 2
