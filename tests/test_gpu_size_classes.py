@@ -503,3 +503,52 @@ def test_launch_count_of_sorts(ctx):
 
     assert launches(4096) == launches(4095)
     assert launches(4097) == launches(4096) + 2
+
+
+@pytest.mark.parametrize("n", [63, 64, 65, 2047, 2048, 2049, 4095, 4096, 4097, 8192, 8193, 12288, 32767, 32768, 32769])
+def test_sorts_and_scans_of_exact_lengths(ctx, n):
+    # Stars, a path over some of their leaves and isolated vertices up to n of them.
+    rng = np.random.default_rng(n)
+    size = max(2, n // 5)
+    edges = [(h * size, h * size + i) for h in range(3) for i in range(1, size)]
+    edges += [(int(i), int(i) + 1) for i in rng.choice(3 * size - 1, size // 2, replace=False)]
+    rp, col = (t.numpy() for t in gg.from_edges(n, edges))
+    assert len(rp) - 1 == n
+    degree = np.diff(rp)
+    limits = (len(col) // n) * np.array([1, 2, 4, 8, 16, 32, 64]) // 2
+    order = np.argsort(-np.searchsorted(limits, degree, side="left"), kind="stable")
+    ids, _ = ctx.dbg_mapping(rp, col)
+    np.testing.assert_array_equal(ids[order], np.arange(n))
+    new_rp, _, _ = ctx.relabel_by_mapping(rp, col, ids)
+    np.testing.assert_array_equal(new_rp, np.concatenate([[0], np.cumsum(degree[order])]))
+
+
+@pytest.mark.parametrize("order", ["super-rcm", "super-rabbit", "hilbert"])
+@pytest.mark.parametrize("pairs", [1, 2, 4095, 4096, 4097, 8191, 8192, 8193, 12288])
+def test_sorts_of_pairs_of_exact_lengths(ctx, pairs, order):
+    # Every vertex a community and every edge a pair of them: the super-graph's sorts, of
+    # 64-bit keys with and without values and three digits long, have `pairs` of them.
+    rng = np.random.default_rng(pairs)
+    n = 2000
+    pick = rng.choice(n * (n - 1) // 2, pairs, replace=False)
+    hi = ((1 + np.sqrt(1 + 8.0 * pick)) // 2).astype(np.int64)
+    rp, col = (t.numpy() for t in gg.from_edges(n, np.stack([hi, pick - hi * (hi - 1) // 2], axis=1).tolist()))
+    assert len(col) == 2 * pairs
+    memb = np.arange(n, dtype=np.uint32)
+    name = {"super-rcm": "sg_super_rcm", "super-rabbit": "sg_super_rabbit", "hilbert": "sg_hilbert"}[order]
+    recipe = f"leiden:compose:{name}:comm_size_desc:intra_bfs:cd_serial:norefine:2:2"
+    ids, _ = ctx.order_compose(rp, col, memb, recipe)
+    np.testing.assert_array_equal(ids, po.compose(rp, col, memb, "size-desc", "bfs", super_order=order)[0])
+
+
+@pytest.mark.parametrize("kind", ["grid", "grid above", "uniform", "rmat"])
+def test_bfs_on_both_sides_of_the_bitmap(ctx, kind):
+    # Shared memory holds the visited bitmap of 1,310,720 vertices; more of them take the
+    # plain one-CTA levels, with frontiers that outgrow it and come back.
+    rp, col = {"grid": lambda: gg.grid(1280, 1024, 0.1, seed=1, device="cuda"),
+               "grid above": lambda: gg.grid(1280, 1025, 0.1, seed=2, device="cuda"),
+               "uniform": lambda: gg.uniform(21, 2, seed=3, device="cuda"),
+               "rmat": lambda: gg.rmat(21, 8, seed=4, device="cuda")}[kind]()
+    degree = rp[1:] - rp[:-1]
+    for source in {int(torch.argmax(degree)), int(torch.nonzero(degree == 1)[0])}:
+        assert torch.equal(ctx.bfs(rp, col, source)[0], _bfs_levels(rp, col, source))
