@@ -1916,6 +1916,9 @@ __device__ __forceinline__ void init_ctl(const ExactState& a, Ctl* c) {
     const long long n = c->n;
     const long long E = min(n, window_length(c, c->progress));
     window_ranges(a, c, 0, E);
+    // The generation that the last advance left without a table: its share of the slots.
+    if (threadIdx.x < kClearSlots)
+        a.slots[((uint32_t)c->tag * kClearSlots + threadIdx.x) & (kTableSlots - 1)].word = 0;
     __syncthreads();
     if (threadIdx.x == 0) {
         c->P = 0;
