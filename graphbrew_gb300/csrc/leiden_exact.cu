@@ -1828,7 +1828,12 @@ __device__ __forceinline__ void designate(const ExactState& a, Ctl* c) {
 // 400 a round, however long the window: 73 ms with always 65,536 of them, 67 so);
 // where a window is committed in three or four rounds, a shorter one only adds
 // rounds (8 M uniform vertices: 268 ms with 65,536, 345 with always 16,384).
-// A span of 4 left planted communities 3 percent slower, 8 nothing faster.
+// A span of 4 left planted communities 3 percent slower, 8 nothing faster.  The
+// floor stands above what the span asks for on a grid (2,400): decisions far ahead
+// are made again, but a round costs nearly the same and moves on further (511 x 601
+// grid, local moving with windows of 4,096 / 8,192 / 12,288 / 16,384: 89.2 / 69.9 /
+// 63.2 / 59.7 ms in 4,626 / 3,524 / 3,095 / 2,812 rounds; R-MAT scale 16: 4.6 / 3.6 /
+// 3.5 / 3.4 ms).
 constexpr long long kSpan = 6;
 constexpr long long kWindowMin = 16384;
 

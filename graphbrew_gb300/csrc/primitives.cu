@@ -1,8 +1,9 @@
 // primitives.cu -- scan, stable radix sort and fill kernels used by every stage.
 //
-// All of these are bandwidth-bound integer passes: tiles of 2048 elements per
-// 256-thread CTA, coalesced loads, shared-memory staging, grid sizes set by
-// the element count.
+// All of these are bandwidth-bound integer passes: tiles of 2,048 (scans, 256
+// threads) or 4,096 elements (radix passes, 512 threads) per CTA, coalesced loads,
+// shared-memory staging, grid sizes set by the element count; short scans and sorts
+// by one CTA.
 #include <algorithm>
 
 #include "gb_chunks.cuh"
@@ -360,7 +361,7 @@ int radix_sort_impl(K* keys, uint32_t* values, int64_t n, int key_bits, cudaStre
     }
     const int64_t tiles = ceil_div(n, kRadixTile);
     constexpr int smem = radix_scatter_smem<K, kHasValues>();
-    if (smem > 24 * 1024)   // beside some 24 KB of static shared memory
+    if (smem > 24 * 1024)   // beside some 10 KB of static shared memory; the limit without it is 48 KB in all
         GB_CUDA(cudaFuncSetAttribute(k_radix_scatter<K, kHasValues>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     DevBuf<K> kbuf(n, s);
     DevBuf<uint32_t> vbuf(kHasValues ? n : 0, s);

@@ -5,7 +5,9 @@
  * Every entry point takes plain pointers and sizes and returns a gbgpu_status.
  * Graph inputs are undirected CSR graphs as the GAPBS builder produces them
  * (int64 row offsets, int32 neighbour ids, each undirected edge stored in both
- * rows, rows sorted ascending, no duplicates, no self-loops).  Pointers are
+ * rows, rows sorted ascending, no duplicates, no self-loops).  Every call checks
+ * the offsets, the ids' range and the rows' order; that each edge stands in both
+ * rows is not checked, and community detection relies on it.  Pointers are
  * host pointers unless GBGPU_DEVICE_POINTERS is set in `flags`, in which case
  * every array argument of that call is a device pointer on the context's
  * device and the call does no host<->device copies.
